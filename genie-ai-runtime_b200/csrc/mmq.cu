@@ -21,6 +21,7 @@ void* mmq_scratch(size_t bytes, bool may_alloc) {
         if (!may_alloc) return nullptr;
         if (c->mmq_act) cudaFree(c->mmq_act);
         c->mmq_act = nullptr; c->mmq_act_bytes = 0;
+        c->tc_op_x = c->mms_op_x = nullptr;      // the operands that lay there are gone, also when the new buffer gets the old address
         if (cudaMalloc(&c->mmq_act, bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
         c->mmq_act_bytes = bytes;
     }
