@@ -76,7 +76,7 @@ struct LayerDecoder : jllm_b200_decoder {
     int alloc_acts(Acts& a, size_t rows, bool chunk);
     NormStep entry(const Acts& a, const float* w, const float* b) const;
     MoeRoute route(const jllm_b200_layer_spec& w) const;
-    DenseGemm product(const Acts& a) const { DenseGemm g; g.kind = kind; g.part = a.part; g.part_floats = a.part ? gemm_pair_part_floats() : 0; return g; }
+    DenseGemm product(const Acts& a) const { DenseGemm g; g.kind = kind; g.early = true; g.part = a.part; g.part_floats = a.part ? gemm_pair_part_floats() : 0; return g; }
     AttnCall attention_call(int l, const Acts& a) const;
     // parallel layers
     int in_segments(OutSeg* seg, const jllm_b200_layer_spec& w, const Acts& a, int& M) const;
@@ -463,7 +463,7 @@ int LayerDecoder::enqueue_rows(const int* rows, int n, float* out, cudaStream_t 
     f.W = m.width; f.eps = m.eps; f.mult = m.residual_mult; f.rms = m.rms_norm; f.next_w = m.final_w; f.next_b = m.final_b; f.h = a.h; f.x = a.x[last_x]; f.row_index = a.rows;
     DCHK(launch_norm_rows(f, kind, n, st));
     DenseGemm g;
-    g.kind = kind; g.W = m.head ? m.head : m.embed; g.M = m.vocab_size; g.K = m.width; g.N = n; g.x = a.h; g.softcap = m.logit_softcap;
+    g.kind = kind; g.early = true; g.W = m.head ? m.head : m.embed; g.M = m.vocab_size; g.K = m.width; g.N = n; g.x = a.h; g.softcap = m.logit_softcap;
     g.seg[0] = OutSeg{out, m.vocab_size, m.vocab_size, 1, 0};
     return launch_dense_gemm(g, st);
 }

@@ -39,6 +39,7 @@ struct DenseGemv {
     const void* x = nullptr;
     const void* x2 = nullptr; int K2 = 0;
     const float* ls = nullptr; const float* ls2 = nullptr;      // GEMV_TWO: per output row; null: 1
+    bool late = false;                       // GEMV_PLAIN: the kernel in front may still be writing W (the other modes, and a model's weights, do not wait for it)
     LatentRows side;                         // side.z set (GEMV_PAIR): one more CTA stores the token's latent row
     NormStep norm;
     MoeRoute route; const float* z = nullptr; int* ids = nullptr; float* wts = nullptr;
@@ -61,13 +62,14 @@ struct DenseGemm {
     OutSeg seg[MAX_SEG]; int nseg = 1;
     float softcap = 0.f; int swiglu = 0;
     const int* off = nullptr; int n_groups = 1;
+    bool early = false;                      // W was complete before the kernel in front of this one started (a model's weights)
     float* part = nullptr; size_t part_floats = 0;      // optional workspace of K ranges (gemm_pair_part_floats), one per stream
 };
 constexpr int GP_MIN_TOKENS = 128;
 bool gemm_pair_applies(const DenseGemm& a);
 size_t gemm_pair_part_floats();
 int launch_gemm_pair(const DenseGemm& a, cudaStream_t st);       // fp16 (EK_F16) or bf16 operands, pairs of CTAs (gemm_pair.cu)
-int launch_dense_gemm(const DenseGemm& a, cudaStream_t st);      // bf16: tensor cores; fp32: CUDA cores
+int launch_dense_gemm(const DenseGemm& a, cudaStream_t st);      // bf16: tensor cores; fp32: CUDA cores; one token: the decode product
 int launch_dense_gemm_tc(const DenseGemm& a, cudaStream_t st);
 int launch_dense_gemm_simt(const DenseGemm& a, cudaStream_t st);
 

@@ -3,8 +3,8 @@
 // Two CTAs of eight warps per SM; the output rows (or gate / up row pairs) are dealt to the CTAs in contiguous runs and
 // within a CTA to groups of 1, 2, 4 or 8 warps that share a row (as many as make the warps' work most even).  A warp walks R
 // rows at a time and keeps eight 16-byte weight loads per lane in flight, one batch ahead of the arithmetic.
-// Where the rows do not depend on the previous kernel (all modes but the expert ones) the first batch is requested before
-// griddepcontrol.wait, so the weights stream in while the input vector is still being produced and normed.  The input
+// Where the rows do not depend on the previous kernel (all modes but the expert ones, and not where the caller says `late`) the first
+// batch is requested before griddepcontrol.wait, so the weights stream in while the input vector is still being produced and normed.  The input
 // vector is held in shared memory in the activation type (what the prompt path multiplies), sums are fp32.
 #include "dense.cuh"
 
@@ -93,6 +93,7 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dense_gemv_kernel(const DgArgs 
     };
 
     uint4 cur[DG_LOADS], nxt[DG_LOADS];
+    if (MODE == GEMV_PLAIN && g.late) pdl_wait();
     if (MODE != GEMV_MOE_UP && MODE != GEMV_MOE_DOWN) { if (n_batches > 0) load(0, 0, cur); }
     if (NORM) norm_prefetch<DG_THREADS>(g.norm);
     pdl_wait();

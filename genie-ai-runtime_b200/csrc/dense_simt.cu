@@ -112,7 +112,7 @@ static bool ds_one_token(const DenseGemm& a) {
 int launch_dense_gemm(const DenseGemm& a, cudaStream_t st) {
     if (ds_one_token(a)) {
         DenseGemv g;
-        g.kind = a.kind; g.W = a.W; g.M = a.M; g.K = a.K; g.x = a.x; g.softcap = a.softcap; g.nseg = a.nseg;
+        g.kind = a.kind; g.W = a.W; g.M = a.M; g.K = a.K; g.x = a.x; g.softcap = a.softcap; g.nseg = a.nseg; g.late = !a.early;
         for (int i = 0; i < a.nseg; ++i) g.seg[i] = a.seg[i];
         return launch_dense_gemv(g, st);
     }

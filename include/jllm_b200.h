@@ -359,7 +359,9 @@ int jllm_b200_sink_attention(void* out, const void* q, const void* k, const void
 int jllm_b200_moe_route(int* ids, float* weights, int* rank, int* counts, const float* z, const float* correction, int rows, int n_experts, int top,
                         int n_groups, int keep_groups, void* stream);
 /* y[t][r] = W[r] . x[t]; with W_up, silu(W[r] . x[t]) * (W_up[r] . x[t]).  n_groups > 1: W holds n_groups matrices of M rows and
- * group g takes token rows group_offsets[g] .. group_offsets[g + 1] - 1 (device array).  y rows: M fp32 or pad8(M) elements. */
+ * group g takes token rows group_offsets[g] .. group_offsets[g + 1] - 1 (device array).  y rows: M fp32 or pad8(M) elements.
+ * W may be the output of the call in front.  (The *_matvec calls are for weights that stay: they may read W while the kernel in front
+ * of them in the stream still runs.) */
 int jllm_b200_dense_matmul(void* y, const void* W, const void* W_up, const void* x, const int* group_offsets, int n_groups, int kind, int out_f32, int M,
                            int N, int K, float softcap, void* stream);
 int jllm_b200_dense_matvec(void* y, const void* W, const void* x, int kind, int out_f32, int M, int K, float softcap, void* stream);

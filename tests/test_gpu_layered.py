@@ -216,6 +216,29 @@ def test_dense_product(M, N, K, dtype):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_one_token_product_over_the_output_of_the_product_in_front(dtype):
+    """keys = x . A^T, then keys . q, with nothing between the two calls: the second may not read the keys before they are there.  Many keys, so that the
+    first product still runs when the second is launched; the outputs of the sequence with a wait in between are the reference."""
+    import torch
+    jb, r = pkg(), rng(21)
+    for n_keys, dim, K in ((4096, 1024, 512), (130, 256, 2048), (70, 64, 64)):
+        x, A, q = (up(rounded(r.standard_normal(s), dtype), dtype, True) for s in ((n_keys, K), (dim, K), (1, dim)))
+        keys, out = torch.zeros((n_keys, dim), dtype=getattr(torch, dtype), device="cuda"), torch.zeros(n_keys, dtype=torch.float32, device="cuda")
+        def scores(between):
+            keys.zero_()
+            torch.cuda.synchronize()
+            jb.dense_matmul(keys, A, x, dim, n_keys, K)
+            between()
+            jb.dense_matmul(out, keys, q, n_keys, 1, dim)
+            torch.cuda.synchronize()
+            return out.clone()
+        want = scores(torch.cuda.synchronize)
+        assert want.abs().max() > 1
+        for _ in range(8):
+            assert torch.equal(scores(lambda: None), want)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_grouped_product_with_empty_and_uneven_groups(dtype):
     import torch
     jb, r = pkg(), rng(9)
