@@ -90,6 +90,7 @@ struct jllm_b200_batch_decoder {
     void** lists = nullptr;            // device: [layer][4 (k, v, k scales, v scales)][B] pointers
     std::vector<unsigned char> maps;   // host: [layer][B][K, V] TMA tensor maps of the caches (128 bytes each), passed to the kernel as parameters
     void* slab = nullptr;
+    MmqWork mmq;                       // the captured step holds its addresses: all of it is there from the start
     int kernels_per_step = 0;
     cudaGraphExec_t graph_exec = nullptr;   // one decode step from the device-side state
     int host_pos = -1;                      // host mirror of the device-side position (-1 until generate has run): the bound of step_device
@@ -109,9 +110,9 @@ static int bdec_enqueue_step(jllm_b200_batch_decoder* d, const int* prompt, int 
         const jllm_b200_layer_desc& w = d->layers[l];
         void** L = d->lists + (size_t)l * 4 * B;
         BCHK(launch_rmsnorm(d->normed, d->x, nullptr, w.rms_attn, true, B, H, m.rms_eps, st));
-        BCHK(launch_mmq(d->q, resolve_weight(w.wq), w.type_wq, d->normed, QD, B, H, nullptr, st));
-        BCHK(launch_mmq_ex(d->k, resolve_weight(w.wk), w.type_wk, d->normed, KVD, B, H, nullptr, true, st));      // same activations as Q
-        BCHK(launch_mmq_ex(d->v, resolve_weight(w.wv), w.type_wv, d->normed, KVD, B, H, nullptr, true, st));
+        BCHK(launch_mmq(d->q, resolve_weight(w.wq), w.type_wq, d->normed, QD, B, H, nullptr, st, &d->mmq));
+        BCHK(launch_mmq_ex(d->k, resolve_weight(w.wk), w.type_wk, d->normed, KVD, B, H, nullptr, true, st, &d->mmq));      // same activations as Q
+        BCHK(launch_mmq_ex(d->v, resolve_weight(w.wv), w.type_wv, d->normed, KVD, B, H, nullptr, true, st, &d->mmq));
         BCHK(launch_qkv_prep_batched(d->q, d->k, d->v, w.q_norm, w.k_norm, m.rms_eps, (int8_t* const*)L, (int8_t* const*)(L + B),
                                      (float* const*)(L + 2 * B), (float* const*)(L + 3 * B), B, m.n_heads, m.n_kv_heads, m.head_dim,
                                      d->state, m.rope_theta, m.rope_neox != 0, st));
@@ -123,14 +124,14 @@ static int bdec_enqueue_step(jllm_b200_batch_decoder* d, const int* prompt, int 
         c.scale = scale; c.kv_int8 = 1;
         c.n_splits = 1;      // the step is one captured graph for every position: no slices (the streams of a step are short or many)
         BCHK(launch_attention(c, st));
-        BCHK(launch_mmq_ex(d->x2, resolve_weight(w.wo), w.type_wo, d->att, H, B, QD, d->x, false, st));           // + residual
+        BCHK(launch_mmq_ex(d->x2, resolve_weight(w.wo), w.type_wo, d->att, H, B, QD, d->x, false, st, &d->mmq));           // + residual
         BCHK(launch_rmsnorm(d->normed, d->x2, nullptr, w.rms_ffn, true, B, H, m.rms_eps, st));
-        BCHK(launch_mmq_pair(d->gate, d->up, resolve_weight(w.w_gate), w.type_w_gate, resolve_weight(w.w_up), w.type_w_up, d->normed, I, I, B, H, st));   // one launch where the tensor-core kernel serves both
+        BCHK(launch_mmq_pair(d->gate, d->up, resolve_weight(w.w_gate), w.type_w_gate, resolve_weight(w.w_up), w.type_w_up, d->normed, I, I, B, H, st, &d->mmq));   // one launch where the tensor-core kernel serves both
         BCHK(launch_glu(d->sw, d->gate, d->up, B, I, false, st));
-        BCHK(launch_mmq_ex(d->x, resolve_weight(w.w_down), w.type_w_down, d->sw, H, B, I, d->x2, false, st));     // + residual
+        BCHK(launch_mmq_ex(d->x, resolve_weight(w.w_down), w.type_w_down, d->sw, H, B, I, d->x2, false, st, &d->mmq));     // + residual
     }
     BCHK(launch_rmsnorm(d->normed, d->x, nullptr, m.output_norm, true, B, H, m.rms_eps, st));
-    BCHK(launch_mmq(d->logits, resolve_weight(m.output), m.output_type, d->normed, V, B, H, nullptr, st));
+    BCHK(launch_mmq(d->logits, resolve_weight(m.output), m.output_type, d->normed, V, B, H, nullptr, st, &d->mmq));
     JB_CUDA(launch_k(argmax_rows_kernel, dim3(B), dim3(1024), 0, st, pdl_enabled(), (const __half*)d->logits, V, d->tokens, d->state,
                      d->out_tokens, d->out_cap, B));
     count_launch();
@@ -194,16 +195,19 @@ jllm_b200_batch_decoder* jllm_b200_batch_decoder_create(const jllm_b200_model_de
                      attn_tma_encode(&maps[(((size_t)l * B + b) * 2 + 1) * 128], d->kv[b].val_ptr(l, 0), model->max_context, model->n_kv_heads);
         if (ok) d->maps.swap(maps);       // else: the general attention kernel serves the pointer lists
     }
-    // scratch the kernels would otherwise grow on first use
+    // product scratch of every step: nothing of it may move once a step is captured
+    const struct { size_t M, M2, K; } products[6] = { { QD, 0, H }, { KVD, 0, H }, { H, 0, QD }, { I, I, H }, { H, 0, I }, { V, 0, H } };
     size_t need = 0;
-    const int Ms[4] = { (int)QD, (int)I, (int)H, (int)V }; const int Ks[4] = { (int)H, (int)H, (int)I, (int)H };
-    for (int i = 0; i < 4; ++i) {
-        const size_t a = mmq_tc_scratch_bytes(T_Q6K, Ms[i], B, Ks[i]), b2 = mmq_tc_scratch_bytes(T_Q4K, Ms[i], B, Ks[i]), c2 = mmq_scratch_bytes(B, Ks[i]);
-        need = a > need ? a : need; need = b2 > need ? b2 : need; need = c2 > need ? c2 : need;
+    bool wide = false;
+    for (const auto& g : products) {
+        const int M = (int)g.M, M2 = (int)g.M2, K = (int)g.K;
+        for (int t : { T_Q4K, T_Q6K })
+            for (size_t b : { mmq_tc_scratch_bytes(t, M, B, K), mmq_tc_scratch_bytes_pair(t, M, M2, B, K), mmq_stream_scratch_bytes(t, M, B, K), mmq_scratch_bytes(B, K) })
+                if (b > need) need = b;
+        wide = wide || mmq_wide_applies(M, M2, B, K);
     }
-    { const size_t a = mmq_tc_scratch_bytes(T_Q6K, (int)H, B, (int)QD), b2 = mmq_tc_scratch_bytes(T_Q4K, (int)H, B, (int)QD); need = a > need ? a : need; need = b2 > need ? b2 : need; }
-    { const size_t a = mmq_tc_scratch_bytes_pair(T_Q6K, (int)I, (int)I, B, (int)H), b2 = mmq_tc_scratch_bytes_pair(T_Q4K, (int)I, (int)I, B, (int)H); need = a > need ? a : need; need = b2 > need ? b2 : need; }
-    mmq_scratch(need, true);
+    if (!d->mmq.scratch(need, false)) { set_error(JB_ERR_NOMEM, "batch decoder: %zu B of product scratch", need); jllm_b200_batch_decoder_destroy(d); return nullptr; }
+    if (wide) d->mmq.wide_scratch(false);
     splitk_buffer((size_t)B * model->n_heads * 64 * (model->head_dim + 4), true);
     return d;
 }
@@ -211,6 +215,7 @@ void jllm_b200_batch_decoder_destroy(jllm_b200_batch_decoder* d) {
     if (!d) return;
     if (d->graph_exec) cudaGraphExecDestroy(d->graph_exec);
     if (d->slab) cudaFree(d->slab);
+    d->mmq.release();
     for (auto& p : d->kv) p.destroy();
     delete d;
 }

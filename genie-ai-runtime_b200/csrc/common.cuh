@@ -36,6 +36,21 @@ int  cuda_error(cudaError_t e, const char* what);
 // ── per-device context ──────────────────────────────────────────────────
 // Library-owned scratch is per device (the reference keeps process-global statics,
 // src/kernels/gemv_q4.cu:1309-1321, attention.cu:975-988, rope.cu:29-40).
+// What the batched K-quant products need beside their arguments (mmq.cu).  A captured graph holds the addresses, so a buffer that was
+// handed out under capture is never freed or moved; a session whose step is captured has an object of its own.
+struct MmqOperand {                     // quantised activations: what they were made from, and where they lie
+    const void* x = nullptr; const void* at = nullptr; void* stream = nullptr; int n = 0, k = 0, ds4 = -1;
+    bool is(const MmqOperand& o) const { return x && x == o.x && at == o.at && stream == o.stream && n == o.n && k == o.k && ds4 == o.ds4; }
+};
+struct MmqWork {
+    void* act = nullptr; size_t act_bytes = 0;       // quantised activations, K ranges of the fused kernel
+    void* wide = nullptr; bool no_wide = false;      // expanded weights and K ranges of the paired kernel; no_wide: the memory was refused once
+    bool held = false;                               // act was handed out under capture
+    MmqOperand few, many;                            // the operands quantised last, in the layouts of mmq_stream.cu and of mmq_tc.cu
+    void* scratch(size_t bytes, bool capturing);     // null: not there (a captured call does not allocate)
+    void* wide_scratch(bool capturing);
+    void  release();
+};
 struct RopeTable { float theta; int half_dim; int max_seq; float* cos; float* sin; };
 struct DeviceCtx {
     int   device = -1;
@@ -43,14 +58,10 @@ struct DeviceCtx {
     int   max_smem_optin = 0;
     int*  d_status = nullptr;           // device status word written by bounded waits
     float* splitk = nullptr; size_t splitk_floats = 0;
-    void*  mmq_act = nullptr; size_t mmq_act_bytes = 0;
+    MmqWork mmq;                        // of the calls outside the sessions that have their own
     RopeTable rope[8]; int n_rope = 0;
     bool gemv_attr[12] = {};
     bool mms_attr[16] = {};
-    // the activation operand the few-token GEMM quantised last (see launch_mmq_stream: reuse_operand)
-    const void* mms_op_x = nullptr; void* mms_op_scratch = nullptr; void* mms_op_stream = nullptr; int mms_op_n = 0, mms_op_k = 0, mms_op_ds4 = -1;
-    const void* tc_op_x = nullptr; void* tc_op_xq = nullptr; void* tc_op_stream = nullptr; int tc_op_n = 0, tc_op_k = 0, tc_op_ds4 = -1;   // the same for the tensor-core GEMM's operand
-    void* wide = nullptr;               // expanded weights and partial sums of the batched GEMM over many tokens (mmq_wide_scratch)
     bool gemm_pair_attr[2] = { false, false };
     bool gemv_chain_attr = false;
     bool attn_tma_attr[6] = { false, false, false, false, false, false };

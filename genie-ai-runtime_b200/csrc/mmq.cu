@@ -14,18 +14,28 @@ struct ActQ { int8_t* q; float* d; float* s; };   // [N][K] codes, [N][K/32] sca
 
 size_t mmq_scratch_bytes(int N, int K) { return (size_t)N * K + 2 * (size_t)N * (K / 32) * sizeof(float) + 256; }
 
-void* mmq_scratch(size_t bytes, bool may_alloc) {
-    DeviceCtx* c = ctx();
-    if (!c) return nullptr;
-    if (bytes > c->mmq_act_bytes) {
-        if (!may_alloc) return nullptr;
-        if (c->mmq_act) cudaFree(c->mmq_act);
-        c->mmq_act = nullptr; c->mmq_act_bytes = 0;
-        c->tc_op_x = c->mms_op_x = nullptr;      // the operands that lay there are gone, also when the new buffer gets the old address
-        if (cudaMalloc(&c->mmq_act, bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-        c->mmq_act_bytes = bytes;
+void* MmqWork::scratch(size_t bytes, bool capturing) {
+    if (bytes > act_bytes) {
+        if (capturing) return nullptr;
+        few = many = MmqOperand();               // the operands that lay there are gone, also when the new buffer gets the old address
+        size_t want = bytes;
+        if (held && want < 2 * act_bytes) want = 2 * act_bytes;      // the old buffer stays: all of them together take less than the newest
+        if (act && !held) cudaFree(act);
+        act = nullptr; act_bytes = 0; held = false;
+        if (cudaMalloc(&act, want) != cudaSuccess) {
+            cudaGetLastError();
+            want = bytes;
+            if (cudaMalloc(&act, want) != cudaSuccess) { cudaGetLastError(); act = nullptr; return nullptr; }
+        }
+        act_bytes = want;
     }
-    return c->mmq_act;
+    held = held || capturing;
+    return act;
+}
+void MmqWork::release() {
+    if (act) cudaFree(act);
+    if (wide) cudaFree(wide);
+    *this = MmqWork();
 }
 
 // one warp per 32-element group of one token
@@ -106,67 +116,72 @@ static bool capturing(cudaStream_t st) {
 int launch_add_half(__half* out, const __half* a, const __half* b, long long n, cudaStream_t st);      // elementwise.cu
 
 static int launch_mmq_impl(__half* y, const void* W, int type, const __half* x, int M, int N, int K, int32_t* dbg, const __half* residual,
-                           bool same_x, cudaStream_t st);
-
-int launch_mmq(__half* y, const void* W, int type, const __half* x, int M, int N, int K, int32_t* dbg, cudaStream_t st) {
-    return launch_mmq_impl(y, W, type, x, M, N, K, dbg, nullptr, false, st);
+                           bool same_x, cudaStream_t st, MmqWork* w);
+static MmqWork* work_of(MmqWork* own) {
+    if (own) return own;
+    DeviceCtx* c = ctx();
+    return c ? &c->mmq : nullptr;
 }
-int launch_mmq_ex(__half* y, const void* W, int type, const __half* x, int M, int N, int K, const __half* residual, bool same_x, cudaStream_t st) {
-    return launch_mmq_impl(y, W, type, x, M, N, K, nullptr, residual, same_x, st);
+
+int launch_mmq(__half* y, const void* W, int type, const __half* x, int M, int N, int K, int32_t* dbg, cudaStream_t st, MmqWork* own) {
+    return launch_mmq_impl(y, W, type, x, M, N, K, dbg, nullptr, false, st, work_of(own));
+}
+int launch_mmq_ex(__half* y, const void* W, int type, const __half* x, int M, int N, int K, const __half* residual, bool same_x, cudaStream_t st, MmqWork* own) {
+    return launch_mmq_impl(y, W, type, x, M, N, K, nullptr, residual, same_x, st, work_of(own));
 }
 
 // Two products over the same activations (gate and up): one launch of the tensor-core kernel when both matrices are of one
 // type and that kernel is the one each would get on its own; else one product after the other, the second reusing the
 // quantised operand of the first.
 int launch_mmq_pair(__half* y1, __half* y2, const void* W1, int type1, const void* W2, int type2, const __half* x, int M1, int M2, int N, int K,
-                    cudaStream_t st) {
+                    cudaStream_t st, MmqWork* own) {
+    MmqWork* w = work_of(own);
     static const bool tc_off = [] { const char* e = getenv("JLLM_B200_MMQ"); return e && !strcmp(e, "cuda"); }();
     static const bool pair_off = [] { const char* e = getenv("JLLM_B200_MMQ_PAIR"); return e && e[0] == '0'; }();
     const bool ok = !tc_off && !pair_off && type1 == type2 && M1 > 0 && M2 > 0 && N > 0 && K > 0 && K % QK_K == 0 && y1 && y2 && W1 && W2 && x &&
                     (type1 == T_Q4K || type1 == T_Q6K) && !mmq_stream_applies(W1, type1, M1, N, K) && !mmq_stream_applies(W2, type2, M2, N, K) &&
                     mmq_tc_applies(W1, type1, M1, N, K) && mmq_tc_applies(W2, type2, M2, N, K);
     if (!ok) {
-        const int rc = launch_mmq_impl(y1, W1, type1, x, M1, N, K, nullptr, nullptr, false, st);
-        return rc ? rc : launch_mmq_impl(y2, W2, type2, x, M2, N, K, nullptr, nullptr, true, st);
+        const int rc = launch_mmq_impl(y1, W1, type1, x, M1, N, K, nullptr, nullptr, false, st, w);
+        return rc ? rc : launch_mmq_impl(y2, W2, type2, x, M2, N, K, nullptr, nullptr, true, st, w);
     }
     const size_t need = mmq_tc_scratch_bytes_pair(type1, M1, M2, N, K);
-    __half* xq = (__half*)mmq_scratch(need, !capturing(st));
+    const bool cap = capturing(st);
+    __half* xq = w ? (__half*)w->scratch(need, cap) : nullptr;
     if (!xq) return set_error(JB_ERR_NOMEM, "batched gemm: %zu B of activation scratch unavailable", need);
-    if (DeviceCtx* c = ctx()) c->mms_op_x = nullptr;
-    return launch_mmq_tc_pair(y1, y2, W1, W2, type1, x, xq, M1, M2, N, K, false, st, mmq_wide_applies(M1, M2, N, K) ? mmq_wide_scratch(!capturing(st)) : nullptr);
+    return launch_mmq_tc_pair(y1, y2, W1, W2, type1, x, xq, M1, M2, N, K, false, st, *w, mmq_wide_applies(M1, M2, N, K) ? w->wide_scratch(cap) : nullptr);
 }
 
 static int launch_mmq_impl(__half* y, const void* W, int type, const __half* x, int M, int N, int K, int32_t* dbg, const __half* residual,
-                           bool same_x, cudaStream_t st) {
+                           bool same_x, cudaStream_t st, MmqWork* w) {
     if (M <= 0 || N <= 0) return JB_OK;
     if (K <= 0 || K % QK_K) return set_error(JB_ERR_ARG, "batched gemm: K=%d is not a positive multiple of 256", K);
     if (type != T_Q4K && type != T_Q6K) return set_error(JB_ERR_TYPE, "batched gemm: ggml type %d", type);
     if (!y || !W || !x) return set_error(JB_ERR_PTR, "batched gemm: null pointer");
     if (type == T_Q4K && ((uintptr_t)W & 3)) return set_error(JB_ERR_PTR, "batched gemm: Q4_K weights must be 4-byte aligned");
+    const bool cap = capturing(st);
     // JLLM_B200_MMQ=cuda keeps the CUDA-core kernel (the one that can also export the integer accumulators)
     static const bool tc_off = [] { const char* e = getenv("JLLM_B200_MMQ"); return e && !strcmp(e, "cuda"); }();
     if (!dbg && !tc_off && mmq_stream_applies(W, type, M, N, K)) {
         const size_t need_s = mmq_stream_scratch_bytes(type, M, N, K);
-        void* sc = mmq_scratch(need_s, !capturing(st));
+        void* sc = w ? w->scratch(need_s, cap) : nullptr;
         if (!sc) return set_error(JB_ERR_NOMEM, "batched gemm: %zu B of activation scratch unavailable", need_s);
-        if (DeviceCtx* c = ctx()) c->tc_op_x = nullptr;          // the scratch is shared: the other path's operand is gone
-        return launch_mmq_stream(y, W, type, x, sc, M, N, K, residual, same_x, st);
+        return launch_mmq_stream(y, W, type, x, sc, M, N, K, residual, same_x, st, *w);
     }
     if (residual) {          // the other kernels have no fused exit: product, then the add (in place)
-        const int rc = launch_mmq_impl(y, W, type, x, M, N, K, dbg, nullptr, false, st);
+        const int rc = launch_mmq_impl(y, W, type, x, M, N, K, dbg, nullptr, false, st, w);
         return rc ? rc : launch_add_half(y, residual, y, (long long)N * M, st);
     }
     if (!dbg && !tc_off && mmq_tc_applies(W, type, M, N, K)) {
         const size_t need_tc = mmq_tc_scratch_bytes(type, M, N, K);
-        __half* xq = (__half*)mmq_scratch(need_tc, !capturing(st));
+        __half* xq = w ? (__half*)w->scratch(need_tc, cap) : nullptr;
         if (!xq) return set_error(JB_ERR_NOMEM, "batched gemm: %zu B of activation scratch unavailable", need_tc);
-        if (DeviceCtx* c = ctx()) c->mms_op_x = nullptr;
-        return launch_mmq_tc(y, W, type, x, xq, M, N, K, same_x, st, mmq_wide_applies(M, 0, N, K) ? mmq_wide_scratch(!capturing(st)) : nullptr);
+        return launch_mmq_tc_pair(y, nullptr, W, nullptr, type, x, xq, M, 0, N, K, same_x, st, *w, mmq_wide_applies(M, 0, N, K) ? w->wide_scratch(cap) : nullptr);
     }
-    if (DeviceCtx* c = ctx()) { c->tc_op_x = nullptr; c->mms_op_x = nullptr; }
     const size_t need = mmq_scratch_bytes(N, K);
-    uint8_t* base = (uint8_t*)mmq_scratch(need, !capturing(st));
+    uint8_t* base = w ? (uint8_t*)w->scratch(need, cap) : nullptr;
     if (!base) return set_error(JB_ERR_NOMEM, "batched gemm: %zu B of activation scratch unavailable", need);
+    w->few = w->many = MmqOperand();
     ActQ a;
     a.q = (int8_t*)base;
     a.d = (float*)(base + (((size_t)N * K + 255) & ~(size_t)255));

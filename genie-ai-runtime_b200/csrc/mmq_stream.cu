@@ -329,7 +329,7 @@ size_t mmq_stream_scratch_bytes(int type, int M, int N, int K) {
 // the previous call on this stream (Q and K, gate and up): the quantised operand in `scratch` is still valid and the quantise
 // launch is skipped; the library checks pointer, shape, flavour and scratch address and quantises again if anything differs.
 int launch_mmq_stream(__half* y, const void* W, int type, const __half* x, void* scratch, int M, int N, int K, const __half* residual,
-                      bool reuse_operand, cudaStream_t st) {
+                      bool reuse_operand, cudaStream_t st, MmqWork& work) {
     DeviceCtx* cx = ctx();
     if (!cx) return JB_ERR_CUDA;
     const int nb = K / QK_K, NT = ms_tiles(N);
@@ -337,12 +337,12 @@ int launch_mmq_stream(__half* y, const void* W, int type, const __half* x, void*
     __half* xb = reinterpret_cast<__half*>(scratch);
     const long long groups = (long long)NPk * (K / 32);
     const int ds4 = type == T_Q4K;
-    const bool same = reuse_operand && cx->mms_op_x == (const void*)x && cx->mms_op_scratch == scratch && cx->mms_op_n == N && cx->mms_op_k == K &&
-                      cx->mms_op_ds4 == ds4 && cx->mms_op_stream == (void*)st;
-    if (!same) {
+    const MmqOperand op = {x, scratch, (void*)st, N, K, ds4};
+    if (!reuse_operand || !work.few.is(op)) {
         JB_CUDA(launch_k(mms_quantize_kernel, dim3((unsigned)((groups + 3) / 4)), dim3(32, 4), 0, st, pdl_enabled(), x, xb, N, NPk, K, ds4));
         count_launch();
-        cx->mms_op_x = x; cx->mms_op_scratch = scratch; cx->mms_op_n = N; cx->mms_op_k = K; cx->mms_op_ds4 = ds4; cx->mms_op_stream = (void*)st;
+        work.few = op;
+        work.many = MmqOperand();                        // the scratch is shared: the other layout's operand is gone
     }
     MsArgs a = {};
     a.y = y; a.res = residual; a.W = (const uint8_t*)W; a.xb = xb; a.M = M; a.N = N; a.NP = NPk; a.nb = nb;

@@ -557,11 +557,11 @@ constexpr int MW_MIN_TOKENS = 384;      // 256 tokens: Q6_K 2560 x 9728 46 us th
 bool mmq_wide_applies(int M, int M2, int N, int K) {
     return N >= MW_MIN_TOKENS && (long long)M + M2 >= 256 && (size_t)(K + K / 16 + TC_K) * sizeof(__half) * 256 <= MW_WEIGHT_BYTES;
 }
-void* mmq_wide_scratch(bool may_alloc) {
-    DeviceCtx* c = ctx();
-    if (!c || c->wide || !may_alloc) return c ? c->wide : nullptr;
-    if (cudaMalloc(&c->wide, MW_WEIGHT_BYTES + gemm_pair_part_floats() * sizeof(float)) != cudaSuccess) { cudaGetLastError(); c->wide = nullptr; }
-    return c->wide;
+// Asked for once: an object whose request was refused stays with the fused kernel, whose results differ in their last bits.
+void* MmqWork::wide_scratch(bool capturing) {
+    if (wide || no_wide || capturing) return wide;
+    if (cudaMalloc(&wide, MW_WEIGHT_BYTES + gemm_pair_part_floats() * sizeof(float)) != cudaSuccess) { cudaGetLastError(); wide = nullptr; no_wide = true; }
+    return wide;
 }
 
 // Rows [r0, r0 + rows) of the operand, Kp halves each; a thread takes 8 bytes of packed codes: 16 weights of a Q4_K block, 32 of a
@@ -676,13 +676,10 @@ bool mmq_tc_applies(const void* W, int type, int M, int N, int K) {
     return N >= 2 && M >= 1 && K % QK_K == 0 && encode_tiled_fn() != nullptr;
 }
 
-int launch_mmq_tc(__half* y, const void* W, int type, const __half* x, __half* xq, int M, int N, int K, bool same_x, cudaStream_t st, void* wide) {
-    return launch_mmq_tc_pair(y, nullptr, W, nullptr, type, x, xq, M, 0, N, K, same_x, st, wide);
-}
 // y = x . W^T and, when W2 is given, y2 = x . W2^T in the same launch: the row tiles of both matrices are one list of work, so
 // two products that share their activations (gate and up) fill the grid together instead of one after the other.
 int launch_mmq_tc_pair(__half* y, __half* y2, const void* W, const void* W2, int type, const __half* x, __half* xq, int M, int M2, int N, int K,
-                       bool same_x, cudaStream_t st, void* wide) {
+                       bool same_x, cudaStream_t st, MmqWork& work, void* wide) {
     DeviceCtx* c = ctx();
     if (!c) return set_error(JB_ERR_STATE, "batched gemm: library not initialised");
     TcArgs a;
@@ -717,8 +714,8 @@ int launch_mmq_tc_pair(__half* y, __half* y2, const void* W, const void* W2, int
     // The operand of the previous call is still in the scratch when the caller says x has not changed since and everything
     // that shapes it (tokens, K, the Q4_K extras) is the same: the products that share an input quantise it once.
     const int ds4 = (int)(type == T_Q4K);
-    const bool reuse = same_x && c->tc_op_x == x && c->tc_op_xq == xq && c->tc_op_stream == (void*)st && c->tc_op_n == N && c->tc_op_k == K && c->tc_op_ds4 == ds4;
-    if (!reuse) {
+    const MmqOperand op = {x, xq, (void*)st, N, K, ds4};
+    if (!same_x || !work.many.is(op)) {
         if (((uintptr_t)x & 15) == 0) {
             const long long warps = (long long)N * (K / QK_K);
             JB_CUDA(launch_k(mmq_tc_quantize_kernel, dim3((unsigned)((warps + 3) / 4)), dim3(32, 4), 0, st, pdl_enabled(), x, xq, N, K, Kp, ds4));
@@ -727,7 +724,8 @@ int launch_mmq_tc_pair(__half* y, __half* y2, const void* W, const void* W2, int
             JB_CUDA(launch_k(mmq_tc_quantize1_kernel, dim3((unsigned)((groups + 3) / 4)), dim3(32, 4), 0, st, pdl_enabled(), x, xq, N, K, Kp, ds4));
         }
         count_launch();
-        c->tc_op_x = x; c->tc_op_xq = xq; c->tc_op_stream = (void*)st; c->tc_op_n = N; c->tc_op_k = K; c->tc_op_ds4 = ds4;
+        work.many = op;
+        work.few = MmqOperand();
     }
     if (wide) return launch_wide(a, xq, Kp, wide, st);
     const int n_work = a.n_full + (tiles - a.n_full) * a.ksplit;

@@ -130,3 +130,43 @@ def test_batch_decoder_step_device_is_bounded_by_the_context():
     assert e.value.code == 6 and jb.launch_count() == n0
     assert jb.device_status(st) == 0
     d.close()
+
+
+def test_captured_step_keeps_its_product_scratch():
+    """step_device replays a captured step.  Between two of its steps other work of the process asks for more product scratch than the batch session ever did
+    (a long prompt in another session, a large product) and allocates what it can get: the logits have to be those of an undisturbed session."""
+    import torch
+    jb = pkg()
+    wide = dict(n_layers=1, hidden=2560, n_heads=32, n_kv=8, hd=128, ffn=9728, vocab=512)
+    m = orc.gen_model(80, **wide)
+    w = jb.decoder.upload(m)
+    rng = np.random.Generator(np.random.PCG64(80))
+    st = torch.cuda.Stream()
+    def steps(B, disturb):
+        prompts = np.random.Generator(np.random.PCG64(B)).integers(0, wide["vocab"], (B, 3)).astype(np.int32)
+        d = jb.decoder.BatchDecoder(m["cfg"], w, 16, B)
+        d.generate(prompts, 1, st)
+        out = []
+        for i in range(3):
+            d.step_device(st)
+            out.append(d.logits().clone())
+            if i == 0:
+                disturb()
+        d.close()
+        return out
+    def disturb():
+        p = jb.decoder.Decoder(m["cfg"], w, 1100, jb.decoder.FUSED | jb.decoder.PREFILL)
+        p.prefill(rng.integers(0, wide["vocab"], 512), 0)
+        torch.cuda.synchronize()
+        keep = [torch.full((1 << n,), 0x5A, dtype=torch.uint8, device="cuda") for n in range(20, 28)]      # takes the place of what was freed
+        N = 1500
+        y = torch.zeros(N * 9728, dtype=torch.float16, device="cuda")
+        jb.gemm_quant_batched(y, w["layers"][0]["gate"][0], 12, torch.ones(N * 2560, dtype=torch.float16, device="cuda"), 9728, N, 2560)
+        torch.cuda.synchronize()
+        p.close()
+        del keep
+    for B in (2, 8, 50):
+        want = steps(B, lambda: None)
+        got = steps(B, disturb)
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), B
+    assert jb.device_status(st) == 0

@@ -141,3 +141,34 @@ def test_n_equal_one_routes_to_gemv():
     jb.gemm_quant_batched(a, W, 12, x, M, 1, K)
     jb.gemv_quant(b, W, 12, x, M, K)
     assert torch.equal(a, b)
+
+
+def test_captured_product_replays_after_larger_calls():
+    """A caller's own graph holds the address of the product's scratch: replayed after calls that ask for more of it, it gives what it gave before."""
+    import torch
+    jb = pkg()
+    rng = np.random.Generator(np.random.PCG64(1011))
+    M, K = 1024, 1024
+    W = dev(orc.gen_weight(rng, 12, M, K))
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for N in (8, 100, 400):
+        with torch.cuda.stream(st):
+            X = dev(orc.gen_act(rng, N * K))
+            y = torch.zeros(N * M, dtype=torch.float16, device="cuda")
+            jb.gemm_quant_batched(y, W, 12, X, M, N, K, stream=st)
+            torch.cuda.synchronize()
+            want = y.clone()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=st):
+                jb.gemm_quant_batched(y, W, 12, X, M, N, K, stream=st)
+            for n in (800 + N, 2000 + N):
+                big = torch.zeros(n * M, dtype=torch.float16, device="cuda")
+                jb.gemm_quant_batched(big, W, 12, torch.ones(n * K, dtype=torch.float16, device="cuda"), M, n, K, stream=st)
+            keep = [torch.full((1 << i,), 0x5A, dtype=torch.uint8, device="cuda") for i in range(18, 27)]
+            y.zero_()
+            g.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(y, want), N
+            del keep, g
+    assert jb.device_status() == 0
