@@ -75,15 +75,21 @@ __global__ void attn_reduce_kernel(QT* out, const float* part, int n_heads, int 
     ag_merge_slices(out + (size_t)z * ldo + (size_t)head * hd, part + ((size_t)z * n_heads + head) * n_splits * (hd + 2), hd, n_splits, sink ? sink + head : nullptr, head_gate(gate, ldg, z, head));
 }
 
+// Captured decode steps hold the buffer's address: it is never freed, a larger one is put beside it (at least twice as large, so that
+// all that was outgrown takes less than the newest).
 float* splitk_buffer(size_t floats, bool may_alloc) {
     DeviceCtx* c = ctx();
     if (!c) return nullptr;
     if (floats > c->splitk_floats) {
         if (!may_alloc) return nullptr;
-        if (c->splitk) cudaFree(c->splitk);
-        c->splitk = nullptr; c->splitk_floats = 0;
-        if (cudaMalloc(&c->splitk, floats * sizeof(float)) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-        c->splitk_floats = floats;
+        float* p = nullptr;
+        size_t want = floats > 2 * c->splitk_floats ? floats : 2 * c->splitk_floats;
+        if (cudaMalloc(&p, want * sizeof(float)) != cudaSuccess) {
+            cudaGetLastError();
+            want = floats;
+            if (cudaMalloc(&p, want * sizeof(float)) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        }
+        c->splitk = p; c->splitk_floats = want;
     }
     return c->splitk;
 }
