@@ -36,8 +36,9 @@ int  cuda_error(cudaError_t e, const char* what);
 // ── per-device context ──────────────────────────────────────────────────
 // Library-owned scratch is per device (the reference keeps process-global statics,
 // src/kernels/gemv_q4.cu:1309-1321, attention.cu:975-988, rope.cu:29-40).
-// What the batched K-quant products need beside their arguments (mmq.cu).  A captured graph holds the addresses, so a buffer that was
-// handed out under capture is never freed or moved; a session whose step is captured has an object of its own.
+// What the batched K-quant products need beside their arguments.  One object serves one order of launches: a stream's (the library keeps
+// them, mmq.cu), or that of a session whose captured step holds the addresses and which reserves all it needs first.  A buffer that was
+// handed out under capture is never freed or moved.
 struct MmqOperand {                     // quantised activations: what they were made from, and where they lie
     const void* x = nullptr; const void* at = nullptr; void* stream = nullptr; int n = 0, k = 0, ds4 = -1;
     bool is(const MmqOperand& o) const { return x && x == o.x && at == o.at && stream == o.stream && n == o.n && k == o.k && ds4 == o.ds4; }
@@ -46,8 +47,9 @@ struct MmqWork {
     void* act = nullptr; size_t act_bytes = 0;       // quantised activations, K ranges of the fused kernel
     void* wide = nullptr; bool no_wide = false;      // expanded weights and K ranges of the paired kernel; no_wide: the memory was refused once
     bool held = false;                               // act was handed out under capture
+    size_t capture_limit = 0;                        // a captured call may allocate up to this much: what an uncaptured one has asked for before
     MmqOperand few, many;                            // the operands quantised last, in the layouts of mmq_stream.cu and of mmq_tc.cu
-    void* scratch(size_t bytes, bool capturing);     // null: not there (a captured call does not allocate)
+    void* scratch(size_t bytes, bool capturing);     // null: not to be had
     void* wide_scratch(bool capturing);
     void  release();
 };
@@ -58,7 +60,6 @@ struct DeviceCtx {
     int   max_smem_optin = 0;
     int*  d_status = nullptr;           // device status word written by bounded waits
     float* splitk = nullptr; size_t splitk_floats = 0;
-    MmqWork mmq;                        // of the calls outside the sessions that have their own
     RopeTable rope[8]; int n_rope = 0;
     bool gemv_attr[12] = {};
     bool mms_attr[16] = {};

@@ -333,6 +333,7 @@ int KquantDecoder::enqueue_chunk(const int* dev_tokens, int N, int start, cudaSt
         DCHK(launch_mmq(pf_y, resolve_weight(w.w_down), w.type_w_down, pf_sw, H, N, I, nullptr, st));
         DCHK(launch_add_half(pf_x, pf_x2, pf_y, (long long)N * H, st));
     }
+    mmq_mark(st);
     return JB_OK;
 }
 // logits of single rows of the chunk (src/engine/decode.cu:2019-2050 computes them for the last prompt token only)

@@ -7,6 +7,7 @@
 #include "mmq.cuh"
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 
 namespace jb {
 
@@ -14,19 +15,23 @@ struct ActQ { int8_t* q; float* d; float* s; };   // [N][K] codes, [N][K/32] sca
 
 size_t mmq_scratch_bytes(int N, int K) { return (size_t)N * K + 2 * (size_t)N * (K / 32) * sizeof(float) + 256; }
 
+cudaError_t mmq_alloc(void** p, size_t bytes, bool capturing) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;       // a captured call may allocate when its thread says so
+    if (capturing) cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) { cudaGetLastError(); *p = nullptr; }
+    if (capturing) cudaThreadExchangeStreamCaptureMode(&mode);
+    return e;
+}
 void* MmqWork::scratch(size_t bytes, bool capturing) {
     if (bytes > act_bytes) {
-        if (capturing) return nullptr;
+        if (capturing && bytes > capture_limit) return nullptr;
         few = many = MmqOperand();               // the operands that lay there are gone, also when the new buffer gets the old address
-        size_t want = bytes;
-        if (held && want < 2 * act_bytes) want = 2 * act_bytes;      // the old buffer stays: all of them together take less than the newest
-        if (act && !held) cudaFree(act);
+        const bool keep = held || capturing;     // the old buffer stays: all of them together take less than the newest
+        size_t want = keep && bytes < 2 * act_bytes ? 2 * act_bytes : bytes;
+        if (act && !keep) cudaFree(act);
         act = nullptr; act_bytes = 0; held = false;
-        if (cudaMalloc(&act, want) != cudaSuccess) {
-            cudaGetLastError();
-            want = bytes;
-            if (cudaMalloc(&act, want) != cudaSuccess) { cudaGetLastError(); act = nullptr; return nullptr; }
-        }
+        if (mmq_alloc(&act, want, capturing) != cudaSuccess && mmq_alloc(&act, want = bytes, capturing) != cudaSuccess) return nullptr;
         act_bytes = want;
     }
     held = held || capturing;
@@ -116,18 +121,102 @@ static bool capturing(cudaStream_t st) {
 int launch_add_half(__half* out, const __half* a, const __half* b, long long n, cudaStream_t st);      // elementwise.cu
 
 static int launch_mmq_impl(__half* y, const void* W, int type, const __half* x, int M, int N, int K, int32_t* dbg, const __half* residual,
-                           bool same_x, cudaStream_t st, MmqWork* w);
-static MmqWork* work_of(MmqWork* own) {
-    if (own) return own;
+                           bool same_x, cudaStream_t st, MmqWork* w, bool cap);
+
+// The library's scratch: an object per stream, so that calls on different streams do not meet.  A call holds the lock while it enqueues
+// its launches (quantiser, product, sum), so that threads that share a stream do not mix theirs.  A stream that has none takes one
+// whose last work is known to be over (sessions record an event at the end of a prompt: mmq_mark), else a new one; when there are
+// MMQ_STREAMS, the one that was not used for the longest time, after a wait for the device.
+// Captured calls have objects apart from these, which their graphs keep: one per stream handle (a stream's id cannot be asked for under
+// capture); a handle beyond MMQ_GRAPHS shares the one that was captured into least recently.
+constexpr int MMQ_STREAMS = 32, MMQ_GRAPHS = 32;
+struct MmqPool {
+    struct Entry { unsigned long long id = 0, used = 0; cudaEvent_t done = nullptr; bool marked = false; MmqWork work; };
+    std::mutex mu;
+    Entry streams[MMQ_STREAMS], graphs[MMQ_GRAPHS];
+    int n_streams = 0, n_graphs = 0;
+    unsigned long long clock = 0;
+    size_t asked = 0;                            // most scratch that a call has asked for outside of captures
+
+    static Entry* oldest(Entry* e, int n) {
+        Entry* o = e;
+        for (int i = 1; i < n; ++i) if (e[i].used < o->used) o = &e[i];
+        return o;
+    }
+    static bool id_of(cudaStream_t st, unsigned long long& id) {
+        id = 0;                                  // the default stream, which has two handles
+        if (!st || st == cudaStreamLegacy || cudaStreamGetId(st, &id) == cudaSuccess) return true;
+        cudaGetLastError();
+        return false;
+    }
+    Entry* find(unsigned long long id) {
+        for (int i = 0; i < n_streams; ++i) if (streams[i].id == id) return &streams[i];
+        return nullptr;
+    }
+    MmqWork* of_graph(cudaStream_t st) {
+        const unsigned long long id = (unsigned long long)(uintptr_t)st;
+        Entry* e = nullptr;
+        for (int i = 0; i < n_graphs; ++i) if (graphs[i].id == id) e = &graphs[i];
+        if (!e) e = n_graphs < MMQ_GRAPHS ? &graphs[n_graphs++] : oldest(graphs, n_graphs);
+        e->id = id; e->used = ++clock;
+        e->work.capture_limit = asked;
+        return &e->work;
+    }
+    MmqWork* of_stream(cudaStream_t st) {
+        unsigned long long id;
+        if (!id_of(st, id)) return nullptr;
+        Entry* e = find(id);
+        if (!e) {
+            for (int i = 0; i < n_streams && !e; ++i) if (streams[i].marked && cudaEventQuery(streams[i].done) == cudaSuccess) e = &streams[i];
+            cudaGetLastError();                  // "not ready" is an answer
+            if (!e && n_streams < MMQ_STREAMS) e = &streams[n_streams++];
+            if (!e) {
+                if (cudaDeviceSynchronize() != cudaSuccess) { cudaGetLastError(); return nullptr; }
+                e = oldest(streams, n_streams);
+            }
+            e->work.few = e->work.many = MmqOperand();
+        }
+        e->id = id; e->used = ++clock; e->marked = false;
+        return &e->work;
+    }
+    void mark(cudaStream_t st) {
+        unsigned long long id;
+        Entry* e = id_of(st, id) ? find(id) : nullptr;
+        if (!e || (!e->done && cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming) != cudaSuccess)) { cudaGetLastError(); return; }
+        e->marked = cudaEventRecord(e->done, st) == cudaSuccess;
+        if (!e->marked) cudaGetLastError();
+    }
+};
+static MmqPool g_mmq_pool[16];                   // per device
+struct MmqLease {
+    std::unique_lock<std::mutex> lock;
+    MmqPool* pool = nullptr;
+    MmqWork* w = nullptr;
+    bool cap;
+    MmqLease(MmqWork* own, cudaStream_t st) : w(own), cap(capturing(st)) {
+        DeviceCtx* c = own ? nullptr : ctx();
+        if (!c) return;
+        pool = &g_mmq_pool[c->device];
+        lock = std::unique_lock<std::mutex>(pool->mu);
+        w = cap ? pool->of_graph(st) : pool->of_stream(st);
+    }
+    ~MmqLease() { if (pool && w && !cap && w->act_bytes > pool->asked) pool->asked = w->act_bytes; }
+};
+
+void mmq_mark(cudaStream_t st) {
     DeviceCtx* c = ctx();
-    return c ? &c->mmq : nullptr;
+    if (!c || capturing(st)) return;
+    std::lock_guard<std::mutex> lock(g_mmq_pool[c->device].mu);
+    g_mmq_pool[c->device].mark(st);
 }
 
 int launch_mmq(__half* y, const void* W, int type, const __half* x, int M, int N, int K, int32_t* dbg, cudaStream_t st, MmqWork* own) {
-    return launch_mmq_impl(y, W, type, x, M, N, K, dbg, nullptr, false, st, work_of(own));
+    const MmqLease l(own, st);
+    return launch_mmq_impl(y, W, type, x, M, N, K, dbg, nullptr, false, st, l.w, l.cap);
 }
 int launch_mmq_ex(__half* y, const void* W, int type, const __half* x, int M, int N, int K, const __half* residual, bool same_x, cudaStream_t st, MmqWork* own) {
-    return launch_mmq_impl(y, W, type, x, M, N, K, nullptr, residual, same_x, st, work_of(own));
+    const MmqLease l(own, st);
+    return launch_mmq_impl(y, W, type, x, M, N, K, nullptr, residual, same_x, st, l.w, l.cap);
 }
 
 // Two products over the same activations (gate and up): one launch of the tensor-core kernel when both matrices are of one
@@ -135,31 +224,30 @@ int launch_mmq_ex(__half* y, const void* W, int type, const __half* x, int M, in
 // quantised operand of the first.
 int launch_mmq_pair(__half* y1, __half* y2, const void* W1, int type1, const void* W2, int type2, const __half* x, int M1, int M2, int N, int K,
                     cudaStream_t st, MmqWork* own) {
-    MmqWork* w = work_of(own);
+    const MmqLease l(own, st);
+    MmqWork* w = l.w;
     static const bool tc_off = [] { const char* e = getenv("JLLM_B200_MMQ"); return e && !strcmp(e, "cuda"); }();
     static const bool pair_off = [] { const char* e = getenv("JLLM_B200_MMQ_PAIR"); return e && e[0] == '0'; }();
     const bool ok = !tc_off && !pair_off && type1 == type2 && M1 > 0 && M2 > 0 && N > 0 && K > 0 && K % QK_K == 0 && y1 && y2 && W1 && W2 && x &&
                     (type1 == T_Q4K || type1 == T_Q6K) && !mmq_stream_applies(W1, type1, M1, N, K) && !mmq_stream_applies(W2, type2, M2, N, K) &&
                     mmq_tc_applies(W1, type1, M1, N, K) && mmq_tc_applies(W2, type2, M2, N, K);
     if (!ok) {
-        const int rc = launch_mmq_impl(y1, W1, type1, x, M1, N, K, nullptr, nullptr, false, st, w);
-        return rc ? rc : launch_mmq_impl(y2, W2, type2, x, M2, N, K, nullptr, nullptr, true, st, w);
+        const int rc = launch_mmq_impl(y1, W1, type1, x, M1, N, K, nullptr, nullptr, false, st, w, l.cap);
+        return rc ? rc : launch_mmq_impl(y2, W2, type2, x, M2, N, K, nullptr, nullptr, true, st, w, l.cap);
     }
     const size_t need = mmq_tc_scratch_bytes_pair(type1, M1, M2, N, K);
-    const bool cap = capturing(st);
-    __half* xq = w ? (__half*)w->scratch(need, cap) : nullptr;
+    __half* xq = w ? (__half*)w->scratch(need, l.cap) : nullptr;
     if (!xq) return set_error(JB_ERR_NOMEM, "batched gemm: %zu B of activation scratch unavailable", need);
-    return launch_mmq_tc_pair(y1, y2, W1, W2, type1, x, xq, M1, M2, N, K, false, st, *w, mmq_wide_applies(M1, M2, N, K) ? w->wide_scratch(cap) : nullptr);
+    return launch_mmq_tc_pair(y1, y2, W1, W2, type1, x, xq, M1, M2, N, K, false, st, *w, mmq_wide_applies(M1, M2, N, K) ? w->wide_scratch(l.cap) : nullptr);
 }
 
 static int launch_mmq_impl(__half* y, const void* W, int type, const __half* x, int M, int N, int K, int32_t* dbg, const __half* residual,
-                           bool same_x, cudaStream_t st, MmqWork* w) {
+                           bool same_x, cudaStream_t st, MmqWork* w, bool cap) {
     if (M <= 0 || N <= 0) return JB_OK;
     if (K <= 0 || K % QK_K) return set_error(JB_ERR_ARG, "batched gemm: K=%d is not a positive multiple of 256", K);
     if (type != T_Q4K && type != T_Q6K) return set_error(JB_ERR_TYPE, "batched gemm: ggml type %d", type);
     if (!y || !W || !x) return set_error(JB_ERR_PTR, "batched gemm: null pointer");
     if (type == T_Q4K && ((uintptr_t)W & 3)) return set_error(JB_ERR_PTR, "batched gemm: Q4_K weights must be 4-byte aligned");
-    const bool cap = capturing(st);
     // JLLM_B200_MMQ=cuda keeps the CUDA-core kernel (the one that can also export the integer accumulators)
     static const bool tc_off = [] { const char* e = getenv("JLLM_B200_MMQ"); return e && !strcmp(e, "cuda"); }();
     if (!dbg && !tc_off && mmq_stream_applies(W, type, M, N, K)) {
@@ -169,7 +257,7 @@ static int launch_mmq_impl(__half* y, const void* W, int type, const __half* x, 
         return launch_mmq_stream(y, W, type, x, sc, M, N, K, residual, same_x, st, *w);
     }
     if (residual) {          // the other kernels have no fused exit: product, then the add (in place)
-        const int rc = launch_mmq_impl(y, W, type, x, M, N, K, dbg, nullptr, false, st, w);
+        const int rc = launch_mmq_impl(y, W, type, x, M, N, K, dbg, nullptr, false, st, w, cap);
         return rc ? rc : launch_add_half(y, residual, y, (long long)N * M, st);
     }
     if (!dbg && !tc_off && mmq_tc_applies(W, type, M, N, K)) {

@@ -7,7 +7,7 @@ namespace jb {
 // y[N x M] half (token-major) = x[N x K] half . W^T, W in Q4_K / Q6_K blocks, with the
 // arithmetic of the reference's default prefill path (gemm_quant_batched,
 // src/kernels/gemv_q4.cu:2478-2495 -> mmq_q4k_llama.cu / mmq_q6k_llama.cu).
-// own: the scratch of a session that has one; else the library's.
+// own: the scratch of a session that has one; else the library's for this stream.
 // dbg_dots (optional): integer accumulators [N][M][K/32] (Q4_K) or [N][M][K/16] (Q6_K).
 int launch_mmq(__half* y, const void* W, int type, const __half* x, int M, int N, int K, int32_t* dbg_dots, cudaStream_t st, MmqWork* own = nullptr);
 // the same with a residual added on the way out (y = half(float(residual) + float(half(product))), residual [N][M] or null)
@@ -17,6 +17,8 @@ int launch_mmq_ex(__half* y, const void* W, int type, const __half* x, int M, in
 int launch_mmq_pair(__half* y1, __half* y2, const void* W1, int type1, const void* W2, int type2, const __half* x, int M1, int M2, int N, int K,
                     cudaStream_t st, MmqWork* own = nullptr);
 size_t mmq_scratch_bytes(int N, int K);
+void mmq_mark(cudaStream_t st);       // all products on st so far may be taken for over once the stream has come here
+cudaError_t mmq_alloc(void** p, size_t bytes, bool capturing);      // cudaMalloc, also under capture
 // tensor-core path (mmq_tc.cu): tcgen05.mma over fp16 operands built from the same quantised values
 bool   mmq_tc_applies(const void* W, int type, int M, int N, int K);
 size_t mmq_tc_scratch_bytes(int type, int M, int N, int K);

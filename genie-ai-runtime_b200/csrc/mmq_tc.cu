@@ -557,10 +557,11 @@ constexpr int MW_MIN_TOKENS = 384;      // 256 tokens: Q6_K 2560 x 9728 46 us th
 bool mmq_wide_applies(int M, int M2, int N, int K) {
     return N >= MW_MIN_TOKENS && (long long)M + M2 >= 256 && (size_t)(K + K / 16 + TC_K) * sizeof(__half) * 256 <= MW_WEIGHT_BYTES;
 }
-// Asked for once: an object whose request was refused stays with the fused kernel, whose results differ in their last bits.
+// Asked for once: an object whose request was refused stays with the fused kernel, whose results differ in their last bits.  A captured
+// call asks too, so that it takes the way an uncaptured one takes.
 void* MmqWork::wide_scratch(bool capturing) {
-    if (wide || no_wide || capturing) return wide;
-    if (cudaMalloc(&wide, MW_WEIGHT_BYTES + gemm_pair_part_floats() * sizeof(float)) != cudaSuccess) { cudaGetLastError(); wide = nullptr; no_wide = true; }
+    if (wide || no_wide || (capturing && !capture_limit)) return wide;
+    no_wide = mmq_alloc(&wide, MW_WEIGHT_BYTES + gemm_pair_part_floats() * sizeof(float), capturing) != cudaSuccess;
     return wide;
 }
 

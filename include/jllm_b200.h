@@ -76,7 +76,10 @@ int jllm_b200_gemv_quant_triple(void* y0, const void* W0, int type0, int M0, voi
                                 void* y2, const void* W2, int type2, int M2, const void* x, int K, void* stream);
 /* gemv_quant_f32 — :148-156, gemv_q4.cu:2755-2775.  fp32 output (logits). */
 int jllm_b200_gemv_quant_f32(float* y, const void* W, int ggml_type, const void* x, int M, int K, void* stream);
-/* gemm_quant_batched — :135-144, gemv_q4.cu:2478-2517.  y[N x M] = x[N x K] . W^T; N == 1 is gemv_quant. */
+/* gemm_quant_batched — :135-144, gemv_q4.cu:2478-2517.  y[N x M] = x[N x K] . W^T; N == 1 is gemv_quant.
+ * Scratch is the library's, one object per stream: calls on different streams, and from different threads, may run at the same time.
+ * Under capture a call may ask for no more scratch than an earlier call on the device did outside of captures (else ERR_NOMEM).  Graphs
+ * keep scratch of their own, one object per stream that was captured on: order the replays of graphs captured on the same stream. */
 int jllm_b200_gemm_quant_batched(void* y, const void* W, int ggml_type, const void* x, int M, int N, int K, void* stream);
 /* dequant_embedding_row — :160-167, gemv_q4.cu:2777-2809.  Returns 0 on success (the C++ symbol returns bool). */
 int jllm_b200_dequant_embedding_row(void* dst, const void* W, int ggml_type, int token_id, int hidden_dim, void* stream);

@@ -1,6 +1,8 @@
 """GPU parity of the batched K-quant GEMM (prefill) against the oracle and the reference's own
 golden vectors (tests/golden/q4k_int8.npz, q6k_int8.npz)."""
 import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -172,3 +174,120 @@ def test_captured_product_replays_after_larger_calls():
             assert torch.equal(y, want), N
             del keep, g
     assert jb.device_status() == 0
+
+
+def _stream_products(jb, seed, sizes, W, M, K, st):
+    """(launch, outputs): launch() enqueues one product per size on st."""
+    import torch
+    rng = np.random.Generator(np.random.PCG64(seed))
+    with torch.cuda.stream(st):
+        xs = [dev(orc.gen_act(rng, n * K)) for n in sizes]
+        ys = [torch.zeros(n * M, dtype=torch.float16, device="cuda") for n in sizes]
+    def launch():
+        for n, x, y in zip(sizes, xs, ys):
+            jb.gemm_quant_batched(y, W, 12, x, M, n, K, stream=st)
+    return launch, ys
+
+
+@pytest.mark.parametrize("count,threads", [(2, False), (40, False), (4, True)])
+def test_products_on_several_streams_at_once(count, threads):
+    """Products of every path (few tokens, fused, expanded) on several streams at the same time, more of them than the library keeps scratch for, and from
+    several threads: the bits of each stream's products run alone."""
+    import threading
+    import torch
+    jb = pkg()
+    M, K, sizes = 4096, 2560, (512, 8, 100, 400, 30)
+    W = dev(orc.gen_weight(np.random.Generator(np.random.PCG64(1012)), 12, M, K))
+    torch.cuda.synchronize()
+    # not torch.cuda.Stream: it hands out 32 streams in turn
+    import ctypes
+    rt = ctypes.CDLL("libcudart.so")
+    handles = []
+    for _ in range(count):
+        h = ctypes.c_void_p()
+        assert rt.cudaStreamCreateWithFlags(ctypes.byref(h), 1) == 0
+        handles.append(h)
+    work = [_stream_products(jb, 1013 + i, sizes, W, M, K, torch.cuda.ExternalStream(h.value)) for i, h in enumerate(handles)]
+    want = []
+    for launch, ys in work:
+        launch()
+        torch.cuda.synchronize()
+        want.append([y.clone() for y in ys])
+        for y in ys:
+            y.zero_()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        if threads:
+            ts = [threading.Thread(target=launch) for launch, _ in work]
+            for t in ts: t.start()
+            for t in ts: t.join()
+        else:
+            for launch, _ in work:
+                launch()
+        torch.cuda.synchronize()
+        for (_, ys), w in zip(work, want):
+            assert all(torch.equal(a, b) for a, b in zip(ys, w))
+    assert jb.device_status() == 0
+
+
+def test_two_sessions_prompt_at_once():
+    """Prompts of two decoder sessions on two streams, long enough for the expanded weights, give what they give one after the other."""
+    import torch
+    jb = pkg()
+    m = orc.gen_model(81, n_layers=2, hidden=1024, n_heads=8, n_kv=2, hd=128, ffn=2048, vocab=512)
+    w = jb.decoder.upload(m)
+    st = [torch.cuda.Stream() for _ in range(2)]
+    d = [jb.decoder.Decoder(m["cfg"], w, 1600, jb.decoder.FUSED | jb.decoder.PREFILL) for _ in range(2)]
+    prompts = [np.random.Generator(np.random.PCG64(1300 + i)).integers(0, 512, n) for i, n in enumerate((1500, 700))]
+    torch.cuda.synchronize()
+    want = []
+    for i in range(2):
+        d[i].prefill(prompts[i], 0, st[i])
+        want.append(d[i].logits().clone())
+    for _ in range(4):
+        for i in range(2):
+            d[i].prefill(prompts[i], 0, st[i])
+        assert all(torch.equal(d[i].logits(), want[i]) for i in range(2))
+    for x in d:
+        x.close()
+    assert jb.device_status() == 0
+
+
+def test_capture_on_another_stream_than_the_warm_up():
+    """A product captured on a stream that has no scratch yet: refused while the device has not seen a call that asked for as much (in a process of its own),
+    else the graph gives the uncaptured result, by the expanded path too."""
+    code = """
+import numpy as np, torch
+from oracle import oracle as orc
+from gpu_util import pkg, dev
+jb = pkg()
+jb.lib.jllm_b200_init(-1)
+M, K = 1024, 512
+W = dev(orc.gen_weight(np.random.Generator(np.random.PCG64(9)), 14, M, K))
+def graph(N, x, y):
+    st, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    rc = 0
+    with torch.cuda.graph(g, stream=st):
+        try:
+            jb.gemm_quant_batched(y, W, 14, x, M, N, K, stream=st)
+        except jb.JllmError as e:
+            rc = e.code
+    return g, rc
+for N in (40, 200, 500):
+    x, y = dev(orc.gen_act(np.random.Generator(np.random.PCG64(N)), N * K)), torch.zeros(N * M, dtype=torch.float16, device="cuda")
+    g, rc = graph(N, x, y)
+    assert rc == 5, (N, rc)
+    jb.gemm_quant_batched(y, W, 14, x, M, N, K)
+    torch.cuda.synchronize()
+    want = y.clone()
+    y.zero_()
+    g, rc = graph(N, x, y)
+    assert rc == 0, (N, rc, jb.last_error())
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want), N
+assert jb.device_status() == 0
+"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, env=dict(os.environ, PYTHONPATH=os.pathsep.join([os.path.dirname(here), here])))
+    assert r.returncode == 0, r.stderr[-2000:]
