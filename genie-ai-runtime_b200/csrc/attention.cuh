@@ -46,6 +46,7 @@ bool   attn_tma_encode(void* map_out128, const void* cache_base, int rows, int n
 bool   attention_prefill_fast_applies(const AttnCall& c);          // causal prefill (causal_start >= 0), INT8 KV, head_dim 128, GQA 1/2/4
 int    launch_attention_prefill_fast(const AttnCall& c, cudaStream_t st);
 // causal prefill on tcgen05 (attention_tc.cu): BF16 caches, and INT8 caches with a workspace (c.scratch, attention_tc_scratch bytes)
+constexpr int AT_MIN_TOKENS = 64;
 bool   attention_tc_applies(const AttnCall& c);
 int    launch_attention_tc(const AttnCall& c, cudaStream_t st);
 size_t attention_tc_scratch(int n_kv, int positions);

@@ -331,7 +331,6 @@ size_t attention_tc_scratch(int n_kv, int positions) {
 
 // Query rows in groups that divide a tile, head sizes in whole 16-byte rows that fill their 64-element chunks but for the last, tiles
 // of 64 keys worth the fixed cost (from AT_MIN_TOKENS on).  INT8: a workspace for the widened codes.
-constexpr int AT_MIN_TOKENS = 64;
 bool attention_tc_applies(const AttnCall& c) {
     const int kind = c.kind(), R = c.n_kv > 0 ? c.n_heads / c.n_kv : 0;
     if ((kind != EK_BF16 && kind != EK_INT8) || c.causal_start < 0 || c.batch < AT_MIN_TOKENS || c.window || c.records || c.k_list || R < 1 || R > 128 || (R & (R - 1)) || c.n_heads != R * c.n_kv) return false;

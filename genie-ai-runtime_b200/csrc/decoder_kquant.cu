@@ -35,14 +35,13 @@ struct KquantDecoder : jllm_b200_decoder {
     uint32_t* seq = nullptr;
     // batched prompt prefill (flag bit 4): activations of up to pf_cap prompt tokens, allocated on first use
     void* pf_slab = nullptr;
-    void* pf_codes = nullptr;          // one layer's cache, widened for the prompt attention; null: the context is too long to hold it
+    void* pf_codes = nullptr;          // in the slab: one layer's cache, widened for the prompt attention; null: too short a chunk, too long a context, or no memory
     __half *pf_x = nullptr, *pf_x2 = nullptr, *pf_normed = nullptr, *pf_y = nullptr, *pf_q = nullptr, *pf_att = nullptr, *pf_k = nullptr,
            *pf_v = nullptr, *pf_gate = nullptr, *pf_up = nullptr, *pf_sw = nullptr;
 
     ~KquantDecoder() override {
         if (slab) cudaFree(slab);
         if (pf_slab) cudaFree(pf_slab);
-        if (pf_codes) cudaFree(pf_codes);
         if (seq) cudaFree(seq);
         kv.destroy();
     }
@@ -288,15 +287,16 @@ static int dec_enqueue_step_tp(KquantDecoder* d, int n_splits, cudaStream_t st) 
 // gate/up, SwiGLU, W_down, residual.  After the last chunk: final norm and logits of the last token only, greedy token.
 int KquantDecoder::reserve_chunk(int cap) {
     if (cap <= pf_cap) return JB_OK;
-    if (pf_slab) { cudaFree(pf_slab); pf_slab = nullptr; pf_cap = 0; }
+    if (pf_slab) { cudaFree(pf_slab); pf_slab = pf_codes = nullptr; pf_cap = 0; }
     const size_t N = (size_t)cap, H = m.hidden_dim, QD = (size_t)m.n_heads * m.head_dim, KVD = (size_t)m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t total = 4 * al(N * H * 2) + 2 * al(N * QD * 2) + 2 * al(N * KVD * 2) + 3 * al(N * I * 2);
-    if (cudaMalloc(&pf_slab, total) != cudaSuccess) { cudaGetLastError(); return set_error(JB_ERR_NOMEM, "decoder: %zu B of prefill activations", total); }
-    if (!pf_codes && m.max_context <= PF_CODES_MAX && m.head_dim == 128 && cudaMalloc(&pf_codes, attention_tc_scratch(m.n_kv_heads, m.max_context)) != cudaSuccess) {
-        cudaGetLastError();
-        pf_codes = nullptr;
-    }
+    // one allocation for all of it: it is made inside a session's first prompt, where each costs 0.4 - 2 ms (512 tokens: the first prompt
+    // took 1064 us more than the next with two, 444 with one)
+    size_t codes = cap >= AT_MIN_TOKENS && m.max_context <= PF_CODES_MAX && m.head_dim == 128 ? attention_tc_scratch(m.n_kv_heads, m.max_context) : 0;
+    if (codes && cudaMalloc(&pf_slab, total + codes) != cudaSuccess) { cudaGetLastError(); pf_slab = nullptr; codes = 0; }
+    if (!pf_slab && cudaMalloc(&pf_slab, total) != cudaSuccess) { cudaGetLastError(); pf_slab = nullptr; return set_error(JB_ERR_NOMEM, "decoder: %zu B of prefill activations", total); }
+    pf_codes = codes ? (char*)pf_slab + total : nullptr;
     char* p = (char*)pf_slab;
     auto take = [&](size_t b) { char* r = p; p += al(b); return r; };
     pf_x = (__half*)take(N * H * 2); pf_x2 = (__half*)take(N * H * 2); pf_normed = (__half*)take(N * H * 2); pf_y = (__half*)take(N * H * 2);

@@ -108,6 +108,7 @@ struct LayerDecoder : jllm_b200_decoder {
 int LayerDecoder::alloc_acts(Acts& a, size_t R, bool chunk) {
     const size_t es = elem_bytes(kind), W = pad8(m.width), T = max_top;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    bool ranges = chunk && kind == EK_BF16;
     for (int pass = 0; pass < 2; ++pass) {
         size_t at = 0;
         auto take = [&](size_t b) { void* r = (char*)a.slab + at; at += al(b); return r; };
@@ -124,12 +125,14 @@ int LayerDecoder::alloc_acts(Acts& a, size_t R, bool chunk) {
         if (chunk) {
             rank = (int*)take(R * T * 4); slots = (int*)take(R * T * 4); counts = (int*)take((size_t)(max_e + 1) * 4); off = (int*)take((size_t)(max_e + 1) * 4);
             rows = (int*)take(R * 4);
-            if (kind == EK_BF16) part = (float*)take(gemm_pair_part_floats() * 4);
             if (!m.parallel) { hp = take(R * T * W * es); ye = take(R * T * W * es); }
         }
+        const size_t acts = at;
+        if (ranges) part = (float*)take(gemm_pair_part_floats() * 4);
         if (pass == 0) {
-            if (cudaMalloc(&a.slab, at) != cudaSuccess) { cudaGetLastError(); a.slab = nullptr; return set_error(JB_ERR_NOMEM, "decoder: %zu B of activations", at); }
-            JB_CUDA(cudaMemset(a.slab, 0, at));           // the padding of every row stays zero
+            if (ranges && cudaMalloc(&a.slab, at) != cudaSuccess) { cudaGetLastError(); a.slab = nullptr; ranges = false; }      // the products do without
+            if (!a.slab && cudaMalloc(&a.slab, acts) != cudaSuccess) { cudaGetLastError(); a.slab = nullptr; return set_error(JB_ERR_NOMEM, "decoder: %zu B of activations", acts); }
+            JB_CUDA(cudaMemset(a.slab, 0, acts));         // the padding of every row stays zero
             continue;
         }
         a.x[0] = x0; a.x[1] = x1; a.y = y; a.h = h; a.q = q; a.att = att; a.z = z; a.wts = wts; a.ids = ids; a.a = ga;
