@@ -189,13 +189,23 @@ int jllm_b200_flash_attention_decode(void* o, const void* q, const void* k, cons
 }
 int jllm_b200_flash_attention_prefill_batched(void* o, const void* q, const void* k, const void* v, int nh, int nkv, int hd, int chd,
                                               int N, int start, float scale, int i8, const float* ks, const float* vs, int window, void* s) {
+    return jllm_b200_flash_attention_prefill_workspace(o, q, k, v, nh, nkv, hd, chd, N, start, scale, i8, ks, vs, window, nullptr, 0, s);
+}
+int64_t jllm_b200_flash_attention_prefill_workspace_bytes(int nkv, int positions) { return nkv > 0 && positions > 0 ? (int64_t)attention_tc_scratch(nkv, positions) : 0; }
+int jllm_b200_flash_attention_prefill_workspace(void* o, const void* q, const void* k, const void* v, int nh, int nkv, int hd, int chd, int N, int start,
+                                                float scale, int i8, const float* ks, const float* vs, int window, void* ws, int64_t ws_bytes, void* s) {
     if (N <= 0) return JB_OK;
     AttnCall c;
     c.out = H(o); c.q = CH(q); c.k = k; c.v = v; c.ks = ks; c.vs = vs; c.n_heads = nh; c.n_kv = nkv; c.hd = hd; c.chd = chd;
     c.scale = scale; c.kv_int8 = i8; c.window = window; c.causal_start = start; c.batch = N; c.n_splits = 1;
     if (start < 0) return set_error(JB_ERR_ARG, "prefill attention: start_pos=%d", start);
     if (!c.out || !c.q || !k || !v) return set_error(JB_ERR_PTR, "prefill attention: null pointer");
-    // INT8 cache with 128-wide heads: query-tiled tensor-core kernel; everything else: the general slice, one CTA per (head, token)
+    if (ws && (((uintptr_t)ws & 15) || ws_bytes < jllm_b200_flash_attention_prefill_workspace_bytes(nkv, start + N)))
+        return set_error(JB_ERR_ARG, "prefill attention: workspace of %lld bytes for %d positions", (long long)ws_bytes, start + N);
+    c.scratch = (float*)ws;
+    // INT8 cache with 128-wide heads: tcgen05 over widened codes, or the query-tiled kernel over the codes; everything else: the general
+    // slice, one CTA per (head, token)
+    if (attention_tc_applies(c)) return launch_attention_tc(c, ST(s));
     return attention_prefill_fast_applies(c) ? launch_attention_prefill_fast(c, ST(s)) : launch_attention_general(c, ST(s));
 }
 int jllm_b200_flash_attention_decode_dyn(void* o, const void* q, const void* k, const void* v, int nh, int nkv, int hd, int chd,

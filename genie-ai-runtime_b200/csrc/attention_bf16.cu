@@ -410,7 +410,6 @@ static int fa_launch(const FaArgs& a, bool prefill, cudaStream_t st) {
 }
 
 int launch_attention_bf16(const AttnCall& c, cudaStream_t st) {
-    if (attention_tc_applies(c)) return launch_attention_tc(c, st);
     FaArgs a = {};
     const bool prefill = c.causal_start >= 0;
     a.out = (__nv_bfloat16*)c.out; a.q = (const __nv_bfloat16*)c.q; a.k = (const __nv_bfloat16*)c.k; a.v = (const __nv_bfloat16*)c.v;
@@ -420,6 +419,7 @@ int launch_attention_bf16(const AttnCall& c, cudaStream_t st) {
     a.ldk = c.ldk > 0 ? c.ldk : c.n_kv * a.dim; a.ldv = c.ldv > 0 ? c.ldv : c.n_kv * a.vdim;
     a.k2 = (const __nv_bfloat16*)c.k2; a.dim1 = a.dim - c.hd2; a.ldk2 = c.ldk2; a.gate = c.gate; a.ldg = c.ldg;
     if (a.k2 && !attention_keys2_applies(c)) return set_error(JB_ERR_ARG, "bf16 attention: keys of %d and %d elements", a.dim1, c.hd2);
+    if (attention_tc_applies(c)) return launch_attention_tc(c, st);
     a.n_tokens = c.batch; a.start = c.causal_start; a.seq_len = c.seq_len; a.d_pos = c.d_pos;
     a.scale = c.scale; a.sink = c.sink; a.qt_coef = c.qt_coef; a.qt_every = c.qt_every;
     a.row_blocks = (a.R + 15) / 16;

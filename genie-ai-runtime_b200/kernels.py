@@ -134,6 +134,20 @@ def flash_attention_prefill_batched(output, q, k_cache, v_cache, n_heads, n_kv_h
                                                         _stream(stream)))
 
 
+def flash_attention_prefill_workspace_bytes(n_kv_heads, positions):
+    lib.jllm_b200_flash_attention_prefill_workspace_bytes.restype = C.c_int64
+    return int(lib.jllm_b200_flash_attention_prefill_workspace_bytes(i32(n_kv_heads), i32(positions)))
+
+
+def flash_attention_prefill_workspace(output, q, k_cache, v_cache, n_heads, n_kv_heads, head_dim, cache_head_dim, N, start_pos, scale,
+                                      kv_int8, k_scales, v_scales, window, workspace, stream=None):
+    size = 0 if workspace is None else workspace.numel() * workspace.element_size()
+    check(lib.jllm_b200_flash_attention_prefill_workspace(_ptr(output), _ptr(q), _ptr(k_cache), _ptr(v_cache), i32(n_heads), i32(n_kv_heads),
+                                                          i32(head_dim), i32(cache_head_dim), i32(N), i32(start_pos), f32(scale),
+                                                          i32(1 if kv_int8 else 0), _ptr(k_scales), _ptr(v_scales), i32(window),
+                                                          _ptr(workspace), C.c_int64(size), _stream(stream)))
+
+
 def flash_attention_decode_dyn(output, q, k_cache, v_cache, n_heads, n_kv_heads, head_dim, cache_head_dim, d_pos, scale, kv_int8,
                                kv_scales, window, n_splits, stream=None):
     check(lib.jllm_b200_flash_attention_decode_dyn(_ptr(output), _ptr(q), _ptr(k_cache), _ptr(v_cache), i32(n_heads), i32(n_kv_heads),

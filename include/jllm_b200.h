@@ -177,6 +177,14 @@ int jllm_b200_gemm_quant_batched_int_dots(void* y, int32_t* dots, const void* W,
  * second reusing the quantised activations.  N >= 2. */
 int jllm_b200_gemm_quant_batched_pair(void* y0, const void* W0, int type0, int M0, void* y1, const void* W1, int type1, int M1,
                                       const void* x, int N, int K, void* stream);
+/* flash_attention_prefill_batched with a workspace of the caller's (16-byte aligned device memory of workspace_bytes(n_kv_heads,
+ * start_pos + N) bytes, used by this call only): from 64 tokens on, INT8 caches with 128-wide heads are widened there and multiplied on
+ * the 5th-generation tensor cores (any power of two of query heads per KV head up to 128, no window).  Null: as without. */
+int64_t jllm_b200_flash_attention_prefill_workspace_bytes(int n_kv_heads, int positions);
+int jllm_b200_flash_attention_prefill_workspace(void* output, const void* q, const void* k_cache, const void* v_cache, int n_heads,
+                                                int n_kv_heads, int head_dim, int cache_head_dim, int N, int start_pos, float scale,
+                                                int kv_int8, const float* k_scales, const float* v_scales, int window, void* workspace,
+                                                int64_t workspace_bytes, void* stream);
 /* RMSNorm fused into the shared-activation GEMVs: x := half(x * rrms * w) is formed in shared
  * memory and quantised there, equal to fused_rmsnorm_residual -> gemv_quant_pair / _triple. */
 int jllm_b200_norm_gemv_quant_pair(void* y0, const void* W0, int type0, int M0, void* y1, const void* W1, int type1, int M1,

@@ -137,3 +137,50 @@ def test_prefill_int8_matches_reference_gpu_record(N):
     got = out.float().cpu().numpy().reshape(N, gc.NH, gc.HD)[sel].reshape(-1, gc.HD)
     want = ref[f"prefill_attn_N{N}_out"].view(np.float16).astype(np.float32).reshape(-1, gc.HD)
     _check(got, want)
+
+
+def _prompt_on_a_workspace(jb, q, k, ks, v, vs, nh, nkv, N, start):
+    import torch
+    out = torch.full((N * nh * 128 + 64,), 7.0, dtype=torch.float16, device="cuda")
+    ws = torch.full((jb.flash_attention_prefill_workspace_bytes(nkv, start + N),), 0x7F, dtype=torch.uint8, device="cuda")      # 0x7F7F: NaN in fp16
+    n0 = jb.launch_count()
+    jb.flash_attention_prefill_workspace(out, dev(q), dev(k), dev(v), nh, nkv, 128, 128, N, start, float(1 / np.sqrt(128)), True, dev(ks), dev(vs), 0, ws)
+    assert jb.launch_count() - n0 == (2 if N >= 64 else 1)               # codes widened, then attention
+    got = out.float().cpu().numpy()
+    assert np.all(got[N * nh * 128:] == 7.0), "wrote past the output"
+    return got[:N * nh * 128].reshape(N, nh, 128)
+
+
+# groups of 1 .. 128 query heads, row tiles of 128 / group tokens and their neighbours, a start inside a key tile, counts around 64, several turns of the
+# five-stage key ring
+@pytest.mark.parametrize("N,start,nh,nkv", [(63, 0, 32, 8), (64, 0, 32, 8), (65, 0, 32, 8), (127, 37, 32, 8), (128, 300, 8, 8), (129, 0, 8, 8), (257, 63, 4, 4), (130, 100, 16, 8),
+                                            (257, 1000, 32, 8), (100, 2000, 16, 2), (70, 500, 16, 1), (66, 64, 64, 2), (64, 130, 128, 1), (65, 1, 128, 1), (300, 0, 2, 1)])
+def test_prefill_int8_on_a_workspace(N, start, nh, nkv):
+    """Causal prefill over an INT8 cache whose codes are widened into a workspace (the tcgen05 kernel from 64 tokens on), to the tolerance of the other kernels.
+    The keys of the last quarter are long: scores rise late and by far more than the 2^8 up to which a maximum is kept."""
+    jb = pkg()
+    rng = np.random.Generator(np.random.PCG64(6000 + 7 * N + start + nh))
+    L = start + N
+    q = orc.gen_act(rng, N * nh * 128)
+    k, ks = orc.gen_kv(rng, L, nkv, 128); v, vs = orc.gen_kv(rng, L, nkv, 128)
+    ks[3 * L // 4:] *= 12
+    got = _prompt_on_a_workspace(jb, q, k, ks, v, vs, nh, nkv, N, start)
+    _check(got, orc.attention_prefill(q, k, v, nh, nkv, 128, N, start, 1 / np.sqrt(128), True, ks, vs))
+    assert jb.device_status() == 0
+
+
+def test_prefill_workspace_arguments():
+    import torch
+    jb = pkg()
+    t, f = torch.zeros(64 * 4 * 128, dtype=torch.float16, device="cuda"), torch.zeros(64 * 4, dtype=torch.float32, device="cuda")
+    c = torch.zeros(64 * 4 * 128, dtype=torch.int8, device="cuda")
+    need = jb.flash_attention_prefill_workspace_bytes(4, 64)
+    for ws in (torch.zeros(need - 1, dtype=torch.uint8, device="cuda"), torch.zeros(need + 1, dtype=torch.uint8, device="cuda")[1:]):
+        with pytest.raises(jb.JllmError) as e:
+            jb.flash_attention_prefill_workspace(t, t, c, c, 4, 4, 128, 128, 64, 0, 1.0, True, f, f, 0, ws)
+        assert e.value.code == 1
+    a, b = torch.ones_like(t), torch.ones_like(t)                        # no workspace: the call without one
+    q = dev(orc.gen_act(np.random.Generator(np.random.PCG64(1)), 64 * 4 * 128))
+    jb.flash_attention_prefill_workspace(a, q, c, c, 4, 4, 128, 128, 64, 0, 1.0, True, f, f, 0, None)
+    jb.flash_attention_prefill_batched(b, q, c, c, 4, 4, 128, 128, 64, 0, 1.0, True, f, f, 0)
+    assert torch.equal(a, b)

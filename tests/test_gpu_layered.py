@@ -136,6 +136,19 @@ def test_prompt_attention(H, G, dim, vdim, dtype):
         assert np.abs(got - want).max() < tol * max(1.0, np.abs(want).max()), (start, T)
 
 
+@pytest.mark.parametrize("H,G,dim,vdim,start,T", [(8, 2, 128, 128, 600, 130), (8, 1, 64, 64, 0, 257), (16, 1, 128, 64, 1000, 64), (4, 4, 192, 128, 70, 260), (32, 1, 72, 40, 333, 65),
+                                                  (128, 1, 64, 128, 5, 66), (3, 3, 128, 128, 1500, 129)])
+def test_long_prompt_attention_in_groups(H, G, dim, vdim, start, T):
+    """bf16 prompts of 64 tokens and more: groups of 1 .. 128 query heads, several turns of the key ring, scores that rise late and by far more than the 2^8 up to
+    which a row's maximum is kept (queries aim at ever longer keys)."""
+    jb, r = pkg(), rng(H * 999 + T)
+    q, k, v = _planted(r, T, start + T, H, G, dim, vdim, start, "bfloat16")
+    grow = np.linspace(0.2, 3.0, start + T)[:, None, None]
+    k = rounded(k * grow, "bfloat16")
+    got, want = _attend(jb, q, k, v, "bfloat16", 1.7 / np.sqrt(dim), start, None, (0.4, 100)), _want(q, k, v, 1.7 / np.sqrt(dim), start, None, (0.4, 100))
+    assert np.abs(got - want).max() < 1.5e-2 * max(1.0, np.abs(want).max())
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H,G,dim,vdim", HEADS)
 def test_decode_attention_and_its_slices(H, G, dim, vdim, dtype):
