@@ -27,9 +27,10 @@ constexpr float AT_LAZY = 8.0f;
 constexpr int at_stages(int qc, int vc) { const int s = (224 * 1024 - 2 * qc * AT_QCHUNK) / ((qc + vc) * AT_KCHUNK); return s > 6 ? 6 : s; }
 
 struct AtArgs {
-    void* out; int n_heads, R, dim1, vdim, ldo, n_tokens, start, stages;
+    void* out; int R, dim1, vdim, ldo, n_tokens, start;
     float scale; const float* sink; float qt_coef; double qt_every; const float* gate; int ldg;
     const float* ks; const float* vs; int lds;       // INT8: scales [kv head][lds]
+    const __nv_bfloat16 *q, *k, *k2, *v; long long ldq, ldk, ldk2, ldv; int dim;      // BF16: what the maps describe, for at_row
     int* status;
 };
 
@@ -60,6 +61,43 @@ __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile
     int ok = 1;
     if ((threadIdx.x & 31) == 0) { ok = tc_wait(bar, parity) && !*fail; if (!ok) tc_fail(fail, status); }
     return __shfl_sync(0xFFFFFFFFu, ok, 0) != 0;
+}
+
+__device__ __forceinline__ float at_dot8(uint4 x, uint4 y, float s) {
+    const uint32_t a[4] = {x.x, x.y, x.z, x.w}, b[4] = {y.x, y.y, y.z, y.w};
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        s = fmaf(__uint_as_float(a[i] << 16), __uint_as_float(b[i] << 16), s);
+        s = fmaf(__uint_as_float(a[i] & 0xFFFF0000u), __uint_as_float(b[i] & 0xFFFF0000u), s);
+    }
+    return s;
+}
+// One output row by one warp, over the keys that the row sees and no others: for rows whose tile holds an infinite or NaN value of a
+// LATER token, which the products above multiply with a weight of zero.  fsc, m: score factor and maximum in base 2; inv: 1 / sum.
+__device__ __noinline__ void at_row(const AtArgs& a, int g, int tok, int head, float fsc, float m, float inv) {
+    const int lane = threadIdx.x & 31, pos = a.start + tok, d0 = 4 * lane;
+    const __nv_bfloat16* q = a.q + tok * a.ldq + (long long)head * a.dim;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int base = 0; base <= pos; base += 32) {
+        const int key = min(base + lane, pos);
+        float s = 0.f;
+        for (int d = 0; d < a.dim; d += 8) {
+            const __nv_bfloat16* k = d < a.dim1 ? a.k + key * a.ldk + (long long)g * a.dim1 + d : a.k2 + key * a.ldk2 + d - a.dim1;
+            s = at_dot8(*reinterpret_cast<const uint4*>(q + d), *reinterpret_cast<const uint4*>(k), s);
+        }
+        const float p = __bfloat162float(__float2bfloat16_rn(at_exp2(s * fsc - m)));
+        for (int j = 0; j < 32 && base + j <= pos; ++j) {
+            const float w = __shfl_sync(0xFFFFFFFFu, p, j);
+            if (d0 < a.vdim) {
+                const uint2 v = *reinterpret_cast<const uint2*>(a.v + (base + j) * a.ldv + (long long)g * a.vdim + d0);
+                acc[0] = fmaf(w, __uint_as_float(v.x << 16), acc[0]); acc[1] = fmaf(w, __uint_as_float(v.x & 0xFFFF0000u), acc[1]);
+                acc[2] = fmaf(w, __uint_as_float(v.y << 16), acc[2]); acc[3] = fmaf(w, __uint_as_float(v.y & 0xFFFF0000u), acc[3]);
+            }
+        }
+    }
+    if (d0 < a.vdim)
+        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)tok * a.ldo + (size_t)head * a.vdim + d0) =
+            make_uint2(fa_pack(acc[0] * inv, acc[1] * inv), fa_pack(acc[2] * inv, acc[3] * inv));
 }
 
 // QC: 64-element chunks of a query (and key) row, VC of a value row
@@ -187,7 +225,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                 #pragma unroll
                 for (int i = 0; i < 64; ++i) v[i] *= fsc;
             }
-            if (k0 + AT_KEYS - 1 > first_pos) {
+            const bool diagonal = k0 + AT_KEYS - 1 > first_pos;
+            if (diagonal) {
                 #pragma unroll
                 for (int i = 0; i < 64; ++i) if (k0 + i > pos) v[i] = -INFINITY;
             }
@@ -205,17 +244,23 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             uint32_t hi[32], lo[32];
             if (INT8) {
                 const float4* vs = reinterpret_cast<const float4*>(a.vs + (size_t)g * a.lds + k0);
-                #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const float4 f = vs[i];
-                    const float w[4] = {v[4 * i] * f.x, v[4 * i + 1] * f.y, v[4 * i + 2] * f.z, v[4 * i + 3] * f.w};
+                // `seen`: a masked weight is zero whatever the scale of its value (infinite where a later token overflowed)
+                auto planes = [&](auto seen) {
                     #pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const uint32_t h = fa_pack(w[2 * e], w[2 * e + 1]);
-                        hi[2 * i + e] = h;
-                        lo[2 * i + e] = fa_pack(w[2 * e] - __uint_as_float(h << 16), w[2 * e + 1] - __uint_as_float(h & 0xFFFF0000u));
+                    for (int i = 0; i < 16; ++i) {
+                        const float4 f = vs[i];
+                        const float w[4] = {seen(4 * i) ? v[4 * i] * f.x : 0.f, seen(4 * i + 1) ? v[4 * i + 1] * f.y : 0.f,
+                                            seen(4 * i + 2) ? v[4 * i + 2] * f.z : 0.f, seen(4 * i + 3) ? v[4 * i + 3] * f.w : 0.f};
+                        #pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const uint32_t h = fa_pack(w[2 * e], w[2 * e + 1]);
+                            hi[2 * i + e] = h;
+                            lo[2 * i + e] = fa_pack(w[2 * e] - __uint_as_float(h << 16), w[2 * e + 1] - __uint_as_float(h & 0xFFFF0000u));
+                        }
                     }
-                }
+                };
+                if (diagonal) planes([&](int i) { return k0 + i <= pos; });
+                else          planes([](int) { return true; });
             } else {
                 #pragma unroll
                 for (int i = 0; i < 32; ++i) hi[i] = fa_pack(v[2 * i], v[2 * i + 1]);
@@ -248,11 +293,16 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             const float inv = sink_norm(m / FA_LOG2E, l, a.sink ? a.sink + head : nullptr) * head_gate(a.gate, a.ldg, tok, head);
             __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)tok * a.ldo + (size_t)head * a.vdim;
             __half* oh = reinterpret_cast<__half*>(a.out) + (size_t)tok * a.ldo + (size_t)head * a.vdim;
+            bool finite = true;
             #pragma unroll 1
             for (int c = 0; c < VC * 64; c += 32) {
                 uint32_t o[32];
                 __syncwarp();
                 tc_ld32(tm + 128u + (uint32_t)c, o);
+                if (!INT8) {
+                    #pragma unroll
+                    for (int i = 0; i < 32; ++i) finite = finite && (o[i] & 0x7F800000u) != 0x7F800000u;
+                }
                 if (fr < total) {
                     #pragma unroll
                     for (int i = 0; i < 4; ++i) {
@@ -268,6 +318,15 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                             else      *reinterpret_cast<uint4*>(ob + c + 8 * i) = make_uint4(w[0], w[1], w[2], w[3]);
                         }
                     }
+                }
+            }
+            // sums of scores that are finite over outputs that are not: some value is infinite or NaN, and it may be one that the row does not see
+            if (!INT8) {
+                __syncwarp();
+                for (unsigned rows = __ballot_sync(0xFFFFFFFFu, fr < total && !finite && isfinite(l)); rows; rows &= rows - 1) {
+                    const int r = __ffs(rows) - 1;
+                    at_row(a, g, __shfl_sync(0xFFFFFFFFu, tok, r), __shfl_sync(0xFFFFFFFFu, head, r), __shfl_sync(0xFFFFFFFFu, fsc, r), __shfl_sync(0xFFFFFFFFu, m == -INFINITY ? 0.f : m, r),
+                           __shfl_sync(0xFFFFFFFFu, inv, r));
                 }
             }
         }
@@ -358,10 +417,13 @@ int launch_attention_tc(const AttnCall& c, cudaStream_t st) {
     const int R = c.n_heads / c.n_kv, vd = c.vhd > 0 ? c.vhd : c.hd, d1 = c.hd - (c.k2 ? c.hd2 : 0), keys = c.causal_start + c.batch;
     const long long ldq = c.ldq > 0 ? c.ldq : (long long)c.n_heads * c.hd, ldk = c.ldk > 0 ? c.ldk : (long long)c.n_kv * d1, ldv = c.ldv > 0 ? c.ldv : (long long)c.n_kv * vd;
     AtArgs a = {};
-    a.out = c.out; a.n_heads = c.n_heads; a.R = R; a.dim1 = d1; a.vdim = vd; a.ldo = c.ldo > 0 ? c.ldo : c.n_heads * vd; a.n_tokens = c.batch; a.start = c.causal_start;
+    a.out = c.out; a.R = R; a.dim1 = d1; a.vdim = vd; a.ldo = c.ldo > 0 ? c.ldo : c.n_heads * vd; a.n_tokens = c.batch; a.start = c.causal_start;
     a.scale = c.scale; a.sink = c.sink; a.qt_coef = c.qt_coef; a.qt_every = c.qt_every; a.gate = c.gate; a.ldg = c.ldg; a.status = cx->d_status;
     const void *kp = c.k, *vp = c.v;
-    if (int8) {
+    if (!int8) {
+        a.q = (const __nv_bfloat16*)c.q; a.k = (const __nv_bfloat16*)c.k; a.k2 = (const __nv_bfloat16*)c.k2; a.v = (const __nv_bfloat16*)c.v;
+        a.ldq = ldq; a.ldk = ldk; a.ldk2 = c.ldk2; a.ldv = ldv; a.dim = c.hd;
+    } else {
         const int padded = (keys + AT_KEYS - 1) / AT_KEYS * AT_KEYS;
         char* s = reinterpret_cast<char*>(c.scratch);
         const size_t plane = (size_t)padded * c.n_kv * 128 * 2, sc = (size_t)padded * c.n_kv * sizeof(float);

@@ -184,3 +184,23 @@ def test_prefill_workspace_arguments():
     jb.flash_attention_prefill_workspace(a, q, c, c, 4, 4, 128, 128, 64, 0, 1.0, True, f, f, 0, None)
     jb.flash_attention_prefill_batched(b, q, c, c, 4, 4, 128, 128, 64, 0, 1.0, True, f, f, 0)
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("late,nh,nkv", [(1, 32, 8), (70, 8, 8), (199, 16, 2)])
+def test_prefill_int8_is_not_spoiled_by_later_tokens(late, nh, nkv):
+    """A token whose values overflowed (an infinite scale) leaves the tokens before it as they were, bit for bit, and is not hidden from those that see it."""
+    jb = pkg()
+    rng = np.random.Generator(np.random.PCG64(6500 + late))
+    N = 200
+    q = orc.gen_act(rng, N * nh * 128)
+    k, ks = orc.gen_kv(rng, N, nkv, 128); v, vs = orc.gen_kv(rng, N, nkv, 128)
+    clean = _prompt_on_a_workspace(jb, q, k, ks, v, vs, nh, nkv, N, 0)
+    for a in (vs, ks):
+        keep = a[late, nkv - 1]
+        a[late, nkv - 1] = np.inf
+        got = _prompt_on_a_workspace(jb, q, k, ks, v, vs, nh, nkv, N, 0)
+        a[late, nkv - 1] = keep
+        assert np.array_equal(got[:late], clean[:late])
+        hit = got[late:, nh - nh // nkv:]
+        assert not np.isfinite(hit).all() and np.array_equal(got[late:, :nh - nh // nkv], clean[late:, :nh - nh // nkv])
+    assert jb.device_status() == 0

@@ -149,6 +149,40 @@ def test_long_prompt_attention_in_groups(H, G, dim, vdim, start, T):
     assert np.abs(got - want).max() < 1.5e-2 * max(1.0, np.abs(want).max())
 
 
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("H,G,dim,vdim,start", [(4, 4, 128, 128, 0), (8, 2, 64, 96, 70), (2, 1, 192, 64, 3)])
+def test_prompt_attention_is_not_spoiled_by_later_tokens(H, G, dim, vdim, start, bad):
+    """A value that is infinite or NaN reaches the tokens that see it, in its own element, and no token before it."""
+    jb, r = pkg(), rng(dim + start)
+    T, late, e = 300, start + 131, 5
+    q, k, v = _planted(r, T, start + T, H, G, dim, vdim, start, "bfloat16")
+    scale = 1.0 / np.sqrt(dim)
+    sink = r.standard_normal(H)
+    clean = _want(q, k, v, scale, start, sink, None).reshape(T, H, vdim)
+    v[late, G - 1, e] = bad
+    got = _attend(jb, q, k, v, "bfloat16", scale, start, sink, None).reshape(T, H, vdim)
+    hit = np.zeros((T, H, vdim), bool)
+    hit[late - start:, H - H // G:, e] = True
+    assert not np.isfinite(got[hit]).any()
+    assert np.abs(got[~hit] - clean[~hit]).max() < 1.5e-2 * max(1.0, np.abs(clean).max())
+
+
+def test_prompt_attention_over_keys_in_two_parts_is_not_spoiled_by_later_tokens():
+    import torch
+    jb, r = pkg(), rng(77)
+    T, H, d1, d2, vd, late = 200, 2, 64, 32, 64, 120
+    q, k1, k2, v = (rounded(r.standard_normal(s), "bfloat16") for s in ((T, H, d1 + d2), (T, H, d1), (T, d2), (T, H, vd)))
+    k = np.concatenate([k1, np.broadcast_to(k2[:, None], (T, H, d2))], -1)
+    want = _want(q, k, v, 0.1, 0, None, None).reshape(T, H, vd)
+    v[late, 1, 9] = np.inf
+    out = torch.zeros((T, H * vd), dtype=torch.bfloat16, device="cuda")
+    jb.split_key_attention(out, up(q.reshape(T, -1), "bfloat16"), up(k1.reshape(T, -1), "bfloat16"), up(k2, "bfloat16"), d2, up(v.reshape(T, -1), "bfloat16"), H, d1, d2, vd, 0.1, T, 0)
+    got = as_np(out).reshape(T, H, vd)
+    hit = np.zeros((T, H, vd), bool)
+    hit[late:, 1, 9] = True
+    assert not np.isfinite(got[hit]).any() and np.abs(got[~hit] - want[~hit]).max() < 1.5e-2 * max(1.0, np.abs(want).max())
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H,G,dim,vdim", HEADS)
 def test_decode_attention_and_its_slices(H, G, dim, vdim, dtype):
