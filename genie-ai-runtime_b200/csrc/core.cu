@@ -47,6 +47,7 @@ DeviceCtx* ctx() {
     cudaMemset(c->d_status, 0, 256);
     if (cudaMalloc(&c->attn_tickets, ATTN_TICKET_WORDS * sizeof(unsigned int)) != cudaSuccess) { cuda_error(cudaGetLastError(), "cudaMalloc(tickets)"); return nullptr; }
     cudaMemset(c->attn_tickets, 0, ATTN_TICKET_WORDS * sizeof(unsigned int));
+    cudaStreamSynchronize(cudaStreamLegacy);      // zeroed before the first kernel of a stream that does not wait for the default one
     c->device = dev;
     return c;
 }

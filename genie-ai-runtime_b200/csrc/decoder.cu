@@ -89,6 +89,7 @@ int jllm_b200_decoder::session_alloc() {
     out_tokens = (int*)take((size_t)out_cap * 4);
     prompt_dev = (int*)take((size_t)prompt_cap * 4);
     pf_tokens = prompt_dev;
+    JB_CUDA(cudaStreamSynchronize(cudaStreamLegacy));      // this slab and the family's are zeroed before a stream that does not wait for the default one uses them
     return JB_OK;
 }
 void jllm_b200_decoder::session_free() {
@@ -151,7 +152,7 @@ static int feed_chunks(jllm_b200_decoder* d, const int* tokens, int n, int start
     DCHK(check_tokens(d, tokens, n, start));
     DCHK(advance_state(d, start, n));
     const int chunk = d->pf_chunk < 2 ? 2 : d->pf_chunk;
-    DCHK(d->reserve_chunk(n < chunk ? n : chunk));
+    DCHK(d->reserve_chunk(n < chunk ? n : chunk, st));
     std::vector<int> rows;
     int done = 0, w = 0;
     while (done < n) {
@@ -176,6 +177,7 @@ void jllm_b200_decoder_destroy(jllm_b200_decoder* d) {
 }
 int jllm_b200_decoder_reset(jllm_b200_decoder* d) {
     JB_CUDA(cudaMemset(d->state, 0, 64));
+    JB_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     d->held = 0;
     d->clear_cache();
     return JB_OK;

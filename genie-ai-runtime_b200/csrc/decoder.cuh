@@ -32,7 +32,7 @@ struct jllm_b200_decoder {
     virtual ~jllm_b200_decoder() = default;
     // ── the model family ──
     virtual int enqueue_step(int n_splits, cudaStream_t st) = 0;              // token and position from `state`; leaves logits, then launch_argmax_advance (or its own)
-    virtual int reserve_chunk(int tokens) = 0;                                // buffers of a chunk (grown on first use)
+    virtual int reserve_chunk(int tokens, cudaStream_t st) = 0;               // buffers of a chunk (grown on first use)
     virtual int enqueue_chunk(const int* dev_tokens, int n, int start, cudaStream_t st) = 0;
     virtual int enqueue_rows(const int* host_rows, int n, float* out, cudaStream_t st) = 0;   // final norm + logits [n][vocab] of rows of the chunk just enqueued
     virtual int attn_splits(int seq_len) const = 0;                           // KV slices of a step at this length (a graph is captured per value)

@@ -47,7 +47,7 @@ struct KquantDecoder : jllm_b200_decoder {
     }
     int alloc();
     int enqueue_step(int n_splits, cudaStream_t st) override;
-    int reserve_chunk(int tokens) override;
+    int reserve_chunk(int tokens, cudaStream_t st) override;
     int enqueue_chunk(const int* dev_tokens, int n, int start, cudaStream_t st) override;
     int enqueue_rows(const int* host_rows, int n, float* out, cudaStream_t st) override;
     int attn_splits(int seq_len) const override { return attn_splits_for(seq_len); }
@@ -285,7 +285,7 @@ static int dec_enqueue_step_tp(KquantDecoder* d, int n_splits, cudaStream_t st) 
 // N >= 2 prompt tokens at positions start .. start+N-1: RMSNorm over rows, batched K-quant products (prefill arithmetic),
 // QK-norm + RoPE + INT8 KV store for all tokens in one launch, query-tiled causal attention, Wo, residual, RMSNorm,
 // gate/up, SwiGLU, W_down, residual.  After the last chunk: final norm and logits of the last token only, greedy token.
-int KquantDecoder::reserve_chunk(int cap) {
+int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     if (cap <= pf_cap) return JB_OK;
     if (pf_slab) { cudaFree(pf_slab); pf_slab = pf_codes = nullptr; pf_cap = 0; }
     const size_t N = (size_t)cap, H = m.hidden_dim, QD = (size_t)m.n_heads * m.head_dim, KVD = (size_t)m.n_kv_heads * m.head_dim, I = m.intermediate_dim;

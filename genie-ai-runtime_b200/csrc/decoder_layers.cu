@@ -73,7 +73,7 @@ struct LayerDecoder : jllm_b200_decoder {
     NormStep pending;                           // the last sublayer's exit of the chunk, still to be applied
 
     ~LayerDecoder() override { if (one.slab) cudaFree(one.slab); if (many.slab) cudaFree(many.slab); if (kexp) cudaFree(kexp); if (vexp) cudaFree(vexp); for (auto& r : rotations) cudaFree(r.table); kv.destroy(); }
-    int alloc_acts(Acts& a, size_t rows, bool chunk);
+    int alloc_acts(Acts& a, size_t rows, bool chunk, cudaStream_t st);
     NormStep entry(const Acts& a, const float* w, const float* b) const;
     MoeRoute route(const jllm_b200_layer_spec& w) const;
     DenseGemm product(const Acts& a) const { DenseGemm g; g.kind = kind; g.early = true; g.part = a.part; g.part_floats = a.part ? gemm_pair_part_floats() : 0; return g; }
@@ -89,7 +89,7 @@ struct LayerDecoder : jllm_b200_decoder {
     int latent_chunk(int l, const Acts& a, int n, int start, cudaStream_t st);
     bool keeps_state() const override { return recurrent; }
     int enqueue_step(int n_splits, cudaStream_t st) override;
-    int reserve_chunk(int tokens) override;
+    int reserve_chunk(int tokens, cudaStream_t st) override;
     int enqueue_chunk(const int* dev_tokens, int n, int start, cudaStream_t st) override;
     int enqueue_rows(const int* host_rows, int n, float* out, cudaStream_t st) override;
     int attn_splits(int seq_len) const override {
@@ -105,7 +105,7 @@ struct LayerDecoder : jllm_b200_decoder {
     const void* buffer(int which) override { return which == 0 ? one.x[0] : which == 7 ? kv.key_ptr(0, 0) : nullptr; }
 };
 
-int LayerDecoder::alloc_acts(Acts& a, size_t R, bool chunk) {
+int LayerDecoder::alloc_acts(Acts& a, size_t R, bool chunk, cudaStream_t st) {
     const size_t es = elem_bytes(kind), W = pad8(m.width), T = max_top;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
     bool ranges = chunk && kind == EK_BF16;
@@ -132,7 +132,7 @@ int LayerDecoder::alloc_acts(Acts& a, size_t R, bool chunk) {
         if (pass == 0) {
             if (ranges && cudaMalloc(&a.slab, at) != cudaSuccess) { cudaGetLastError(); a.slab = nullptr; ranges = false; }      // the products do without
             if (!a.slab && cudaMalloc(&a.slab, acts) != cudaSuccess) { cudaGetLastError(); a.slab = nullptr; return set_error(JB_ERR_NOMEM, "decoder: %zu B of activations", acts); }
-            JB_CUDA(cudaMemset(a.slab, 0, acts));         // the padding of every row stays zero
+            JB_CUDA(cudaMemsetAsync(a.slab, 0, acts, st));         // the padding of every row stays zero; on the stream of the kernels that follow
             continue;
         }
         a.x[0] = x0; a.x[1] = x1; a.y = y; a.h = h; a.q = q; a.att = att; a.z = z; a.wts = wts; a.ids = ids; a.a = ga;
@@ -382,10 +382,10 @@ int LayerDecoder::enqueue_step(int n_splits, cudaStream_t st) {
     return JB_OK;
 }
 
-int LayerDecoder::reserve_chunk(int tokens) {
+int LayerDecoder::reserve_chunk(int tokens, cudaStream_t st) {
     if (tokens <= pf_cap) return JB_OK;
     if (many.slab) { JB_CUDA(cudaDeviceSynchronize()); cudaFree(many.slab); many = Acts(); pf_cap = 0; }
-    DCHK(alloc_acts(many, tokens, true));
+    DCHK(alloc_acts(many, tokens, true, st));
     pf_cap = tokens;
     return JB_OK;
 }
@@ -567,6 +567,6 @@ extern "C" jllm_b200_decoder* jllm_b200_decoder_create_layered(const jllm_b200_l
     }
     // scratch that must exist before any graph capture
     for (const auto& w : d->layers) grow(vmax, w.v_dim);
-    if (d->session_alloc() || d->alloc_acts(d->one, 1, false) || !splitk_buffer((size_t)d->max_heads * 64 * (vmax + 2), true)) { jllm_b200_decoder_destroy(d); return nullptr; }
+    if (d->alloc_acts(d->one, 1, false, cudaStreamLegacy) || d->session_alloc() || !splitk_buffer((size_t)d->max_heads * 64 * (vmax + 2), true)) { jllm_b200_decoder_destroy(d); return nullptr; }
     return d;
 }

@@ -40,6 +40,7 @@ bool KVCachePool::init(const Config& cfg) {
             cudaMemset(kv_scales_, 0, (size_t)sb);
         }
     }
+    cudaStreamSynchronize(cudaStreamLegacy);      // zeroed before a stream that does not wait for the default one stores its first rows
     return true;
 }
 
@@ -144,6 +145,7 @@ bool LayeredKVCache::init(int n_layers, const int* k_width, const int* v_width, 
     bytes_ = at;
     if (cudaMalloc(&base_, (size_t)at) != cudaSuccess) { cudaGetLastError(); base_ = nullptr; destroy(); return false; }
     if (cudaMemset(base_, 0, (size_t)at) != cudaSuccess) { cudaGetLastError(); destroy(); return false; }
+    cudaStreamSynchronize(cudaStreamLegacy);      // as above
     return true;
 }
 void LayeredKVCache::destroy() {
