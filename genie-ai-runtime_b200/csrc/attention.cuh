@@ -47,6 +47,7 @@ bool   attention_prefill_fast_applies(const AttnCall& c);          // causal pre
 int    launch_attention_prefill_fast(const AttnCall& c, cudaStream_t st);
 // causal prefill on tcgen05 (attention_tc.cu): BF16 caches, and INT8 caches with a workspace (c.scratch, attention_tc_scratch bytes)
 constexpr int AT_MIN_TOKENS = 64;
+int    attention_tc_min_tokens(int n_heads, int n_kv);            // INT8 caches
 bool   attention_tc_applies(const AttnCall& c);
 int    launch_attention_tc(const AttnCall& c, cudaStream_t st);
 size_t attention_tc_scratch(int n_kv, int positions);

@@ -2,15 +2,17 @@
 // in tensor memory.  BF16 caches (keys in one or two parts, values of their own size), and INT8 caches whose codes were widened to
 // 16 bits first (exactly: a code has 7 bits), with the scale of a key applied to its scores and the scale of a value to its weights.
 //
-// What bounds it: the exponentials (16 per clock and SM), then the instructions around them; the products take 320 of the 512 clocks
-// that 128 x 64 exponentials do.  The kernels on mma.sync ran at 130 - 150 TFLOP/s (bf16) and 90 (int8), bound by instruction issue.
+// What bounds it: the instructions and the latency of the softmax.  Per tile of 128 rows x 64 keys the products take 512 clocks (heads of
+// 128; 640 at 192 / 128; 768 for int8, whose weights are two planes) and the exponentials 512 (16 per clock and SM), and neither pipe is
+// more than 31 % busy: 2048 tokens, 32 / 8 heads of 128: 89.6 us (bf16) and 121.4 (int8, widening included) against 198.9 and 412.4 of
+// the kernels on mma.sync.
 //   * a CTA owns two tiles of 128 query rows, (token, head of the group) pairs, so that one tile's products run under the other's
 //     softmax and both read the same tile of 64 keys;
 //   * S = Q K^T, 128 x 64 in fp32, goes to tensor memory; a thread reads its row, frees S for the next tile at once, and writes the
 //     weights as the A operand of O += P V back to tensor memory: bf16 for bf16 caches, as the older kernel has it; two bf16 planes
 //     (rounding and remainder, 16 bits of mantissa) for int8 caches, whose older kernel held them in 15 bits;
-//   * O stays in tensor memory; it is rescaled only when a row's maximum has risen by more than 2^8 since the last time, which leaves
-//     weights and sums in range and the result unchanged up to rounding;
+//   * O stays in tensor memory; it is rescaled only when a row's maximum has risen by more than 2^8 since the last time (the conditional
+//     rescaling that FlashAttention-4 describes), which leaves weights and sums in range and the result unchanged up to rounding;
 //   * V is read as it lies, [key][dim]: the B operand of the second product is MN-major.
 // Warps: 0 TMA, 1 MMA issuer, 2-3 idle, 4-7 and 8-11 the softmax of the two tiles (a warp's index modulo 4 is its quarter of tensor
 // memory).  Every mbarrier wait is bounded.
@@ -51,6 +53,7 @@ __device__ __forceinline__ void at_st32(uint32_t taddr, const uint32_t (&r)[32])
                    "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr) : "memory");
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
+// the bits of exp2f wherever the result is at least 2^-126 (compared for every float in [-150, 16]); zero below
 __device__ __forceinline__ float at_exp2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 // MN-major operand tile: rows of 64 elements (128 bytes, swizzled), eight rows 1024 bytes apart, the next 64 elements one chunk further
 __device__ __forceinline__ uint64_t at_desc_mn(uint32_t saddr) {
@@ -388,22 +391,42 @@ size_t attention_tc_scratch(int n_kv, int positions) {
     return rows * n_kv * (2 * 128 * 2 + 2 * sizeof(float));
 }
 
-// Query rows in groups that divide a tile, head sizes in whole 16-byte rows that fill their 64-element chunks but for the last, tiles
-// of 64 keys worth the fixed cost (from AT_MIN_TOKENS on).  INT8: a workspace for the widened codes.
+// From how many tokens on a chunk over an INT8 cache gains.  Here a CTA walks all keys of 256 rows alone, 2.3 us per 64 keys, and 64 tokens
+// in groups of four are one CTA per KV head; the kernel of attention_prefill.cu deals two tokens to a CTA and is the faster one until
+// tokens x KV heads fill the machine with them.  32 / 8 heads after 2000 positions, 64 / 192 /
+// 256 tokens: 41 / 84 / 110 us there, 85 / 88 / 89 here; 8 / 2 heads, 512 / 1024 tokens: 76 / 130 and 95 / 112; 32 / 32 heads, 64 tokens:
+// 121 and 95.  Groups it does not take go to the general kernel without this one (32 / 2 heads, 64 tokens: 2250 us, 78 here).
+int attention_tc_min_tokens(int n_heads, int n_kv) {
+    const int R = n_kv > 0 ? n_heads / n_kv : 0;
+    if (R > 4) return AT_MIN_TOKENS;
+    const int n = (2048 + n_kv - 1) / (n_kv > 0 ? n_kv : 1);
+    return n > AT_MIN_TOKENS ? n : AT_MIN_TOKENS;
+}
+// Query rows in groups that divide a tile, head sizes in whole 16-byte rows that fill their 64-element chunks but for the last, more keys
+// than one tile.  INT8: a workspace for the widened codes.
 bool attention_tc_applies(const AttnCall& c) {
     const int kind = c.kind(), R = c.n_kv > 0 ? c.n_heads / c.n_kv : 0;
     if ((kind != EK_BF16 && kind != EK_INT8) || c.causal_start < 0 || c.batch < AT_MIN_TOKENS || c.window || c.records || c.k_list || R < 1 || R > 128 || (R & (R - 1)) || c.n_heads != R * c.n_kv) return false;
     if (!c.out || !c.q || !c.k || !c.v || !al16(c.out) || !al16(c.q) || !al16(c.k) || !al16(c.v) || c.n_kv > 65535) return false;
-    if (kind == EK_INT8) return c.hd == 128 && c.chd == 128 && c.ks && c.vs && c.scratch && !c.sink && !c.gate && c.qt_coef == 0.f;
+    if (kind == EK_INT8) return c.batch >= attention_tc_min_tokens(c.n_heads, c.n_kv) && c.hd == 128 && c.chd == 128 && c.ks && c.vs && c.scratch && !c.sink && !c.gate && c.qt_coef == 0.f;
     const int vd = c.vhd > 0 ? c.vhd : c.hd, d1 = c.hd - c.hd2;
     if (c.hd % 8 || vd % 8 || c.hd > 192 || vd > 128 || c.chd != c.hd || (c.k2 ? d1 % 64 || c.hd2 <= 0 || c.hd2 > 64 || !al16(c.k2) || c.ldk2 % 8 : c.hd2 != 0)) return false;
+    // heads of 64 have a kernel of their own size on mma.sync, whose CTAs are shorter: this one needs the rows to fill the machine (32 / 8 heads,
+    // 256 / 512 / 1024 tokens: 8.1 / 15.8 / 36.1 us there, 9.7 / 15.6 / 27.5 here; 8 / 2 heads, 1024 / 2048: 21.5 / 51.5 and 26.9 / 50.0)
+    if (c.hd == 64 && vd == 64 && (long long)c.batch * c.n_heads < 16384) return false;
+    // so have heads of 128; over one tile of keys it is the faster one (64 tokens: 6.1 us there, 7.0 here; 80: 8.0 and 7.0)
+    if (c.hd == 128 && vd == 128 && c.causal_start + c.batch <= AT_KEYS) return false;
     return c.ldq % 8 == 0 && c.ldo % 8 == 0 && c.ldk % 8 == 0 && c.ldv % 8 == 0;
 }
 
 template <int QC, int VC, bool INT8>
 static int at_go(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& k2, const CUtensorMap& v, const AtArgs& a, int n_kv, cudaStream_t st) {
     const size_t smem = (size_t)2 * QC * AT_QCHUNK + (size_t)at_stages(QC, VC) * (QC + VC) * AT_KCHUNK + 1024;
-    JB_CUDA(cudaFuncSetAttribute(attn_tc_kernel<QC, VC, INT8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    bool& attr = ctx()->attn_tc_attr[INT8 ? 6 : 2 * (QC - 1) + VC - 1];
+    if (!attr) {
+        JB_CUDA(cudaFuncSetAttribute(attn_tc_kernel<QC, VC, INT8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        attr = true;
+    }
     const long long rows = (long long)a.n_tokens * a.R;
     JB_CUDA(launch_k(attn_tc_kernel<QC, VC, INT8>, dim3((unsigned)((rows + 2 * AT_ROWS - 1) / (2 * AT_ROWS)), n_kv), dim3(AT_THREADS), smem, st, pdl_enabled(), q, k, k2, v, a));
     count_launch();

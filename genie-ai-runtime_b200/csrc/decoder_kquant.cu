@@ -293,7 +293,7 @@ int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     const size_t total = 4 * al(N * H * 2) + 2 * al(N * QD * 2) + 2 * al(N * KVD * 2) + 3 * al(N * I * 2);
     // one allocation for all of it: it is made inside a session's first prompt, where each costs 0.4 - 2 ms (512 tokens: the first prompt
     // took 1064 us more than the next with two, 444 with one)
-    size_t codes = cap >= AT_MIN_TOKENS && m.max_context <= PF_CODES_MAX && m.head_dim == 128 ? attention_tc_scratch(m.n_kv_heads, m.max_context) : 0;
+    size_t codes = cap >= attention_tc_min_tokens(m.n_heads, m.n_kv_heads) && m.max_context <= PF_CODES_MAX && m.head_dim == 128 ? attention_tc_scratch(m.n_kv_heads, m.max_context) : 0;
     if (codes && cudaMalloc(&pf_slab, total + codes) != cudaSuccess) { cudaGetLastError(); pf_slab = nullptr; codes = 0; }
     if (!pf_slab && cudaMalloc(&pf_slab, total) != cudaSuccess) { cudaGetLastError(); pf_slab = nullptr; return set_error(JB_ERR_NOMEM, "decoder: %zu B of prefill activations", total); }
     pf_codes = codes ? (char*)pf_slab + total : nullptr;

@@ -145,7 +145,8 @@ def _prompt_on_a_workspace(jb, q, k, ks, v, vs, nh, nkv, N, start):
     ws = torch.full((jb.flash_attention_prefill_workspace_bytes(nkv, start + N),), 0x7F, dtype=torch.uint8, device="cuda")      # 0x7F7F: NaN in fp16
     n0 = jb.launch_count()
     jb.flash_attention_prefill_workspace(out, dev(q), dev(k), dev(v), nh, nkv, 128, 128, N, start, float(1 / np.sqrt(128)), True, dev(ks), dev(vs), 0, ws)
-    assert jb.launch_count() - n0 == (2 if N >= 64 else 1)               # codes widened, then attention
+    widened = N >= 64 if nh // nkv > 4 else N >= 64 and N * nkv >= 2048  # elsewhere the kernel over the codes is the faster one
+    assert jb.launch_count() - n0 == (2 if widened else 1)
     got = out.float().cpu().numpy()
     assert np.all(got[N * nh * 128:] == 7.0), "wrote past the output"
     return got[:N * nh * 128].reshape(N, nh, 128)
@@ -153,10 +154,11 @@ def _prompt_on_a_workspace(jb, q, k, ks, v, vs, nh, nkv, N, start):
 
 # groups of 1 .. 128 query heads, row tiles of 128 / group tokens and their neighbours, a start inside a key tile, counts around 64, several turns of the
 # five-stage key ring
-@pytest.mark.parametrize("N,start,nh,nkv", [(63, 0, 32, 8), (64, 0, 32, 8), (65, 0, 32, 8), (127, 37, 32, 8), (128, 300, 8, 8), (129, 0, 8, 8), (257, 63, 4, 4), (130, 100, 16, 8),
-                                            (257, 1000, 32, 8), (100, 2000, 16, 2), (70, 500, 16, 1), (66, 64, 64, 2), (64, 130, 128, 1), (65, 1, 128, 1), (300, 0, 2, 1)])
+@pytest.mark.parametrize("N,start,nh,nkv", [(63, 0, 32, 32), (64, 130, 32, 32), (65, 0, 32, 32), (129, 300, 16, 16), (512, 0, 4, 4), (255, 0, 32, 8), (256, 0, 32, 8), (257, 63, 32, 8),
+                                            (300, 1000, 32, 8), (256, 100, 16, 8), (130, 63, 32, 16), (2048, 0, 2, 1), (64, 0, 16, 2), (127, 37, 16, 2), (100, 2000, 16, 2),
+                                            (70, 500, 16, 1), (66, 64, 64, 2), (64, 130, 128, 1), (65, 1, 128, 1)])
 def test_prefill_int8_on_a_workspace(N, start, nh, nkv):
-    """Causal prefill over an INT8 cache whose codes are widened into a workspace (the tcgen05 kernel from 64 tokens on), to the tolerance of the other kernels.
+    """Causal prefill over an INT8 cache whose codes are widened into a workspace (the tcgen05 kernel where it gains), to the tolerance of the other kernels.
     The keys of the last quarter are long: scores rise late and by far more than the 2^8 up to which a maximum is kept."""
     jb = pkg()
     rng = np.random.Generator(np.random.PCG64(6000 + 7 * N + start + nh))
@@ -186,12 +188,12 @@ def test_prefill_workspace_arguments():
     assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("late,nh,nkv", [(1, 32, 8), (70, 8, 8), (199, 16, 2)])
+@pytest.mark.parametrize("late,nh,nkv", [(1, 32, 8), (70, 8, 8), (299, 16, 2)])
 def test_prefill_int8_is_not_spoiled_by_later_tokens(late, nh, nkv):
     """A token whose values overflowed (an infinite scale) leaves the tokens before it as they were, bit for bit, and is not hidden from those that see it."""
     jb = pkg()
     rng = np.random.Generator(np.random.PCG64(6500 + late))
-    N = 200
+    N = 300
     q = orc.gen_act(rng, N * nh * 128)
     k, ks = orc.gen_kv(rng, N, nkv, 128); v, vs = orc.gen_kv(rng, N, nkv, 128)
     clean = _prompt_on_a_workspace(jb, q, k, ks, v, vs, nh, nkv, N, 0)
