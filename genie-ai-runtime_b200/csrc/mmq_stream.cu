@@ -30,7 +30,7 @@ constexpr int MS_WARPS = 8;                        // per CTA, at most
 struct MsArgs {
     __half* y; const __half* res;                 // output; optional residual [N][M]: y = half(float(res) + float(half(product)))
     const uint8_t* W; const __half* xb;           // weights; activation operand, block-major
-    int M, N, NP, nb;                             // NP = tokens padded to a multiple of 8
+    int M, N, NP, nb;                             // NP = tokens padded to whole pairs of 8-token tiles (one: 8)
     int rt, ks;                                   // row tiles of a CTA, K ranges of a row tile (a warp each)
 };
 
@@ -203,20 +203,22 @@ __device__ __forceinline__ void ms_block6(float (&acc)[NT][4], uint32_t pA, uint
     }
 }
 
+// NT: 8-token tiles of a CTA.  Two CTAs share an SM up to 128 registers.  At four and six tiles that has to be asked for: Q4_K 9728 x 2560 over
+// 48 tokens 36.4 -> 28.9 us, Q6_K 2560 x 9728 over 32 tokens 32.5 -> 24.6; elsewhere the compiler's own choice is the faster one.
 template <int TYPE, int NT>
-__global__ void __launch_bounds__(MS_WARPS * 32) mms_kernel(const MsArgs a) {
+__global__ void __launch_bounds__(MS_WARPS * 32, NT == 4 || NT == 6 ? 2 : 0) mms_kernel(const MsArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int BB = TYPE == T_Q4K ? Q4K_BYTES : Q6K_BYTES;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
     const int rt = warp / a.ks, ks = warp - rt * a.ks;                       // row tile of the CTA, K range
-    const int row0 = (blockIdx.x * a.rt + rt) * 16;
+    const int row0 = (blockIdx.x * a.rt + rt) * 16, tok0 = blockIdx.y * NT * 8;
     const bool live = row0 < a.M;
     const int kb0 = (int)((long long)ks * a.nb / a.ks), kb1 = (int)((long long)(ks + 1) * a.nb / a.ks);
     const size_t rb = (size_t)a.nb * BB;
     float acc[NT][4];
     #pragma unroll
     for (int t = 0; t < NT; ++t) { acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f; }
-    const uint8_t* xb = reinterpret_cast<const uint8_t*>(a.xb) + (size_t)g * MS_XROWB + c * 16;
+    const uint8_t* xb = reinterpret_cast<const uint8_t*>(a.xb) + (size_t)(tok0 + g) * MS_XROWB + c * 16;
     const size_t x_block = (size_t)a.NP * MS_XROWB;
     // a row past M multiplies the last row's weights and is never stored
     const uint8_t *wA = a.W + (size_t)min(row0 + g, a.M - 1) * rb, *wB = a.W + (size_t)min(row0 + g + 8, a.M - 1) * rb;
@@ -286,7 +288,7 @@ __global__ void __launch_bounds__(MS_WARPS * 32) mms_kernel(const MsArgs a) {
     for (int t = 0; t < NT; ++t) {
         #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int row = row0 + g + 8 * (e >> 1), tok = 8 * t + 2 * c + (e & 1);
+            const int row = row0 + g + 8 * (e >> 1), tok = tok0 + 8 * t + 2 * c + (e & 1);
             if (row < a.M && tok < a.N) {
                 const size_t o = (size_t)tok * a.M + row;
                 const __half pr = __float2half_rn(acc[t][e]);
@@ -300,9 +302,10 @@ __global__ void __launch_bounds__(MS_WARPS * 32) mms_kernel(const MsArgs a) {
 bool mmq_stream_applies(const void* W, int type, int M, int N, int K) {
     static const bool off = [] { const char* e = getenv("JLLM_B200_MMQ_STREAM"); return e && e[0] == '0'; }();
     if (off || N < 2 || N > 64 || M < 16 || K % QK_K) return false;
-    // the largest matrices at more than 48 tokens: the tensor-core kernel is faster (64 tokens, Q4_K 9728 x 2560: 29.5 against
-    // 36.6 us; Q6_K 2560 x 9728: 30.7 against 35.7 us; equal at 32 tokens, and the smaller matrices stay faster here)
-    if (N > 48 && (long long)M * K >= (1ll << 24) && mmq_tc_applies(W, type, M, N, K)) return false;
+    // the largest matrices at more than 40 tokens: the tensor-core kernel is as fast or faster (here / there, us: Q4_K 9728 x 2560, 40 tokens
+    // 24.9 / 28.5, 48: 28.9 / 28.6, 64: 36.8 / 28.8; Q6_K 2560 x 9728 28.9 / 27.9, 34.9 / 27.9, 44.6 / 28.2; Q6_K 151936 x 2560 274 / 279, 283 / 279,
+    // 304 / 280); the smaller ones stay faster here (Q4_K 2560 x 4096, 64 tokens: 17.0 / 20.5)
+    if (N > 40 && (long long)M * K >= (1ll << 24) && mmq_tc_applies(W, type, M, N, K)) return false;
     if (type == T_Q4K) return ((uintptr_t)W & 15) == 0;
     return type == T_Q6K && ((uintptr_t)W & 1) == 0;
 }
@@ -318,10 +321,19 @@ static void ms_shape(int M, int nb, int sm_count, int& rt, int& ks) {
 }
 
 static int ms_tiles(int N) { return N <= 48 ? (N + 7) / 8 : 8; }       // 8-token MMA tiles the kernel is built for
+static int ms_padded(int N) { const int t = ms_tiles(N); return t == 1 ? 1 : (t + 1) & ~1; }
+// Few rows leave SMs idle (1024 rows: 64 CTAs): the token tiles are then dealt to two or four CTAs, each with the weights to itself.
+// 1024 x 2560 over 16 / 32 / 48 / 64 tokens: Q4_K 9.3 / 9.3 / 12.0 / 15.1 us with one, 6.8 / 7.9 / 8.7 / 8.6 dealt; Q6_K 8.1 / 11.2 / 13.4 /
+// 12.8 and 7.5 / 9.1 / 9.3 / 9.7.
+static int ms_split(int N, int ctas, int sm_count) {
+    int ty = 1;
+    while (ctas * ty < sm_count && ty < 4 && ms_padded(N) % (2 * ty) == 0) ty *= 2;
+    return ty;
+}
 
 size_t mmq_stream_scratch_bytes(int type, int M, int N, int K) {
     (void)type; (void)M;
-    return (((size_t)(K / QK_K) * 8 * ms_tiles(N) * MS_XROWB + 255) & ~(size_t)255) + 256;
+    return (((size_t)(K / QK_K) * 8 * ms_padded(N) * MS_XROWB + 255) & ~(size_t)255) + 256;
 }
 
 // `residual` (optional, [N][M]): the residual exit of a layer fused in (add_half arithmetic: the product is rounded to fp16
@@ -332,8 +344,7 @@ int launch_mmq_stream(__half* y, const void* W, int type, const __half* x, void*
                       bool reuse_operand, cudaStream_t st, MmqWork& work) {
     DeviceCtx* cx = ctx();
     if (!cx) return JB_ERR_CUDA;
-    const int nb = K / QK_K, NT = ms_tiles(N);
-    const int NPk = NT * 8;                               // tokens the kernel multiplies (padded ones are zero columns)
+    const int nb = K / QK_K, NPk = ms_padded(N) * 8;      // tokens of the operand (padded ones are zero columns)
     __half* xb = reinterpret_cast<__half*>(scratch);
     const long long groups = (long long)NPk * (K / 32);
     const int ds4 = type == T_Q4K;
@@ -347,19 +358,21 @@ int launch_mmq_stream(__half* y, const void* W, int type, const __half* x, void*
     MsArgs a = {};
     a.y = y; a.res = residual; a.W = (const uint8_t*)W; a.xb = xb; a.M = M; a.N = N; a.NP = NPk; a.nb = nb;
     ms_shape(M, nb, cx->sm_count, a.rt, a.ks);
+    const int tiles = (M + 15) / 16, ctas = (tiles + a.rt - 1) / a.rt, ty = ms_split(N, ctas, cx->sm_count);
+    const int NT = ty > 1 ? ms_padded(N) / ty : ms_tiles(N);
     typedef void (*Kern)(MsArgs);
     static const Kern k4[8] = { mms_kernel<T_Q4K, 1>, mms_kernel<T_Q4K, 2>, mms_kernel<T_Q4K, 3>, mms_kernel<T_Q4K, 4>, mms_kernel<T_Q4K, 5>, mms_kernel<T_Q4K, 6>, nullptr, mms_kernel<T_Q4K, 8> };
     static const Kern k6[8] = { mms_kernel<T_Q6K, 1>, mms_kernel<T_Q6K, 2>, mms_kernel<T_Q6K, 3>, mms_kernel<T_Q6K, 4>, mms_kernel<T_Q6K, 5>, mms_kernel<T_Q6K, 6>, nullptr, mms_kernel<T_Q6K, 8> };
     const Kern kern = ds4 ? k4[NT - 1] : k6[NT - 1];
-    const int ki = (ds4 ? 0 : 8) + NT - 1, warps = a.rt * a.ks, tiles = (M + 15) / 16;
+    const int ki = (ds4 ? 0 : 8) + NT - 1, warps = a.rt * a.ks;
     const size_t red = (size_t)a.rt * (a.ks - 1) * NT * 4 * 32 * sizeof(float), slots = ds4 ? 0 : (size_t)warps * 2 * 16 * MS_W6SLOT, smem = red > slots ? red : slots;
     if (!cx->mms_attr[ki]) {
         JB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MS_WARPS * 2 * 16 * MS_W6SLOT));
         cx->mms_attr[ki] = true;
     }
     static const bool verbose = getenv("JLLM_B200_MMQ_DEBUG") != nullptr;
-    if (verbose) fprintf(stderr, "[mmq_stream] type %d M=%d N=%d K=%d: %d CTAs of %d row tiles x %d K ranges, smem %zu\n", type, M, N, K, (tiles + a.rt - 1) / a.rt, a.rt, a.ks, smem);
-    JB_CUDA(launch_k(kern, dim3((tiles + a.rt - 1) / a.rt), dim3(warps * 32), smem, st, pdl_enabled(), a));
+    if (verbose) fprintf(stderr, "[mmq_stream] type %d M=%d N=%d K=%d: %d x %d CTAs of %d row tiles x %d K ranges, smem %zu\n", type, M, N, K, ctas, ty, a.rt, a.ks, smem);
+    JB_CUDA(launch_k(kern, dim3(ctas, ty), dim3(warps * 32), smem, st, pdl_enabled(), a));
     count_launch();
     return JB_OK;
 }
