@@ -552,10 +552,11 @@ static void tc_pick(int tiles_m, int N, int n_main_tiles, int sm_count, int& n_t
 // memory.  From MW_MIN_TOKENS on the same fp16 operand, bit for bit, is written to memory once, in pieces that stay in L2, and
 // multiplied by the paired kernel of gemm_pair.cu (2048 tokens: 9728 x 2560 131 -> 110 us, Q6_K 2560 x 9728 171 -> 121 us).
 constexpr size_t MW_WEIGHT_BYTES = (size_t)64 << 20;
-constexpr int MW_MIN_TOKENS = 384;      // 256 tokens: Q6_K 2560 x 9728 46 us this way, 38 fused; 512 tokens: 54 and 65; Q4_K 9728 x 2560 equal at both
+constexpr int MW_MIN_TOKENS = 384;      // 256 tokens: Q6_K 2560 x 9728 46 us this way, 38 fused; 512 tokens: 54 and 65; Q4_K 9728 x 2560 equal at both;
+                                        // 1024 x 2560, 384 / 448 tokens: Q4_K 19.5 / 20.0 this way, 18.5 / 21.3 fused, Q6_K 18.8 / 19.2 and 17.3 / 19.5
 
 bool mmq_wide_applies(int M, int M2, int N, int K) {
-    return N >= MW_MIN_TOKENS && (long long)M + M2 >= 256 && (size_t)(K + K / 16 + TC_K) * sizeof(__half) * 256 <= MW_WEIGHT_BYTES;
+    return N >= ((long long)M + M2 < 2048 ? MW_MIN_TOKENS + 64 : MW_MIN_TOKENS) && (long long)M + M2 >= 256 && (size_t)(K + K / 16 + TC_K) * sizeof(__half) * 256 <= MW_WEIGHT_BYTES;
 }
 // Asked for once: an object whose request was refused stays with the fused kernel, whose results differ in their last bits.  A captured
 // call asks too, so that it takes the way an uncaptured one takes.

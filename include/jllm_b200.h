@@ -173,13 +173,15 @@ int jllm_b200_gemv_quant_int_dots(void* y, int32_t* dots, const void* W, int ggm
 int jllm_b200_gemm_quant_batched_int_dots(void* y, int32_t* dots, const void* W, int ggml_type, const void* x, int M, int N, int K, void* stream);
 /* Two batched products over the same activations (the gate and up projections of a layer): y0[N x M0] = x . W0^T and
  * y1[N x M1] = x . W1^T, equal to two jllm_b200_gemm_quant_batched calls.  With more than 64 tokens (or the large matrices
- * from 49) and both matrices Q4_K or both Q6_K the row tiles of the two share one launch; otherwise two launches, the
- * second reusing the quantised activations.  N >= 2. */
+ * from 41) and both matrices Q4_K or both Q6_K the row tiles of the two are one list of work: one launch below 384 tokens, from there
+ * on pieces of the two whose weights are expanded first; otherwise one product after the other, the second reusing the quantised
+ * activations.  N >= 2. */
 int jllm_b200_gemm_quant_batched_pair(void* y0, const void* W0, int type0, int M0, void* y1, const void* W1, int type1, int M1,
                                       const void* x, int N, int K, void* stream);
 /* flash_attention_prefill_batched with a workspace of the caller's (16-byte aligned device memory of workspace_bytes(n_kv_heads,
- * start_pos + N) bytes, used by this call only): from 64 tokens on, INT8 caches with 128-wide heads are widened there and multiplied on
- * the 5th-generation tensor cores (any power of two of query heads per KV head up to 128, no window).  Null: as without. */
+ * start_pos + N) bytes, used by this call only): where it gains, INT8 caches with 128-wide heads are widened there and multiplied on the
+ * 5th-generation tensor cores (up to four query heads per KV head: from N * n_kv_heads = 2048 on; 8 to 128, a power of two: from 64
+ * tokens on; no window).  Else, and with a null workspace, as without. */
 int64_t jllm_b200_flash_attention_prefill_workspace_bytes(int n_kv_heads, int positions);
 int jllm_b200_flash_attention_prefill_workspace(void* output, const void* q, const void* k_cache, const void* v_cache, int n_heads,
                                                 int n_kv_heads, int head_dim, int cache_head_dim, int N, int start_pos, float scale,

@@ -35,9 +35,13 @@ def test_gemm_quant_batched_matches_oracle(t, M, N, K):
 
 # weights expanded once for many tokens: the first size that takes that way and its neighbours, ragged rows (groups of four, and not), K ranges of tail tiles,
 # a last row tile that is mostly beyond the matrix, a matrix in two pieces
-WIDE = [(12, 300, 383, 512), (12, 300, 384, 768), (14, 300, 384, 512), (12, 515, 385, 512), (14, 513, 400, 768), (12, 256, 511, 2560), (14, 772, 390, 4096), (12, 66000, 384, 512)]
+WIDE = [(12, 300, 383, 512), (12, 300, 384, 768), (14, 300, 384, 512), (12, 515, 385, 512), (14, 513, 400, 768), (12, 256, 511, 2560), (14, 772, 390, 4096), (12, 66000, 384, 512),
+        # fewer than 2048 rows: from 448 tokens on
+        (12, 300, 447, 768), (12, 300, 448, 768), (12, 515, 449, 512), (14, 513, 450, 768), (14, 772, 460, 4096), (14, 2047, 448, 512), (14, 2048, 384, 512)]
 # few tokens: every number of token tiles, one row, rows that do not fill a tile, one super-block, more super-blocks than ranges
-FEW = [(t, M, N, K) for t in (12, 14) for M, N, K in ((40, 8, 512), (16, 9, 256), (2500, 17, 2560), (100, 25, 768), (33, 33, 9728), (1000, 41, 1024), (18, 48, 5120), (70, 49, 512), (64, 64, 2560), (17, 2, 4096))]
+FEW = [(t, M, N, K) for t in (12, 14) for M, N, K in ((40, 8, 512), (16, 9, 256), (2500, 17, 2560), (100, 25, 768), (33, 33, 9728), (1000, 41, 1024), (18, 48, 5120), (70, 49, 512), (64, 64, 2560), (17, 2, 4096),
+                                              # token tiles dealt to two and to four CTAs, and not
+                                              (1024, 12, 2560), (1024, 40, 2560), (1024, 57, 2560), (512, 31, 256), (2360, 32, 256), (2384, 32, 2560), (4096, 48, 2560))]
 
 
 @pytest.mark.parametrize("t,M,N,K", WIDE + FEW)
