@@ -213,9 +213,9 @@ static int dt_pick(int tiles_m, int tokens_per_group, int groups, int max_tile, 
 
 int launch_dense_gemm_tc(const DenseGemm& a, cudaStream_t st) {
     if (a.N <= 0 || a.M <= 0) return JB_OK;
-    if (a.kind == EK_BF16 && gemm_pair_applies(a)) return launch_gemm_pair(a, st);
     DeviceCtx* c = ctx();
     if (!c) return set_error(JB_ERR_STATE, "dense gemm: library not initialised");
+    if (a.kind == EK_BF16 && gemm_pair_applies(a) && !(dt_pick((a.M + DT_M - 1) / DT_M, a.N, 1, 256, c->sm_count) <= 192 && gemm_pair_one_round(a))) return launch_gemm_pair(a, st);
     if (a.kind != EK_BF16) return set_error(JB_ERR_TYPE, "dense gemm: element kind %d", a.kind);
     if (!a.W || !a.x || (a.swiglu && !a.W_up) || (a.n_groups > 1 && !a.off && (a.x_step <= 0 || a.x_step % 8))) return set_error(JB_ERR_PTR, "dense gemm: null pointer");
     if (a.n_groups < 1 || a.n_groups > DT_MAX_GROUPS || a.K <= 0) return set_error(JB_ERR_LIMIT, "dense gemm: %d groups, K=%d", a.n_groups, a.K);

@@ -254,6 +254,17 @@ bool gemm_pair_applies(const DenseGemm& a) {
     return (a.kind == EK_BF16 || a.kind == EK_F16) && !a.swiglu && !a.off && a.n_groups == 1 && a.N >= GP_MIN_TOKENS && a.M >= 256;
 }
 
+// One round of pairs without K ranges: the one-CTA kernel spreads the same rows over twice as many, narrower tiles and starts faster
+// (2560 x 9728 over 256 / 1024 tokens 49 / 54 us there, 58 / 61 here; 6144 x 2560 over 512: 19.3 and 22.2).  From a second round on, or where its
+// tiles would be wider than 192 tokens, the pairs gain (21632 x 2560 over 160 tokens 38.0 against 44.2, 12288 x 2560 over 256: 23.5 and 30.2).
+bool gemm_pair_one_round(const DenseGemm& a) {
+    DeviceCtx* c = ctx();
+    if (!c) return false;
+    GpArgs p = {};
+    gp_pick((a.M + 255) / 256, a.N, (a.K + GP_K - 1) / GP_K, c->sm_count / 2, a.part != nullptr && a.part_floats >= gemm_pair_part_floats(), p);
+    return p.ksplit == 1 && p.n_items <= c->sm_count / 2;
+}
+
 int launch_gemm_pair(const DenseGemm& a, cudaStream_t st) {
     DeviceCtx* c = ctx();
     if (!c) return set_error(JB_ERR_STATE, "paired gemm: library not initialised");

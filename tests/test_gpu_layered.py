@@ -262,6 +262,19 @@ def test_dense_product(M, N, K, dtype):
     assert np.abs(as_np(y1) - W @ x[0]).max() < 1e-5 * np.sqrt(K)
 
 
+@pytest.mark.parametrize("M,N,K", [(19200, 130, 64), (19200, 128, 200), (2560, 256, 520), (1024, 640, 512), (300, 2000, 200), (256, 128, 64), (12000, 250, 136), (2600, 2048, 328)])
+def test_bf16_products_of_one_round_and_of_more(M, N, K):
+    """dense_matmul without room for K ranges: one round of pairs goes to the one-CTA kernel unless its tiles were wider than 192 tokens, more than one to the pairs."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    W, x = (torch.randn(s, device="cuda", generator=g).bfloat16() for s in ((M, K), (N, K)))
+    y = torch.full((N + 1, M), 7.0, device="cuda")
+    pkg().dense_matmul(y, W, x, M, N, K)
+    want = x.double() @ W.double().T
+    assert (y[:N].double() - want).abs().max() < 1e-5 * np.sqrt(K) * 4 and (y[N] == 7).all()
+    assert pkg().device_status() == 0
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_one_token_product_over_the_output_of_the_product_in_front(dtype):
     """keys = x . A^T, then keys . q, with nothing between the two calls: the second may not read the keys before they are there.  Many keys, so that the
