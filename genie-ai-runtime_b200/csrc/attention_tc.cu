@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             uint32_t hi[32], lo[32];
             if (INT8) {
                 const float4* vs = reinterpret_cast<const float4*>(a.vs + (size_t)g * a.lds + k0);
-                // `seen`: a masked weight is zero whatever the scale of its value (infinite where a later token overflowed)
+                // `seen`: a masked weight is zero whatever the scale of its value; asked where some scale of a diagonal tile is not finite
                 auto planes = [&](auto seen) {
                     #pragma unroll
                     for (int i = 0; i < 16; ++i) {
@@ -262,8 +262,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                         }
                     }
                 };
-                if (diagonal) planes([&](int i) { return k0 + i <= pos; });
-                else          planes([](int) { return true; });
+                const float* sc = reinterpret_cast<const float*>(vs);
+                if (diagonal && __any_sync(0xFFFFFFFFu, !(isfinite(sc[lane]) && isfinite(sc[lane + 32])))) planes([&](int i) { return k0 + i <= pos; });
+                else planes([](int) { return true; });
             } else {
                 #pragma unroll
                 for (int i = 0; i < 32; ++i) hi[i] = fa_pack(v[2 * i], v[2 * i + 1]);
