@@ -90,7 +90,7 @@ struct jllm_b200_batch_decoder {
     void** lists = nullptr;            // device: [layer][4 (k, v, k scales, v scales)][B] pointers
     std::vector<unsigned char> maps;   // host: [layer][B][K, V] TMA tensor maps of the caches (128 bytes each), passed to the kernel as parameters
     void* slab = nullptr;
-    MmqWork mmq;                       // the captured step holds its addresses: all of it is there from the start
+    MmqWork mmq;                       // in the slab: the captured step holds its addresses, all of it is there from the start
     int kernels_per_step = 0;
     cudaGraphExec_t graph_exec = nullptr;   // one decode step from the device-side state
     int host_pos = -1;                      // host mirror of the device-side position (-1 until generate has run): the bound of step_device
@@ -165,7 +165,19 @@ jllm_b200_batch_decoder* jllm_b200_batch_decoder_create(const jllm_b200_model_de
     d->out_cap = model->max_context + 8; d->prompt_cap = model->max_context + 8;
     const size_t total = 4 * al(B * H * 2) + 2 * al(B * QD * 2) + 2 * al(B * KVD * 2) + 3 * al(B * I * 2) + al(B * V * 2) + al(64) + 2 * al((size_t)B * 4) +
                          al((size_t)d->out_cap * B * 4) + al((size_t)d->prompt_cap * B * 4) + al((size_t)model->n_layers * 4 * B * sizeof(void*));
-    if (cudaMalloc(&d->slab, total) != cudaSuccess) { cudaGetLastError(); set_error(JB_ERR_NOMEM, "batch decoder: %zu B of activations", total); jllm_b200_batch_decoder_destroy(d); return nullptr; }
+    // product scratch of every step: nothing of it may move once a step is captured
+    const struct { size_t M, M2, K; } products[6] = { { QD, 0, H }, { KVD, 0, H }, { H, 0, QD }, { I, I, H }, { H, 0, I }, { V, 0, H } };
+    size_t need = 0;
+    bool wide = false;
+    for (const auto& g : products) {
+        const int M = (int)g.M, M2 = (int)g.M2, K = (int)g.K;
+        for (int t : { T_Q4K, T_Q6K })
+            for (size_t b : { mmq_tc_scratch_bytes(t, M, B, K), mmq_tc_scratch_bytes_pair(t, M, M2, B, K), mmq_stream_scratch_bytes(t, M, B, K), mmq_scratch_bytes(B, K) })
+                if (b > need) need = b;
+        wide = wide || mmq_wide_applies(M, M2, B, K);
+    }
+    if (cudaMalloc(&d->slab, total + need) != cudaSuccess) { cudaGetLastError(); d->slab = nullptr; set_error(JB_ERR_NOMEM, "batch decoder: %zu B of activations and product scratch", total + need); jllm_b200_batch_decoder_destroy(d); return nullptr; }
+    d->mmq.act = (char*)d->slab + total; d->mmq.act_bytes = need; d->mmq.held = true;
     cudaMemset(d->slab, 0, total);
     char* p = (char*)d->slab;
     auto take = [&](size_t b) { char* r = p; p += al(b); return r; };
@@ -195,18 +207,6 @@ jllm_b200_batch_decoder* jllm_b200_batch_decoder_create(const jllm_b200_model_de
                      attn_tma_encode(&maps[(((size_t)l * B + b) * 2 + 1) * 128], d->kv[b].val_ptr(l, 0), model->max_context, model->n_kv_heads);
         if (ok) d->maps.swap(maps);       // else: the general attention kernel serves the pointer lists
     }
-    // product scratch of every step: nothing of it may move once a step is captured
-    const struct { size_t M, M2, K; } products[6] = { { QD, 0, H }, { KVD, 0, H }, { H, 0, QD }, { I, I, H }, { H, 0, I }, { V, 0, H } };
-    size_t need = 0;
-    bool wide = false;
-    for (const auto& g : products) {
-        const int M = (int)g.M, M2 = (int)g.M2, K = (int)g.K;
-        for (int t : { T_Q4K, T_Q6K })
-            for (size_t b : { mmq_tc_scratch_bytes(t, M, B, K), mmq_tc_scratch_bytes_pair(t, M, M2, B, K), mmq_stream_scratch_bytes(t, M, B, K), mmq_scratch_bytes(B, K) })
-                if (b > need) need = b;
-        wide = wide || mmq_wide_applies(M, M2, B, K);
-    }
-    if (!d->mmq.scratch(need, false)) { set_error(JB_ERR_NOMEM, "batch decoder: %zu B of product scratch", need); jllm_b200_batch_decoder_destroy(d); return nullptr; }
     if (wide) d->mmq.wide_scratch(false);
     splitk_buffer((size_t)B * model->n_heads * 64 * (model->head_dim + 4), true);
     return d;
@@ -215,7 +215,7 @@ void jllm_b200_batch_decoder_destroy(jllm_b200_batch_decoder* d) {
     if (!d) return;
     if (d->graph_exec) cudaGraphExecDestroy(d->graph_exec);
     if (d->slab) cudaFree(d->slab);
-    d->mmq.release();
+    if (d->mmq.wide) cudaFree(d->mmq.wide);
     for (auto& p : d->kv) p.destroy();
     delete d;
 }

@@ -51,7 +51,6 @@ struct MmqWork {
     MmqOperand few, many;                            // the operands quantised last, in the layouts of mmq_stream.cu and of mmq_tc.cu
     void* scratch(size_t bytes, bool capturing);     // null: not to be had
     void* wide_scratch(bool capturing);
-    void  release();
 };
 struct RopeTable { float theta; int half_dim; int max_seq; float* cos; float* sin; };
 struct DeviceCtx {

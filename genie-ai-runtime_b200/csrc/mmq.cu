@@ -37,12 +37,6 @@ void* MmqWork::scratch(size_t bytes, bool capturing) {
     held = held || capturing;
     return act;
 }
-void MmqWork::release() {
-    if (act) cudaFree(act);
-    if (wide) cudaFree(wide);
-    *this = MmqWork();
-}
-
 // one warp per 32-element group of one token
 __global__ void mmq_quantize_kernel(const __half* x, ActQ a, int N, int K, int ds4) {
     pdl_wait();

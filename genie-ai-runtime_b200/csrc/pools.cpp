@@ -40,7 +40,6 @@ bool KVCachePool::init(const Config& cfg) {
             cudaMemset(kv_scales_, 0, (size_t)sb);
         }
     }
-    cudaStreamSynchronize(cudaStreamLegacy);      // zeroed before a stream that does not wait for the default one stores its first rows
     return true;
 }
 
@@ -145,7 +144,6 @@ bool LayeredKVCache::init(int n_layers, const int* k_width, const int* v_width, 
     bytes_ = at;
     if (cudaMalloc(&base_, (size_t)at) != cudaSuccess) { cudaGetLastError(); base_ = nullptr; destroy(); return false; }
     if (cudaMemset(base_, 0, (size_t)at) != cudaSuccess) { cudaGetLastError(); destroy(); return false; }
-    cudaStreamSynchronize(cudaStreamLegacy);      // as above
     return true;
 }
 void LayeredKVCache::destroy() {
@@ -194,6 +192,7 @@ jllm_b200_kv_pool* jllm_b200_kv_pool_create(int n_layers, int n_kv_heads, int he
     if (!h) return nullptr;
     jllm::KVCachePool::Config c = { n_layers, n_kv_heads, head_dim, max_context, overflow_context, kv_type_bytes };
     if (!h->pool.init(c)) { delete h; return nullptr; }
+    cudaStreamSynchronize(cudaStreamLegacy);      // zeroed before a stream that does not wait for the default one stores rows (sessions wait once, for all they clear)
     return h;
 }
 void    jllm_b200_kv_pool_destroy(jllm_b200_kv_pool* p) { if (p) { p->pool.destroy(); delete p; } }
