@@ -30,7 +30,7 @@ constexpr int MS_WARPS = 8;                        // per CTA, at most
 struct MsArgs {
     __half* y; const __half* res;                 // output; optional residual [N][M]: y = half(float(res) + float(half(product)))
     const uint8_t* W; const __half* xb;           // weights; activation operand, block-major
-    int M, N, NP, nb;                             // NP = tokens padded to whole pairs of 8-token tiles (one: 8)
+    int M, N, NP, nb;                             // NP = tokens padded to a multiple of 8
     int rt, ks;                                   // row tiles of a CTA, K ranges of a row tile (a warp each)
 };
 
@@ -211,7 +211,8 @@ __global__ void __launch_bounds__(MS_WARPS * 32, NT == 4 || NT == 6 ? 2 : 0) mms
     constexpr int BB = TYPE == T_Q4K ? Q4K_BYTES : Q6K_BYTES;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
     const int rt = warp / a.ks, ks = warp - rt * a.ks;                       // row tile of the CTA, K range
-    const int row0 = (blockIdx.x * a.rt + rt) * 16, tok0 = blockIdx.y * NT * 8;
+    const int row0 = (blockIdx.x * a.rt + rt) * 16;
+    const int tok0 = NT <= 4 ? blockIdx.y * NT * 8 : 0;                      // more than four token tiles a CTA: they are not dealt
     const bool live = row0 < a.M;
     const int kb0 = (int)((long long)ks * a.nb / a.ks), kb1 = (int)((long long)(ks + 1) * a.nb / a.ks);
     const size_t rb = (size_t)a.nb * BB;
@@ -321,19 +322,20 @@ static void ms_shape(int M, int nb, int sm_count, int& rt, int& ks) {
 }
 
 static int ms_tiles(int N) { return N <= 48 ? (N + 7) / 8 : 8; }       // 8-token MMA tiles the kernel is built for
-static int ms_padded(int N) { const int t = ms_tiles(N); return t == 1 ? 1 : (t + 1) & ~1; }
-// Few rows leave SMs idle (1024 rows: 64 CTAs): the token tiles are then dealt to two or four CTAs, each with the weights to itself.
-// 1024 x 2560 over 16 / 32 / 48 / 64 tokens: Q4_K 9.3 / 9.3 / 12.0 / 15.1 us with one, 6.8 / 7.9 / 8.7 / 8.6 dealt; Q6_K 8.1 / 11.2 / 13.4 /
-// 12.8 and 7.5 / 9.1 / 9.3 / 9.7.
+// Few rows leave SMs idle (1024 rows: 64 CTAs): the token tiles are then dealt evenly to as many CTAs as it takes, each with the weights to
+// itself.  1024 x 2560 over 16 / 32 / 48 / 64 tokens: Q4_K 9.3 / 9.3 / 12.0 / 15.1 us with one, 6.8 / 7.9 / 8.7 / 8.6 dealt; Q6_K 8.1 / 11.2 /
+// 13.4 / 12.8 and 7.5 / 9.1 / 9.3 / 9.7.
 static int ms_split(int N, int ctas, int sm_count) {
+    const int t = ms_tiles(N);
     int ty = 1;
-    while (ctas * ty < sm_count && ty < 4 && ms_padded(N) % (2 * ty) == 0) ty *= 2;
+    for (int d = 2; d <= t && ctas * ty < sm_count; ++d)
+        if (t % d == 0) ty = d;
     return ty;
 }
 
 size_t mmq_stream_scratch_bytes(int type, int M, int N, int K) {
     (void)type; (void)M;
-    return (((size_t)(K / QK_K) * 8 * ms_padded(N) * MS_XROWB + 255) & ~(size_t)255) + 256;
+    return (((size_t)(K / QK_K) * 8 * ms_tiles(N) * MS_XROWB + 255) & ~(size_t)255) + 256;
 }
 
 // `residual` (optional, [N][M]): the residual exit of a layer fused in (add_half arithmetic: the product is rounded to fp16
@@ -344,7 +346,7 @@ int launch_mmq_stream(__half* y, const void* W, int type, const __half* x, void*
                       bool reuse_operand, cudaStream_t st, MmqWork& work) {
     DeviceCtx* cx = ctx();
     if (!cx) return JB_ERR_CUDA;
-    const int nb = K / QK_K, NPk = ms_padded(N) * 8;      // tokens of the operand (padded ones are zero columns)
+    const int nb = K / QK_K, NPk = ms_tiles(N) * 8;      // tokens of the operand (padded ones are zero columns)
     __half* xb = reinterpret_cast<__half*>(scratch);
     const long long groups = (long long)NPk * (K / 32);
     const int ds4 = type == T_Q4K;
@@ -359,7 +361,7 @@ int launch_mmq_stream(__half* y, const void* W, int type, const __half* x, void*
     a.y = y; a.res = residual; a.W = (const uint8_t*)W; a.xb = xb; a.M = M; a.N = N; a.NP = NPk; a.nb = nb;
     ms_shape(M, nb, cx->sm_count, a.rt, a.ks);
     const int tiles = (M + 15) / 16, ctas = (tiles + a.rt - 1) / a.rt, ty = ms_split(N, ctas, cx->sm_count);
-    const int NT = ty > 1 ? ms_padded(N) / ty : ms_tiles(N);
+    const int NT = ms_tiles(N) / ty;
     typedef void (*Kern)(MsArgs);
     static const Kern k4[8] = { mms_kernel<T_Q4K, 1>, mms_kernel<T_Q4K, 2>, mms_kernel<T_Q4K, 3>, mms_kernel<T_Q4K, 4>, mms_kernel<T_Q4K, 5>, mms_kernel<T_Q4K, 6>, nullptr, mms_kernel<T_Q4K, 8> };
     static const Kern k6[8] = { mms_kernel<T_Q6K, 1>, mms_kernel<T_Q6K, 2>, mms_kernel<T_Q6K, 3>, mms_kernel<T_Q6K, 4>, mms_kernel<T_Q6K, 5>, mms_kernel<T_Q6K, 6>, nullptr, mms_kernel<T_Q6K, 8> };
