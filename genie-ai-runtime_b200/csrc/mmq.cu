@@ -15,12 +15,17 @@ struct ActQ { int8_t* q; float* d; float* s; };   // [N][K] codes, [N][K/32] sca
 
 size_t mmq_scratch_bytes(int N, int K) { return (size_t)N * K + 2 * (size_t)N * (K / 32) * sizeof(float) + 256; }
 
-cudaError_t mmq_alloc(void** p, size_t bytes, bool capturing) {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;       // a captured call may allocate when its thread says so
-    if (capturing) cudaThreadExchangeStreamCaptureMode(&mode);
+// While it lives, this thread's allocations, waits and event queries neither fail under its own capture nor invalidate the capture of
+// another thread (which they do in the default mode).
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+cudaError_t mmq_alloc(void** p, size_t bytes) {
+    const RelaxedCapture relaxed;
     const cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) { cudaGetLastError(); *p = nullptr; }
-    if (capturing) cudaThreadExchangeStreamCaptureMode(&mode);
     return e;
 }
 void* MmqWork::scratch(size_t bytes, bool capturing) {
@@ -29,9 +34,9 @@ void* MmqWork::scratch(size_t bytes, bool capturing) {
         few = many = MmqOperand();               // the operands that lay there are gone, also when the new buffer gets the old address
         const bool keep = held || capturing;     // the old buffer stays: all of them together take less than the newest
         size_t want = keep && bytes < 2 * act_bytes ? 2 * act_bytes : bytes;
-        if (act && !keep) cudaFree(act);
+        if (act && !keep) { const RelaxedCapture relaxed; cudaFree(act); }
         act = nullptr; act_bytes = 0; held = false;
-        if (mmq_alloc(&act, want, capturing) != cudaSuccess && mmq_alloc(&act, want = bytes, capturing) != cudaSuccess) return nullptr;
+        if (mmq_alloc(&act, want) != cudaSuccess && mmq_alloc(&act, want = bytes) != cudaSuccess) return nullptr;
         act_bytes = want;
     }
     held = held || capturing;
@@ -120,7 +125,8 @@ static int launch_mmq_impl(__half* y, const void* W, int type, const __half* x, 
 // The library's scratch: an object per stream, so that calls on different streams do not meet.  A call holds the lock while it enqueues
 // its launches (quantiser, product, sum), so that threads that share a stream do not mix theirs.  A stream that has none takes one
 // whose last work is known to be over (sessions record an event at the end of a prompt: mmq_mark), else a new one; when there are
-// MMQ_STREAMS, the one that was not used for the longest time, after a wait for the device.
+// MMQ_STREAMS, the one that was not used for the longest time, behind its event (every call records one from half of them on).  Nothing
+// here waits on the host: a wait for the device would invalidate any capture in the process.
 // Captured calls have objects apart from these, which their graphs keep: one per stream handle (a stream's id cannot be asked for under
 // capture); a handle beyond MMQ_GRAPHS shares the one that was captured into least recently.
 constexpr int MMQ_STREAMS = 32, MMQ_GRAPHS = 32;
@@ -132,9 +138,9 @@ struct MmqPool {
     unsigned long long clock = 0;
     size_t asked = 0;                            // most scratch that a call has asked for outside of captures
 
-    static Entry* oldest(Entry* e, int n) {
-        Entry* o = e;
-        for (int i = 1; i < n; ++i) if (e[i].used < o->used) o = &e[i];
+    static Entry* oldest(Entry* e, int n, bool marked) {
+        Entry* o = nullptr;
+        for (int i = 0; i < n; ++i) if ((e[i].marked || !marked) && (!o || e[i].used < o->used)) o = &e[i];
         return o;
     }
     static bool id_of(cudaStream_t st, unsigned long long& id) {
@@ -151,12 +157,13 @@ struct MmqPool {
         const unsigned long long id = (unsigned long long)(uintptr_t)st;
         Entry* e = nullptr;
         for (int i = 0; i < n_graphs; ++i) if (graphs[i].id == id) e = &graphs[i];
-        if (!e) e = n_graphs < MMQ_GRAPHS ? &graphs[n_graphs++] : oldest(graphs, n_graphs);
+        if (!e) e = n_graphs < MMQ_GRAPHS ? &graphs[n_graphs++] : oldest(graphs, n_graphs, false);
         e->id = id; e->used = ++clock;
         e->work.capture_limit = asked;
         return &e->work;
     }
     MmqWork* of_stream(cudaStream_t st) {
+        const RelaxedCapture relaxed;
         unsigned long long id;
         if (!id_of(st, id)) return nullptr;
         Entry* e = find(id);
@@ -165,8 +172,8 @@ struct MmqPool {
             cudaGetLastError();                  // "not ready" is an answer
             if (!e && n_streams < MMQ_STREAMS) e = &streams[n_streams++];
             if (!e) {
-                if (cudaDeviceSynchronize() != cudaSuccess) { cudaGetLastError(); return nullptr; }
-                e = oldest(streams, n_streams);
+                e = oldest(streams, n_streams, true);
+                if (!e || cudaStreamWaitEvent(st, e->done, 0) != cudaSuccess) { cudaGetLastError(); return nullptr; }
             }
             e->work.few = e->work.many = MmqOperand();
         }
@@ -174,6 +181,7 @@ struct MmqPool {
         return &e->work;
     }
     void mark(cudaStream_t st) {
+        const RelaxedCapture relaxed;
         unsigned long long id;
         Entry* e = id_of(st, id) ? find(id) : nullptr;
         if (!e || (!e->done && cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming) != cudaSuccess)) { cudaGetLastError(); return; }
@@ -186,15 +194,20 @@ struct MmqLease {
     std::unique_lock<std::mutex> lock;
     MmqPool* pool = nullptr;
     MmqWork* w = nullptr;
+    cudaStream_t st;
     bool cap;
-    MmqLease(MmqWork* own, cudaStream_t st) : w(own), cap(capturing(st)) {
+    MmqLease(MmqWork* own, cudaStream_t stream) : w(own), st(stream), cap(capturing(stream)) {
         DeviceCtx* c = own ? nullptr : ctx();
         if (!c) return;
         pool = &g_mmq_pool[c->device];
         lock = std::unique_lock<std::mutex>(pool->mu);
         w = cap ? pool->of_graph(st) : pool->of_stream(st);
     }
-    ~MmqLease() { if (pool && w && !cap && w->act_bytes > pool->asked) pool->asked = w->act_bytes; }
+    ~MmqLease() {
+        if (!pool || !w || cap) return;
+        if (w->act_bytes > pool->asked) pool->asked = w->act_bytes;
+        if (pool->n_streams > MMQ_STREAMS / 2) pool->mark(st);
+    }
 };
 
 void mmq_mark(cudaStream_t st) {

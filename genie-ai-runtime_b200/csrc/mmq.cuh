@@ -18,7 +18,7 @@ int launch_mmq_pair(__half* y1, __half* y2, const void* W1, int type1, const voi
                     cudaStream_t st, MmqWork* own = nullptr);
 size_t mmq_scratch_bytes(int N, int K);
 void mmq_mark(cudaStream_t st);       // all products on st so far may be taken for over once the stream has come here
-cudaError_t mmq_alloc(void** p, size_t bytes, bool capturing);      // cudaMalloc, also under capture
+cudaError_t mmq_alloc(void** p, size_t bytes);      // cudaMalloc, whether this thread or another one captures
 // tensor-core path (mmq_tc.cu): tcgen05.mma over fp16 operands built from the same quantised values
 bool   mmq_tc_applies(const void* W, int type, int M, int N, int K);
 size_t mmq_tc_scratch_bytes(int type, int M, int N, int K);

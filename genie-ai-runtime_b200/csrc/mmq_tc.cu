@@ -562,7 +562,7 @@ bool mmq_wide_applies(int M, int M2, int N, int K) {
 // call asks too, so that it takes the way an uncaptured one takes.
 void* MmqWork::wide_scratch(bool capturing) {
     if (wide || no_wide || (capturing && !capture_limit)) return wide;
-    no_wide = mmq_alloc(&wide, MW_WEIGHT_BYTES + gemm_pair_part_floats() * sizeof(float), capturing) != cudaSuccess;
+    no_wide = mmq_alloc(&wide, MW_WEIGHT_BYTES + gemm_pair_part_floats() * sizeof(float)) != cudaSuccess;
     return wide;
 }
 
