@@ -295,3 +295,46 @@ assert jb.device_status() == 0
     here = os.path.dirname(os.path.abspath(__file__))
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, env=dict(os.environ, PYTHONPATH=os.pathsep.join([os.path.dirname(here), here])))
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_products_beside_another_threads_capture():
+    """Products on new streams, one of which needs more scratch than there is, while another thread captures: both are as they are alone."""
+    import ctypes
+    import threading
+    import torch
+    jb = pkg()
+    M, K = 1024, 1024
+    rng = np.random.Generator(np.random.PCG64(1014))
+    W = dev(orc.gen_weight(rng, 12, M, K))
+    rt, sizes = ctypes.CDLL("libcudart.so"), (30, 500, 6000)
+    xs, ys = [dev(orc.gen_act(rng, n * K)) for n in sizes], [torch.zeros(n * M, dtype=torch.float16, device="cuda") for n in sizes]
+    x, y = dev(orc.gen_act(rng, 40 * K)), torch.zeros(40 * M, dtype=torch.float16, device="cuda")
+    jb.gemm_quant_batched(y, W, 12, x, M, 40, K)
+    torch.cuda.synchronize()
+    want, failed, handles = y.clone(), [], [ctypes.c_void_p() for _ in sizes]
+    assert all(rt.cudaStreamCreateWithFlags(ctypes.byref(h), 1) == 0 for h in handles)
+    torch.cuda.synchronize()
+    def other():
+        try:
+            for n, a, b, h in zip(sizes, xs, ys, handles):
+                jb.gemm_quant_batched(b, W, 12, a, M, n, K, stream=h.value)
+        except Exception as e:
+            failed.append(e)
+    g, st = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(g, stream=st):
+        t = threading.Thread(target=other)
+        t.start()
+        t.join()
+        jb.gemm_quant_batched(y, W, 12, x, M, 40, K, stream=st)
+    assert not failed, failed
+    torch.cuda.synchronize()
+    y.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+    for n, a, b in zip(sizes, xs, ys):
+        again = torch.zeros_like(b)
+        jb.gemm_quant_batched(again, W, 12, a, M, n, K)
+        torch.cuda.synchronize()
+        assert torch.equal(again, b), n
+    assert jb.device_status() == 0
