@@ -13,6 +13,7 @@
 #include "attention.cuh"
 #include "mmq.cuh"
 #include "gemv.cuh"
+#include "mmq_few.cuh"
 #include <cmath>
 #include <new>
 #include <vector>
@@ -90,6 +91,7 @@ struct jllm_b200_batch_decoder {
     void** lists = nullptr;            // device: [layer][4 (k, v, k scales, v scales)][B] pointers
     std::vector<unsigned char> maps;   // host: [layer][B][K, V] TMA tensor maps of the caches (128 bytes each), passed to the kernel as parameters
     void* slab = nullptr;
+    MfModel few;                       // the products of up to MF_MAX_TOKENS streams; its scratch is in the slab too
     MmqWork mmq;                       // in the slab: the captured step holds its addresses, all of it is there from the start
     int kernels_per_step = 0;
     cudaGraphExec_t graph_exec = nullptr;   // one decode step from the device-side state
@@ -106,9 +108,19 @@ static int bdec_enqueue_step(jllm_b200_batch_decoder* d, const int* prompt, int 
     JB_CUDA(launch_k(batch_begin_kernel, dim3(1), dim3(128), 0, st, pdl_enabled(), d->state, d->seq_lens, d->tokens, prompt, n_prompt, B));
     count_launch();
     BCHK(launch_embed_rows(d->x, m.tok_embd, m.embd_type, d->tokens, B, H, st));
+    MfModel& f = d->few;
+    const bool few = !f.layers.empty();
+    if (few) BCHK(launch_mf_norm(nullptr, nullptr, d->x, nullptr, d->layers[0].rms_attn, m.rms_eps, H, mf_operand(f.layers[0].qkv, f.xh4, f.xh6), B, st));
     for (int l = 0; l < m.n_layers; ++l) {
         const jllm_b200_layer_desc& w = d->layers[l];
         void** L = d->lists + (size_t)l * 4 * B;
+        if (few) {
+            const MfPrep pr = { d->q, w.q_norm, w.k_norm, m.rms_eps, (int8_t* const*)L, (int8_t* const*)(L + B), (float* const*)(L + 2 * B), (float* const*)(L + 3 * B),
+                                nullptr, nullptr, nullptr, nullptr, d->state, 0, 0, m.n_heads, m.n_kv_heads, m.rope_neox != 0 };
+            const MfProduct& qkv = f.layers[l].qkv;
+            BCHK(launch_mf_sums(qkv, mf_operand(qkv, f.xh4, f.xh6), f.part, B, st));
+            BCHK(launch_mf_prep(qkv, f.part, pr, m.rope_theta, B, st));
+        } else {
         BCHK(launch_rmsnorm(d->normed, d->x, nullptr, w.rms_attn, true, B, H, m.rms_eps, st));
         BCHK(launch_mmq(d->q, resolve_weight(w.wq), w.type_wq, d->normed, QD, B, H, nullptr, st, &d->mmq));
         BCHK(launch_mmq_ex(d->k, resolve_weight(w.wk), w.type_wk, d->normed, KVD, B, H, nullptr, true, st, &d->mmq));      // same activations as Q
@@ -116,6 +128,7 @@ static int bdec_enqueue_step(jllm_b200_batch_decoder* d, const int* prompt, int 
         BCHK(launch_qkv_prep_batched(d->q, d->k, d->v, w.q_norm, w.k_norm, m.rms_eps, (int8_t* const*)L, (int8_t* const*)(L + B),
                                      (float* const*)(L + 2 * B), (float* const*)(L + 3 * B), B, m.n_heads, m.n_kv_heads, m.head_dim,
                                      d->state, m.rope_theta, m.rope_neox != 0, st));
+        }
         AttnCall c;
         c.out = d->att; c.q = d->q; c.k_list = (const void* const*)L; c.v_list = (const void* const*)(L + B);
         c.ks_list = (const float* const*)(L + 2 * B); c.vs_list = (const float* const*)(L + 3 * B); c.seq_lens = d->seq_lens;
@@ -124,14 +137,31 @@ static int bdec_enqueue_step(jllm_b200_batch_decoder* d, const int* prompt, int 
         c.scale = scale; c.kv_int8 = 1;
         c.n_splits = 1;      // the step is one captured graph for every position: no slices (the streams of a step are short or many)
         BCHK(launch_attention(c, st));
+        if (few) {
+            const MfLayer& p = f.layers[l];
+            BCHK(launch_mf_quantise(d->att, mf_operand(p.wo, f.xa, f.xa), QD, B, st));
+            BCHK(launch_mf_sums(p.wo, mf_operand(p.wo, f.xa, f.xa), f.part, B, st));
+            BCHK(launch_mf_norm(&p.wo, f.part, d->x, d->x2, w.rms_ffn, m.rms_eps, H, mf_operand(p.gate_up, f.xh4, f.xh6), B, st));
+            BCHK(launch_mf_sums(p.gate_up, mf_operand(p.gate_up, f.xh4, f.xh6), f.part, B, st));
+            BCHK(launch_mf_glu(p.gate_up, f.part, mf_operand(p.down, f.xi, f.xi), B, st));
+            BCHK(launch_mf_sums(p.down, mf_operand(p.down, f.xi, f.xi), f.part, B, st));
+            const bool more = l + 1 < m.n_layers;
+            const MfOperand next = mf_operand(more ? f.layers[l + 1].qkv : f.out, f.xh4, f.xh6);
+            BCHK(launch_mf_norm(&p.down, f.part, d->x2, d->x, more ? d->layers[l + 1].rms_attn : m.output_norm, m.rms_eps, H, next, B, st));
+            continue;
+        }
         BCHK(launch_mmq_ex(d->x2, resolve_weight(w.wo), w.type_wo, d->att, H, B, QD, d->x, false, st, &d->mmq));           // + residual
         BCHK(launch_rmsnorm(d->normed, d->x2, nullptr, w.rms_ffn, true, B, H, m.rms_eps, st));
         BCHK(launch_mmq_pair(d->gate, d->up, resolve_weight(w.w_gate), w.type_w_gate, resolve_weight(w.w_up), w.type_w_up, d->normed, I, I, B, H, st, &d->mmq));   // one launch where the tensor-core kernel serves both
         BCHK(launch_glu(d->sw, d->gate, d->up, B, I, false, st));
         BCHK(launch_mmq_ex(d->x, resolve_weight(w.w_down), w.type_w_down, d->sw, H, B, I, d->x2, false, st, &d->mmq));     // + residual
     }
+    if (few) {
+        BCHK(launch_mf_out(f.out, mf_operand(f.out, f.xh4, f.xh6), d->logits, nullptr, f.part, B, st));
+    } else {
     BCHK(launch_rmsnorm(d->normed, d->x, nullptr, m.output_norm, true, B, H, m.rms_eps, st));
     BCHK(launch_mmq(d->logits, resolve_weight(m.output), m.output_type, d->normed, V, B, H, nullptr, st, &d->mmq));
+    }
     JB_CUDA(launch_k(argmax_rows_kernel, dim3(B), dim3(1024), 0, st, pdl_enabled(), (const __half*)d->logits, V, d->tokens, d->state,
                      d->out_tokens, d->out_cap, B));
     count_launch();
@@ -176,8 +206,10 @@ jllm_b200_batch_decoder* jllm_b200_batch_decoder_create(const jllm_b200_model_de
                 if (b > need) need = b;
         wide = wide || mmq_wide_applies(M, M2, B, K);
     }
+    if (B <= MF_MAX_TOKENS && d->few.plan(d->m, true)) { need = al(d->few.bytes(B)); wide = false; }
     if (cudaMalloc(&d->slab, total + need) != cudaSuccess) { cudaGetLastError(); d->slab = nullptr; set_error(JB_ERR_NOMEM, "batch decoder: %zu B of activations and product scratch", total + need); jllm_b200_batch_decoder_destroy(d); return nullptr; }
-    d->mmq.act = (char*)d->slab + total; d->mmq.act_bytes = need; d->mmq.held = true;
+    if (d->few.layers.empty()) { d->mmq.act = (char*)d->slab + total; d->mmq.act_bytes = need; d->mmq.held = true; }
+    else d->few.place((char*)d->slab + total, B);
     cudaMemset(d->slab, 0, total);
     char* p = (char*)d->slab;
     auto take = [&](size_t b) { char* r = p; p += al(b); return r; };

@@ -62,6 +62,7 @@ struct DeviceCtx {
     RopeTable rope[8]; int n_rope = 0;
     bool gemv_attr[12] = {};
     bool mms_attr[16] = {};
+    bool mf_attr[2] = {};
     bool gemm_pair_attr[2] = { false, false };
     bool gemv_chain_attr = false;
     bool attn_tma_attr[6] = { false, false, false, false, false, false };

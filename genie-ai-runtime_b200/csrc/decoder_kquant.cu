@@ -8,6 +8,7 @@
 #include "elementwise.cuh"
 #include "attention.cuh"
 #include "mmq.cuh"
+#include "mmq_few.cuh"
 #include "tp.cuh"
 #include <cfloat>
 #include <cstdlib>
@@ -38,6 +39,7 @@ struct KquantDecoder : jllm_b200_decoder {
     void* pf_codes = nullptr;          // in the slab: one layer's cache, widened for the prompt attention; null: too short a chunk, too long a context, or no memory
     __half *pf_x = nullptr, *pf_x2 = nullptr, *pf_normed = nullptr, *pf_y = nullptr, *pf_q = nullptr, *pf_att = nullptr, *pf_k = nullptr,
            *pf_v = nullptr, *pf_gate = nullptr, *pf_up = nullptr, *pf_sw = nullptr;
+    MfModel few;                       // products of chunks of up to MF_MAX_TOKENS tokens; its scratch is in pf_slab
 
     ~KquantDecoder() override {
         if (slab) cudaFree(slab);
@@ -49,6 +51,7 @@ struct KquantDecoder : jllm_b200_decoder {
     int enqueue_step(int n_splits, cudaStream_t st) override;
     int reserve_chunk(int tokens, cudaStream_t st) override;
     int enqueue_chunk(const int* dev_tokens, int n, int start, cudaStream_t st) override;
+    int enqueue_few_mlp(int l, int N, cudaStream_t st);
     int enqueue_rows(const int* host_rows, int n, float* out, cudaStream_t st) override;
     int attn_splits(int seq_len) const override { return attn_splits_for(seq_len); }
     bool has_chunks() const override { return !tp_on; }
@@ -290,7 +293,8 @@ int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     if (pf_slab) { cudaFree(pf_slab); pf_slab = pf_codes = nullptr; pf_cap = 0; }
     const size_t N = (size_t)cap, H = m.hidden_dim, QD = (size_t)m.n_heads * m.head_dim, KVD = (size_t)m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    const size_t total = 4 * al(N * H * 2) + 2 * al(N * QD * 2) + 2 * al(N * KVD * 2) + 3 * al(N * I * 2);
+    const int few_tokens = few.layers.empty() ? 0 : cap < MF_MAX_TOKENS ? cap : MF_MAX_TOKENS;
+    const size_t few_bytes = few_tokens ? al(few.bytes(few_tokens)) : 0, total = 4 * al(N * H * 2) + 2 * al(N * QD * 2) + 2 * al(N * KVD * 2) + 3 * al(N * I * 2) + few_bytes;
     // one allocation for all of it: it is made inside a session's first prompt, where each costs 0.4 - 2 ms (512 tokens: the first prompt
     // took 1064 us more than the next with two, 444 with one)
     size_t codes = cap >= attention_tc_min_tokens(m.n_heads, m.n_kv_heads) && m.max_context <= PF_CODES_MAX && m.head_dim == 128 ? attention_tc_scratch(m.n_kv_heads, m.max_context) : 0;
@@ -303,28 +307,56 @@ int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     pf_q = (__half*)take(N * QD * 2); pf_att = (__half*)take(N * QD * 2);
     pf_k = (__half*)take(N * KVD * 2); pf_v = (__half*)take(N * KVD * 2);
     pf_gate = (__half*)take(N * I * 2); pf_up = (__half*)take(N * I * 2); pf_sw = (__half*)take(N * I * 2);
+    if (few_tokens) few.place(take(few_bytes), few_tokens);
     pf_cap = cap;
     return JB_OK;
+}
+
+// what follows attention in a layer of few tokens: Wo, residual and norm, gate and up, SwiGLU, W_down, residual and the next layer's norm
+int KquantDecoder::enqueue_few_mlp(int l, int N, cudaStream_t st) {
+    const MfLayer& p = few.layers[l];
+    const bool more = l + 1 < m.n_layers;
+    const int H = m.hidden_dim;
+    DCHK(launch_mf_quantise(pf_att, mf_operand(p.wo, few.xa, few.xa), m.n_heads * m.head_dim, N, st));
+    DCHK(launch_mf_sums(p.wo, mf_operand(p.wo, few.xa, few.xa), few.part, N, st));
+    DCHK(launch_mf_norm(&p.wo, few.part, pf_x, pf_x2, layers[l].rms_ffn, m.rms_eps, H, mf_operand(p.gate_up, few.xh4, few.xh6), N, st));
+    DCHK(launch_mf_sums(p.gate_up, mf_operand(p.gate_up, few.xh4, few.xh6), few.part, N, st));
+    DCHK(launch_mf_glu(p.gate_up, few.part, mf_operand(p.down, few.xi, few.xi), N, st));
+    DCHK(launch_mf_sums(p.down, mf_operand(p.down, few.xi, few.xi), few.part, N, st));
+    return launch_mf_norm(&p.down, few.part, pf_x2, pf_x, more ? layers[l + 1].rms_attn : nullptr, m.rms_eps, H, more ? mf_operand(few.layers[l + 1].qkv, few.xh4, few.xh6) : MfOperand(), N, st);
 }
 
 int KquantDecoder::enqueue_chunk(const int* dev_tokens, int N, int start, cudaStream_t st) {
     const int H = m.hidden_dim, QD = m.n_heads * m.head_dim, KVD = m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
     const float scale = 1.0f / sqrtf((float)m.head_dim);
     DCHK(launch_embed_rows(pf_x, m.tok_embd, m.embd_type, dev_tokens, N, H, st));
+    const bool by_few = !few.layers.empty() && N <= MF_MAX_TOKENS;
+    if (by_few) DCHK(launch_mf_norm(nullptr, nullptr, pf_x, nullptr, layers[0].rms_attn, m.rms_eps, H, mf_operand(few.layers[0].qkv, few.xh4, few.xh6), N, st));
     for (int l = 0; l < m.n_layers; ++l) {
         const jllm_b200_layer_desc& w = layers[l];
         int8_t* kc = (int8_t*)kv.key_ptr(l, 0); int8_t* vc = (int8_t*)kv.val_ptr(l, 0);
         float* ks = kv.kv_scale_ptr(l, 0, false); float* vs = kv.kv_scale_ptr(l, 0, true);
+        if (by_few) {
+            const MfProduct& qkv = few.layers[l].qkv;
+            const MfPrep pr = { pf_q, w.q_norm, w.k_norm, m.rms_eps, nullptr, nullptr, nullptr, nullptr, kc, vc, ks, vs, nullptr, start, 1, m.n_heads, m.n_kv_heads, m.rope_neox != 0 };
+            DCHK(launch_mf_sums(qkv, mf_operand(qkv, few.xh4, few.xh6), few.part, N, st));
+            DCHK(launch_mf_prep(qkv, few.part, pr, m.rope_theta, N, st));
+        } else {
         DCHK(launch_rmsnorm(pf_normed, pf_x, nullptr, w.rms_attn, true, N, H, m.rms_eps, st));
         DCHK(launch_mmq_pair(pf_q, pf_k, resolve_weight(w.wq), w.type_wq, resolve_weight(w.wk), w.type_wk, pf_normed, QD, KVD, N, H, st));
         DCHK(launch_mmq_ex(pf_v, resolve_weight(w.wv), w.type_wv, pf_normed, KVD, N, H, nullptr, true, st));      // the operand of the product before
         DCHK(launch_qkv_prep_tokens(pf_q, pf_k, pf_v, w.q_norm, w.k_norm, m.rms_eps, kc, vc, ks, vs, N, m.n_heads, m.n_kv_heads,
                                     m.head_dim, start, m.rope_theta, m.rope_neox != 0, st));
+        }
         AttnCall c;
         c.out = pf_att; c.q = pf_q; c.k = kc; c.v = vc; c.ks = ks; c.vs = vs; c.n_heads = m.n_heads; c.n_kv = m.n_kv_heads;
         c.hd = m.head_dim; c.chd = m.head_dim; c.scale = scale; c.kv_int8 = 1; c.causal_start = start; c.batch = N; c.n_splits = 1;
         c.scratch = (float*)pf_codes;
         DCHK(attention_tc_applies(c) ? launch_attention_tc(c, st) : attention_prefill_fast_applies(c) ? launch_attention_prefill_fast(c, st) : launch_attention_general(c, st));
+        if (by_few) {
+            DCHK(enqueue_few_mlp(l, N, st));
+            continue;
+        }
         DCHK(launch_mmq(pf_y, resolve_weight(w.wo), w.type_wo, pf_att, H, N, QD, nullptr, st));
         DCHK(launch_add_half(pf_x2, pf_x, pf_y, (long long)N * H, st));
         DCHK(launch_rmsnorm(pf_normed, pf_x2, nullptr, w.rms_ffn, true, N, H, m.rms_eps, st));
@@ -366,6 +398,7 @@ jllm_b200_decoder* jllm_b200_decoder_create(const jllm_b200_model_desc* model, i
     jllm::KVCachePool::Config c = { model->n_layers, model->n_kv_heads, model->head_dim, model->max_context, 0, 1 };
     if (!d->kv.init(c) || !d->kv.kv_scale_ptr(0, 0, false)) { set_error(JB_ERR_NOMEM, "decoder: KV pool allocation failed"); jllm_b200_decoder_destroy(d); return nullptr; }
     if (d->alloc()) { jllm_b200_decoder_destroy(d); return nullptr; }
+    d->few.plan(d->m, false);
     // scratch that must exist before any graph capture
     splitk_buffer((size_t)model->n_heads * 64 * (model->head_dim + 4), true);
     return d;

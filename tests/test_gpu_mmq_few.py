@@ -1,0 +1,118 @@
+"""Products of a few tokens (2..128: prompt chunks and lock-step streams) on the split-by-units tensor-core kernel, against the kernels
+that serve weights it does not take (a Q6_K matrix that starts at an odd multiple of two bytes).
+
+Both sides build the same fp16 operands and sum them in fp32 in another order.  What that may do: a key, formed by one product from
+identical operands, differs by the last fp16 bit of a few values, which moves a cache code by one at most and its head's scale by 2^-10
+of itself.  Further on, one such bit re-rounds the codes of a group of activations (tests/test_gpu_batch_decoder.py: error RMS 0.05 and
+maximum 0.43 of the logit RMS against the oracle over the streams of a model of this size), so their logits are held to that file's
+bounds; the logits of one token, where a flipped group weighs more than in the mean over streams, to the error RMS of 0.15 that
+tests/test_gpu_decoder.py derives for them."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+from gpu_util import pkg
+
+pytestmark = pytest.mark.gpu
+
+ERR_RMS, ERR_MAX, ONE_TOKEN_RMS = 0.08, 0.6, 0.15
+# super-blocks of a row, in the order hidden, heads' outputs, MLP: Q6_K rows of 1, 2, 4 and 8 to a multiple of 16 bytes; tiles cut off at their last rows
+SHAPES = {
+    "even": dict(n_layers=2, hidden=512, n_heads=4, n_kv=2, hd=128, ffn=1024, vocab=2048),
+    "odd": dict(n_layers=2, hidden=768, n_heads=6, n_kv=2, hd=128, ffn=1280, vocab=1000),
+    "whole": dict(n_layers=1, hidden=2048, n_heads=2, n_kv=1, hd=128, ffn=2048, vocab=2056),
+}
+
+
+def weights(shape, swap):
+    """The model's weights on the device; swap: Q6_K where the benchmark's mix has Q4_K and the other way round."""
+    c = dict(SHAPES[shape])
+    m = orc.gen_model(5, **c)
+    if swap:
+        r = np.random.Generator(np.random.PCG64(6))
+        four = lambda rows, K: (orc.gen_q4k(r, rows, K, orc.model_sigma(orc.Q4_K, K), orc.MODEL_MIN_RATIO), orc.Q4_K)
+        six = lambda rows, K: (orc.gen_q6k(r, rows, K, orc.model_sigma(orc.Q6_K, K)), orc.Q6_K)
+        H, Q, KV, I = c["hidden"], c["n_heads"] * 128, c["n_kv"] * 128, c["ffn"]
+        for lw in m["layers"]:
+            lw.update(wq=six(Q, H), wk=six(KV, H), wv=four(KV, H), wo=six(H, Q), gate=six(I, H), up=four(I, H), down=four(H, I))
+    return m["cfg"], pkg().decoder.upload(m)
+
+
+def elsewhere(w):
+    """The same weights with one Q6_K matrix two bytes further on: taken by the general kernels alone."""
+    import torch
+    w = dict(w, layers=[dict(l) for l in w["layers"]])
+    name = next(n for n in ("wv", "wq") if w["layers"][0][n][1] == orc.Q6_K)
+    for l in w["layers"]:
+        t = l[name][0].reshape(-1)
+        buf = torch.empty(t.numel() + 16, dtype=torch.uint8, device="cuda")
+        buf[2:2 + t.numel()] = t
+        l[name] = (buf[2:2 + t.numel()], l[name][1])
+    return w
+
+
+def device_bytes(ptr, n):
+    import torch
+    out = torch.empty(n, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    C.CDLL("libcudart.so").cudaMemcpy(C.c_void_p(out.data_ptr()), C.c_void_p(ptr), C.c_size_t(n), 3)
+    return out.cpu().numpy()
+
+
+def check_logits(got, want, bound):
+    rms = float(np.sqrt(np.mean(want ** 2)))
+    err = np.abs(got - want)
+    print("logit error: max %.4f, rms %.4f of the logit RMS" % (float(err.max()) / rms, float(np.sqrt(np.mean(err ** 2))) / rms))
+    assert np.isfinite(got).all() and np.sqrt(np.mean(err ** 2)) <= bound * rms and err.max() <= ERR_MAX * rms
+
+
+# padded to 16 tokens; two accumulators up to 48, three super-blocks of weights in tensor memory up to 96, two above, two accumulators again up to 112
+@pytest.mark.parametrize("shape,swap", [("even", False), ("odd", False), ("odd", True), ("whole", False)])
+@pytest.mark.parametrize("n", [2, 16, 17, 48, 49, 96, 97, 112, 113, 128])
+def test_prompt_chunk_as_the_general_kernels(shape, swap, n):
+    import torch
+    jb = pkg()
+    cfg, w = weights(shape, swap)
+    prompt = np.random.Generator(np.random.PCG64(n)).integers(0, cfg["vocab"], n)
+    kv = cfg["n_kv_heads"]
+    sides = []
+    for ws in (w, elsewhere(w)):
+        d = jb.decoder.Decoder(cfg, ws, 160, jb.decoder.FUSED | jb.decoder.PREFILL)
+        st = torch.cuda.Stream()
+        n0 = jb.launch_count()
+        d.prefill(prompt, 0, st)
+        launches = jb.launch_count() - n0
+        buf = jb.lib.jllm_b200_decoder_buffer
+        buf.restype = C.c_void_p
+        codes = device_bytes(buf(C.c_void_p(d._h), 7), n * kv * 128).view(np.int8).reshape(n, kv, 128).astype(np.int32)
+        scales = device_bytes(buf(C.c_void_p(d._h), 8), n * kv * 4).view(np.float32).reshape(n, kv)
+        sides.append((codes, scales, d.logits().cpu().numpy().astype(np.float64), launches))
+        assert jb.device_status(st) == 0
+        d.close()
+    (codes, scales, logits, few), (codes0, scales0, logits0, many) = sides
+    assert few < many                                      # the general kernels need a launch for every quantiser, sum and residual
+    assert np.all(np.abs(scales - scales0) <= 2.0 ** -10 * np.abs(scales0))
+    assert np.abs(codes - codes0).max() <= 1 and np.mean(codes != codes0) <= 0.05
+    check_logits(logits, logits0, ONE_TOKEN_RMS)
+
+
+@pytest.mark.parametrize("shape,swap,streams", [("even", False, 2), ("odd", True, 33), ("odd", False, 96), ("whole", False, 128), ("even", True, 113)])
+def test_streams_as_the_general_kernels(shape, swap, streams):
+    import torch
+    jb = pkg()
+    cfg, w = weights(shape, swap)
+    prompts = np.random.Generator(np.random.PCG64(streams)).integers(0, cfg["vocab"], (streams, 3)).astype(np.int32)
+    sides = []
+    for ws in (w, elsewhere(w)):
+        d = jb.decoder.BatchDecoder(cfg, ws, 16, streams)
+        st = torch.cuda.Stream()
+        d.generate(prompts, 1, st)
+        first = d.logits()
+        d.generate(prompts, 1, st)
+        assert torch.equal(first, d.logits())              # a session can be used again, and sums in a fixed order
+        sides.append(first.double().cpu().numpy())
+        assert jb.device_status(st) == 0
+        d.close()
+    check_logits(*sides, ERR_RMS)
