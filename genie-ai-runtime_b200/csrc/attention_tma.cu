@@ -34,10 +34,10 @@ constexpr int AM_SCALE_BYTES = AM_WARPS * AM_STAGES * 2 * AM_TILE * 4;          
 constexpr int AM_SMEM = AM_RING_BYTES + AM_WARPS * 256 + 1024 + 64 + AM_SCALE_BYTES + 1024;   // + PV weight bytes, query planes, scales, alignment slack
 
 constexpr int AM_PREC = AM_HD + 4;                    // floats of a slice's partial record: m, l, two pad words, acc[128] (16-byte aligned)
-constexpr int AM_BATCH_SEQS = 14;                     // sequences per launch of a ragged batch: 28 tensor maps fit the 4 KB of kernel parameters
-
 // Tensor maps travel as kernel parameters (constant bank).  Maps read from global memory work but were measured at several
-// microseconds per tensor copy, so a ragged batch is launched in groups of AM_BATCH_SEQS sequences instead.
+// microseconds per tensor copy, so a ragged batch is launched in groups of sequences whose maps fit there: 14 (in 4 KB, the least to
+// copy for a small batch), 64 or 120 (of the 32764 bytes that sm_100 takes).
+constexpr int AM_GROUP_S = 14, AM_GROUP_M = 64, AM_GROUP_L = 120;
 template <int NSEQ> struct AmMaps { CUtensorMap m[2 * NSEQ]; };
 
 struct AmArgs {
@@ -444,10 +444,25 @@ bool attention_tma_applies(const AttnCall& c) {
 template <int NSEQ>
 static int am_launch(const AmMaps<NSEQ>& mp, const AmArgs& a, int G, dim3 grid, DeviceCtx* cx, cudaStream_t st) {
     auto kern = G == 4 ? attn_tma_kernel<4, NSEQ> : (G == 2 ? attn_tma_kernel<2, NSEQ> : attn_tma_kernel<1, NSEQ>);
-    const int gi = (G == 4 ? 2 : (G == 2 ? 1 : 0)) + (NSEQ == 1 ? 0 : 3);
+    const int gi = (G == 4 ? 2 : (G == 2 ? 1 : 0)) + (NSEQ == 1 ? 0 : NSEQ == AM_GROUP_S ? 3 : NSEQ == AM_GROUP_M ? 6 : 9);
     if (!cx->attn_tma_attr[gi]) { JB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AM_SMEM)); cx->attn_tma_attr[gi] = true; }
     JB_CUDA(launch_k(kern, grid, dim3(AM_WARPS * 32), (size_t)AM_SMEM, st, pdl_enabled(), mp, a));
     count_launch();
+    return JB_OK;
+}
+
+template <int NSEQ>
+static int am_launch_groups(const AttnCall& c, AmArgs& a, int G, int batch, DeviceCtx* cx, cudaStream_t st) {
+    const CUtensorMap* hm = reinterpret_cast<const CUtensorMap*>(c.tma_maps);
+    for (int z0 = 0; z0 < batch; z0 += NSEQ) {
+        const int n = batch - z0 < NSEQ ? batch - z0 : NSEQ;
+        alignas(64) AmMaps<NSEQ> mp;
+        memcpy(mp.m, hm + 2 * z0, (size_t)n * 2 * sizeof(CUtensorMap));
+        for (int i = 2 * n; i < 2 * NSEQ; ++i) mp.m[i] = mp.m[0];
+        a.z0 = z0;
+        const int rc = am_launch<NSEQ>(mp, a, G, dim3(c.n_kv, a.n_splits, n), cx, st);
+        if (rc) return rc;
+    }
     return JB_OK;
 }
 
@@ -479,18 +494,9 @@ int launch_attention_tma(const AttnCall& c, cudaStream_t st) {
             return set_error(JB_ERR_CUDA, "attention: tensor map for the KV cache refused");
         return am_launch<1>(mp, a, G, dim3(c.n_kv, n_splits, 1), cx, st);
     }
-    // ragged batch: c.tma_maps is a HOST array of [batch][K, V] maps; groups of AM_BATCH_SEQS sequences per launch
-    const CUtensorMap* hm = reinterpret_cast<const CUtensorMap*>(c.tma_maps);
-    for (int z0 = 0; z0 < batch; z0 += AM_BATCH_SEQS) {
-        const int n = batch - z0 < AM_BATCH_SEQS ? batch - z0 : AM_BATCH_SEQS;
-        alignas(64) AmMaps<AM_BATCH_SEQS> mp;
-        memcpy(mp.m, hm + 2 * z0, (size_t)n * 2 * sizeof(CUtensorMap));
-        for (int i = 2 * n; i < 2 * AM_BATCH_SEQS; ++i) mp.m[i] = mp.m[0];
-        a.z0 = z0;
-        const int rc = am_launch<AM_BATCH_SEQS>(mp, a, G, dim3(c.n_kv, n_splits, n), cx, st);
-        if (rc) return rc;
-    }
-    return JB_OK;
+    // ragged batch: c.tma_maps is a HOST array of [batch][K, V] maps
+    return batch <= AM_GROUP_S ? am_launch_groups<AM_GROUP_S>(c, a, G, batch, cx, st) : batch <= AM_GROUP_M ? am_launch_groups<AM_GROUP_M>(c, a, G, batch, cx, st)
+                                                                                                    : am_launch_groups<AM_GROUP_L>(c, a, G, batch, cx, st);
 }
 
 }  // namespace jb

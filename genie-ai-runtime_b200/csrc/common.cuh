@@ -65,7 +65,7 @@ struct DeviceCtx {
     bool mf_attr[2] = {};
     bool gemm_pair_attr[2] = { false, false };
     bool gemv_chain_attr = false;
-    bool attn_tma_attr[6] = { false, false, false, false, false, false };
+    bool attn_tma_attr[12] = {};
     bool attn_prefill_attr[3] = { false, false, false };
     bool attn_tc_attr[7] = {};
     unsigned int* attn_tickets = nullptr;   // ATTN_TICKET_WORDS zeroed words: slice counters of the TMA attention kernel
