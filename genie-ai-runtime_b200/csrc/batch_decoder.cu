@@ -20,18 +20,34 @@
 
 namespace jb {
 
-// greedy argmax of every row of fp16 logits [B][V] (lowest index among equal maxima, non-finite skipped); block b = row b.
-// Also records the tokens of this step and, in block 0, advances the shared position.
-__global__ void __launch_bounds__(1024) argmax_rows_kernel(const __half* logits, int V, int* tokens, int* state, int* out, int out_cap, int B) {
+// greedy argmax of every row of fp16 logits [B][V] (lowest index among equal maxima, non-finite skipped); CTA (slice, row).
+// One CTA per row left most of the machine idle (8 rows of 151936: 12.7 us, all of it the latency of a CTA's loads), so a row is cut into
+// slices; the last CTA of a row to finish settles it, the last of all moves the step on: state[0] = position, state[2] = steps recorded,
+// seq_lens[b] = position + 1 for the attention of the next step, tokens[b] = its prompt token while there are some.
+constexpr int AR_SLICES = 16;
+struct ArArgs {
+    const __half* logits; int V, B; int* tokens; int* state; int* out; int out_cap; int* seq_lens; const int* prompt; int n_prompt;
+    float* best; int* index; unsigned int* tickets;       // [B][AR_SLICES], [B][AR_SLICES], [1 + B], zero between steps
+};
+__device__ __forceinline__ void ar_take(float& best, int& bi, float v, int i) { if (v > best || (v == best && i < bi)) { best = v; bi = i; } }
+__device__ __forceinline__ void ar_warp(float& best, int& bi) {
+    #pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, o); const int oi = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
+        ar_take(best, bi, ov, oi);
+    }
+}
+__global__ void __launch_bounds__(1024) argmax_rows_kernel(const ArArgs a) {
+    pdl_launch();
     pdl_wait();
-    __shared__ float sv[32]; __shared__ int si[32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b = blockIdx.x;
-    const __half* row = logits + (size_t)b * V;
+    __shared__ float sv[32]; __shared__ int si[32]; __shared__ bool last_row, last;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b = blockIdx.y, S = gridDim.x, threads = S * blockDim.x, t0 = blockIdx.x * blockDim.x + tid;
+    const __half* row = a.logits + (size_t)b * a.V;
     float best = -INFINITY; int bi = 0x7FFFFFFF;
-    auto take = [&](float v, int i) { if (isfinite(v) && (v > best || (v == best && i < bi))) { best = v; bi = i; } };
-    if (V % 8 == 0 && ((uintptr_t)row & 15) == 0) {       // one CTA per row: its loads in flight set the time (2 bytes at a time: 68 us for 151936 logits)
+    auto take = [&](float v, int i) { if (isfinite(v)) ar_take(best, bi, v, i); };
+    if (a.V % 8 == 0 && ((uintptr_t)row & 15) == 0) {
         #pragma unroll 4
-        for (int i = tid; i < V / 8; i += blockDim.x) {
+        for (int i = t0; i < a.V / 8; i += threads) {
             const uint4 w = reinterpret_cast<const uint4*>(row)[i];
             const uint32_t u[4] = {w.x, w.y, w.z, w.w};
             #pragma unroll
@@ -41,31 +57,47 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(const __half* logits,
             }
         }
     } else {
-        for (int i = tid; i < V; i += blockDim.x) take(__half2float(row[i]), i);
+        for (int i = t0; i < a.V; i += threads) take(__half2float(row[i]), i);
     }
-    #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, o); const int oi = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
-        if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
+    ar_warp(best, bi);
     if (lane == 0) { sv[warp] = best; si[warp] = bi; }
     __syncthreads();
-    if (tid == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-            if (sv[w] > best || (sv[w] == best && si[w] < bi)) { best = sv[w]; bi = si[w]; }
-        if (bi == 0x7FFFFFFF) bi = 0;
-        tokens[b] = bi;
-        const int k = state[2];                       // steps recorded so far (read by every block before block 0 bumps it: see below)
-        if (out && k < out_cap) out[(size_t)k * B + b] = bi;
+    if (warp == 0) {
+        best = lane < (int)(blockDim.x >> 5) ? sv[lane] : -INFINITY; bi = lane < (int)(blockDim.x >> 5) ? si[lane] : 0x7FFFFFFF;
+        ar_warp(best, bi);
+        if (lane == 0) {
+            a.best[b * AR_SLICES + blockIdx.x] = best; a.index[b * AR_SLICES + blockIdx.x] = bi;
+            __threadfence();
+            last_row = atomicAdd(&a.tickets[1 + b], 1u) == (unsigned)S - 1;
+        }
+        __syncwarp();
+        if (last_row) {
+            __threadfence();
+            best = lane < S ? __ldcg(&a.best[b * AR_SLICES + lane]) : -INFINITY; bi = lane < S ? __ldcg(&a.index[b * AR_SLICES + lane]) : 0x7FFFFFFF;
+            ar_warp(best, bi);
+            if (lane == 0) {
+                if (bi == 0x7FFFFFFF) bi = 0;
+                a.tickets[1 + b] = 0u;
+                a.tokens[b] = bi;
+                const int k = a.state[2];                 // every row reads it before the last of them moves it on
+                if (a.out && k < a.out_cap) a.out[(size_t)k * a.B + b] = bi;
+                __threadfence();
+            }
+        }
+        if (lane == 0) last = last_row && atomicAdd(&a.tickets[0], 1u) == (unsigned)a.B - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int p = a.state[0] + 1;
+    __syncthreads();
+    if (tid == 0) { a.tickets[0] = 0u; a.state[0] = p; a.state[2] = a.state[2] + 1; }
+    for (int i = tid; i < a.B; i += blockDim.x) {
+        a.seq_lens[i] = p + 1;
+        if (a.prompt && p < a.n_prompt) a.tokens[i] = a.prompt[(size_t)i * a.n_prompt + p];
     }
 }
-// state[0] = position, state[2] = steps recorded; seq_lens[b] = position + 1 for the attention of the NEXT step
-__global__ void batch_advance_kernel(int* state, int* seq_lens, int B) {
-    pdl_wait();
-    const int p = state[0] + 1;
-    if (threadIdx.x == 0) { state[0] = p; state[2] = state[2] + 1; }
-    for (int b = threadIdx.x; b < B; b += blockDim.x) seq_lens[b] = p + 1;
-}
+// the first step of a request: position 0
 __global__ void batch_begin_kernel(int* state, int* seq_lens, int* tokens, const int* prompt, int n_prompt, int B) {
     pdl_wait();
     const int p = state[0];
@@ -86,6 +118,7 @@ struct jllm_b200_batch_decoder {
     int B = 0;
     __half *x = nullptr, *x2 = nullptr, *normed = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *att = nullptr, *gate = nullptr,
            *up = nullptr, *sw = nullptr, *y = nullptr, *logits = nullptr;
+    float* best = nullptr; int* best_at = nullptr; unsigned int* tickets = nullptr;      // argmax_rows_kernel
     int *state = nullptr, *tokens = nullptr, *seq_lens = nullptr, *out_tokens = nullptr, *prompt_dev = nullptr;
     int out_cap = 0, prompt_cap = 0;
     void** lists = nullptr;            // device: [layer][4 (k, v, k scales, v scales)][B] pointers
@@ -105,8 +138,6 @@ static int bdec_enqueue_step(jllm_b200_batch_decoder* d, const int* prompt, int 
     const int B = d->B, H = m.hidden_dim, QD = m.n_heads * m.head_dim, KVD = m.n_kv_heads * m.head_dim, I = m.intermediate_dim, V = m.vocab_size;
     const float scale = 1.0f / sqrtf((float)m.head_dim);
     const long long l0 = jllm_b200_launch_count();
-    JB_CUDA(launch_k(batch_begin_kernel, dim3(1), dim3(128), 0, st, pdl_enabled(), d->state, d->seq_lens, d->tokens, prompt, n_prompt, B));
-    count_launch();
     BCHK(launch_embed_rows(d->x, m.tok_embd, m.embd_type, d->tokens, B, H, st));
     MfModel& f = d->few;
     const bool few = !f.layers.empty();
@@ -162,10 +193,9 @@ static int bdec_enqueue_step(jllm_b200_batch_decoder* d, const int* prompt, int 
     BCHK(launch_rmsnorm(d->normed, d->x, nullptr, m.output_norm, true, B, H, m.rms_eps, st));
     BCHK(launch_mmq(d->logits, resolve_weight(m.output), m.output_type, d->normed, V, B, H, nullptr, st, &d->mmq));
     }
-    JB_CUDA(launch_k(argmax_rows_kernel, dim3(B), dim3(1024), 0, st, pdl_enabled(), (const __half*)d->logits, V, d->tokens, d->state,
-                     d->out_tokens, d->out_cap, B));
-    count_launch();
-    JB_CUDA(launch_k(batch_advance_kernel, dim3(1), dim3(128), 0, st, pdl_enabled(), d->state, d->seq_lens, B));
+    const ArArgs ar = { d->logits, V, B, d->tokens, d->state, d->out_tokens, d->out_cap, d->seq_lens, prompt, n_prompt, d->best, d->best_at, d->tickets };
+    const int slices = B >= 2 * AR_SLICES ? (B >= 148 ? 1 : 4) : AR_SLICES;      // one to two CTAs of 1024 threads per SM
+    JB_CUDA(launch_k(argmax_rows_kernel, dim3(slices, B), dim3(1024), 0, st, pdl_enabled(), ar));
     count_launch();
     d->kernels_per_step = (int)(jllm_b200_launch_count() - l0);
     return JB_OK;
@@ -193,7 +223,7 @@ jllm_b200_batch_decoder* jllm_b200_batch_decoder_create(const jllm_b200_model_de
         if (!d->kv[b].init(c) || !d->kv[b].kv_scale_ptr(0, 0, false)) { set_error(JB_ERR_NOMEM, "batch decoder: KV pool %d", b); jllm_b200_batch_decoder_destroy(d); return nullptr; }
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
     d->out_cap = model->max_context + 8; d->prompt_cap = model->max_context + 8;
-    const size_t total = 4 * al(B * H * 2) + 2 * al(B * QD * 2) + 2 * al(B * KVD * 2) + 3 * al(B * I * 2) + al(B * V * 2) + al(64) + 2 * al((size_t)B * 4) +
+    const size_t total = 4 * al(B * H * 2) + 2 * al(B * QD * 2) + 2 * al(B * KVD * 2) + 3 * al(B * I * 2) + al(B * V * 2) + al(64) + 2 * al((size_t)B * 4) + 2 * al((size_t)B * AR_SLICES * 4) + al((size_t)(1 + B) * 4) +
                          al((size_t)d->out_cap * B * 4) + al((size_t)d->prompt_cap * B * 4) + al((size_t)model->n_layers * 4 * B * sizeof(void*));
     // product scratch of every step: nothing of it may move once a step is captured
     const struct { size_t M, M2, K; } products[6] = { { QD, 0, H }, { KVD, 0, H }, { H, 0, QD }, { I, I, H }, { H, 0, I }, { V, 0, H } };
@@ -220,6 +250,7 @@ jllm_b200_batch_decoder* jllm_b200_batch_decoder_create(const jllm_b200_model_de
     d->logits = (__half*)take(B * V * 2);
     d->state = (int*)take(64); d->tokens = (int*)take((size_t)B * 4); d->seq_lens = (int*)take((size_t)B * 4);
     d->out_tokens = (int*)take((size_t)d->out_cap * B * 4); d->prompt_dev = (int*)take((size_t)d->prompt_cap * B * 4);
+    d->best = (float*)take((size_t)B * AR_SLICES * 4); d->best_at = (int*)take((size_t)B * AR_SLICES * 4); d->tickets = (unsigned int*)take((size_t)(1 + B) * 4);
     d->lists = (void**)take((size_t)model->n_layers * 4 * B * sizeof(void*));
     std::vector<void*> host((size_t)model->n_layers * 4 * B);
     for (int l = 0; l < model->n_layers; ++l)
@@ -263,6 +294,8 @@ int jllm_b200_batch_decoder_generate(jllm_b200_batch_decoder* d, const int* host
     for (auto& p : d->kv) p.clear();
     const int total_steps = n_prompt + (n_new > 0 ? n_new - 1 : 0);
     d->host_pos = -1;
+    JB_CUDA(launch_k(batch_begin_kernel, dim3(1), dim3(128), 0, st, pdl_enabled(), d->state, d->seq_lens, d->tokens, (const int*)d->prompt_dev, n_prompt, B));
+    count_launch();
     for (int s = 0; s < total_steps; ++s) BCHK(bdec_enqueue_step(d, d->prompt_dev, n_prompt, st));
     d->host_pos = total_steps;              // every step advances the device-side position by one
     if (n_new > 0 && host_out)

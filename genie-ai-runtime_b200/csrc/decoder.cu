@@ -15,13 +15,16 @@ namespace jb {
 // [32+G..32+2G) indices, G = gridDim.x <= 64.
 __global__ void __launch_bounds__(1024) argmax_advance_kernel(const float* logits, int n, int* state, int* out, int out_cap, unsigned int* scratch) {
     pdl_wait();
-    __shared__ float sv[32]; __shared__ int si[32]; __shared__ int last;
+    __shared__ float sv[32]; __shared__ int si[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, G = gridDim.x;
     float best = -INFINITY; int bi = 0x7FFFFFFF;
-    for (int i = blockIdx.x * blockDim.x + tid; i < n; i += G * blockDim.x) {
-        const float v = logits[i];
-        if (isfinite(v) && (v > best || (v == best && i < bi))) { best = v; bi = i; }
+    auto take = [&](float v, int i) { if (isfinite(v) && (v > best || (v == best && i < bi))) { best = v; bi = i; } };
+    const int n4 = ((uintptr_t)logits & 15) == 0 ? n / 4 : 0;
+    for (int i = blockIdx.x * blockDim.x + tid; i < n4; i += G * blockDim.x) {
+        const float4 v = reinterpret_cast<const float4*>(logits)[i];
+        take(v.x, 4 * i); take(v.y, 4 * i + 1); take(v.z, 4 * i + 2); take(v.w, 4 * i + 3);
     }
+    for (int i = 4 * n4 + blockIdx.x * blockDim.x + tid; i < n; i += G * blockDim.x) take(logits[i], i);
     #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, o); const int oi = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
@@ -29,23 +32,35 @@ __global__ void __launch_bounds__(1024) argmax_advance_kernel(const float* logit
     }
     if (lane == 0) { sv[warp] = best; si[warp] = bi; }
     __syncthreads();
-    if (tid == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-            if (sv[w] > best || (sv[w] == best && si[w] < bi)) { best = sv[w]; bi = si[w]; }
+    // the warps', then the CTAs' candidates by one warp (by one thread, a load after the other, this end took half of the kernel's 10.4 us)
+    if (warp != 0) return;
+    auto reduce = [&]() {
+        #pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, o); const int oi = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
+            if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
+        }
+    };
+    const bool have = lane < (int)(blockDim.x >> 5);
+    best = have ? sv[lane] : -INFINITY; bi = have ? si[lane] : 0x7FFFFFFF;
+    reduce();
+    int last = 0;
+    if (lane == 0) {
         reinterpret_cast<float*>(scratch)[32 + blockIdx.x] = best;
         reinterpret_cast<int*>(scratch)[32 + G + blockIdx.x] = bi;
         __threadfence();
         last = atomicAdd(scratch, 1u) == (unsigned)G - 1;
     }
-    __syncthreads();
-    if (!last || tid != 0) return;
+    if (!__shfl_sync(0xFFFFFFFFu, last, 0)) return;
     __threadfence();
-    scratch[0] = 0u;
     best = -INFINITY; bi = 0x7FFFFFFF;
-    for (int g = 0; g < G; ++g) {
-        const float v = reinterpret_cast<volatile float*>(scratch)[32 + g]; const int i = reinterpret_cast<volatile int*>(scratch)[32 + G + g];
+    for (int g = lane; g < G; g += 32) {
+        const float v = __ldcg(reinterpret_cast<const float*>(scratch) + 32 + g); const int i = __ldcg(reinterpret_cast<const int*>(scratch) + 32 + G + g);
         if (i != 0x7FFFFFFF && (v > best || (v == best && i < bi))) { best = v; bi = i; }
     }
+    reduce();
+    if (lane != 0) return;
+    scratch[0] = 0u;
     if (bi == 0x7FFFFFFF) bi = 0;
     const int k = state[2];
     if (out && k < out_cap) out[k] = bi;
