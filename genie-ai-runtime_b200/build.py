@@ -18,7 +18,7 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 COMMON = ["core.cu", "decoder.cu", "pools.cpp", "attention_general.cu"]
 LAYERS = ["decoder_layers.cu", "layernorm.cu", "dense_gemv.cu", "dense_simt.cu", "dense_tc.cu", "gemm_pair.cu", "moe.cu", "attention_bf16.cu", "attention_tc.cu", "attention_latent.cu", "latent.cu", "mlstm.cu", "mlstm_chunk.cu"]
 KQUANT = ["api.cu", "gemv.cu", "elementwise.cu", "attention.cu", "attention_tma.cu", "attention_prefill.cu", "attention_noalloc.cu", "mmq.cu", "mmq_tc.cu",
-          "mmq_stream.cu", "mmq_few.cu", "tp.cu", "decoder_kquant.cu", "batch_decoder.cu", "layers_api.cu"]
+          "mmq_stream.cu", "mmq_few.cu", "mmq_rows.cu", "tp.cu", "decoder_kquant.cu", "batch_decoder.cu", "layers_api.cu"]
 SOURCES = COMMON + LAYERS + KQUANT
 # A command that serves one model in a fresh checkout builds only the part its architecture needs, as a library of its own.
 LAYERS_OUT = os.path.join(HERE, "libjllm_b200_layers.so")

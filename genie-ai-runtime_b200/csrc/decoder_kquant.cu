@@ -39,7 +39,8 @@ struct KquantDecoder : jllm_b200_decoder {
     void* pf_codes = nullptr;          // in the slab: one layer's cache, widened for the prompt attention; null: too short a chunk, too long a context, or no memory
     __half *pf_x = nullptr, *pf_x2 = nullptr, *pf_normed = nullptr, *pf_y = nullptr, *pf_q = nullptr, *pf_att = nullptr, *pf_k = nullptr,
            *pf_v = nullptr, *pf_gate = nullptr, *pf_up = nullptr, *pf_sw = nullptr;
-    MfModel few;                       // products of chunks of up to MF_MAX_TOKENS tokens; its scratch is in pf_slab
+    MfModel few;                       // products of chunks of up to MF_MAX_TOKENS tokens
+    void* pf_operands = nullptr;       // in the slab: quantised activations and partial sums of such a chunk, or the operands of a longer one
 
     ~KquantDecoder() override {
         if (slab) cudaFree(slab);
@@ -52,6 +53,8 @@ struct KquantDecoder : jllm_b200_decoder {
     int reserve_chunk(int tokens, cudaStream_t st) override;
     int enqueue_chunk(const int* dev_tokens, int n, int start, cudaStream_t st) override;
     int enqueue_few_mlp(int l, int N, cudaStream_t st);
+    int enqueue_rows_chunk(int N, int start, cudaStream_t st);
+    int enqueue_attention(int l, int N, int start, cudaStream_t st);
     int enqueue_rows(const int* host_rows, int n, float* out, cudaStream_t st) override;
     int attn_splits(int seq_len) const override { return attn_splits_for(seq_len); }
     bool has_chunks() const override { return !tp_on; }
@@ -293,8 +296,12 @@ int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     if (pf_slab) { cudaFree(pf_slab); pf_slab = pf_codes = nullptr; pf_cap = 0; }
     const size_t N = (size_t)cap, H = m.hidden_dim, QD = (size_t)m.n_heads * m.head_dim, KVD = (size_t)m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    const int few_tokens = few.layers.empty() ? 0 : cap < MF_MAX_TOKENS ? cap : MF_MAX_TOKENS;
-    const size_t few_bytes = few_tokens ? al(few.bytes(few_tokens)) : 0, total = 4 * al(N * H * 2) + 2 * al(N * QD * 2) + 2 * al(N * KVD * 2) + 3 * al(N * I * 2) + few_bytes;
+    // Where the weights allow it (by_rows), every chunk goes through the kernels that hand one product's results to the next as its operand: up to
+    // MF_MAX_TOKENS tokens the products of few tokens, beyond those of mmq_tc.cu; the scratch of one serves the other.
+    const bool by_rows = !few.layers.empty(), many = !by_rows || cap > MF_MAX_TOKENS;
+    const size_t few_bytes = by_rows ? al(few.bytes(cap < MF_MAX_TOKENS ? cap : MF_MAX_TOKENS)) : 0, row_bytes = by_rows && many ? al(few.row_bytes(cap)) : 0;
+    const size_t operands = few_bytes > row_bytes ? few_bytes : row_bytes;
+    const size_t total = 2 * al(N * H * 2) + 2 * al(N * QD * 2) + (many ? al(N * H * 2) + 2 * al(N * KVD * 2) + 2 * al(N * I * 2) : 0) + (by_rows ? operands : al(N * H * 2) + al(N * I * 2));
     // one allocation for all of it: it is made inside a session's first prompt, where each costs 0.4 - 2 ms (512 tokens: the first prompt
     // took 1064 us more than the next with two, 444 with one)
     size_t codes = cap >= attention_tc_min_tokens(m.n_heads, m.n_kv_heads) && m.max_context <= PF_CODES_MAX && m.head_dim == 128 ? attention_tc_scratch(m.n_kv_heads, m.max_context) : 0;
@@ -303,12 +310,63 @@ int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     pf_codes = codes ? (char*)pf_slab + total : nullptr;
     char* p = (char*)pf_slab;
     auto take = [&](size_t b) { char* r = p; p += al(b); return r; };
-    pf_x = (__half*)take(N * H * 2); pf_x2 = (__half*)take(N * H * 2); pf_normed = (__half*)take(N * H * 2); pf_y = (__half*)take(N * H * 2);
+    pf_x = (__half*)take(N * H * 2); pf_x2 = (__half*)take(N * H * 2);
     pf_q = (__half*)take(N * QD * 2); pf_att = (__half*)take(N * QD * 2);
-    pf_k = (__half*)take(N * KVD * 2); pf_v = (__half*)take(N * KVD * 2);
-    pf_gate = (__half*)take(N * I * 2); pf_up = (__half*)take(N * I * 2); pf_sw = (__half*)take(N * I * 2);
-    if (few_tokens) few.place(take(few_bytes), few_tokens);
+    if (many) {
+        pf_y = (__half*)take(N * H * 2);
+        pf_k = (__half*)take(N * KVD * 2); pf_v = (__half*)take(N * KVD * 2);
+        pf_gate = (__half*)take(N * I * 2); pf_up = (__half*)take(N * I * 2);
+    }
+    if (by_rows) {
+        pf_operands = take(operands);
+    } else {
+        pf_normed = (__half*)take(N * H * 2); pf_sw = (__half*)take(N * I * 2);
+    }
     pf_cap = cap;
+    return JB_OK;
+}
+
+// causal attention of a chunk over layer l's cache
+int KquantDecoder::enqueue_attention(int l, int N, int start, cudaStream_t st) {
+    AttnCall c;
+    c.out = pf_att; c.q = pf_q; c.k = kv.key_ptr(l, 0); c.v = kv.val_ptr(l, 0); c.ks = kv.kv_scale_ptr(l, 0, false); c.vs = kv.kv_scale_ptr(l, 0, true); c.n_heads = m.n_heads; c.n_kv = m.n_kv_heads;
+    c.hd = m.head_dim; c.chd = m.head_dim; c.scale = 1.0f / sqrtf((float)m.head_dim); c.kv_int8 = 1; c.causal_start = start; c.batch = N; c.n_splits = 1;
+    c.scratch = (float*)pf_codes;
+    return attention_tc_applies(c) ? launch_attention_tc(c, st) : attention_prefill_fast_applies(c) ? launch_attention_prefill_fast(c, st) : launch_attention_general(c, st);
+}
+
+// The layers of a chunk of many tokens: between two products one kernel adds, norms, rotates or gates and writes the next one's operand (before:
+// a launch for each, and a quantiser in front of every product).
+int KquantDecoder::enqueue_rows_chunk(int N, int start, cudaStream_t st) {
+    const int H = m.hidden_dim, QD = m.n_heads * m.head_dim, KVD = m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
+    few.place_rows(pf_operands, N);
+    auto product = [&](__half* y, const void* W, int type, int M, int K, const MfOperand& x) { return launch_mmq_ready(y, nullptr, W, nullptr, type, type == T_Q6K ? x.x6 : x.x4, M, 0, N, K, st); };
+    auto pair = [&](__half* y1, __half* y2, const void* W1, int t1, const void* W2, int t2, int M1, int M2, int K, const MfOperand& x) {
+        if (t1 == t2) return launch_mmq_ready(y1, y2, W1, W2, t1, t1 == T_Q6K ? x.x6 : x.x4, M1, M2, N, K, st);
+        const int rc = product(y1, W1, t1, M1, K, x);
+        return rc ? rc : product(y2, W2, t2, M2, K, x);
+    };
+    DCHK(launch_mr_norm(pf_x, nullptr, nullptr, layers[0].rms_attn, m.rms_eps, H, mf_operand(few.layers[0].qkv, few.xh4, few.xh6), N, st));
+    for (int l = 0; l < m.n_layers; ++l) {
+        const jllm_b200_layer_desc& w = layers[l];
+        const MfLayer& p = few.layers[l];
+        const bool more = l + 1 < m.n_layers;
+        const MfOperand in = mf_operand(p.qkv, few.xh4, few.xh6), at = mf_operand(p.wo, few.xa, few.xa), mid = mf_operand(p.gate_up, few.xh4, few.xh6), act = mf_operand(p.down, few.xi, few.xi);
+        const MrPrep pr = { pf_q, pf_k, pf_v, w.q_norm, w.k_norm, m.rms_eps, (int8_t*)kv.key_ptr(l, 0), (int8_t*)kv.val_ptr(l, 0), kv.kv_scale_ptr(l, 0, false), kv.kv_scale_ptr(l, 0, true),
+                            start, m.n_heads, m.n_kv_heads, m.rope_neox != 0 };
+        DCHK(pair(pf_q, pf_k, w.wq, w.type_wq, w.wk, w.type_wk, QD, KVD, H, in));
+        DCHK(product(pf_v, w.wv, w.type_wv, KVD, H, in));
+        DCHK(launch_mr_prep(pr, m.rope_theta, N, st));
+        DCHK(enqueue_attention(l, N, start, st));
+        DCHK(launch_mr_quantise(pf_att, at, QD, N, st));
+        DCHK(product(pf_y, w.wo, w.type_wo, H, QD, at));
+        DCHK(launch_mr_norm(pf_x, pf_y, pf_x2, w.rms_ffn, m.rms_eps, H, mid, N, st));
+        DCHK(pair(pf_gate, pf_up, w.w_gate, w.type_w_gate, w.w_up, w.type_w_up, I, I, H, mid));
+        DCHK(launch_mr_glu(pf_gate, pf_up, act, I, N, st));
+        DCHK(product(pf_y, w.w_down, w.type_w_down, H, I, act));
+        DCHK(launch_mr_norm(pf_x2, pf_y, pf_x, more ? layers[l + 1].rms_attn : nullptr, m.rms_eps, H, more ? mf_operand(few.layers[l + 1].qkv, few.xh4, few.xh6) : MfOperand(), N, st));
+    }
+    mmq_mark(st);
     return JB_OK;
 }
 
@@ -330,7 +388,9 @@ int KquantDecoder::enqueue_chunk(const int* dev_tokens, int N, int start, cudaSt
     const int H = m.hidden_dim, QD = m.n_heads * m.head_dim, KVD = m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
     const float scale = 1.0f / sqrtf((float)m.head_dim);
     DCHK(launch_embed_rows(pf_x, m.tok_embd, m.embd_type, dev_tokens, N, H, st));
-    const bool by_few = !few.layers.empty() && N <= MF_MAX_TOKENS;
+    if (!few.layers.empty() && N > MF_MAX_TOKENS) return enqueue_rows_chunk(N, start, st);
+    const bool by_few = !few.layers.empty();
+    if (by_few) few.place(pf_operands, N);
     if (by_few) DCHK(launch_mf_norm(nullptr, nullptr, pf_x, nullptr, layers[0].rms_attn, m.rms_eps, H, mf_operand(few.layers[0].qkv, few.xh4, few.xh6), N, st));
     for (int l = 0; l < m.n_layers; ++l) {
         const jllm_b200_layer_desc& w = layers[l];
@@ -348,11 +408,7 @@ int KquantDecoder::enqueue_chunk(const int* dev_tokens, int N, int start, cudaSt
         DCHK(launch_qkv_prep_tokens(pf_q, pf_k, pf_v, w.q_norm, w.k_norm, m.rms_eps, kc, vc, ks, vs, N, m.n_heads, m.n_kv_heads,
                                     m.head_dim, start, m.rope_theta, m.rope_neox != 0, st));
         }
-        AttnCall c;
-        c.out = pf_att; c.q = pf_q; c.k = kc; c.v = vc; c.ks = ks; c.vs = vs; c.n_heads = m.n_heads; c.n_kv = m.n_kv_heads;
-        c.hd = m.head_dim; c.chd = m.head_dim; c.scale = scale; c.kv_int8 = 1; c.causal_start = start; c.batch = N; c.n_splits = 1;
-        c.scratch = (float*)pf_codes;
-        DCHK(attention_tc_applies(c) ? launch_attention_tc(c, st) : attention_prefill_fast_applies(c) ? launch_attention_prefill_fast(c, st) : launch_attention_general(c, st));
+        DCHK(enqueue_attention(l, N, start, st));
         if (by_few) {
             DCHK(enqueue_few_mlp(l, N, st));
             continue;

@@ -248,6 +248,16 @@ int launch_mmq_pair(__half* y1, __half* y2, const void* W1, int type1, const voi
     return launch_mmq_tc_pair(y1, y2, W1, W2, type1, x, xq, M1, M2, N, K, false, st, *w, mmq_wide_applies(M1, M2, N, K) ? w->wide_scratch(l.cap) : nullptr);
 }
 
+int launch_mmq_ready(__half* y1, __half* y2, const void* W1, const void* W2, int type, const __half* xq, int M1, int M2, int N, int K, cudaStream_t st, MmqWork* own) {
+    const MmqLease l(own, st);
+    if (!mmq_tc_applies(W1, type, M1, N, K) || (W2 && !mmq_tc_applies(W2, type, M2, N, K))) return set_error(JB_ERR_ARG, "batched gemm: %d x %d over %d tokens is not for the tensor-core path", M1, K, N);
+    const size_t need = mmq_tc_scratch_bytes_pair(type, M1, M2, N, K);
+    __half* scratch = l.w ? (__half*)l.w->scratch(need, l.cap) : nullptr;
+    if (!scratch) return set_error(JB_ERR_NOMEM, "batched gemm: %zu B of scratch unavailable", need);
+    l.w->few = l.w->many = MmqOperand();         // sums of K ranges may lie where another call left its operand
+    return launch_mmq_tc_pair(y1, y2, W1, W2, type, nullptr, scratch, M1, M2, N, K, false, st, *l.w, mmq_wide_applies(M1, M2, N, K) ? l.w->wide_scratch(l.cap) : nullptr, xq);
+}
+
 static int launch_mmq_impl(__half* y, const void* W, int type, const __half* x, int M, int N, int K, int32_t* dbg, const __half* residual,
                            bool same_x, cudaStream_t st, MmqWork* w, bool cap) {
     if (M <= 0 || N <= 0) return JB_OK;

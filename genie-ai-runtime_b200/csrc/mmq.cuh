@@ -16,6 +16,8 @@ int launch_mmq_ex(__half* y, const void* W, int type, const __half* x, int M, in
                   cudaStream_t st, MmqWork* own = nullptr);
 int launch_mmq_pair(__half* y1, __half* y2, const void* W1, int type1, const void* W2, int type2, const __half* x, int M1, int M2, int N, int K,
                     cudaStream_t st, MmqWork* own = nullptr);
+// The tensor-core path over activations that are quantised already: xq [N][columns of mmq_tc.cu's operand for `type`]
+int launch_mmq_ready(__half* y1, __half* y2, const void* W1, const void* W2, int type, const __half* xq, int M1, int M2, int N, int K, cudaStream_t st, MmqWork* own = nullptr);
 size_t mmq_scratch_bytes(int N, int K);
 void mmq_mark(cudaStream_t st);       // all products on st so far may be taken for over once the stream has come here
 cudaError_t mmq_alloc(void** p, size_t bytes);      // cudaMalloc, whether this thread or another one captures
@@ -23,7 +25,7 @@ cudaError_t mmq_alloc(void** p, size_t bytes);      // cudaMalloc, whether this 
 bool   mmq_tc_applies(const void* W, int type, int M, int N, int K);
 size_t mmq_tc_scratch_bytes(int type, int M, int N, int K);
 int    launch_mmq_tc_pair(__half* y, __half* y2, const void* W, const void* W2, int type, const __half* x, __half* xq, int M, int M2, int N, int K,
-                          bool same_x_as_last, cudaStream_t st, MmqWork& work, void* wide = nullptr);
+                          bool same_x_as_last, cudaStream_t st, MmqWork& work, void* wide = nullptr, const __half* ready = nullptr);
 size_t mmq_tc_scratch_bytes_pair(int type, int M, int M2, int N, int K);
 // many tokens: the weights are expanded to the fp16 operand once, then multiplied by gemm_pair.cu
 bool   mmq_wide_applies(int M, int M2, int N, int K);

@@ -29,6 +29,8 @@
 #include "mmq_few.cuh"
 #include "mmq.cuh"
 #include "tc.cuh"
+#include <cstdlib>
+#include <cstring>
 
 namespace jb {
 
@@ -784,6 +786,8 @@ int launch_mf_quantise(const __half* x, const MfOperand& q, int K, int N, cudaSt
 static size_t mf_align(size_t b) { return (b + 255) & ~(size_t)255; }
 bool MfModel::plan(const jllm_b200_model_desc& m, bool with_out) {
     layers.clear();
+    const char* only = getenv("JLLM_B200_MMQ");            // "cuda" keeps all products on the CUDA cores
+    if (only && !strcmp(only, "cuda")) return false;
     hidden = m.hidden_dim; q_dim = m.n_heads * m.head_dim; ffn = m.intermediate_dim;
     const int kv_dim = m.n_kv_heads * m.head_dim;
     // a head is a 128-row tile; norms keep a token in one CTA's registers
@@ -815,6 +819,14 @@ void MfModel::place(void* scratch, int N) {
     auto take = [&](size_t b) { char* r = p; p += mf_align(b); return (void*)r; };
     xh4 = take(mf_x_bytes(hidden, N)); xh6 = take(mf_x_bytes(hidden, N)); xa = take(mf_x_bytes(q_dim, N)); xi = take(mf_x_bytes(ffn, N));
     part = (float*)p;
+}
+
+static size_t mr_bytes(int K, int N) { return mf_align((size_t)N * mr_width(K) * sizeof(__half)); }
+size_t MfModel::row_bytes(int N) const { return 2 * mr_bytes(hidden, N) + mr_bytes(q_dim, N) + mr_bytes(ffn, N); }
+void MfModel::place_rows(void* scratch, int N) {
+    char* p = (char*)scratch;
+    auto take = [&](int K) { char* r = p; p += mr_bytes(K, N); return (void*)r; };
+    xh4 = take(hidden); xh6 = take(hidden); xa = take(q_dim); xi = take(ffn);
 }
 
 }  // namespace jb

@@ -60,6 +60,21 @@ int launch_mf_glu(const MfProduct& p, const float* part, const MfOperand& q, int
 // fp16 vectors [N][K], quantised
 int launch_mf_quantise(const __half* x, const MfOperand& q, int K, int N, cudaStream_t st);
 
+// ── the kernels between the products of many tokens (mmq_rows.cu): fp16 results in, rows of mmq_tc.cu's operand out (x4 as for Q4_K, x6 as for
+// Q6_K matrices, null where not asked for) ──
+inline int mr_width(int K) { return K + (K / 16 + 63) / 64 * 64; }       // columns of a Q4_K operand: sums and centring sums of K / 32 groups, in whole K tiles; Q6_K: K
+// x + add (add null: x alone; else x_out) -> RMSNorm with weights w, quantised (w null: the sum alone)
+int launch_mr_norm(const __half* x, const __half* add, __half* x_out, const float* w, float eps, int H, const MfOperand& q, int N, cudaStream_t st);
+// head norms and rotation of q in place, K and V rows of tokens pos .. pos + N - 1 into one cache
+struct MrPrep {
+    __half* q; const __half* k_in; const __half* v_in; const float* q_norm; const float* k_norm; float eps;
+    int8_t* k; int8_t* v; float* ks; float* vs;
+    int pos, n_heads, n_kv, neox;
+};
+int launch_mr_prep(const MrPrep& a, float theta, int N, cudaStream_t st);
+int launch_mr_glu(const __half* gate, const __half* up, const MfOperand& q, int K, int N, cudaStream_t st);
+int launch_mr_quantise(const __half* x, const MfOperand& q, int K, int N, cudaStream_t st);
+
 // ── the layers of a Llama / Qwen3 model over a few tokens ──
 struct MfLayer { MfProduct qkv, wo, gate_up, down; };
 struct MfModel {
@@ -72,6 +87,9 @@ struct MfModel {
     bool plan(const jllm_b200_model_desc& m, bool with_out);
     size_t bytes(int N) const;
     void place(void* scratch, int N);
+    // the same operands as rows of many tokens (mmq_rows.cu)
+    size_t row_bytes(int N) const;
+    void place_rows(void* scratch, int N);
 };
 
 }  // namespace jb

@@ -28,6 +28,7 @@
 // Every mbarrier wait is bounded; a wait that runs out sets the device status word, the kernel still frees
 // its tensor memory and returns.
 #include "mmq.cuh"
+#include "mmq_quant.cuh"
 #include "dense.cuh"
 #include "tc.cuh"
 #include <type_traits>
@@ -223,56 +224,18 @@ __global__ void mmq_tc_quantize1_kernel(const __half* x, __half* xq, int N, int 
     if (gi == 0) for (int c = K + (ds4 ? 2 * G : 0) + lane; c < Kp; c += 32) row[c] = __float2half_rn(0.f);
 }
 
-// The same operand, one warp per (token, super-block of 256): lane 4j + c holds elements 8c..8c+7 of group j, read and
-// written as 16 bytes (the form above moves 2 bytes per lane and needs eight times the warps; on a 2048 x 9728 operand it
-// took as long as half the product).  The sum of x is taken in the order of the 32-lane xor-shuffle tree of that form
-// (partners 16, 8, 4, 2, 1 apart), so both forms, and the CPU restatement of the reference's quantiser, give the same bits.
-// Needs x 16-byte aligned.
+// The same operand, one warp per (token, super-block of 256), see mmq_quant.cuh (the form above moves 2 bytes per lane and needs eight times
+// the warps; on a 2048 x 9728 operand it took as long as half the product).  Needs x 16-byte aligned.
 __global__ void mmq_tc_quantize_kernel(const __half* x, __half* xq, int N, int K, int Kp, int ds4) {
     pdl_wait();
     const long long wi = (long long)blockIdx.x * blockDim.y + threadIdx.y;
-    const int lane = threadIdx.x, nsb = K / QK_K, G = K / 32;
+    const int lane = threadIdx.x, nsb = K / QK_K;
     if (wi >= (long long)N * nsb) return;
     const long long t = wi / nsb; const int sb = (int)(wi - t * nsb);
-    const int c = lane & 3, gi = sb * 8 + (lane >> 2);
-    const uint4 raw = *reinterpret_cast<const uint4*>(x + t * K + (size_t)gi * 32 + 8 * c);
-    const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
-    float v[8], s[8];
-    float amax = 0.f;
-    #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&rw[i]));
-        v[2 * i] = f.x; v[2 * i + 1] = f.y;
-        amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
-    }
-    amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
-    #pragma unroll
-    for (int i = 0; i < 8; ++i) { s[i] = v[i] + __shfl_xor_sync(0xFFFFFFFFu, v[i], 2); }       // elements 16 apart
-    #pragma unroll
-    for (int i = 0; i < 8; ++i) { s[i] = s[i] + __shfl_xor_sync(0xFFFFFFFFu, s[i], 1); }       // 8 apart
-    const float sum = __fadd_rn(__fadd_rn(__fadd_rn(s[0], s[4]), __fadd_rn(s[2], s[6])), __fadd_rn(__fadd_rn(s[1], s[5]), __fadd_rn(s[3], s[7])));   // 4, 2, 1 apart
-    float d = __fdiv_rn(amax, 127.0f);
-    const float dinv = d > 0.f ? __fdiv_rn(1.0f, d) : 0.f;
-    int q[8], qsum = 0;
-    #pragma unroll
-    for (int i = 0; i < 8; ++i) { q[i] = __float2int_rn(__fmul_rn(v[i], dinv)); qsum += q[i]; }
-    qsum += __shfl_xor_sync(0xFFFFFFFFu, qsum, 1);
-    qsum += __shfl_xor_sync(0xFFFFFFFFu, qsum, 2);
-    if (ds4) d = __half2float(__float2half_rn(d));
-    uint32_t ow[4];
-    #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const __half2 h = __halves2half2(__float2half_rn(__fmul_rn(d, (float)q[2 * i])), __float2half_rn(__fmul_rn(d, (float)q[2 * i + 1])));
-        ow[i] = *reinterpret_cast<const uint32_t*>(&h);
-    }
-    __half* row = xq + t * Kp;
-    *reinterpret_cast<uint4*>(row + (size_t)gi * 32 + 8 * c) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
-    if (ds4 && c == 0) {
-        row[K + gi] = __float2half_rn(sum);
-        row[K + G + gi] = __float2half_rn(__fmul_rn(d, (float)qsum));
-    }
-    if (sb == 0) for (int z = K + (ds4 ? 2 * G : 0) + lane; z < Kp; z += 32) row[z] = __float2half_rn(0.f);
+    float v[8];
+    mq_load8(v, x + t * K + sb * QK_K + 8 * lane);
+    if (ds4) mq_rows8(v, xq + t * Kp, nullptr, sb, K, Kp, lane);
+    else     mq_rows8(v, nullptr, xq + t * Kp, sb, K, Kp, lane);
 }
 
 // Persistent kernel: one CTA per SM walks output tiles (token tile fastest, so the CTAs running at one time
@@ -681,7 +644,7 @@ bool mmq_tc_applies(const void* W, int type, int M, int N, int K) {
 // y = x . W^T and, when W2 is given, y2 = x . W2^T in the same launch: the row tiles of both matrices are one list of work, so
 // two products that share their activations (gate and up) fill the grid together instead of one after the other.
 int launch_mmq_tc_pair(__half* y, __half* y2, const void* W, const void* W2, int type, const __half* x, __half* xq, int M, int M2, int N, int K,
-                       bool same_x, cudaStream_t st, MmqWork& work, void* wide) {
+                       bool same_x, cudaStream_t st, MmqWork& work, void* wide, const __half* ready) {
     DeviceCtx* c = ctx();
     if (!c) return set_error(JB_ERR_STATE, "batched gemm: library not initialised");
     TcArgs a;
@@ -702,7 +665,7 @@ int launch_mmq_tc_pair(__half* y, __half* y2, const void* W, const void* W2, int
     const cuuint64_t gstr[1] = {(cuuint64_t)Kp * sizeof(__half)};
     const cuuint32_t box[2] = {(cuuint32_t)TC_K, (cuuint32_t)n_tile};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, xq, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const CUresult r = encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, ready ? const_cast<__half*>(ready) : xq, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(JB_ERR_CUDA, "batched gemm: tensor map for the activation tile refused (driver code %d)", (int)r);
 
@@ -717,7 +680,7 @@ int launch_mmq_tc_pair(__half* y, __half* y2, const void* W, const void* W2, int
     // that shapes it (tokens, K, the Q4_K extras) is the same: the products that share an input quantise it once.
     const int ds4 = (int)(type == T_Q4K);
     const MmqOperand op = {x, xq, (void*)st, N, K, ds4};
-    if (!same_x || !work.many.is(op)) {
+    if (!ready && (!same_x || !work.many.is(op))) {
         if (((uintptr_t)x & 15) == 0) {
             const long long warps = (long long)N * (K / QK_K);
             JB_CUDA(launch_k(mmq_tc_quantize_kernel, dim3((unsigned)((warps + 3) / 4)), dim3(32, 4), 0, st, pdl_enabled(), x, xq, N, K, Kp, ds4));
@@ -729,7 +692,7 @@ int launch_mmq_tc_pair(__half* y, __half* y2, const void* W, const void* W2, int
         work.many = op;
         work.few = MmqOperand();
     }
-    if (wide) return launch_wide(a, xq, Kp, wide, st);
+    if (wide) return launch_wide(a, ready ? ready : xq, Kp, wide, st);
     const int n_work = a.n_full + (tiles - a.n_full) * a.ksplit;
     const dim3 grid(n_work < c->sm_count ? n_work : c->sm_count);
     if (ti == 0) JB_CUDA(launch_k(mmq_tc_kernel<T_Q4K>, grid, dim3(TC_THREADS), TC_SMEM, st, pdl_enabled(), map, a, n_tile));

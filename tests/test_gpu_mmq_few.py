@@ -1,5 +1,6 @@
-"""Products of a few tokens (2..128: prompt chunks and lock-step streams) on the split-by-units tensor-core kernel, against the kernels
-that serve weights it does not take (a Q6_K matrix that starts at an odd multiple of two bytes).
+"""Products of a few tokens (2..128: prompt chunks and lock-step streams) on the split-by-units tensor-core kernel, and longer chunks whose
+kernels between the products write the next product's operand, against the kernels that serve weights these do not take (a Q6_K matrix that
+starts at an odd multiple of two bytes).
 
 Both sides build the same fp16 operands and sum them in fp32 in another order.  What that may do: a key, formed by one product from
 identical operands, differs by the last fp16 bit of a few values, which moves a cache code by one at most and its head's scale by 2^-10
@@ -70,7 +71,8 @@ def check_logits(got, want, bound):
 
 # padded to 16 tokens; two accumulators up to 48, three super-blocks of weights in tensor memory up to 96, two above, two accumulators again up to 112
 @pytest.mark.parametrize("shape,swap", [("even", False), ("odd", False), ("odd", True), ("whole", False)])
-@pytest.mark.parametrize("n", [2, 16, 17, 48, 49, 96, 97, 112, 113, 128])
+# beyond 128: rows of many tokens, tiles of 32..256 tokens with and without K ranges, and from 384 or 448 on the expanded weights
+@pytest.mark.parametrize("n", [2, 16, 17, 48, 49, 96, 97, 112, 113, 128, 129, 257, 450])
 def test_prompt_chunk_as_the_general_kernels(shape, swap, n):
     import torch
     jb = pkg()
@@ -79,7 +81,7 @@ def test_prompt_chunk_as_the_general_kernels(shape, swap, n):
     kv = cfg["n_kv_heads"]
     sides = []
     for ws in (w, elsewhere(w)):
-        d = jb.decoder.Decoder(cfg, ws, 160, jb.decoder.FUSED | jb.decoder.PREFILL)
+        d = jb.decoder.Decoder(cfg, ws, 512, jb.decoder.FUSED | jb.decoder.PREFILL)
         st = torch.cuda.Stream()
         n0 = jb.launch_count()
         d.prefill(prompt, 0, st)
