@@ -9,6 +9,7 @@
 #include "attention.cuh"
 #include "mmq.cuh"
 #include "mmq_few.cuh"
+#include "dense.cuh"
 #include "tp.cuh"
 #include <cfloat>
 #include <cstdlib>
@@ -40,6 +41,7 @@ struct KquantDecoder : jllm_b200_decoder {
     __half *pf_x = nullptr, *pf_x2 = nullptr, *pf_normed = nullptr, *pf_y = nullptr, *pf_q = nullptr, *pf_att = nullptr, *pf_k = nullptr,
            *pf_v = nullptr, *pf_gate = nullptr, *pf_up = nullptr, *pf_sw = nullptr;
     MfModel few;                       // products of chunks of up to MF_MAX_TOKENS tokens
+    void* pf_wide = nullptr;           // in the slab: two buffers of expanded weights and the paired products' partial sums (null: chunks too short, or no memory)
     void* pf_operands = nullptr;       // in the slab: quantised activations and partial sums of such a chunk, or the operands of a longer one
 
     ~KquantDecoder() override {
@@ -54,7 +56,7 @@ struct KquantDecoder : jllm_b200_decoder {
     int enqueue_chunk(const int* dev_tokens, int n, int start, cudaStream_t st) override;
     int enqueue_few_mlp(int l, int N, cudaStream_t st);
     int enqueue_rows_chunk(int N, int start, cudaStream_t st);
-    int enqueue_attention(int l, int N, int start, cudaStream_t st);
+    int enqueue_attention(int l, int N, int start, cudaStream_t st, bool* tc = nullptr);      // tc: whether it was attention_tc.cu's
     int enqueue_rows(const int* host_rows, int n, float* out, cudaStream_t st) override;
     int attn_splits(int seq_len) const override { return attn_splits_for(seq_len); }
     bool has_chunks() const override { return !tp_on; }
@@ -293,7 +295,7 @@ static int dec_enqueue_step_tp(KquantDecoder* d, int n_splits, cudaStream_t st) 
 // gate/up, SwiGLU, W_down, residual.  After the last chunk: final norm and logits of the last token only, greedy token.
 int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     if (cap <= pf_cap) return JB_OK;
-    if (pf_slab) { cudaFree(pf_slab); pf_slab = pf_codes = nullptr; pf_cap = 0; }
+    if (pf_slab) { cudaFree(pf_slab); pf_slab = pf_codes = pf_wide = nullptr; pf_cap = 0; }
     const size_t N = (size_t)cap, H = m.hidden_dim, QD = (size_t)m.n_heads * m.head_dim, KVD = (size_t)m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
     // Where the weights allow it (by_rows), every chunk goes through the kernels that hand one product's results to the next as its operand: up to
@@ -304,10 +306,13 @@ int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     const size_t total = 2 * al(N * H * 2) + 2 * al(N * QD * 2) + (many ? al(N * H * 2) + 2 * al(N * KVD * 2) + 2 * al(N * I * 2) : 0) + (by_rows ? operands : al(N * H * 2) + al(N * I * 2));
     // one allocation for all of it: it is made inside a session's first prompt, where each costs 0.4 - 2 ms (512 tokens: the first prompt
     // took 1064 us more than the next with two, 444 with one)
+    size_t wide = by_rows && mmq_wide_applies(m.hidden_dim, 0, cap, m.hidden_dim) ? 2 * MMQ_WEIGHT_BYTES + al(gemm_pair_part_floats() * sizeof(float)) : 0;
     size_t codes = cap >= attention_tc_min_tokens(m.n_heads, m.n_kv_heads) && m.max_context <= PF_CODES_MAX && m.head_dim == 128 ? attention_tc_scratch(m.n_kv_heads, m.max_context) : 0;
-    if (codes && cudaMalloc(&pf_slab, total + codes) != cudaSuccess) { cudaGetLastError(); pf_slab = nullptr; codes = 0; }
+    if (wide && cudaMalloc(&pf_slab, total + codes + wide) != cudaSuccess) { cudaGetLastError(); pf_slab = nullptr; wide = 0; }
+    if (!pf_slab && codes && cudaMalloc(&pf_slab, total + codes) != cudaSuccess) { cudaGetLastError(); pf_slab = nullptr; codes = 0; }
     if (!pf_slab && cudaMalloc(&pf_slab, total) != cudaSuccess) { cudaGetLastError(); pf_slab = nullptr; return set_error(JB_ERR_NOMEM, "decoder: %zu B of prefill activations", total); }
     pf_codes = codes ? (char*)pf_slab + total : nullptr;
+    pf_wide = wide ? (char*)pf_slab + total + codes : nullptr;
     char* p = (char*)pf_slab;
     auto take = [&](size_t b) { char* r = p; p += al(b); return r; };
     pf_x = (__half*)take(N * H * 2); pf_x2 = (__half*)take(N * H * 2);
@@ -327,11 +332,12 @@ int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
 }
 
 // causal attention of a chunk over layer l's cache
-int KquantDecoder::enqueue_attention(int l, int N, int start, cudaStream_t st) {
+int KquantDecoder::enqueue_attention(int l, int N, int start, cudaStream_t st, bool* tc) {
     AttnCall c;
     c.out = pf_att; c.q = pf_q; c.k = kv.key_ptr(l, 0); c.v = kv.val_ptr(l, 0); c.ks = kv.kv_scale_ptr(l, 0, false); c.vs = kv.kv_scale_ptr(l, 0, true); c.n_heads = m.n_heads; c.n_kv = m.n_kv_heads;
     c.hd = m.head_dim; c.chd = m.head_dim; c.scale = 1.0f / sqrtf((float)m.head_dim); c.kv_int8 = 1; c.causal_start = start; c.batch = N; c.n_splits = 1;
     c.scratch = (float*)pf_codes;
+    if (tc) *tc = attention_tc_applies(c);
     return attention_tc_applies(c) ? launch_attention_tc(c, st) : attention_prefill_fast_applies(c) ? launch_attention_prefill_fast(c, st) : launch_attention_general(c, st);
 }
 
@@ -340,9 +346,47 @@ int KquantDecoder::enqueue_attention(int l, int N, int start, cudaStream_t st) {
 int KquantDecoder::enqueue_rows_chunk(int N, int start, cudaStream_t st) {
     const int H = m.hidden_dim, QD = m.n_heads * m.head_dim, KVD = m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
     few.place_rows(pf_operands, N);
-    auto product = [&](__half* y, const void* W, int type, int M, int K, const MfOperand& x) { return launch_mmq_ready(y, nullptr, W, nullptr, type, type == T_Q6K ? x.x6 : x.x4, M, 0, N, K, st); };
+    // Expanded weights in two buffers by turns: the next product's while the present one runs, or the attention (512 tokens of 8 layers: 0.52 ms of
+    // 2.40 went into expansions in front of products).
+    std::vector<MmqPiece> pieces;
+    std::vector<size_t> ends;                // of the products, in the order they are called in
+    auto add = [&](const void* W1, const void* W2, int type, int M1, int M2, int K) {
+        if (pf_wide && mmq_wide_applies(M1, M2, N, K)) mmq_pieces(pieces, W1, W2, type, M1, M2, K);
+        ends.push_back(pieces.size());
+    };
+    auto add_pair = [&](const void* W1, int t1, const void* W2, int t2, int M1, int M2, int K) {
+        if (t1 == t2) { add(W1, W2, t1, M1, M2, K); return; }
+        add(W1, nullptr, t1, M1, 0, K); add(W2, nullptr, t2, M2, 0, K);
+    };
+    for (const jllm_b200_layer_desc& w : layers) {
+        add_pair(w.wq, w.type_wq, w.wk, w.type_wk, QD, KVD, H);
+        add(w.wv, nullptr, w.type_wv, KVD, 0, H);
+        add(w.wo, nullptr, w.type_wo, H, 0, QD);
+        add_pair(w.w_gate, w.type_w_gate, w.w_up, w.type_w_up, I, I, H);
+        add(w.w_down, nullptr, w.type_w_down, H, 0, I);
+    }
+    size_t expanded = 0, multiplied = 0, called = 0;
+    auto buffer_of = [&](size_t i) { return (char*)pf_wide + (i & 1) * MMQ_WEIGHT_BYTES; };
+    auto ahead = [&]() -> int {              // behind piece multiplied - 1 or the attention: the buffer of the piece before is free
+        if (expanded >= pieces.size() || expanded > multiplied) return JB_OK;
+        const size_t i = expanded++;
+        return launch_mmq_expand(pieces[i], buffer_of(i), true, st);
+    };
+    // wait: the next expansion has a better place than beside this product
+    auto both = [&](__half* y1, __half* y2, const void* W1, const void* W2, int type, int M1, int M2, int K, const MfOperand& x, bool wait) -> int {
+        const __half* xq = type == T_Q6K ? x.x6 : x.x4;
+        const size_t end = ends[called++];
+        if (multiplied == end) return launch_mmq_ready(y1, y2, W1, W2, type, xq, M1, M2, N, K, st);
+        while (multiplied < end) {
+            const size_t n = multiplied++;
+            if (expanded == n) { ++expanded; DCHK(launch_mmq_expand(pieces[n], buffer_of(n), false, st)); }
+            DCHK(launch_mmq_piece(pieces[n], buffer_of(n), xq, y1, y2, N, (float*)((char*)pf_wide + 2 * MMQ_WEIGHT_BYTES), st, wait ? std::function<int()>() : ahead));
+        }
+        return JB_OK;
+    };
+    auto product = [&](__half* y, const void* W, int type, int M, int K, const MfOperand& x, bool wait = false) { return both(y, nullptr, W, nullptr, type, M, 0, K, x, wait); };
     auto pair = [&](__half* y1, __half* y2, const void* W1, int t1, const void* W2, int t2, int M1, int M2, int K, const MfOperand& x) {
-        if (t1 == t2) return launch_mmq_ready(y1, y2, W1, W2, t1, t1 == T_Q6K ? x.x6 : x.x4, M1, M2, N, K, st);
+        if (t1 == t2) return both(y1, y2, W1, W2, t1, M1, M2, K, x, false);
         const int rc = product(y1, W1, t1, M1, K, x);
         return rc ? rc : product(y2, W2, t2, M2, K, x);
     };
@@ -355,9 +399,11 @@ int KquantDecoder::enqueue_rows_chunk(int N, int start, cudaStream_t st) {
         const MrPrep pr = { pf_q, pf_k, pf_v, w.q_norm, w.k_norm, m.rms_eps, (int8_t*)kv.key_ptr(l, 0), (int8_t*)kv.val_ptr(l, 0), kv.kv_scale_ptr(l, 0, false), kv.kv_scale_ptr(l, 0, true),
                             start, m.n_heads, m.n_kv_heads, m.rope_neox != 0 };
         DCHK(pair(pf_q, pf_k, w.wq, w.type_wq, w.wk, w.type_wk, QD, KVD, H, in));
-        DCHK(product(pf_v, w.wv, w.type_wv, KVD, H, in));
+        DCHK(product(pf_v, w.wv, w.type_wv, KVD, H, in, true));      // Wo's weights beside the attention
         DCHK(launch_mr_prep(pr, m.rope_theta, N, st));
-        DCHK(enqueue_attention(l, N, start, st));
+        bool tc = false;
+        DCHK(enqueue_attention(l, N, start, st, &tc));
+        if (tc) DCHK(ahead());
         DCHK(launch_mr_quantise(pf_att, at, QD, N, st));
         DCHK(product(pf_y, w.wo, w.type_wo, H, QD, at));
         DCHK(launch_mr_norm(pf_x, pf_y, pf_x2, w.rms_ffn, m.rms_eps, H, mid, N, st));

@@ -3,6 +3,7 @@
 // CUDA-core product in true fp32 (dense_simt.cu).
 #pragma once
 #include "latent.cuh"
+#include <functional>
 #include "moe.cuh"
 
 namespace jb {
@@ -69,7 +70,7 @@ constexpr int GP_MIN_TOKENS = 128;
 bool gemm_pair_applies(const DenseGemm& a);
 bool gemm_pair_one_round(const DenseGemm& a);
 size_t gemm_pair_part_floats();
-int launch_gemm_pair(const DenseGemm& a, cudaStream_t st);       // fp16 (EK_F16) or bf16 operands, pairs of CTAs (gemm_pair.cu)
+int launch_gemm_pair(const DenseGemm& a, cudaStream_t st, const std::function<int()>& behind = nullptr);       // fp16 (EK_F16) or bf16 operands, pairs of CTAs (gemm_pair.cu)
 int launch_dense_gemm(const DenseGemm& a, cudaStream_t st);      // bf16: tensor cores; fp32: CUDA cores; one token: the decode product
 int launch_dense_gemm_tc(const DenseGemm& a, cudaStream_t st);
 int launch_dense_gemm_simt(const DenseGemm& a, cudaStream_t st);

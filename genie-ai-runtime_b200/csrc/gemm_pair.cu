@@ -265,7 +265,7 @@ bool gemm_pair_one_round(const DenseGemm& a) {
     return p.ksplit == 1 && p.n_items <= c->sm_count / 2;
 }
 
-int launch_gemm_pair(const DenseGemm& a, cudaStream_t st) {
+int launch_gemm_pair(const DenseGemm& a, cudaStream_t st, const std::function<int()>& behind) {
     DeviceCtx* c = ctx();
     if (!c) return set_error(JB_ERR_STATE, "paired gemm: library not initialised");
     if (!a.W || !a.x) return set_error(JB_ERR_PTR, "paired gemm: null pointer");
@@ -291,6 +291,7 @@ int launch_gemm_pair(const DenseGemm& a, cudaStream_t st) {
     const dim3 grid(2u * (unsigned)(p.n_items < n_pairs ? p.n_items : n_pairs));
     JB_CUDA(launch_k(kern, grid, dim3(GP_THREADS), GP_SMEM, st, pdl_enabled(), wm, xm, p));
     count_launch();
+    if (behind) { const int rc = behind(); if (rc) return rc; }
     if (p.ksplit > 1) {
         const dim3 g((p.width + 1) / 2, (p.n_items - p.n_full) / p.ksplit);
         if (half) JB_CUDA(launch_k(gemm_pair_sum_kernel<__half>, g, dim3(256), 0, st, pdl_enabled(), p));

@@ -1,6 +1,8 @@
 // mmq.cuh — prefill / batched K-quant GEMM launchers.
 #pragma once
 #include "common.cuh"
+#include <functional>
+#include <vector>
 
 namespace jb {
 
@@ -29,6 +31,12 @@ int    launch_mmq_tc_pair(__half* y, __half* y2, const void* W, const void* W2, 
 size_t mmq_tc_scratch_bytes_pair(int type, int M, int M2, int N, int K);
 // many tokens: the weights are expanded to the fp16 operand once, then multiplied by gemm_pair.cu
 bool   mmq_wide_applies(int M, int M2, int N, int K);
+constexpr size_t MMQ_WEIGHT_BYTES = (size_t)64 << 20;      // expanded weights of a piece
+struct MmqPiece { const void* W; const void* W2; int type, M, M2, K, r0, rows; };      // rows r0 .. of W's and W2's (null: none) rows in a row
+void   mmq_pieces(std::vector<MmqPiece>& out, const void* W1, const void* W2, int type, int M1, int M2, int K);
+int    launch_mmq_expand(const MmqPiece& p, void* wq, bool ahead, cudaStream_t st);
+// behind: launches to go right behind the product, before the sum of its K ranges; part: gemm_pair_part_floats
+int    launch_mmq_piece(const MmqPiece& p, const void* wq, const __half* xq, __half* y1, __half* y2, int N, float* part, cudaStream_t st, const std::function<int()>& behind = nullptr);
 // few tokens (2..64): weights streamed once, mma.sync on fp16 operands with the tensor-core path's arithmetic (mmq_stream.cu)
 bool   mmq_stream_applies(const void* W, int type, int M, int N, int K);
 size_t mmq_stream_scratch_bytes(int type, int M, int N, int K);

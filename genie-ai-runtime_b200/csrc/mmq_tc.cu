@@ -514,7 +514,7 @@ static void tc_pick(int tiles_m, int N, int n_main_tiles, int sm_count, int& n_t
 // The kernel above dequantises a weight tile again for every 256 tokens, and its producers and the tensor pipe share one SM's shared
 // memory.  From MW_MIN_TOKENS on the same fp16 operand, bit for bit, is written to memory once, in pieces that stay in L2, and
 // multiplied by the paired kernel of gemm_pair.cu (2048 tokens: 9728 x 2560 131 -> 110 us, Q6_K 2560 x 9728 171 -> 121 us).
-constexpr size_t MW_WEIGHT_BYTES = (size_t)64 << 20;
+constexpr size_t MW_WEIGHT_BYTES = MMQ_WEIGHT_BYTES;
 constexpr int MW_MIN_TOKENS = 384;      // 256 tokens: Q6_K 2560 x 9728 46 us this way, 38 fused; 512 tokens: 54 and 65; Q4_K 9728 x 2560 equal at both;
                                         // 1024 x 2560, 384 / 448 tokens: Q4_K 19.5 / 20.0 this way, 18.5 / 21.3 fused, Q6_K 18.8 / 19.2 and 17.3 / 19.5
 
@@ -532,9 +532,7 @@ void* MmqWork::wide_scratch(bool capturing) {
 // Rows [r0, r0 + rows) of the operand, Kp halves each; a thread takes 8 bytes of packed codes: 16 weights of a Q4_K block, 32 of a
 // Q6_K block, or 8 of the extra columns.  Bound by the writes (2 bytes per weight, into L2).
 template <int TYPE>
-__global__ void __launch_bounds__(256) mmq_expand_kernel(const TcArgs a, __half* out, int r0, int rows, int Kp) {
-    pdl_wait();
-    pdl_launch();
+__device__ __forceinline__ void mw_expand(const TcArgs& a, __half* out, int r0, int rows, int Kp) {
     const int nb = a.K / QK_K, per = TYPE == T_Q4K ? nb * 16 + a.n_min * 8 : nb * 8;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)rows * per) return;
@@ -598,23 +596,51 @@ __global__ void __launch_bounds__(256) mmq_expand_kernel(const TcArgs a, __half*
     }
 }
 
-static int launch_wide(const TcArgs& a, const __half* xq, int Kp, void* wide, cudaStream_t st) {
-    __half* wq = reinterpret_cast<__half*>(wide);
-    const long long all = (long long)a.M + a.M2, most = (long long)(MW_WEIGHT_BYTES / ((size_t)Kp * sizeof(__half))) & ~255ll;
+// AHEAD (a prompt's chunk, two buffers by turns: 512 tokens of 8 layers 2399 -> 2131 us, 3001 tokens 9491 -> 9062): beside the product in front, whose CTAs leave room for three of these per SM.  Weights do not depend on it, and what read `out` before is
+// over (see launch_mmq_expand); the last CTA stays until the kernel in front is done, so that what follows this grid follows that one too.
+template <int TYPE, bool AHEAD>
+__global__ void __launch_bounds__(256) mmq_expand_kernel(const TcArgs a, __half* out, int r0, int rows, int Kp) {
+    if (!AHEAD) pdl_wait();
+    pdl_launch();
+    mw_expand<TYPE>(a, out, r0, rows, Kp);
+    if (AHEAD && blockIdx.x == gridDim.x - 1) pdl_wait();
+}
+
+static int mw_width(int type, int K) { return K + (type == T_Q4K ? (2 * (K / 32) + TC_K - 1) / TC_K * TC_K : 0); }
+void mmq_pieces(std::vector<MmqPiece>& out, const void* W1, const void* W2, int type, int M1, int M2, int K) {
+    const long long all = (long long)M1 + M2, most = (long long)(MW_WEIGHT_BYTES / ((size_t)mw_width(type, K) * sizeof(__half))) & ~255ll;
     const long long pieces = (all + most - 1) / most, step = ((all + pieces - 1) / pieces + 255) & ~255ll;
-    for (long long r0 = 0; r0 < all; r0 += step) {
-        const int rows = (int)(all - r0 < step ? all - r0 : step);
-        const long long n = (long long)rows * (a.type == T_Q4K ? a.K / 16 + a.n_min * 8 : a.K / 32);
-        if (a.type == T_Q4K) JB_CUDA(launch_k(mmq_expand_kernel<T_Q4K>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, pdl_enabled(), a, wq, (int)r0, rows, Kp));
-        else                 JB_CUDA(launch_k(mmq_expand_kernel<T_Q6K>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, pdl_enabled(), a, wq, (int)r0, rows, Kp));
-        count_launch();
-        DenseGemm g;
-        g.kind = EK_F16; g.W = wq; g.M = rows; g.K = g.ldw = g.ldx = Kp; g.N = a.N; g.x = xq;
-        g.part = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(wide) + MW_WEIGHT_BYTES); g.part_floats = gemm_pair_part_floats();
-        g.nseg = 0;
-        if (r0 < a.M) g.seg[g.nseg++] = OutSeg{a.y + r0, a.M, (int)(a.M - r0 < rows ? a.M - r0 : rows), 0, 0};
-        if (r0 + rows > a.M) g.seg[g.nseg++] = OutSeg{a.y2 + (r0 > a.M ? r0 - a.M : 0), a.M2, (int)(r0 > a.M ? rows : r0 + rows - a.M), 0, 0};
-        const int rc = launch_gemm_pair(g, st);
+    for (long long r0 = 0; r0 < all; r0 += step) out.push_back(MmqPiece{W1, W2, type, M1, M2, K, (int)r0, (int)(all - r0 < step ? all - r0 : step)});
+}
+// ahead: the launch in front on this stream lets its dependents start only after its own wait for what came before it (gemm_pair.cu and
+// attention_tc.cu do), and the product that read `wq` last lies before that.
+int launch_mmq_expand(const MmqPiece& p, void* wq, bool ahead, cudaStream_t st) {
+    TcArgs a = {};
+    a.W = (const uint8_t*)p.W; a.W2 = (const uint8_t*)p.W2; a.type = p.type; a.M = p.M; a.M2 = p.M2; a.K = p.K;
+    const int Kp = mw_width(p.type, p.K);
+    a.n_min = (Kp - p.K) / TC_K;
+    const long long n = (long long)p.rows * (p.type == T_Q4K ? p.K / 16 + a.n_min * 8 : p.K / 32);
+    auto kern = p.type == T_Q4K ? (ahead ? mmq_expand_kernel<T_Q4K, true> : mmq_expand_kernel<T_Q4K, false>) : ahead ? mmq_expand_kernel<T_Q6K, true> : mmq_expand_kernel<T_Q6K, false>;
+    JB_CUDA(launch_k(kern, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, pdl_enabled(), a, (__half*)wq, p.r0, p.rows, Kp));
+    count_launch();
+    return JB_OK;
+}
+int launch_mmq_piece(const MmqPiece& p, const void* wq, const __half* xq, __half* y1, __half* y2, int N, float* part, cudaStream_t st, const std::function<int()>& behind) {
+    DenseGemm g;
+    g.kind = EK_F16; g.W = wq; g.M = p.rows; g.K = g.ldw = g.ldx = mw_width(p.type, p.K); g.N = N; g.x = xq;
+    g.part = part; g.part_floats = gemm_pair_part_floats();
+    g.nseg = 0;
+    const int r0 = p.r0, rows = p.rows;
+    if (r0 < p.M) g.seg[g.nseg++] = OutSeg{y1 + r0, p.M, p.M - r0 < rows ? p.M - r0 : rows, 0, 0};
+    if (r0 + rows > p.M) g.seg[g.nseg++] = OutSeg{y2 + (r0 > p.M ? r0 - p.M : 0), p.M2, r0 > p.M ? rows : r0 + rows - p.M, 0, 0};
+    return launch_gemm_pair(g, st, behind);
+}
+static int launch_wide(const TcArgs& a, const __half* xq, void* wide, cudaStream_t st) {
+    std::vector<MmqPiece> pieces;
+    mmq_pieces(pieces, a.W, a.W2, a.type, a.M, a.M2, a.K);
+    for (const MmqPiece& p : pieces) {
+        int rc = launch_mmq_expand(p, wide, false, st);
+        if (!rc) rc = launch_mmq_piece(p, wide, xq, a.y, a.y2, a.N, reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(wide) + MW_WEIGHT_BYTES), st);
         if (rc) return rc;
     }
     return JB_OK;
@@ -692,7 +718,7 @@ int launch_mmq_tc_pair(__half* y, __half* y2, const void* W, const void* W2, int
         work.many = op;
         work.few = MmqOperand();
     }
-    if (wide) return launch_wide(a, ready ? ready : xq, Kp, wide, st);
+    if (wide) return launch_wide(a, ready ? ready : xq, wide, st);
     const int n_work = a.n_full + (tiles - a.n_full) * a.ksplit;
     const dim3 grid(n_work < c->sm_count ? n_work : c->sm_count);
     if (ti == 0) JB_CUDA(launch_k(mmq_tc_kernel<T_Q4K>, grid, dim3(TC_THREADS), TC_SMEM, st, pdl_enabled(), map, a, n_tile));
