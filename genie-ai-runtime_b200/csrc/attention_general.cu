@@ -104,6 +104,10 @@ template <typename QT>
 static cudaError_t ag_launch(const AttnArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
     if constexpr (!std::is_same<QT, __half>::value)
         if (a.hd > 32 * AG_MAXD) return launch_k(attn_general_kernel<QT, AG_WIDE>, grid, dim3(AG_THREADS), smem, st, pdl_enabled(), a);
+    // head dimensions per lane: what the keys and values have, so that registers hold several keys
+    const int most = a.hd > a.vhd ? a.hd : a.vhd;
+    if (most <= 128) return launch_k(attn_general_kernel<QT, 4>, grid, dim3(AG_THREADS), smem, st, pdl_enabled(), a);
+    if (most <= 256) return launch_k(attn_general_kernel<QT, 8>, grid, dim3(AG_THREADS), smem, st, pdl_enabled(), a);
     return launch_k(attn_general_kernel<QT, AG_MAXD>, grid, dim3(AG_THREADS), smem, st, pdl_enabled(), a);
 }
 // merges records [rows][heads][slices] into out (rows of ldo elements)

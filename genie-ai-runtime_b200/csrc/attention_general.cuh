@@ -59,22 +59,53 @@ __device__ __forceinline__ void ag_slice_typed(const QT* q, const AgCache& c, in
     for (int i = 0; i < MAXD; ++i) { const int d = lane + 32 * i; qr[i] = d < hd ? to_f32(q[d]) : 0.f; acc[i] = 0.f; }
     float m = -FLT_MAX, l = 0.f;
     const int first = c.window > 0 ? max(kv0, seq - c.window) : kv0;      // keys before the window contribute nothing
-    for (int p = first + warp; p < kv1; p += AG_WARPS) {
-        float kd[MAXD], dot = 0.f;
-        const char* kr = reinterpret_cast<const char*>(c.k) + (size_t)p * krow + koff;
-        const float ksc = scaled && c.ks ? c.ks[(size_t)p * c.n_kv + kvh] : 1.0f;
+    // Small heads: the rows of BATCH keys are requested together and the keys taken in the same order as one by one (a key at a time, each with its
+    // trip to memory, 134 FP32 keys of 128 took 41 us; so 8).
+    constexpr int BATCH = MAXD <= 4 ? 8 : MAXD <= 8 ? 4 : 1;
+    for (int p0 = first + warp; p0 < kv1; p0 += BATCH * AG_WARPS) {
+        float kd[BATCH][MAXD], vd[BATCH][MAXD], s[BATCH];
         #pragma unroll
-        for (int i = 0; i < MAXD; ++i) { const int d = lane + 32 * i; kd[i] = d < hd ? ag_elem<CT>(kr, d, ksc) : 0.f; }
+        for (int j = 0; j < BATCH; ++j) {
+            const int p = min(p0 + j * AG_WARPS, kv1 - 1);
+            const char* kr = reinterpret_cast<const char*>(c.k) + (size_t)p * krow + koff;
+            const float ksc = scaled && c.ks ? c.ks[(size_t)p * c.n_kv + kvh] : 1.0f;
+            #pragma unroll
+            for (int i = 0; i < MAXD; ++i) { const int d = lane + 32 * i; kd[j][i] = d < hd ? ag_elem<CT>(kr, d, ksc) : 0.f; }
+        }
+        if (BATCH > 1) {
+            #pragma unroll
+            for (int j = 0; j < BATCH; ++j) {
+                const int p = min(p0 + j * AG_WARPS, kv1 - 1);
+                const char* vr = reinterpret_cast<const char*>(c.v) + (size_t)p * vrow + voff;
+                const float vsc = scaled && c.vs ? c.vs[(size_t)p * c.n_kv + kvh] : 1.0f;
+                #pragma unroll
+                for (int i = 0; i < MAXD; ++i) { const int d = lane + 32 * i; vd[j][i] = d < vhd ? ag_elem<CT>(vr, d, vsc) : 0.f; }
+            }
+        }
         #pragma unroll
-        for (int i = 0; i < MAXD; ++i) dot += qr[i] * kd[i];
-        const float s = warp_sum(dot) * scale;
-        const float m_new = fmaxf(m, s), corr = expf(m - m_new), pw = expf(s - m_new);
-        m = m_new;
-        l = l * corr + pw;
-        const char* vr = reinterpret_cast<const char*>(c.v) + (size_t)p * vrow + voff;
-        const float vsc = scaled && c.vs ? c.vs[(size_t)p * c.n_kv + kvh] : 1.0f;
+        for (int j = 0; j < BATCH; ++j) {
+            float dot = 0.f;
+            #pragma unroll
+            for (int i = 0; i < MAXD; ++i) dot += qr[i] * kd[j][i];
+            s[j] = warp_sum(dot) * scale;
+        }
         #pragma unroll
-        for (int i = 0; i < MAXD; ++i) { const int d = lane + 32 * i; if (d < vhd) acc[i] = acc[i] * corr + pw * ag_elem<CT>(vr, d, vsc); }
+        for (int j = 0; j < BATCH; ++j) {
+            const int p = p0 + j * AG_WARPS;
+            if (p >= kv1) break;
+            const float m_new = fmaxf(m, s[j]), corr = expf(m - m_new), pw = expf(s[j] - m_new);
+            m = m_new;
+            l = l * corr + pw;
+            if (BATCH > 1) {
+                #pragma unroll
+                for (int i = 0; i < MAXD; ++i) { const int d = lane + 32 * i; if (d < vhd) acc[i] = acc[i] * corr + pw * vd[j][i]; }
+            } else {
+                const char* vr = reinterpret_cast<const char*>(c.v) + (size_t)p * vrow + voff;
+                const float vsc = scaled && c.vs ? c.vs[(size_t)p * c.n_kv + kvh] : 1.0f;
+                #pragma unroll
+                for (int i = 0; i < MAXD; ++i) { const int d = lane + 32 * i; if (d < vhd) acc[i] = acc[i] * corr + pw * ag_elem<CT>(vr, d, vsc); }
+            }
+        }
     }
     // merge the warps' states
     float* sm_m = sm; float* sm_l = sm + AG_WARPS; float* sm_o = sm + 2 * AG_WARPS;     // [warp][vhd]
