@@ -1,106 +1,152 @@
 // dense_simt.cu — dense products over many tokens on the CUDA cores, in true fp32 (FFMA, no reduced-precision matrix mode): the 32-bit
-// path of layer-list models.  64 (rows) x 32 (tokens) output tiles, 4 x 2 per thread, K tiles of 32; groups (experts) on grid.z.
+// path of layer-list models; groups (experts) on grid.z.
 //
-// At the sizes of prompts in this format a launch has few CTAs, so a tile's chain of K tiles sets the time: the next K tile is
-// requested as 16-byte loads before the present one is multiplied and stored into the other half of shared memory after it, one
-// barrier per K tile.  A value is summed over k in ascending order.
+// A launch has few tokens per weight matrix here (an expert of a 130-token prompt: 16), so it is bound by the weights' way from memory and by the
+// tokens that pad a tile.  A WARP holds a tile of 64 rows x 16 tokens, 8 x 4 values per lane, and the warps of a CTA take
+// four k of a K tile in turn; a CTA is 16, 32 or 64 tokens wide (the other warps' tiles) and its warps' sums meet in shared memory in a fixed order.  Operands come by
+// cp.async in four stages, K contiguous as in memory: a lane reads four k of a row at a time, 12 (gate and up: 20) 16-byte reads of shared memory,
+// free of conflicts, for 128 (256) multiply-adds.
+//
+// 130 tokens, width 1024, 32 experts of 768, top 4, us before (64 x 32 tiles, 4 x 2 values a thread, tiles transposed through registers) / here:
+// gate and up 169 / 89 (their weights at the rate of memory: 31), down 108 / 57; 3072 x 1024 and 1024 x 2048 67 and 71 / 47 and 30.  The reads of
+// shared memory, four passes for each of 16 bytes a lane, now take 1.5 times the multiply-adds.  Error against 64 bits of the whole request 5.5e-7 / 3.4e-7.
 #include "dense.cuh"
 
 namespace jb {
 
-constexpr int DS_M = 64, DS_N = 32, DS_K = 32, DS_THREADS = 256;
+constexpr int DS_M = 64, DS_T = 16, DS_WARPS = 8, DS_THREADS = DS_WARPS * 32;
+// K tile and stages: two CTAs per SM; rows K + 4 words apart, so that eight rows' reads lie in different banks
+template <bool GLU> constexpr int DS_K = GLU ? 32 : 64;
+template <bool GLU> constexpr int DS_STAGES = GLU ? 4 : 3;
 
-struct DsTile { float w[DS_K][DS_M + 4], x[DS_K][DS_N + 4]; };
-template <bool GLU> struct DsUp { float u[DS_K][DS_M + 4]; };
-template <> struct DsUp<false> {};
-
-// four elements at k of a row, zero beyond K; vec: 16-byte aligned rows
-__device__ __forceinline__ float4 ds_load(const float* row, bool in, int k, int K, bool vec) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (!in || k >= K) return v;
-    if (vec && k + 4 <= K) return load4(row + k);
-    v.x = row[k];
-    if (k + 1 < K) v.y = row[k + 1];
-    if (k + 2 < K) v.z = row[k + 2];
-    if (k + 3 < K) v.w = row[k + 3];
-    return v;
+template <bool GLU, int WT> constexpr int ds_stage() { return (DS_M * (GLU ? 2 : 1) + DS_T * WT) * (DS_K<GLU> + 4); }      // floats
+template <bool GLU, int WT> constexpr size_t ds_smem() {
+    const size_t stages = (size_t)DS_STAGES<GLU> * ds_stage<GLU, WT>(), sums = (size_t)DS_WARPS * DS_M * DS_T * (GLU ? 2 : 1);
+    return (stages > sums ? stages : sums) * sizeof(float);
 }
-template <int LD>
-__device__ __forceinline__ void ds_put(float (*t)[LD], int k, int j, float4 v) { t[k][j] = v.x; t[k + 1][j] = v.y; t[k + 2][j] = v.z; t[k + 3][j] = v.w; }
 
-template <bool GLU>
-__global__ void __launch_bounds__(DS_THREADS) dense_simt_kernel(const __grid_constant__ DenseGemm a, bool vec) {
+// WT: 16-token tiles of a CTA; its 8 / WT warps on a tile share K
+template <bool GLU, int WT>
+__global__ void __launch_bounds__(DS_THREADS, 2) dense_simt_kernel(const __grid_constant__ DenseGemm a, bool vec) {
     pdl_wait();
-    __shared__ __align__(16) DsTile tile[2];
-    __shared__ __align__(16) DsUp<GLU> up[2];
+    pdl_launch();
+    extern __shared__ __align__(16) float ds_sm[];
+    constexpr int KG = DS_WARPS / WT, ROWS = DS_M * (GLU ? 2 : 1) + DS_T * WT, STAGE = ds_stage<GLU, WT>(), KT = DS_K<GLU>, LD = KT + 4, STAGES = DS_STAGES<GLU>, QUADS = KT / 4, PER = DS_THREADS / QUADS;
     const int grp = blockIdx.z, t_lo = a.off ? a.off[grp] : 0, t_hi = a.off ? a.off[grp + 1] : a.N;
     const int r0 = blockIdx.x * DS_M, ldw = a.ldw > 0 ? a.ldw : pad8(a.K), ldx = a.ldx > 0 ? a.ldx : pad8(a.K);
     const float* W = reinterpret_cast<const float*>(a.W) + (size_t)grp * a.M * ldw;
     const float* V = GLU ? reinterpret_cast<const float*>(a.W_up) + (size_t)grp * a.M * ldw : nullptr;
     const float* x = reinterpret_cast<const float*>(a.x) + (size_t)grp * a.x_step;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;                      // thread: rows 4 tx .., tokens 2 ty ..
-    const int lk = 4 * (threadIdx.x & 7), lj = threadIdx.x >> 3;                 // loads: row (or token) lj and row lj + 32, elements lk ..
-    const bool in0 = r0 + lj < a.M, in1 = r0 + lj + 32 < a.M;
-    const float *w0 = W + (size_t)(r0 + lj) * ldw, *w1 = w0 + (size_t)32 * ldw, *v0 = GLU ? V + (size_t)(r0 + lj) * ldw : nullptr, *v1 = GLU ? v0 + (size_t)32 * ldw : nullptr;
-    for (int t0 = t_lo + blockIdx.y * DS_N; t0 < t_hi; t0 += gridDim.y * DS_N) {
-    const bool inx = t0 + lj < t_hi;
-    const float* xr = x + (size_t)(t0 + lj) * ldx;
-    float4 f[3], h[2];
-    auto fetch = [&](int k) {
-        f[0] = ds_load(w0, in0, k + lk, a.K, vec); f[1] = ds_load(w1, in1, k + lk, a.K, vec); f[2] = ds_load(xr, inx, k + lk, a.K, vec);
-        if (GLU) { h[0] = ds_load(v0, in0, k + lk, a.K, vec); h[1] = ds_load(v1, in1, k + lk, a.K, vec); }
-    };
-    auto put = [&](int b) {
-        ds_put(tile[b].w, lk, lj, f[0]); ds_put(tile[b].w, lk, lj + 32, f[1]); ds_put(tile[b].x, lk, lj, f[2]);
-        if constexpr (GLU) { ds_put(up[b].u, lk, lj, h[0]); ds_put(up[b].u, lk, lj + 32, h[1]); }
-    };
-    float acc[4][2] = {}, acu[4][2] = {};
-    fetch(0);
-    put(0);
-    __syncthreads();
-    for (int k0 = 0, b = 0; k0 < a.K; k0 += DS_K, b ^= 1) {
-        const bool more = k0 + DS_K < a.K;
-        if (more) fetch(k0 + DS_K);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tx = lane & 7, ty = lane >> 3, wt = warp % WT, kg = warp / WT;
+    const int k_tiles = (a.K + KT - 1) / KT;
+    for (int t0 = t_lo + blockIdx.y * DS_T * WT; t0 < t_hi; t0 += gridDim.y * DS_T * WT) {
+        // QUADS pieces of 16 bytes a row: thread's piece of every PER-th row
+        auto fetch = [&](int kt) {
+            float* st = ds_sm + (kt % STAGES) * STAGE;
+            const int k = kt * KT + 4 * (threadIdx.x % QUADS);
+            #pragma unroll
+            for (int j = 0; j < ROWS; j += PER) {
+                const int r = j + threadIdx.x / QUADS;
+                if (r >= ROWS) break;
+                const float* src; bool in;
+                if (j < DS_M) { src = W + (size_t)(r0 + r) * ldw; in = r0 + r < a.M; }
+                else if (GLU && j < 2 * DS_M) { src = V + (size_t)(r0 + r - DS_M) * ldw; in = r0 + r - DS_M < a.M; }
+                else { const int t = t0 + r - DS_M * (GLU ? 2 : 1); src = x + (size_t)t * ldx; in = t < t_hi; }
+                float* dst = st + r * LD + 4 * (threadIdx.x % QUADS);
+                const int left = in ? max(0, min(4, a.K - k)) : 0;               // elements of the piece; the rest is zero
+                if (vec) {
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(left ? src + k : x), "r"(4 * left) : "memory");
+                } else {
+                    #pragma unroll
+                    for (int e = 0; e < 4; ++e) dst[e] = e < left ? src[k + e] : 0.f;
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        float acc[8][4] = {}, acu[GLU ? 8 : 1][4] = {};
         #pragma unroll
-        for (int k = 0; k < DS_K; ++k) {
-            const float4 w = load4(&tile[b].w[k][4 * tx]);
-            const float2 v = *reinterpret_cast<const float2*>(&tile[b].x[k][2 * ty]);
-            acc[0][0] = fmaf(w.x, v.x, acc[0][0]); acc[0][1] = fmaf(w.x, v.y, acc[0][1]); acc[1][0] = fmaf(w.y, v.x, acc[1][0]); acc[1][1] = fmaf(w.y, v.y, acc[1][1]);
-            acc[2][0] = fmaf(w.z, v.x, acc[2][0]); acc[2][1] = fmaf(w.z, v.y, acc[2][1]); acc[3][0] = fmaf(w.w, v.x, acc[3][0]); acc[3][1] = fmaf(w.w, v.y, acc[3][1]);
-            if constexpr (GLU) {
-                const float4 u = load4(&up[b].u[k][4 * tx]);
-                acu[0][0] = fmaf(u.x, v.x, acu[0][0]); acu[0][1] = fmaf(u.x, v.y, acu[0][1]); acu[1][0] = fmaf(u.y, v.x, acu[1][0]); acu[1][1] = fmaf(u.y, v.y, acu[1][1]);
-                acu[2][0] = fmaf(u.z, v.x, acu[2][0]); acu[2][1] = fmaf(u.z, v.y, acu[2][1]); acu[3][0] = fmaf(u.w, v.x, acu[3][0]); acu[3][1] = fmaf(u.w, v.y, acu[3][1]);
+        for (int s = 0; s < STAGES - 1; ++s) { if (s < k_tiles) fetch(s); else asm volatile("cp.async.commit_group;" ::: "memory"); }
+        for (int kt = 0; kt < k_tiles; ++kt) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+            __syncthreads();                             // the tile has landed, and the one before it is read
+            if (kt + STAGES - 1 < k_tiles) fetch(kt + STAGES - 1); else asm volatile("cp.async.commit_group;" ::: "memory");
+            const float* st = ds_sm + (kt % STAGES) * STAGE;
+            #pragma unroll 1
+            for (int q = kg; q < QUADS; q += KG) {
+                float4 xv[4];
+                #pragma unroll
+                for (int j = 0; j < 4; ++j) xv[j] = load4(st + (DS_M * (GLU ? 2 : 1) + DS_T * wt + ty + 4 * j) * LD + 4 * q);
+                #pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float4 w = load4(st + (tx + 8 * i) * LD + 4 * q);
+                    #pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(w.w, xv[j].w, fmaf(w.z, xv[j].z, fmaf(w.y, xv[j].y, fmaf(w.x, xv[j].x, acc[i][j]))));
+                    if constexpr (GLU) {
+                        const float4 u = load4(st + (DS_M + tx + 8 * i) * LD + 4 * q);
+                        #pragma unroll
+                        for (int j = 0; j < 4; ++j) acu[i][j] = fmaf(u.w, xv[j].w, fmaf(u.z, xv[j].z, fmaf(u.y, xv[j].y, fmaf(u.x, xv[j].x, acu[i][j]))));
+                    }
+                }
             }
         }
-        if (more) put(b ^ 1);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-    }
-    #pragma unroll
-    for (int j = 0; j < 2; ++j)
+        // [kg][wt][token 16][row 64] (then the same of `up`): the sums of a value's K groups, in their order
+        constexpr int PART = DS_WARPS * DS_T * DS_M;
+        float* mine = ds_sm + (kg * WT + wt) * DS_T * DS_M;
         #pragma unroll
-        for (int i = 0; i < 4; i += 2) {
-            const int r = r0 + 4 * tx + i, t = t0 + 2 * ty + j;
-            if (r < a.M && t < t_hi)
-                store_rows2<float>(a.seg, a.nseg, a.softcap, nullptr, t, a.start + t, r, a.M, GLU ? silu_f(acc[i][j]) * acu[i][j] : acc[i][j],
-                                   GLU ? silu_f(acc[i + 1][j]) * acu[i + 1][j] : acc[i + 1][j], (long long)grp * a.y_step);
+        for (int i = 0; i < 8; ++i)
+            #pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                mine[(ty + 4 * j) * DS_M + tx + 8 * i] = acc[i][j];
+                if constexpr (GLU) mine[PART + (ty + 4 * j) * DS_M + tx + 8 * i] = acu[i][j];
+            }
+        __syncthreads();
+        for (int e = threadIdx.x; e < WT * DS_T * DS_M / 2; e += DS_THREADS) {
+            const int r = 2 * (e % (DS_M / 2)), tl = e / (DS_M / 2), t = t0 + tl, at = tl * DS_M + r;
+            if (t >= t_hi || r0 + r >= a.M) continue;
+            float2 s = *reinterpret_cast<const float2*>(ds_sm + at), u = make_float2(0.f, 0.f);
+            if (GLU) u = *reinterpret_cast<const float2*>(ds_sm + PART + at);
+            #pragma unroll
+            for (int g = 1; g < KG; ++g) {
+                const float2 v = *reinterpret_cast<const float2*>(ds_sm + g * WT * DS_T * DS_M + at);
+                s.x += v.x; s.y += v.y;
+                if (GLU) { const float2 w = *reinterpret_cast<const float2*>(ds_sm + PART + g * WT * DS_T * DS_M + at); u.x += w.x; u.y += w.y; }
+            }
+            store_rows2<float>(a.seg, a.nseg, a.softcap, nullptr, t, a.start + t, r0 + r, a.M, GLU ? silu_f(s.x) * u.x : s.x, GLU ? silu_f(s.y) * u.y : s.y, (long long)grp * a.y_step);
         }
+        __syncthreads();                                 // before the next tokens' tiles take the place of the sums
     }
 }
 
+template <bool GLU, int WT>
+static int ds_go(const DenseGemm& a, bool vec, cudaStream_t st) {
+    static bool set[16] = {};
+    DeviceCtx* c = ctx();
+    if (!c) return JB_ERR_CUDA;
+    if (!set[c->device]) { JB_CUDA(cudaFuncSetAttribute(dense_simt_kernel<GLU, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ds_smem<GLU, WT>())); set[c->device] = true; }
+    // an expert's tokens are known on the device alone: a few CTAs for each walk its tiles (as many as all tokens would need: 12672 CTAs for 600 tiles)
+    const int all = (a.N + DS_T * WT - 1) / (DS_T * WT), few = a.off ? 2 * ((a.N / a.n_groups + DS_T * WT - 1) / (DS_T * WT)) + 2 : all, tiles = all < few ? all : few;
+    JB_CUDA(launch_k(dense_simt_kernel<GLU, WT>, dim3((a.M + DS_M - 1) / DS_M, tiles < 65535 ? tiles : 65535, a.n_groups), dim3(DS_THREADS), ds_smem<GLU, WT>(), st, pdl_enabled(), a, vec));
+    count_launch();
+    return JB_OK;
+}
 int launch_dense_gemm_simt(const DenseGemm& a, cudaStream_t st) {
     if (a.N <= 0 || a.M <= 0) return JB_OK;
     if (a.kind != EK_F32) return set_error(JB_ERR_TYPE, "dense fp32 gemm: element kind %d", a.kind);
     if (!a.W || !a.x || (a.swiglu && !a.W_up) || (a.n_groups > 1 && !a.off && !a.x_step)) return set_error(JB_ERR_PTR, "dense fp32 gemm: null pointer");
-    const int tiles = (a.N + DS_N - 1) / DS_N;
-    const dim3 grid((a.M + DS_M - 1) / DS_M, tiles < 65535 ? tiles : 65535, a.n_groups);
     const int ldw = a.ldw > 0 ? a.ldw : pad8(a.K), ldx = a.ldx > 0 ? a.ldx : pad8(a.K);
     const bool vec = !(((uintptr_t)a.W | (uintptr_t)a.x | (a.swiglu ? (uintptr_t)a.W_up : 0)) & 15) && ldw % 4 == 0 && ldx % 4 == 0 && a.x_step % 4 == 0;
     if ((a.N + 63) / 64 > 65535) return set_error(JB_ERR_LIMIT, "dense fp32 gemm: %d tokens", a.N);
-    if (a.swiglu) JB_CUDA(launch_k(dense_simt_kernel<true>, grid, dim3(DS_THREADS), 0, st, pdl_enabled(), a, vec));
-    else          JB_CUDA(launch_k(dense_simt_kernel<false>, grid, dim3(DS_THREADS), 0, st, pdl_enabled(), a, vec));
-    count_launch();
-    return JB_OK;
+    DeviceCtx* c = ctx();
+    if (!c) return JB_ERR_CUDA;
+    // Wider tiles read the weights less often, narrower ones make more CTAs and pad less: as wide as still leaves two CTAs per SM, and no
+    // wider than a group's tokens are on average.
+    const long long per_group = a.off ? a.N / a.n_groups : a.N, row_tiles = (long long)((a.M + DS_M - 1) / DS_M) * a.n_groups;
+    int wt = 1;
+    while (wt < 4 && per_group >= 2 * wt * DS_T && row_tiles * ((per_group + 2 * wt * DS_T - 1) / (2 * wt * DS_T)) >= 2 * c->sm_count) wt *= 2;
+    if (a.swiglu) return wt == 1 ? ds_go<true, 1>(a, vec, st) : wt == 2 ? ds_go<true, 2>(a, vec, st) : ds_go<true, 4>(a, vec, st);
+    return wt == 1 ? ds_go<false, 1>(a, vec, st) : wt == 2 ? ds_go<false, 2>(a, vec, st) : ds_go<false, 4>(a, vec, st);
 }
 // One token (the logits after a prompt) is a product of the decode family: 151936 x 2560 in bf16 take 122 us there, the weights at the
 // rate of memory, and 145 us in tiles of 16 tokens; the smallest tile of this file is 32 tokens wide.
