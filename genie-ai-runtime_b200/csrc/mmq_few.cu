@@ -24,7 +24,7 @@
 // 128 x 256 tiles of mmq_tc.cu): gate and up, Q4_K 9728 x 2560 twice, 12.8 / 16.9 / 22.4 (27.2 / 35.4 / -); W_down, Q6_K 2560 x 9728,
 // 11.2 / 13.4 / 18.3 (16.8 / 27.1 / -); Wo, Q4_K 2560 x 4096, 6.7 / 8.9 / 12.4 (7.5 / 20.3 / -); logits, Q6_K 151936 x 2560, 91 / 99 / 123
 // (125 / 280 / -), of which 62 / 75 / 103 are left without the arithmetic on the codes (ALU 63 % and issue slots 73 % busy), and memory needs 49.
-// A prompt chunk of 8 layers: 2 / 33 / 64 / 128 tokens 686 / 749 / 822 / 1083 us (953 / 1311 / 1350 / 1568); above 128 tokens an accumulator and two
+// A prompt chunk of 8 layers: 33 tokens 696 us (1283); above 128 tokens an accumulator and two
 // super-blocks of weights no longer fit into tensor memory.
 #include "mmq_few.cuh"
 #include "mmq.cuh"
@@ -474,34 +474,41 @@ __global__ void __launch_bounds__(256) mf_edge_kernel(const __grid_constant__ Mf
 // ── the kernels between the products ──────────────────────────────────────
 // What they read: sums of rows 4 lane .. 4 lane + 3 of a tile, in order of K.
 struct MfSums { const float* part; MfSeg seg[MF_MAX_SEG]; int nb, N, rows; };
-template <int BATCH>
-__device__ __forceinline__ void mf_sum4(float (&v)[4], const MfSums& a, const MfSeg& s, int tile, int tok, int lane) {
-    const int first = mf_owner(s, tile * a.nb), count = mf_owner(s, (tile + 1) * a.nb - 1) - first + 1;
-    const float* p = a.part + (size_t)tok * a.rows + s.m0 + tile * MF_ROWS;
-    const size_t slot = (size_t)a.N * a.rows;
-    // every sum of a batch is requested before the first is added: one trip to L2 for all (added as they came, nine sums of W_down took 13 us)
-    int at[4];
-    const int per = MF_ROWS / s.perm, shift = __ffs(s.perm) - 1;
+// What a kernel can know before the product in front is done (where its sums lie, angles, weights of a norm) it forms ahead of its wait: rotation and
+// SwiGLU kernels of eight streams 6.1 and 5.1 -> 3.3 us after their product's end.
+struct MfPlace { const float* p; int count, perm; size_t slot; int at[4]; };
+__device__ __forceinline__ MfPlace mf_place(const MfSums& a, const MfSeg& s, int tile, int tok, int lane) {
+    const int first = mf_owner(s, tile * a.nb), per = MF_ROWS / s.perm, shift = __ffs(s.perm) - 1;
+    MfPlace r;
+    r.count = mf_owner(s, (tile + 1) * a.nb - 1) - first + 1;
+    r.p = a.part + (size_t)tok * a.rows + s.m0 + tile * MF_ROWS;
+    r.slot = (size_t)a.N * a.rows;
+    r.perm = s.perm;
     #pragma unroll
-    for (int e = 0; e < 4; ++e) at[e] = ((4 * lane + e) & (s.perm - 1)) * per + ((4 * lane + e) >> shift);
+    for (int e = 0; e < 4; ++e) r.at[e] = s.perm == 1 ? 4 * lane + e : ((4 * lane + e) & (s.perm - 1)) * per + ((4 * lane + e) >> shift);
+    return r;
+}
+template <int BATCH>
+__device__ __forceinline__ void mf_sum4(float (&v)[4], const MfPlace& s) {
+    // every sum of a batch is requested before the first is added: one trip to L2 for all (added as they came, nine sums of W_down took 13 us)
     v[0] = v[1] = v[2] = v[3] = 0.f;
-    for (int c0 = 0; c0 < count; c0 += BATCH) {
+    for (int c0 = 0; c0 < s.count; c0 += BATCH) {
         float w[BATCH][4];
         #pragma unroll
         for (int c = 0; c < BATCH; ++c) {
-            const float* q = p + (c0 + c) * slot;
-            if (c0 + c >= count) w[c][0] = w[c][1] = w[c][2] = w[c][3] = 0.f;
+            const float* q = s.p + (c0 + c) * s.slot;
+            if (c0 + c >= s.count) w[c][0] = w[c][1] = w[c][2] = w[c][3] = 0.f;
             else if (s.perm == 1) {
-                const float4 x = *reinterpret_cast<const float4*>(q + 4 * lane);
+                const float4 x = *reinterpret_cast<const float4*>(q + s.at[0]);
                 w[c][0] = x.x; w[c][1] = x.y; w[c][2] = x.z; w[c][3] = x.w;
             } else {
                 #pragma unroll
-                for (int e = 0; e < 4; ++e) w[c][e] = q[at[e]];
+                for (int e = 0; e < 4; ++e) w[c][e] = q[s.at[e]];
             }
         }
         #pragma unroll
         for (int c = 0; c < BATCH; ++c)
-            if (c0 + c < count) { v[0] += w[c][0]; v[1] += w[c][1]; v[2] += w[c][2]; v[3] += w[c][3]; }
+            if (c0 + c < s.count) { v[0] += w[c][0]; v[1] += w[c][1]; v[2] += w[c][2]; v[3] += w[c][3]; }
     }
 }
 struct MfQuant { __half* x4; __half* x6; int N, NP; };
@@ -562,11 +569,17 @@ __device__ __forceinline__ float mf_half(float v) { return __half2float(__float2
 // One CTA per token, a warp per 128 elements (MF_NORM_TILES per warp at most).  Bound by its launch and one trip to L2: the sums, x and
 // the weights are requested together.
 constexpr int MF_NORM_TILES = 4;
-template <int TILES>
-__global__ void __launch_bounds__(1024) mf_norm_kernel(const __grid_constant__ MfSums sums, const __half* x, __half* x_out, const float* w, float eps, int H, MfQuant q) {
+template <int TILES, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) mf_norm_kernel(const __grid_constant__ MfSums sums, const __half* x, __half* x_out, const float* w, float eps, int H, MfQuant q) {
     __shared__ float red[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, tok = blockIdx.x, tiles = H / MF_ROWS;
     pdl_launch();
+    MfPlace at = {};
+    float4 wn = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (TILES == 1) {                                     // a warp per tile
+        if (sums.part) at = mf_place(sums, sums.seg[0], warp, tok, lane);
+        if (w) wn = *reinterpret_cast<const float4*>(w + warp * MF_ROWS + 4 * lane);
+    }
     pdl_wait();
     float v[TILES][4], ss = 0.f;
     #pragma unroll
@@ -576,7 +589,8 @@ __global__ void __launch_bounds__(1024) mf_norm_kernel(const __grid_constant__ M
         mf_load4(v[i], x + (size_t)tok * H + tile * MF_ROWS + 4 * lane);
         if (sums.part) {
             float y[4];
-            mf_sum4<5>(y, sums, sums.seg[0], tile, tok, lane);
+            if (TILES > 1) at = mf_place(sums, sums.seg[0], tile, tok, lane);
+            mf_sum4<THREADS < 1024 ? 5 : 3>(y, at);
             #pragma unroll
             for (int e = 0; e < 4; ++e) v[i][e] = mf_half(__fadd_rn(v[i][e], mf_half(y[e])));
             mf_store4(x_out + (size_t)tok * H + tile * MF_ROWS + 4 * lane, v[i]);
@@ -595,7 +609,7 @@ __global__ void __launch_bounds__(1024) mf_norm_kernel(const __grid_constant__ M
     for (int i = 0; i < TILES; ++i) {
         const int tile = warp + i * warps;
         if (tile >= tiles) break;
-        const float4 wn = *reinterpret_cast<const float4*>(w + tile * MF_ROWS + 4 * lane);
+        if (TILES > 1) wn = *reinterpret_cast<const float4*>(w + tile * MF_ROWS + 4 * lane);
         const float wv[4] = {wn.x, wn.y, wn.z, wn.w};
         #pragma unroll
         for (int e = 0; e < 4; ++e) v[i][e] = mf_half(__fmul_rn(__fmul_rn(v[i][e], rrms), wv[e]));
@@ -604,16 +618,24 @@ __global__ void __launch_bounds__(1024) mf_norm_kernel(const __grid_constant__ M
 }
 
 // A warp per head of 128 and token: the arithmetic of qkv_prep_kernel (elementwise.cu) on the fp16 results of the products.
-__global__ void __launch_bounds__(256) mf_prep_kernel(const __grid_constant__ MfSums sums, const __grid_constant__ MfPrep a, const __grid_constant__ RopeFreq fr) {
+__global__ void __launch_bounds__(256, 3) mf_prep_kernel(const __grid_constant__ MfSums sums, const __grid_constant__ MfPrep a, const __grid_constant__ RopeFreq fr) {
     const int lane = threadIdx.x & 31, head = blockIdx.x * 8 + (threadIdx.x >> 5), tok = blockIdx.y;
     pdl_launch();
-    pdl_wait();
-    if (head >= a.n_heads + 2 * a.n_kv) return;
+    if (head >= a.n_heads + 2 * a.n_kv) { pdl_wait(); return; }
     const bool is_q = head < a.n_heads, is_k = !is_q && head < a.n_heads + a.n_kv;
     const int hh = is_q ? head : is_k ? head - a.n_heads : head - a.n_heads - a.n_kv;
     const int pos = (a.d_pos ? *a.d_pos : a.pos) + tok * a.pos_step;
+    // Ahead of the wait for the product: the position, which was settled before the kernels of this step (the first of them starts no kernel early),
+    // its angles, and where the sums lie.
+    float c[4], s[4];
+    if (is_q || is_k) {
+        #pragma unroll
+        for (int e = 0; e < 4; ++e) sincosf(__fmul_rn((float)pos, fr.f[a.neox ? 4 * (lane & 15) + e : 2 * lane + e / 2]), &s[e], &c[e]);
+    }
+    const MfPlace at_ = mf_place(sums, sums.seg[is_q ? 0 : is_k ? 1 : 2], hh, tok, lane);
+    pdl_wait();
     float v[4];
-    mf_sum4<3>(v, sums, sums.seg[is_q ? 0 : is_k ? 1 : 2], hh, tok, lane);
+    mf_sum4<4>(v, at_);
     #pragma unroll
     for (int e = 0; e < 4; ++e) v[e] = mf_half(v[e]);
     if (is_q || is_k) {
@@ -630,18 +652,14 @@ __global__ void __launch_bounds__(256) mf_prep_kernel(const __grid_constant__ Mf
             #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float o = __shfl_xor_sync(0xFFFFFFFFu, v[e], 16);
-                float c, s;
-                sincosf(__fmul_rn((float)pos, fr.f[4 * (lane & 15) + e]), &s, &c);
-                v[e] = mf_half(lane < 16 ? __fsub_rn(__fmul_rn(v[e], c), __fmul_rn(o, s)) : __fadd_rn(__fmul_rn(o, s), __fmul_rn(v[e], c)));
+                v[e] = mf_half(lane < 16 ? __fsub_rn(__fmul_rn(v[e], c[e]), __fmul_rn(o, s[e])) : __fadd_rn(__fmul_rn(o, s[e]), __fmul_rn(v[e], c[e])));
             }
         } else {
             #pragma unroll
             for (int e = 0; e < 4; e += 2) {
-                float c, s;
-                sincosf(__fmul_rn((float)pos, fr.f[2 * lane + e / 2]), &s, &c);
                 const float v0 = v[e], v1 = v[e + 1];
-                v[e] = mf_half(__fsub_rn(__fmul_rn(v0, c), __fmul_rn(v1, s)));
-                v[e + 1] = mf_half(__fadd_rn(__fmul_rn(v0, s), __fmul_rn(v1, c)));
+                v[e] = mf_half(__fsub_rn(__fmul_rn(v0, c[e]), __fmul_rn(v1, s[e])));
+                v[e + 1] = mf_half(__fadd_rn(__fmul_rn(v0, s[e]), __fmul_rn(v1, c[e])));
             }
         }
         if (is_q) { mf_store4(a.q + ((size_t)tok * a.n_heads + hh) * 128 + 4 * lane, v); return; }
@@ -663,13 +681,15 @@ template <bool GLU>
 __global__ void __launch_bounds__(256) mf_vec_kernel(const __grid_constant__ MfSums sums, const __half* x, int K, MfQuant q) {
     const int lane = threadIdx.x & 31, tile = blockIdx.x * 8 + (threadIdx.x >> 5), tok = blockIdx.y;
     pdl_launch();
+    if (tile >= K / MF_ROWS) { pdl_wait(); return; }
+    MfPlace g_at, u_at;
+    if (GLU) { g_at = mf_place(sums, sums.seg[0], tile, tok, lane); u_at = mf_place(sums, sums.seg[1], tile, tok, lane); }
     pdl_wait();
-    if (tile >= K / MF_ROWS) return;
     float v[4];
     if (GLU) {
         float u[4];
-        mf_sum4<2>(v, sums, sums.seg[0], tile, tok, lane);
-        mf_sum4<2>(u, sums, sums.seg[1], tile, tok, lane);
+        mf_sum4<2>(v, g_at);
+        mf_sum4<2>(u, u_at);
         #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const float g = mf_half(v[e]);
@@ -760,7 +780,7 @@ static MfSums mf_sums(const MfProduct* p, const float* part, int N) {
 int launch_mf_norm(const MfProduct* p, const float* part, const __half* x, __half* x_out, const float* w, float eps, int H, const MfOperand& q, int N, cudaStream_t st) {
     const int tiles = H / MF_ROWS, warps = tiles < 32 ? tiles : 32;
     if (H % MF_ROWS || tiles > 32 * MF_NORM_TILES) return set_error(JB_ERR_ARG, "few-token norm: width %d", H);
-    auto kern = tiles <= 32 ? mf_norm_kernel<1> : tiles <= 64 ? mf_norm_kernel<2> : mf_norm_kernel<4>;
+    auto kern = tiles <= 20 ? mf_norm_kernel<1, 640> : tiles <= 32 ? mf_norm_kernel<1, 1024> : tiles <= 64 ? mf_norm_kernel<2, 1024> : mf_norm_kernel<4, 1024>;      // by registers
     JB_CUDA(launch_k(kern, dim3(N), dim3(32 * warps), 0, st, pdl_enabled(), mf_sums(p, part, N), x, x_out, w, eps, H, MfQuant{q.x4, q.x6, N, mf_padded(N)}));
     count_launch();
     return JB_OK;
