@@ -83,17 +83,6 @@ __device__ __forceinline__ void mf_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                    "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void mf_mma_ts(uint32_t d, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 b;\n\tmov.b64 b, {%2, %3};\n\tsetp.ne.b32 p, %5, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}\n"
-                 ::"r"(d), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ bool mf_elect() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
-    return p != 0;
-}
-// every lane waits; false on all of them when one's wait ran out
-__device__ __forceinline__ bool mf_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xFFFFFFFFu, tc_wait(bar, parity)); }
 
 __device__ __forceinline__ __half2 mf_h2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
 __device__ __forceinline__ uint32_t mf_u32(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
@@ -277,7 +266,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1) mf_kernel(const __grid_constant
         // fp16 x fp16 -> fp32, A in tensor memory, B without swizzle: chunks of K NP * 16 bytes apart, groups of eight tokens 128.
         // The issue of the MMAs is the longest chain here (17 of them a super-block, each faster than its operands' set-up), so the whole warp
         // runs the loop (its values are then uniform), without divisions, and one lane issues.
-        const bool leader = mf_elect();
+        const bool leader = tc_elect();
         const uint32_t idesc = (1u << 4) | ((uint32_t)(NP >> 3) << 17) | ((uint32_t)(MF_ROWS >> 4) << 24);
         const uint32_t bd_hi = 8u | (1u << 14), bd_lo0 = ((smem_u32(xring) >> 4) & 0x3FFFu) | ((uint32_t)NP << 16);
         const uint32_t step = 2u * NP, x16 = (uint32_t)x_bytes >> 4;       // 16-byte units from one K step, one stage to the next
@@ -286,29 +275,29 @@ __global__ void __launch_bounds__(MF_THREADS, 1) mf_kernel(const __grid_constant
         int kb = u0 % nb;
         bool first = true;
         for (int u = u0; u < u1; ++u) {
-            if (first && !mf_wait(&acc_empty[acc], pacc)) { ok = false; break; }
-            if (!mf_wait(&x_full[sx], px) || !mf_wait(&a_full[sa], pa)) { ok = false; break; }
+            if (first && !tc_wait_all(&acc_empty[acc], pacc)) { ok = false; break; }
+            if (!tc_wait_all(&x_full[sx], px) || !tc_wait_all(&a_full[sa], pa)) { ok = false; break; }
             tc_fence_after();
             uint32_t ta = tmem + sa * MF_ACOLS, bd_lo = bd_lo0 + sx * x16;
             if (++kb == nb) kb = 0;
             const bool last = kb == 0 || u + 1 == u1;
             if (leader) {
                 #pragma unroll
-                for (int k = 0; k < 8; ++k) mf_mma_ts(d, ta + 8 * k, bd_lo + k * step, bd_hi, idesc, (uint32_t)(!first || k));
+                for (int k = 0; k < 8; ++k) tc_mma_ts(d, ta + 8 * k, bd_lo + k * step, bd_hi, idesc, (uint32_t)(!first || k));
             }
             ta += 64; bd_lo += 8 * step;
             if (parts == 2) {
                 if (leader) tc_commit(&x_empty[sx]);
                 __syncwarp();
                 if (++sx == (uint32_t)nx) { sx = 0; px ^= 1; }
-                if (!mf_wait(&x_full[sx], px)) { ok = false; break; }
+                if (!tc_wait_all(&x_full[sx], px)) { ok = false; break; }
                 tc_fence_after();
                 bd_lo = bd_lo0 + sx * x16;
             }
             if (leader) {
                 #pragma unroll
-                for (int k = 0; k < 8; ++k) mf_mma_ts(d, ta + 8 * k, bd_lo + k * step, bd_hi, idesc, 1u);
-                if (!q6) mf_mma_ts(d, ta + 64, bd_lo + 8 * step, bd_hi, idesc, 1u);
+                for (int k = 0; k < 8; ++k) tc_mma_ts(d, ta + 8 * k, bd_lo + k * step, bd_hi, idesc, 1u);
+                if (!q6) tc_mma_ts(d, ta + 64, bd_lo + 8 * step, bd_hi, idesc, 1u);
                 tc_commit(&a_empty[sa]);
                 tc_commit(&x_empty[sx]);
                 if (last) tc_commit(&acc_full[acc]);
@@ -341,7 +330,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1) mf_kernel(const __grid_constant
         int kb = (u0 + set) % nb;
         bool ok = true;
         for (int u = u0 + set; u < u1; u += 2) {
-            if (!mf_wait(&w_full[s], pw_)) { ok = false; break; }
+            if (!tc_wait_all(&w_full[s], pw_)) { ok = false; break; }
             const uint32_t col = lane_base + sa * MF_ACOLS + 64 * f;
             uint32_t o[32];
             if (!q6) {
@@ -350,13 +339,13 @@ __global__ void __launch_bounds__(MF_THREADS, 1) mf_kernel(const __grid_constant
                 const MfS4 sc = mf_scales4(hd, f);
                 const __half2 c02 = __hmul2(mf_h2(0x48004800u), sc.d02), c13 = __hmul2(mf_h2(0x48004800u), sc.d13);      // centring constants: 8 half(d * sc)
                 mf_codes4(o, q0, q1, __low2half2(sc.d02), __low2half2(sc.d13));
-                if (!mf_wait(&a_empty[sa], pa)) { ok = false; break; }
+                if (!tc_wait_all(&a_empty[sa], pa)) { ok = false; break; }
                 tc_fence_after();
+                __syncwarp();
                 mf_st32(col, o);
                 mf_st4(lane_base + sa * MF_ACOLS + 128 + 4 * f, mf_u32(__lows2half2(sc.m02, sc.m13)), mf_u32(__lows2half2(c02, c13)), mf_u32(__highs2half2(sc.m02, sc.m13)), mf_u32(__highs2half2(c02, c13)));
                 mf_codes4(o, q2, q3, __high2half2(sc.d02), __high2half2(sc.d13));
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&w_empty[s]);
                 mf_st32(col + 32, o);
             } else {
                 const uint32_t at = w0 + s * MF_WBYTES6 + ((mis0 + (uint32_t)(kb * Q6K_BYTES)) & 15u);
@@ -364,13 +353,13 @@ __global__ void __launch_bounds__(MF_THREADS, 1) mf_kernel(const __grid_constant
                 mf_scales6(r, at, f);
                 mf_load6(r, at, f, 0);
                 mf_codes6(o, r, 0);
-                if (!mf_wait(&a_empty[sa], pa)) { ok = false; break; }
+                if (!tc_wait_all(&a_empty[sa], pa)) { ok = false; break; }
                 tc_fence_after();
+                __syncwarp();
                 mf_st32(col, o);
                 mf_load6(r, at, f, 1);
                 mf_codes6(o, r, 1);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&w_empty[s]);
                 mf_st32(col + 32, o);
                 kb += 2;
                 while (kb >= nb) kb -= nb;
@@ -378,7 +367,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1) mf_kernel(const __grid_constant
             mf_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&a_full[sa]);
+            if (lane == 0) { mbar_arrive(&w_empty[s]); mbar_arrive(&a_full[sa]); }
             s += 2;
             if (s >= MF_WSTAGES) { s -= MF_WSTAGES; pw_ ^= 1; }
             sa += 2; if (sa >= (uint32_t)na) { sa -= na; pa ^= 1; }
@@ -394,7 +383,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1) mf_kernel(const __grid_constant
         for (int u = u0; u < u1; ++piece) {
             const int tile = u / nb, kb0 = u - tile * nb, len = min(nb - kb0, u1 - u);
             const uint32_t acc = piece % acc_n;
-            if (!mf_wait(&acc_full[acc], (piece / acc_n) & 1)) { if (lane == 0) atomicExch(a.status, JB_ERR_TIMEOUT); break; }
+            if (!tc_wait_all(&acc_full[acc], (piece / acc_n) & 1)) { if (lane == 0) atomicExch(a.status, JB_ERR_TIMEOUT); break; }
             tc_fence_after();
             const bool whole = OUT && len == nb;
             float* dst = OUT ? a.part + ((size_t)(2 * blockIdx.x + (kb0 == 0)) * a.N) * MF_ROWS + pos
@@ -402,6 +391,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1) mf_kernel(const __grid_constant
             const size_t ld = OUT ? MF_ROWS : a.rows;
             for (int t0 = 0; t0 < a.N; t0 += MF_OUT_TOK) {
                 uint32_t r[16];
+                __syncwarp();
                 mf_ld16(acc0 + acc * NP + t0 + ((uint32_t)(32 * quarter) << 16), r);
                 if (!whole) {
                     #pragma unroll

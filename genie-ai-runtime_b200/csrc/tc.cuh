@@ -47,6 +47,31 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uin
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// Issuing MMAs by the whole warp: it runs the loop, so that addresses and descriptors are uniform values, and its elected lane issues.  Issued from a
+// branch of one lane, an MMA took 60 clocks to set up on an idle SM and 100 beside other warps, more than most of them take to run; so 25.
+// Descriptors go in halves, the upper one a constant.
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
+// Every lane waits; false on all of them when one's wait ran out.  No lane waits for the others: a poll in a branch of one lane leaves the warp
+// apart behind it, each part running what follows on its own, and `.aligned` instructions must not meet it so.
+__device__ __forceinline__ bool tc_wait_all(uint64_t* bar, uint32_t parity) {
+    const bool ok = __all_sync(0xFFFFFFFFu, tc_wait(bar, parity));
+    __syncwarp();
+    return ok;
+}
+__device__ __forceinline__ void tc_mma_ss(uint32_t d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\tsetp.ne.b32 p, %6, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}\n"
+                 ::"r"(d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tc_mma_ts(uint32_t d, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 b;\n\tmov.b64 b, {%2, %3};\n\tsetp.ne.b32 p, %5, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}\n"
+                 ::"r"(d), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
+}
+constexpr uint32_t TC_DESC_HI = 64u | (1u << 14) | (2u << 29);       // upper half of tc_smem_desc
+__device__ __forceinline__ uint32_t tc_desc_lo(uint32_t saddr) { return ((saddr >> 4) & 0x3FFFu) | (1u << 16); }
 // K-major operand tile, 128-byte rows, 128-byte swizzle, 8-row atoms 1024 bytes apart
 __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t saddr) {
     return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
