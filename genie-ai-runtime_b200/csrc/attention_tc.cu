@@ -4,8 +4,9 @@
 //
 // What bounds it: the instructions and the latency of the softmax.  Per tile of 128 rows x 64 keys the products take 512 clocks (heads of
 // 128; 640 at 192 / 128; 768 for int8, whose weights are two planes) and the exponentials 512 (16 per clock and SM), and neither pipe is
-// more than 31 % busy: 2048 tokens, 32 / 8 heads of 128: 89.6 us (bf16) and 121.4 (int8, widening included) against 198.9 and 412.4 of
-// the kernels on mma.sync.
+// half busy: 1024 tokens behind 1024 others, 32 heads of 128: 52.4 us (bf16, 32 key heads) and 77 to 80 (int8, 8 key heads, widening not
+// included).  With 64-bit descriptors formed by one lane, which issues an MMA every 60 to 100 clocks, where a whole warp's uniform values let one
+// go every 25, and with the scales of int8 caches fetched by every softmax thread from global memory, they took 63.3 and 88.0.
 //   * a CTA owns two tiles of 128 query rows, (token, head of the group) pairs, so that one tile's products run under the other's
 //     softmax and both read the same tile of 64 keys;
 //   * S = Q K^T, 128 x 64 in fp32, goes to tensor memory; a thread reads its row, frees S for the next tile at once, and writes the
@@ -14,8 +15,8 @@
 //   * O stays in tensor memory; it is rescaled only when a row's maximum has risen by more than 2^8 since the last time (the conditional
 //     rescaling that FlashAttention-4 describes), which leaves weights and sums in range and the result unchanged up to rounding;
 //   * V is read as it lies, [key][dim]: the B operand of the second product is MN-major.
-// Warps: 0 TMA, 1 MMA issuer, 2-3 idle, 4-7 and 8-11 the softmax of the two tiles (a warp's index modulo 4 is its quarter of tensor
-// memory).  Every mbarrier wait is bounded.
+// Warps: 0 TMA (int8: the scales too), 1 MMA issuer (bf16: 1 and 2, a tile each), 3 idle, 4-7 and 8-11 the softmax of the two tiles (a warp's
+// index modulo 4 is its quarter of tensor memory).  Every mbarrier wait is bounded.
 #include "attention.cuh"
 #include "attention_general.cuh"
 #include "mma.cuh"
@@ -26,7 +27,9 @@ namespace jb {
 constexpr int AT_ROWS = 128, AT_KEYS = 64, AT_THREADS = 384;
 constexpr int AT_QCHUNK = AT_ROWS * 128, AT_KCHUNK = AT_KEYS * 128;      // bytes of 64 elements of a tile's rows
 constexpr float AT_LAZY = 8.0f;
-constexpr int at_stages(int qc, int vc) { const int s = (224 * 1024 - 2 * qc * AT_QCHUNK) / ((qc + vc) * AT_KCHUNK); return s > 6 ? 6 : s; }
+// INT8: the tile's 64 key and 64 value scales lie behind the ring
+constexpr int AT_SCALES = 2 * AT_KEYS * 4;
+constexpr int at_stages(int qc, int vc, bool int8) { const int s = (224 * 1024 - 2 * qc * AT_QCHUNK) / ((qc + vc) * AT_KCHUNK + (int8 ? AT_SCALES : 0)); return s > 6 ? 6 : s; }
 
 struct AtArgs {
     void* out; int R, dim1, vdim, ldo, n_tokens, start;
@@ -40,10 +43,6 @@ __device__ __forceinline__ void at_load_3d(uint32_t dst, const CUtensorMap* map,
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void at_mma_ts(uint32_t d, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
-                 ::"r"(d), "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void at_st32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
                  "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};"
@@ -55,10 +54,9 @@ __device__ __forceinline__ void at_st32(uint32_t taddr, const uint32_t (&r)[32])
 }
 // the bits of exp2f wherever the result is at least 2^-126 (compared for every float in [-150, 16]); zero below
 __device__ __forceinline__ float at_exp2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-// MN-major operand tile: rows of 64 elements (128 bytes, swizzled), eight rows 1024 bytes apart, the next 64 elements one chunk further
-__device__ __forceinline__ uint64_t at_desc_mn(uint32_t saddr) {
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(AT_KCHUNK >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
+// lower half of the descriptor of an MN-major operand tile: rows of 64 elements (128 bytes, swizzled), eight rows 1024 bytes apart, the next 64
+// elements one chunk further
+__device__ __forceinline__ uint32_t at_desc_mn(uint32_t saddr) { return ((saddr >> 4) & 0x3FFFu) | ((uint32_t)(AT_KCHUNK >> 4) << 16); }
 // the warp's wait: false on every lane when it ran out or another role gave up
 __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int* status) {
     int ok = 1;
@@ -109,18 +107,21 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                                                                 const __grid_constant__ CUtensorMap k2map, const __grid_constant__ CUtensorMap vmap,
                                                                 const __grid_constant__ AtArgs a) {
     extern __shared__ uint8_t at_smem_raw[];
-    constexpr int ST = at_stages(QC, VC), STAGE = (QC + VC) * AT_KCHUNK;
+    // Waits, 12 to 20 MMAs and commits of a turn take about 1400 clocks of an issuing warp: a warp per tile where the softmax takes less (heads of
+    // 128, bf16: 63 us with one, 52 with two); int8 tiles, whose softmax takes more, run better out of step behind one (77 us; 84 with two).
+    constexpr int ST = at_stages(QC, VC, INT8), STAGE = (QC + VC) * AT_KCHUNK, ISSUERS = INT8 ? 1 : 2;
     __shared__ uint64_t q_full, full[ST], empty[ST], s_full[2], s_free[2], p_full[2], o_done[2];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int fail;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = blockIdx.y;
     const uint32_t qs = (smem_u32(at_smem_raw) + 1023u) & ~1023u, ring = qs + 2 * QC * AT_QCHUNK;
+    float* scales = reinterpret_cast<float*>(at_smem_raw + (ring - smem_u32(at_smem_raw)) + ST * STAGE);       // [stage][keys 64 | values 64]
     const int total = a.n_tokens * a.R, row0 = (gridDim.x - 1 - blockIdx.x) * 2 * AT_ROWS;        // longest tiles first
     const int n_keys = a.start + (min(row0 + 2 * AT_ROWS, total) - 1) / a.R + 1, tiles = (n_keys + AT_KEYS - 1) / AT_KEYS;
 
     if (threadIdx.x == 0) {
         mbar_init(&q_full, 1);
-        for (int s = 0; s < ST; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < ST; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], ISSUERS); }
         for (int x = 0; x < 2; ++x) { mbar_init(&s_full[x], 1); mbar_init(&s_free[x], 4); mbar_init(&p_full[x], 4); mbar_init(&o_done[x], 1); }
         fence_mbar_init();
         fail = 0;
@@ -146,7 +147,11 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                 const int s = t % ST;
                 if (!tc_wait(&empty[s], ((t / ST) & 1) ^ 1) || fail) { tc_fail(&fail, a.status); break; }
                 const uint32_t st = ring + s * STAGE;
-                mbar_expect_tx(&full[s], STAGE);
+                mbar_expect_tx(&full[s], STAGE + (INT8 ? AT_SCALES : 0));
+                if (INT8) {
+                    bulk_g2s(scales + s * 2 * AT_KEYS, a.ks + (size_t)g * a.lds + t * AT_KEYS, AT_SCALES / 2, &full[s]);
+                    bulk_g2s(scales + s * 2 * AT_KEYS + AT_KEYS, a.vs + (size_t)g * a.lds + t * AT_KEYS, AT_SCALES / 2, &full[s]);
+                }
                 for (int c = 0; c < QC; ++c) {
                     if (c * 64 < a.dim1) at_load_3d(st + c * AT_KCHUNK, &kmap, c * 64, g, t * AT_KEYS, &full[s]);
                     else                 at_load_3d(st + c * AT_KCHUNK, &k2map, c * 64 - a.dim1, 0, t * AT_KEYS, &full[s]);
@@ -156,57 +161,74 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             tc_wait(&q_full, 0);                      // its own copies are not in flight when it leaves
             for (int t = max(0, tiles - ST); t < tiles && !fail; ++t) if (!tc_wait(&full[t % ST], (t / ST) & 1)) break;
         }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t kind = INT8 ? 0u : (1u << 7) | (1u << 10), m128 = (uint32_t)(AT_ROWS >> 4) << 24;
-            const uint32_t i_qk = (1u << 4) | kind | ((uint32_t)(AT_KEYS >> 3) << 17) | m128;
-            const uint32_t i_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(VC * 64 >> 3) << 17) | m128;
-            bool ok = tc_wait(&q_full, 0);
-            auto scores = [&](int t, int x) {         // S of tile x over keys t
-                if (t >= tiles) return;
-                const int s = t % ST;
-                ok = ok && tc_wait(&full[s], (t / ST) & 1) && tc_wait(&s_free[x], (t & 1) ^ 1);
-                if (!ok) return;
-                tc_fence_after();
-                const uint64_t qd = tc_smem_desc(qs + x * QC * AT_QCHUNK), kd = tc_smem_desc(ring + s * STAGE);
-                #pragma unroll
-                for (int c = 0; c < QC; ++c)
-                    #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        tc_mma_f16(tmem + x * 256u, qd + (uint64_t)(c * (AT_QCHUNK >> 4) + 2 * k), kd + (uint64_t)(c * (AT_KCHUNK >> 4) + 2 * k), i_qk, (uint32_t)(c != 0 || k != 0));
-                tc_commit(&s_full[x]);
-            };
-            scores(0, 0);
-            scores(0, 1);
-            for (int t = 0; t < tiles && ok; ++t) {
-                const uint64_t vd = at_desc_mn(ring + (t % ST) * STAGE + QC * AT_KCHUNK);
-                for (int x = 0; x < 2 && ok; ++x) {
-                    scores(t + 1, x);
-                    ok = ok && tc_wait(&p_full[x], t & 1);
-                    if (!ok) break;
+    } else if (warp <= ISSUERS) {
+        // The whole warp runs the loop (its values are then uniform), one lane waits and issues; a wait that ran out leaves it idle for the rest.
+        const bool leader = tc_elect();
+        const uint32_t kind = INT8 ? 0u : (1u << 7) | (1u << 10), m128 = (uint32_t)(AT_ROWS >> 4) << 24;
+        const uint32_t i_qk = (1u << 4) | kind | ((uint32_t)(AT_KEYS >> 3) << 17) | m128;
+        const uint32_t i_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(VC * 64 >> 3) << 17) | m128;
+        const uint32_t q_lo = tc_desc_lo(qs), k_lo = tc_desc_lo(ring), v_lo = at_desc_mn(ring + QC * AT_KCHUNK);
+        bool ok = true;
+        auto wait = [&](uint64_t* bar, uint32_t parity) {
+            if (leader && ok && !tc_wait(bar, parity)) { ok = false; tc_fail(&fail, a.status); }
+            __syncwarp();
+        };
+        wait(&q_full, 0);
+        uint32_t s = 0, sn = 0, pn = 0;               // stage of key tile t; stage and parity of the one whose scores come next
+        for (int t = -1; t < tiles; ++t) {
+            #pragma unroll
+            for (int i = 0; i < 2 / ISSUERS; ++i) {
+                const int x = ISSUERS == 2 ? warp - 1 : i;
+                const uint32_t d = tmem + x * 256u, p = d + 64u, o = d + 128u;
+                if (t + 1 < tiles) {                  // scores over the next keys, as soon as the present ones are read
+                    if (i == 0) wait(&full[sn], pn);
+                    wait(&s_free[x], (t + 1) & 1 ^ 1);
+                    if (leader && ok) {
+                        tc_fence_after();
+                        const uint32_t qd = q_lo + x * QC * (AT_QCHUNK >> 4), kd = k_lo + sn * (STAGE >> 4);
+                        #pragma unroll
+                        for (int c = 0; c < QC; ++c)
+                            #pragma unroll
+                            for (int k = 0; k < 4; ++k)
+                                tc_mma_ss(d, qd + (uint32_t)(c * (AT_QCHUNK >> 4) + 2 * k), TC_DESC_HI, kd + (uint32_t)(c * (AT_KCHUNK >> 4) + 2 * k), TC_DESC_HI, i_qk, (uint32_t)(c != 0 || k != 0));
+                        tc_commit(&s_full[x]);
+                    }
+                    __syncwarp();
+                }
+                if (t < 0) continue;
+                wait(&p_full[x], t & 1);
+                if (leader && ok) {
                     tc_fence_after();
-                    const uint32_t p = tmem + x * 256u + 64u, o = tmem + x * 256u + 128u;
+                    const uint32_t vd = v_lo + s * (STAGE >> 4);
                     #pragma unroll
-                    for (int k = 0; k < 4; ++k) at_mma_ts(o, p + 8 * k, vd + (uint64_t)(k * (2048 >> 4)), i_pv, (uint32_t)(t != 0 || k != 0));
+                    for (int k = 0; k < 4; ++k) tc_mma_ts(o, p + 8 * k, vd + (uint32_t)(k * (2048 >> 4)), TC_DESC_HI, i_pv, (uint32_t)(t != 0 || k != 0));
                     if (INT8) {
                         #pragma unroll
-                        for (int k = 0; k < 4; ++k) at_mma_ts(o, p + 32 + 8 * k, vd + (uint64_t)(k * (2048 >> 4)), i_pv, 1u);
+                        for (int k = 0; k < 4; ++k) tc_mma_ts(o, p + 32 + 8 * k, vd + (uint32_t)(k * (2048 >> 4)), TC_DESC_HI, i_pv, 1u);
                     }
                     tc_commit(&o_done[x]);
+                    if (i == 2 / ISSUERS - 1) tc_commit(&empty[s]);
                 }
-                tc_commit(&empty[t % ST]);
+                __syncwarp();
             }
-            if (!ok) tc_fail(&fail, a.status);
+            if (++sn == ST) { sn = 0; pn ^= 1; }
+            if (t >= 0 && ++s == ST) s = 0;
         }
     } else if (warp >= 4) {
         const int x = (warp - 4) >> 2, q = warp & 3, fr = row0 + x * AT_ROWS + q * 32 + lane, frc = min(fr, total - 1);
         const int tok = frc / a.R, head = g * a.R + frc - tok * a.R, pos = a.start + tok;
         const int first_pos = a.start + min(row0 + x * AT_ROWS + q * 32, total - 1) / a.R;        // least position among the warp's rows
+        // Scores in units of log2 are raw scores (times their key's scale) times fsc.  Where that is positive it waits for the exponent's subtraction,
+        // a multiply-add; else scores are multiplied by it first and the factor left is 1.
         const float fsc = a.scale * q_temp_factor(pos, a.qt_coef, a.qt_every) * FA_LOG2E;
+        const bool late = __all_sync(0xFFFFFFFFu, fsc > 0.f && fsc < INFINITY);
+        const float early = late ? 1.f : fsc, f2 = late ? fsc : 1.f;
         const uint32_t tm = tmem + x * 256u + ((uint32_t)(q * 32) << 16);
-        float m = -INFINITY, l = 0.f;
+        float m = -INFINITY, l = 0.f;                 // m: in units of the scores before f2
         bool good = true;
+        uint32_t stage = 0, stage_parity = 0;
         for (int t = 0; t < tiles; ++t) {
+            if (INT8 && !at_wait(&full[stage], stage_parity, &fail, a.status)) { good = false; break; }       // the scales are there to see
             if (!at_wait(&s_full[x], t & 1, &fail, a.status)) { good = false; break; }
             tc_fence_after();
             uint32_t s0[32], s1[32];
@@ -216,17 +238,22 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&s_free[x]);
+            __syncwarp();
             float v[64];
             #pragma unroll
             for (int i = 0; i < 32; ++i) { v[i] = __uint_as_float(s0[i]); v[32 + i] = __uint_as_float(s1[i]); }
             const int k0 = t * AT_KEYS;
+            const float* tile_scales = scales + stage * 2 * AT_KEYS;
             if (INT8) {
-                const float4* ks = reinterpret_cast<const float4*>(a.ks + (size_t)g * a.lds + k0);
                 #pragma unroll
-                for (int i = 0; i < 16; ++i) { const float4 f = ks[i]; v[4 * i] *= fsc * f.x; v[4 * i + 1] *= fsc * f.y; v[4 * i + 2] *= fsc * f.z; v[4 * i + 3] *= fsc * f.w; }
-            } else {
+                for (int i = 0; i < 16; ++i) {
+                    const float4 f = *reinterpret_cast<const float4*>(tile_scales + 4 * i);
+                    v[4 * i] *= f.x; v[4 * i + 1] *= f.y; v[4 * i + 2] *= f.z; v[4 * i + 3] *= f.w;
+                }
+            }
+            if (!late) {
                 #pragma unroll
-                for (int i = 0; i < 64; ++i) v[i] *= fsc;
+                for (int i = 0; i < 64; ++i) v[i] *= early;
             }
             const bool diagonal = k0 + AT_KEYS - 1 > first_pos;
             if (diagonal) {
@@ -238,15 +265,15 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             for (int i = 4; i < 64; ++i) mx[i & 3] = fmaxf(mx[i & 3], v[i]);
             const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
             float corr = 1.f;
-            if (top > m + AT_LAZY) { corr = at_exp2(m - top); m = top; }          // the first tile: every row sees key 0
-            const float base = m == -INFINITY ? 0.f : m;
+            if ((top - m) * f2 > AT_LAZY) { corr = at_exp2((m - top) * f2); m = top; }          // the first tile: every row sees key 0
+            const float base = m == -INFINITY ? 0.f : -m * f2;
             float sum[4] = {0.f, 0.f, 0.f, 0.f};
             #pragma unroll
-            for (int i = 0; i < 64; ++i) { v[i] = at_exp2(v[i] - base); sum[i & 3] += v[i]; }
+            for (int i = 0; i < 64; ++i) { v[i] = at_exp2(fmaf(v[i], f2, base)); sum[i & 3] += v[i]; }
             l = l * corr + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
             uint32_t hi[32], lo[32];
             if (INT8) {
-                const float4* vs = reinterpret_cast<const float4*>(a.vs + (size_t)g * a.lds + k0);
+                const float4* vs = reinterpret_cast<const float4*>(tile_scales + AT_KEYS);
                 // `seen`: a masked weight is zero whatever the scale of its value; asked where some scale of a diagonal tile is not finite
                 auto planes = [&](auto seen) {
                     #pragma unroll
@@ -290,7 +317,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_full[x]);
+            if (INT8 && ++stage == ST) { stage = 0; stage_parity ^= 1; }
         }
+        m *= f2;
         if (good) good = at_wait(&o_done[x], (tiles - 1) & 1, &fail, a.status);
         if (good) {
             tc_fence_after();
@@ -422,7 +451,7 @@ bool attention_tc_applies(const AttnCall& c) {
 
 template <int QC, int VC, bool INT8>
 static int at_go(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& k2, const CUtensorMap& v, const AtArgs& a, int n_kv, cudaStream_t st) {
-    const size_t smem = (size_t)2 * QC * AT_QCHUNK + (size_t)at_stages(QC, VC) * (QC + VC) * AT_KCHUNK + 1024;
+    const size_t smem = (size_t)2 * QC * AT_QCHUNK + (size_t)at_stages(QC, VC, INT8) * ((QC + VC) * AT_KCHUNK + (INT8 ? AT_SCALES : 0)) + 1024;
     bool& attr = ctx()->attn_tc_attr[INT8 ? 6 : 2 * (QC - 1) + VC - 1];
     if (!attr) {
         JB_CUDA(cudaFuncSetAttribute(attn_tc_kernel<QC, VC, INT8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
