@@ -1,0 +1,57 @@
+"""The memory's prompt kernel at the edges of its chunks of 128 tokens, its 64 dimensions and its 32 value columns, and with values that are not finite."""
+import numpy as np
+import pytest
+
+from gpu_util import pkg
+from oracle import delizen as orc
+from test_gpu_delizen import f32, memory_case, zeros
+from test_gpu_layered import as_np, pad8, rng, up
+
+pytestmark = pytest.mark.gpu
+
+
+def run(jb, q, k, v, zi, zf, cuts):
+    """raw outputs [T][H][V] and the state left behind"""
+    T, H, D = q.shape
+    V = v.shape[2]
+    a, b = pad8(H * D), pad8(H * V)
+    proj = np.zeros((T, 2 * a + 2 * b))
+    proj[:, :H * D], proj[:, a:a + H * D], proj[:, 2 * a:2 * a + H * V] = q.reshape(T, -1), k.reshape(T, -1), v.reshape(T, -1)
+    gates = np.zeros((T, pad8(2 * H)))
+    gates[:, :H], gates[:, H:2 * H] = zi, zf
+    pd, gd, bd, wd, state = up(proj, "bfloat16"), f32(gates), f32(np.zeros(2 * H), False), f32(np.ones(H * V), False), zeros(jb.mlstm_state_floats(H, D, V))
+    got, at = [], 0
+    for c in cuts:
+        out, raw = zeros((c, b), "bfloat16"), zeros((c, H * V))
+        jb.mlstm(out, raw, state, pd[at:at + c].contiguous(), gd[at:at + c].contiguous(), bd, wd, H, D, V, 13.0, 1e-4, c, at)
+        got.append(as_np(raw).reshape(c, H, V))
+        at += c
+    assert at == T
+    return np.concatenate(got), as_np(state)
+
+
+@pytest.mark.parametrize("H,D,V", [(1, 8, 8), (2, 64, 32), (1, 72, 40), (3, 128, 64), (2, 136, 24), (1, 192, 96), (1, 256, 72)])
+@pytest.mark.parametrize("kind", ["plain", "drop", "far"])
+@pytest.mark.parametrize("cuts", [[16], [127], [128], [129], [256, 16], [257, 383, 17]])
+def test_edges(H, D, V, kind, cuts):
+    jb, T = pkg(), sum(cuts)
+    q, k, v, _, zi, zf = memory_case(rng(D + T), H, D, V, T, kind, "bfloat16")
+    want = np.stack([orc.mlstm_memory(q[:, h] * D ** -0.5, k[:, h], v[:, h], orc.capped(zi[:, h], 13.0), orc.log_sigmoid(orc.capped(zf[:, h], 13.0)))[0] for h in range(H)], 1)
+    got, _ = run(jb, q, k, v, zi, zf, cuts)
+    assert (np.abs(got - want) / np.abs(want).max(axis=(0, 2))[None, :, None]).max() < 2e-4      # as in the general test: two bf16 parts, and n . q may cancel
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("at", [0, 31, 100, 127, 128, 200])
+def test_a_value_that_is_not_finite_reaches_no_earlier_token(at, value):
+    jb, T = pkg(), 300
+    q, k, v, _, zi, zf = memory_case(rng(at), 2, 64, 40, T, "plain", "bfloat16")
+    clean, _ = run(jb, q, k, v, zi, zf, [T])
+    v = v.copy()
+    v[at, 1, 33] = value
+    got, _ = run(jb, q, k, v, zi, zf, [T])
+    other = np.arange(40) != 33
+    # the chunk's part is then added up in fp32 one token after the other: 2^-24 of up to 128 terms
+    for a, b in ((got[:at], clean[:at]), (got[:, 0], clean[:, 0]), (got[:, 1, other], clean[:, 1, other])):
+        assert np.isfinite(a).all() and np.abs(a - b).max(initial=0) <= 1e-4 * np.abs(clean).max()
+    assert not np.isfinite(got[at:, 1, 33]).any()
