@@ -803,9 +803,13 @@ bool MfModel::plan(const jllm_b200_model_desc& m, bool with_out) {
     // a head is a 128-row tile; norms keep a token in one CTA's registers
     if (m.head_dim != MF_ROWS || hidden % QK_K || q_dim % QK_K || ffn % QK_K || hidden > 32 * MF_NORM_TILES * MF_ROWS) return false;
     auto own = [](const void* W) { return resolve_weight(W) == W ? W : nullptr; };       // weights in host memory are read by the other kernels
+    // norm vectors are read as float4; others (from inside a file, say) are read element by element by the other kernels, which also refuse null ones
+    auto norm = [](const float* w) { return w && !((uintptr_t)w & 15); };
+    if (with_out && !norm(m.output_norm)) return false;
     std::vector<MfLayer> all(m.n_layers);
     for (int l = 0; l < m.n_layers; ++l) {
         const jllm_b200_layer_desc& w = m.layers[l];
+        if (!norm(w.rms_attn) || !norm(w.rms_ffn) || (w.q_norm && !norm(w.q_norm)) || (w.k_norm && !norm(w.k_norm))) return false;
         const MfWeight qkv[3] = {{own(w.wq), w.type_wq, q_dim}, {own(w.wk), w.type_wk, kv_dim}, {own(w.wv), w.type_wv, kv_dim}};
         const MfWeight wo = {own(w.wo), w.type_wo, hidden}, gu[2] = {{own(w.w_gate), w.type_w_gate, ffn}, {own(w.w_up), w.type_w_up, ffn}}, down = {own(w.w_down), w.type_w_down, hidden};
         if (!mf_plan(all[l].qkv, qkv, 3, hidden) || !mf_plan(all[l].wo, &wo, 1, q_dim) || !mf_plan(all[l].gate_up, gu, 2, hidden) || !mf_plan(all[l].down, &down, 1, ffn)) return false;

@@ -54,6 +54,14 @@ def elsewhere(w):
     return w
 
 
+def shifted(v):
+    """The vector one element further on than a 16-byte boundary."""
+    import torch
+    buf = torch.empty(v.numel() + 4, dtype=v.dtype, device="cuda")
+    buf[1:1 + v.numel()] = v
+    return buf[1:1 + v.numel()]
+
+
 def device_bytes(ptr, n):
     import torch
     out = torch.empty(n, dtype=torch.uint8, device="cuda")
@@ -118,3 +126,51 @@ def test_streams_as_the_general_kernels(shape, swap, streams):
         assert jb.device_status(st) == 0
         d.close()
     check_logits(*sides, ERR_RMS)
+
+
+@pytest.mark.parametrize("name", ["rms_attn", "rms_ffn", "q_norm", "k_norm", "out_norm"])
+def test_norm_vectors_may_start_at_any_element(name):
+    """The kernels between the products read norm vectors 16 bytes at a time: a model whose vectors start elsewhere stays with the general ones."""
+    import torch
+    jb = pkg()
+    cfg, w = weights("even", False)
+    moved = dict(w, layers=[dict(l, **({name: shifted(l[name])} if name in l else {})) for l in w["layers"]])
+    if name == "out_norm":
+        moved["out_norm"] = shifted(w["out_norm"])
+    st = torch.cuda.Stream()
+    for n in (20, 150):
+        prompt = np.random.Generator(np.random.PCG64(n)).integers(0, cfg["vocab"], n)
+        got = []
+        for ws in (moved, elsewhere(w)):
+            d = jb.decoder.Decoder(cfg, ws, 256, jb.decoder.FUSED | jb.decoder.PREFILL)
+            d.prefill(prompt, 0, st)
+            got.append(d.logits().cpu().numpy().astype(np.float64))
+            assert jb.device_status(st) == 0
+            d.close()
+        check_logits(*got, ONE_TOKEN_RMS)
+    prompts = np.random.Generator(np.random.PCG64(7)).integers(0, cfg["vocab"], (5, 3)).astype(np.int32)
+    got = []
+    for ws in (moved, elsewhere(w)):
+        d = jb.decoder.BatchDecoder(cfg, ws, 16, 5)
+        d.generate(prompts, 1, st)
+        got.append(d.logits().double().cpu().numpy())
+        assert jb.device_status(st) == 0
+        d.close()
+    check_logits(*got, ERR_RMS)
+
+
+@pytest.mark.parametrize("name", ["rms_attn", "rms_ffn"])
+def test_a_missing_norm_vector_is_refused(name):
+    jb = pkg()
+    cfg, w = weights("even", False)
+    w = dict(w, layers=[dict(l) for l in w["layers"]])
+    w["layers"][1][name] = None
+    d = jb.decoder.Decoder(cfg, w, 256, jb.decoder.FUSED | jb.decoder.PREFILL)
+    for n in (20, 150):
+        with pytest.raises(jb.JllmError):
+            d.prefill(np.zeros(n, np.int32), 0)
+    d.close()
+    d = jb.decoder.BatchDecoder(cfg, w, 16, 5)
+    with pytest.raises(jb.JllmError):
+        d.generate(np.zeros((5, 3), np.int32), 1)
+    d.close()
