@@ -84,6 +84,13 @@ __device__ __forceinline__ void mf_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// whether all four drain warps say so: they meet at barriers, so they leave together or not at all
+__device__ __forceinline__ bool mf_drains_all(bool ok) {
+    int x;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n" : "=r"(x) : "r"((int)ok) : "memory");
+    return x != 0;
+}
+
 __device__ __forceinline__ __half2 mf_h2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
 __device__ __forceinline__ uint32_t mf_u32(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
 // bytes 0 and 2 of a word as two halves
@@ -383,7 +390,8 @@ __global__ void __launch_bounds__(MF_THREADS, 1) mf_kernel(const __grid_constant
         for (int u = u0; u < u1; ++piece) {
             const int tile = u / nb, kb0 = u - tile * nb, len = min(nb - kb0, u1 - u);
             const uint32_t acc = piece % acc_n;
-            if (!tc_wait_all(&acc_full[acc], (piece / acc_n) & 1)) { if (lane == 0) atomicExch(a.status, JB_ERR_TIMEOUT); break; }
+            const bool full = tc_wait_all(&acc_full[acc], (piece / acc_n) & 1);
+            if (OUT ? !mf_drains_all(full) : !full) { if (lane == 0) atomicExch(a.status, JB_ERR_TIMEOUT); break; }
             tc_fence_after();
             const bool whole = OUT && len == nb;
             float* dst = OUT ? a.part + ((size_t)(2 * blockIdx.x + (kb0 == 0)) * a.N) * MF_ROWS + pos
