@@ -303,7 +303,8 @@ int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     const bool by_rows = !few.layers.empty(), many = !by_rows || cap > MF_MAX_TOKENS;
     const size_t few_bytes = by_rows ? al(few.bytes(cap < MF_MAX_TOKENS ? cap : MF_MAX_TOKENS)) : 0, row_bytes = by_rows && many ? al(few.row_bytes(cap)) : 0;
     const size_t operands = few_bytes > row_bytes ? few_bytes : row_bytes;
-    const size_t total = 2 * al(N * H * 2) + 2 * al(N * QD * 2) + (many ? al(N * H * 2) + 2 * al(N * KVD * 2) + 2 * al(N * I * 2) : 0) + (by_rows ? operands : al(N * H * 2) + al(N * I * 2));
+    const size_t rows = many ? N : 1, general = by_rows ? 1 : N;        // a chunk of one token is the general kernels' too
+    const size_t total = 2 * al(N * H * 2) + 2 * al(N * QD * 2) + al(rows * H * 2) + 2 * al(rows * KVD * 2) + 2 * al(rows * I * 2) + al(general * H * 2) + al(general * I * 2) + (by_rows ? operands : 0);
     // one allocation for all of it: it is made inside a session's first prompt, where each costs 0.4 - 2 ms (512 tokens: the first prompt
     // took 1064 us more than the next with two, 444 with one)
     size_t wide = by_rows && mmq_wide_applies(m.hidden_dim, 0, cap, m.hidden_dim) ? 2 * MMQ_WEIGHT_BYTES + al(gemm_pair_part_floats() * sizeof(float)) : 0;
@@ -317,16 +318,11 @@ int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     auto take = [&](size_t b) { char* r = p; p += al(b); return r; };
     pf_x = (__half*)take(N * H * 2); pf_x2 = (__half*)take(N * H * 2);
     pf_q = (__half*)take(N * QD * 2); pf_att = (__half*)take(N * QD * 2);
-    if (many) {
-        pf_y = (__half*)take(N * H * 2);
-        pf_k = (__half*)take(N * KVD * 2); pf_v = (__half*)take(N * KVD * 2);
-        pf_gate = (__half*)take(N * I * 2); pf_up = (__half*)take(N * I * 2);
-    }
-    if (by_rows) {
-        pf_operands = take(operands);
-    } else {
-        pf_normed = (__half*)take(N * H * 2); pf_sw = (__half*)take(N * I * 2);
-    }
+    pf_y = (__half*)take(rows * H * 2);
+    pf_k = (__half*)take(rows * KVD * 2); pf_v = (__half*)take(rows * KVD * 2);
+    pf_gate = (__half*)take(rows * I * 2); pf_up = (__half*)take(rows * I * 2);
+    pf_normed = (__half*)take(general * H * 2); pf_sw = (__half*)take(general * I * 2);
+    if (by_rows) pf_operands = take(operands);
     pf_cap = cap;
     return JB_OK;
 }
@@ -432,10 +428,9 @@ int KquantDecoder::enqueue_few_mlp(int l, int N, cudaStream_t st) {
 
 int KquantDecoder::enqueue_chunk(const int* dev_tokens, int N, int start, cudaStream_t st) {
     const int H = m.hidden_dim, QD = m.n_heads * m.head_dim, KVD = m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
-    const float scale = 1.0f / sqrtf((float)m.head_dim);
     DCHK(launch_embed_rows(pf_x, m.tok_embd, m.embd_type, dev_tokens, N, H, st));
     if (!few.layers.empty() && N > MF_MAX_TOKENS) return enqueue_rows_chunk(N, start, st);
-    const bool by_few = !few.layers.empty();
+    const bool by_few = !few.layers.empty() && N > 1;       // one token: integer dots summed in fp32, by the general kernels
     if (by_few) few.place(pf_operands, N);
     if (by_few) DCHK(launch_mf_norm(nullptr, nullptr, pf_x, nullptr, layers[0].rms_attn, m.rms_eps, H, mf_operand(few.layers[0].qkv, few.xh4, few.xh6), N, st));
     for (int l = 0; l < m.n_layers; ++l) {

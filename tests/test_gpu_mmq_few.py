@@ -108,6 +108,24 @@ def test_prompt_chunk_as_the_general_kernels(shape, swap, n):
     check_logits(logits, logits0, ONE_TOKEN_RMS)
 
 
+def test_a_chunk_of_one_token_keeps_its_integer_products():
+    """Three tokens in chunks of two: the last one alone.  Its key codes of the first layer are those of the general kernels, bit for bit."""
+    import torch
+    jb = pkg()
+    cfg, w = weights("odd", False)
+    st = torch.cuda.Stream()
+    kv, sides = cfg["n_kv_heads"], []
+    for ws in (w, elsewhere(w)):
+        d = jb.decoder.Decoder(cfg, ws, 64, jb.decoder.FUSED | jb.decoder.PREFILL)
+        d.prefill(np.array([5, 6, 7]), 0, st, chunk=2)
+        buf = jb.lib.jllm_b200_decoder_buffer
+        buf.restype = C.c_void_p
+        sides.append((device_bytes(buf(C.c_void_p(d._h), 7), 3 * kv * 128)[2 * kv * 128:], device_bytes(buf(C.c_void_p(d._h), 8), 3 * kv * 4)[2 * kv * 4:]))
+        assert jb.device_status(st) == 0
+        d.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*sides))
+
+
 @pytest.mark.parametrize("shape,swap,streams", [("even", False, 2), ("odd", True, 33), ("odd", False, 96), ("whole", False, 128), ("even", True, 113)])
 def test_streams_as_the_general_kernels(shape, swap, streams):
     import torch
