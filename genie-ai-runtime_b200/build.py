@@ -16,7 +16,7 @@ OUT = os.path.join(HERE, "libjllm_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 # What every model family needs, what the layer-list models add, and what the K-quant kernels and the reference's API add.
 COMMON = ["core.cu", "decoder.cu", "pools.cpp", "attention_general.cu"]
-LAYERS = ["decoder_layers.cu", "layernorm.cu", "dense_gemv.cu", "dense_simt.cu", "dense_tc.cu", "gemm_pair.cu", "moe.cu", "attention_bf16.cu", "attention_tc.cu", "attention_latent.cu", "latent.cu", "mlstm.cu", "mlstm_chunk.cu"]
+LAYERS = ["decoder_layers.cu", "layernorm.cu", "dense_gemv.cu", "dense_simt.cu", "dense_tc.cu", "gemm_pair.cu", "moe.cu", "attention_bf16.cu", "attention_tc.cu", "attention_latent.cu", "latent.cu", "mlstm.cu", "mlstm_chunk.cu", "mlstm_short.cu"]
 KQUANT = ["api.cu", "gemv.cu", "elementwise.cu", "attention.cu", "attention_tma.cu", "attention_prefill.cu", "attention_noalloc.cu", "mmq.cu", "mmq_tc.cu",
           "mmq_stream.cu", "mmq_few.cu", "mmq_rows.cu", "tp.cu", "decoder_kquant.cu", "batch_decoder.cu", "layers_api.cu"]
 SOURCES = COMMON + LAYERS + KQUANT

@@ -68,6 +68,7 @@ struct DeviceCtx {
     bool attn_tma_attr[12] = {};
     bool attn_prefill_attr[3] = { false, false, false };
     bool attn_tc_attr[7] = {};
+    bool mlstm_short_attr[3] = {};
     unsigned int* attn_tickets = nullptr;   // ATTN_TICKET_WORDS zeroed words: slice counters of the TMA attention kernel
     int  gemv_smem_budget = 0;          // dynamic shared memory of a GEMV CTA that shares its SM with one other CTA
 };

@@ -23,8 +23,13 @@ struct MlstmCall {
 size_t mlstm_state_floats(int heads, int dim, int vdim);
 // Tokens start .. start + n - 1 of one sequence (a state older than position 0 is not read).  d_pos: one token at *d_pos instead.
 int launch_mlstm(const MlstmCall& a, int n, int start, const int* d_pos, cudaStream_t st);
-bool mlstm_chunks_apply(const MlstmCall& a, int n);                       // tensor-core kernel for prompts: bf16, sizes it holds
+bool mlstm_chunks_apply(const MlstmCall& a, int n);                       // tensor-core kernels for prompts: bf16, sizes they hold
 int launch_mlstm_chunks(const MlstmCall& a, int n, int start, cudaStream_t st);   // leaves `raw`, S, and the next n and m
+
+// Up to how many tokens one chunk of mlstm_short.cu serves.  us with the norm that follows, there / in mlstm_chunk.cu, 16 and 64 tokens: 8 heads of 256 x 512
+// 12.1 and 13.5 / 16.4 and 17.4, 4 heads of 128 x 256 8.7 and 9.5 / 12.3 and 12.4.
+constexpr int MLSTM_SHORT = 64;
+int launch_mlstm_short(const MlstmCall& a, int n, int start, cudaStream_t st);
 
 // floats from n (or m) to its next value
 __host__ __device__ inline size_t mlstm_next(const MlstmCall& a) { return (size_t)a.heads * a.dim + pad8(a.heads); }

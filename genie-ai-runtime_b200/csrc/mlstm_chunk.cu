@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mlstm_chunk_kernel(const __grid
 
 bool mlstm_chunks_apply(const MlstmCall& a, int n) {
     return a.kind == EK_BF16 && n >= 16 && a.dim % 8 == 0 && a.dim <= MC_MAX_DIM && a.vdim % 8 == 0 && a.ld % 8 == 0 && a.off_q % 8 == 0 && a.off_k % 8 == 0 && a.off_v % 8 == 0 &&
-           !((uintptr_t)a.proj & 15) && !((uintptr_t)a.raw & 15) && !((uintptr_t)a.state & 15) && encode_tiled_fn();
+           !((uintptr_t)a.proj & 15) && !((uintptr_t)a.state & 15) && (n <= MLSTM_SHORT ? !((uintptr_t)a.raw & 7) : !((uintptr_t)a.raw & 15) && encode_tiled_fn());
 }
 // [head][token][column] of a part of the projections, boxes of 64 columns x a chunk, zero outside a head's columns and behind the last token
 static bool mc_map(CUtensorMap* map, const MlstmCall& a, int off, int cols, int n) {
@@ -624,6 +624,7 @@ int launch_mlstm_chunks(const MlstmCall& a, int n, int start, cudaStream_t st) {
     DeviceCtx* x = ctx();
     if (!x) return set_error(JB_ERR_STATE, "mlstm chunks: library not initialised");
     if (!mlstm_chunks_apply(a, n)) return set_error(JB_ERR_ARG, "mlstm chunks: %d tokens, heads of %d x %d", n, a.dim, a.vdim);
+    if (n <= MLSTM_SHORT) return launch_mlstm_short(a, n, start, st);
     return a.dim <= 128 ? mc_go<2>(a, n, start, x->d_status, st) : mc_go<4>(a, n, start, x->d_status, st);
 }
 

@@ -1,4 +1,5 @@
-"""The memory's prompt kernel at the edges of its chunks of 128 tokens, its 64 dimensions and its 32 value columns, and with values that are not finite."""
+"""The memory's prompt kernels at the edges of their chunks (16 to 64 tokens in one, 128 in a row), their 64 dimensions and 32 value columns, and with values
+that are not finite."""
 import numpy as np
 import pytest
 
@@ -32,7 +33,7 @@ def run(jb, q, k, v, zi, zf, cuts):
 
 @pytest.mark.parametrize("H,D,V", [(1, 8, 8), (2, 64, 32), (1, 72, 40), (3, 128, 64), (2, 136, 24), (1, 192, 96), (1, 256, 72)])
 @pytest.mark.parametrize("kind", ["plain", "drop", "far"])
-@pytest.mark.parametrize("cuts", [[16], [127], [128], [129], [256, 16], [257, 383, 17]])
+@pytest.mark.parametrize("cuts", [[16], [17], [33], [64], [65], [127], [128], [129], [256, 16], [257, 383, 17], [64, 48, 100, 20]])
 def test_edges(H, D, V, kind, cuts):
     jb, T = pkg(), sum(cuts)
     q, k, v, _, zi, zf = memory_case(rng(D + T), H, D, V, T, kind, "bfloat16")
@@ -42,9 +43,9 @@ def test_edges(H, D, V, kind, cuts):
 
 
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
-@pytest.mark.parametrize("at", [0, 31, 100, 127, 128, 200])
-def test_a_value_that_is_not_finite_reaches_no_earlier_token(at, value):
-    jb, T = pkg(), 300
+@pytest.mark.parametrize("T,at", [(300, 0), (300, 31), (300, 100), (300, 127), (300, 128), (300, 200), (50, 0), (50, 20), (50, 49), (64, 63), (16, 5)])
+def test_a_value_that_is_not_finite_reaches_no_earlier_token(T, at, value):
+    jb = pkg()
     q, k, v, _, zi, zf = memory_case(rng(at), 2, 64, 40, T, "plain", "bfloat16")
     clean, _ = run(jb, q, k, v, zi, zf, [T])
     v = v.copy()
