@@ -4,7 +4,7 @@
 // A launch has few tokens per weight matrix here (an expert of a 130-token prompt: 16), so it is bound by the weights' way from memory and by the
 // tokens that pad a tile.  A WARP holds a tile of 64 rows x 16 tokens, 8 x 4 values per lane, and the warps of a CTA take
 // four k of a K tile in turn; a CTA is 16, 32 or 64 tokens wide (the other warps' tiles) and its warps' sums meet in shared memory in a fixed order.  Operands come by
-// cp.async in four stages, K contiguous as in memory: a lane reads four k of a row at a time, 12 (gate and up: 20) 16-byte reads of shared memory,
+// cp.async in three stages (gate and up: four), K contiguous as in memory: a lane reads four k of a row at a time, 12 (gate and up: 20) 16-byte reads of shared memory,
 // free of conflicts, for 128 (256) multiply-adds.
 //
 // 130 tokens, width 1024, 32 experts of 768, top 4, us before (64 x 32 tiles, 4 x 2 values a thread, tiles transposed through registers) / here:
@@ -25,21 +25,39 @@ template <bool GLU, int WT> constexpr size_t ds_smem() {
     return (stages > sums ? stages : sums) * sizeof(float);
 }
 
+// Groups of unlike sizes, known on the device alone: the tiles of group g start at item off[g] / width + g, which leaves room for as many as the tokens
+// before it can fill, with a part of a tile in every group.  False: no tile there.
+template <int WIDTH>
+__device__ __forceinline__ bool ds_find(const int* off, int n_groups, int item, int& grp, int& t0, int& t_hi) {
+    const int lane = threadIdx.x & 31;
+    for (int base = 0;; base += 32) {
+        const int g = min(base + lane, n_groups - 1), lo = off[g], hi = off[g + 1], first = lo / WIDTH + g;
+        const unsigned begun = __ballot_sync(0xFFFFFFFFu, base + lane < n_groups && first <= item);
+        if (begun == 0xFFFFFFFFu && base + 32 < n_groups && off[base + 32] / WIDTH + base + 32 <= item) continue;
+        const int at = 31 - __clz(begun);
+        grp = base + at;
+        t0 = __shfl_sync(0xFFFFFFFFu, lo + (item - first) * WIDTH, at);
+        t_hi = __shfl_sync(0xFFFFFFFFu, hi, at);
+        return t0 < t_hi;
+    }
+}
+
 // WT: 16-token tiles of a CTA; its 8 / WT warps on a tile share K
 template <bool GLU, int WT>
-__global__ void __launch_bounds__(DS_THREADS, 2) dense_simt_kernel(const __grid_constant__ DenseGemm a, bool vec) {
+__global__ void __launch_bounds__(DS_THREADS, 2) dense_simt_kernel(const __grid_constant__ DenseGemm a, int tiles, bool vec) {
     pdl_wait();
     pdl_launch();
     extern __shared__ __align__(16) float ds_sm[];
     constexpr int KG = DS_WARPS / WT, ROWS = DS_M * (GLU ? 2 : 1) + DS_T * WT, STAGE = ds_stage<GLU, WT>(), KT = DS_K<GLU>, LD = KT + 4, STAGES = DS_STAGES<GLU>, QUADS = KT / 4, PER = DS_THREADS / QUADS;
-    const int grp = blockIdx.z, t_lo = a.off ? a.off[grp] : 0, t_hi = a.off ? a.off[grp + 1] : a.N;
     const int r0 = blockIdx.x * DS_M, ldw = a.ldw > 0 ? a.ldw : pad8(a.K), ldx = a.ldx > 0 ? a.ldx : pad8(a.K);
-    const float* W = reinterpret_cast<const float*>(a.W) + (size_t)grp * a.M * ldw;
-    const float* V = GLU ? reinterpret_cast<const float*>(a.W_up) + (size_t)grp * a.M * ldw : nullptr;
-    const float* x = reinterpret_cast<const float*>(a.x) + (size_t)grp * a.x_step;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tx = lane & 7, ty = lane >> 3, wt = warp % WT, kg = warp / WT;
     const int k_tiles = (a.K + KT - 1) / KT;
-    for (int t0 = t_lo + blockIdx.y * DS_T * WT; t0 < t_hi; t0 += gridDim.y * DS_T * WT) {
+    for (int item = blockIdx.y; item < tiles; item += gridDim.y) {
+        int grp = blockIdx.z, t0 = item * DS_T * WT, t_hi = a.N;
+        if (a.off && !ds_find<DS_T * WT>(a.off, a.n_groups, item, grp, t0, t_hi)) continue;
+        const float* W = reinterpret_cast<const float*>(a.W) + (size_t)grp * a.M * ldw;
+        const float* V = GLU ? reinterpret_cast<const float*>(a.W_up) + (size_t)grp * a.M * ldw : nullptr;
+        const float* x = reinterpret_cast<const float*>(a.x) + (size_t)grp * a.x_step;
         // QUADS pieces of 16 bytes a row: thread's piece of every PER-th row
         auto fetch = [&](int kt) {
             float* st = ds_sm + (kt % STAGES) * STAGE;
@@ -125,9 +143,10 @@ static int ds_go(const DenseGemm& a, bool vec, cudaStream_t st) {
     DeviceCtx* c = ctx();
     if (!c) return JB_ERR_CUDA;
     if (!set[c->device]) { JB_CUDA(cudaFuncSetAttribute(dense_simt_kernel<GLU, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ds_smem<GLU, WT>())); set[c->device] = true; }
-    // an expert's tokens are known on the device alone: a few CTAs for each walk its tiles (as many as all tokens would need: 12672 CTAs for 600 tiles)
-    const int all = (a.N + DS_T * WT - 1) / (DS_T * WT), few = a.off ? 2 * ((a.N / a.n_groups + DS_T * WT - 1) / (DS_T * WT)) + 2 : all, tiles = all < few ? all : few;
-    JB_CUDA(launch_k(dense_simt_kernel<GLU, WT>, dim3((a.M + DS_M - 1) / DS_M, tiles < 65535 ? tiles : 65535, a.n_groups), dim3(DS_THREADS), ds_smem<GLU, WT>(), st, pdl_enabled(), a, vec));
+    // Groups of unlike sizes have no more tiles than this (see ds_find), wherever their tokens are (a few CTAs for each group, walking its tiles, took twice as long as
+    // before where all tokens went to one expert of many: 2048 tokens, gate and up of 768 x 1024, 316 -> 673 us; so 203).
+    const int width = DS_T * WT, tiles = a.off ? a.N / width + a.n_groups : (a.N + width - 1) / width;
+    JB_CUDA(launch_k(dense_simt_kernel<GLU, WT>, dim3((a.M + DS_M - 1) / DS_M, tiles < 65535 ? tiles : 65535, a.off ? 1 : a.n_groups), dim3(DS_THREADS), ds_smem<GLU, WT>(), st, pdl_enabled(), a, tiles, vec));
     count_launch();
     return JB_OK;
 }
@@ -149,7 +168,7 @@ int launch_dense_gemm_simt(const DenseGemm& a, cudaStream_t st) {
     return wt == 1 ? ds_go<false, 1>(a, vec, st) : wt == 2 ? ds_go<false, 2>(a, vec, st) : ds_go<false, 4>(a, vec, st);
 }
 // One token (the logits after a prompt) is a product of the decode family: 151936 x 2560 in bf16 take 122 us there, the weights at the
-// rate of memory, and 145 us in tiles of 16 tokens; the smallest tile of this file is 32 tokens wide.
+// rate of memory, and 145 us in tiles of 16 tokens, the narrowest of this file.
 static bool ds_one_token(const DenseGemm& a) {
     if (a.N != 1 || a.n_groups != 1 || a.off || a.swiglu || a.M <= 0 || a.K <= 0 || a.K % 8 || a.K > 8192 || (a.ldw > 0 && a.ldw != a.K) || (((uintptr_t)a.W | (uintptr_t)a.x) & 15)) return false;
     for (int i = 0; i < a.nseg; ++i) if (a.seg[i].pair != PAIR_NONE) return false;

@@ -40,7 +40,8 @@ def test_products(M, N, K, glu, aligned):
     assert (y[N] == 7).all()
 
 
-@pytest.mark.parametrize("counts", [[0, 16, 17, 0, 33, 1], [300, 0, 0, 0], [5] * 20])
+@pytest.mark.parametrize("counts", [[0, 16, 17, 0, 33, 1], [300, 0, 0, 0], [5] * 20, [0] * 31 + [40] + [0] * 32 + [17, 0, 3], [1] * 33, [3] * 31 + [500, 2] + [0] * 64 + [16],
+                                    [0] * 63 + [900]])
 def test_grouped_products(counts):
     import torch
     jb = pkg()
