@@ -270,7 +270,7 @@ jllm_b200_batch_decoder* jllm_b200_batch_decoder_create(const jllm_b200_model_de
                      attn_tma_encode(&maps[(((size_t)l * B + b) * 2 + 1) * 128], d->kv[b].val_ptr(l, 0), model->max_context, model->n_kv_heads);
         if (ok) d->maps.swap(maps);       // else: the general attention kernel serves the pointer lists
     }
-    if (wide) d->mmq.wide_scratch(false);
+    if (wide) d->mmq.wide_scratch(MMQ_WEIGHT_BYTES, false);
     splitk_buffer((size_t)B * model->n_heads * 64 * (model->head_dim + 4), true);
     return d;
 }

@@ -45,12 +45,12 @@ struct MmqOperand {                     // quantised activations: what they were
 };
 struct MmqWork {
     void* act = nullptr; size_t act_bytes = 0;       // quantised activations, K ranges of the fused kernel
-    void* wide = nullptr; bool no_wide = false;      // expanded weights and K ranges of the paired kernel; no_wide: the memory was refused once
+    void* wide = nullptr; size_t wide_bytes = 0, wide_refused = (size_t)-1;      // expanded weights, then K ranges of the paired kernel; the least that was refused once
     bool held = false;                               // act was handed out under capture
     size_t capture_limit = 0;                        // a captured call may allocate up to this much: what an uncaptured one has asked for before
     MmqOperand few, many;                            // the operands quantised last, in the layouts of mmq_stream.cu and of mmq_tc.cu
     void* scratch(size_t bytes, bool capturing);     // null: not to be had
-    void* wide_scratch(bool capturing);
+    void* wide_scratch(size_t weights, bool capturing);      // `weights` bytes (a multiple of 256) in front of the K ranges; null: not to be had
 };
 struct RopeTable { float theta; int half_dim; int max_seq; float* cos; float* sin; };
 struct DeviceCtx {

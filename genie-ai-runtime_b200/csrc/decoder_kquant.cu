@@ -11,6 +11,7 @@
 #include "mmq_few.cuh"
 #include "dense.cuh"
 #include "tp.cuh"
+#include <algorithm>
 #include <cfloat>
 #include <cstdlib>
 #include <new>
@@ -41,7 +42,6 @@ struct KquantDecoder : jllm_b200_decoder {
     __half *pf_x = nullptr, *pf_x2 = nullptr, *pf_normed = nullptr, *pf_y = nullptr, *pf_q = nullptr, *pf_att = nullptr, *pf_k = nullptr,
            *pf_v = nullptr, *pf_gate = nullptr, *pf_up = nullptr, *pf_sw = nullptr;
     MfModel few;                       // products of chunks of up to MF_MAX_TOKENS tokens
-    void* pf_wide = nullptr;           // in the slab: two buffers of expanded weights and the paired products' partial sums (null: chunks too short, or no memory)
     void* pf_operands = nullptr;       // in the slab: quantised activations and partial sums of such a chunk, or the operands of a longer one
 
     ~KquantDecoder() override {
@@ -295,7 +295,7 @@ static int dec_enqueue_step_tp(KquantDecoder* d, int n_splits, cudaStream_t st) 
 // gate/up, SwiGLU, W_down, residual.  After the last chunk: final norm and logits of the last token only, greedy token.
 int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     if (cap <= pf_cap) return JB_OK;
-    if (pf_slab) { cudaFree(pf_slab); pf_slab = pf_codes = pf_wide = nullptr; pf_cap = 0; }
+    if (pf_slab) { cudaFree(pf_slab); pf_slab = pf_codes = nullptr; pf_cap = 0; }
     const size_t N = (size_t)cap, H = m.hidden_dim, QD = (size_t)m.n_heads * m.head_dim, KVD = (size_t)m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
     // Where the weights allow it (by_rows), every chunk goes through the kernels that hand one product's results to the next as its operand: up to
@@ -307,13 +307,10 @@ int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     const size_t total = 2 * al(N * H * 2) + 2 * al(N * QD * 2) + al(rows * H * 2) + 2 * al(rows * KVD * 2) + 2 * al(rows * I * 2) + al(general * H * 2) + al(general * I * 2) + (by_rows ? operands : 0);
     // one allocation for all of it: it is made inside a session's first prompt, where each costs 0.4 - 2 ms (512 tokens: the first prompt
     // took 1064 us more than the next with two, 444 with one)
-    size_t wide = by_rows && mmq_wide_applies(m.hidden_dim, 0, cap, m.hidden_dim) ? 2 * MMQ_WEIGHT_BYTES + al(gemm_pair_part_floats() * sizeof(float)) : 0;
     size_t codes = cap >= attention_tc_min_tokens(m.n_heads, m.n_kv_heads) && m.max_context <= PF_CODES_MAX && m.head_dim == 128 ? attention_tc_scratch(m.n_kv_heads, m.max_context) : 0;
-    if (wide && cudaMalloc(&pf_slab, total + codes + wide) != cudaSuccess) { cudaGetLastError(); pf_slab = nullptr; wide = 0; }
-    if (!pf_slab && codes && cudaMalloc(&pf_slab, total + codes) != cudaSuccess) { cudaGetLastError(); pf_slab = nullptr; codes = 0; }
+    if (codes && cudaMalloc(&pf_slab, total + codes) != cudaSuccess) { cudaGetLastError(); pf_slab = nullptr; codes = 0; }
     if (!pf_slab && cudaMalloc(&pf_slab, total) != cudaSuccess) { cudaGetLastError(); pf_slab = nullptr; return set_error(JB_ERR_NOMEM, "decoder: %zu B of prefill activations", total); }
     pf_codes = codes ? (char*)pf_slab + total : nullptr;
-    pf_wide = wide ? (char*)pf_slab + total + codes : nullptr;
     char* p = (char*)pf_slab;
     auto take = [&](size_t b) { char* r = p; p += al(b); return r; };
     pf_x = (__half*)take(N * H * 2); pf_x2 = (__half*)take(N * H * 2);
@@ -343,11 +340,11 @@ int KquantDecoder::enqueue_rows_chunk(int N, int start, cudaStream_t st) {
     const int H = m.hidden_dim, QD = m.n_heads * m.head_dim, KVD = m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
     few.place_rows(pf_operands, N);
     // Expanded weights in two buffers by turns: the next product's while the present one runs, or the attention (512 tokens of 8 layers: 0.52 ms of
-    // 2.40 went into expansions in front of products).
+    // 2.40 went into expansions in front of products).  They are the stream's, which later sessions take over, and as large as the model's largest piece.
     std::vector<MmqPiece> pieces;
     std::vector<size_t> ends;                // of the products, in the order they are called in
     auto add = [&](const void* W1, const void* W2, int type, int M1, int M2, int K) {
-        if (pf_wide && mmq_wide_applies(M1, M2, N, K)) mmq_pieces(pieces, W1, W2, type, M1, M2, K);
+        if (mmq_wide_applies(M1, M2, N, K)) mmq_pieces(pieces, W1, W2, type, M1, M2, K);
         ends.push_back(pieces.size());
     };
     auto add_pair = [&](const void* W1, int t1, const void* W2, int t2, int M1, int M2, int K) {
@@ -361,8 +358,13 @@ int KquantDecoder::enqueue_rows_chunk(int N, int start, cudaStream_t st) {
         add_pair(w.w_gate, w.type_w_gate, w.w_up, w.type_w_up, I, I, H);
         add(w.w_down, nullptr, w.type_w_down, H, 0, I);
     }
+    size_t largest = 0;
+    for (const MmqPiece& p : pieces) largest = std::max(largest, (mmq_piece_bytes(p) + 255) & ~(size_t)255);
+    const MmqLease lease(nullptr, st);
+    char* wide = largest && lease.w ? (char*)lease.w->wide_scratch(2 * largest, lease.cap) : nullptr;
+    if (!wide) { pieces.clear(); std::fill(ends.begin(), ends.end(), 0); }       // product by product, with what memory there is
     size_t expanded = 0, multiplied = 0, called = 0;
-    auto buffer_of = [&](size_t i) { return (char*)pf_wide + (i & 1) * MMQ_WEIGHT_BYTES; };
+    auto buffer_of = [&](size_t i) { return wide + (i & 1) * largest; };
     auto ahead = [&]() -> int {              // behind piece multiplied - 1 or the attention: the buffer of the piece before is free
         if (expanded >= pieces.size() || expanded > multiplied) return JB_OK;
         const size_t i = expanded++;
@@ -376,7 +378,7 @@ int KquantDecoder::enqueue_rows_chunk(int N, int start, cudaStream_t st) {
         while (multiplied < end) {
             const size_t n = multiplied++;
             if (expanded == n) { ++expanded; DCHK(launch_mmq_expand(pieces[n], buffer_of(n), false, st)); }
-            DCHK(launch_mmq_piece(pieces[n], buffer_of(n), xq, y1, y2, N, (float*)((char*)pf_wide + 2 * MMQ_WEIGHT_BYTES), st, wait ? std::function<int()>() : ahead));
+            DCHK(launch_mmq_piece(pieces[n], buffer_of(n), xq, y1, y2, N, (float*)(wide + 2 * largest), st, wait ? std::function<int()>() : ahead));
         }
         return JB_OK;
     };
@@ -408,7 +410,6 @@ int KquantDecoder::enqueue_rows_chunk(int N, int start, cudaStream_t st) {
         DCHK(product(pf_y, w.w_down, w.type_w_down, H, I, act));
         DCHK(launch_mr_norm(pf_x2, pf_y, pf_x, more ? layers[l + 1].rms_attn : nullptr, m.rms_eps, H, more ? mf_operand(few.layers[l + 1].qkv, few.xh4, few.xh6) : MfOperand(), N, st));
     }
-    mmq_mark(st);
     return JB_OK;
 }
 
@@ -429,7 +430,11 @@ int KquantDecoder::enqueue_few_mlp(int l, int N, cudaStream_t st) {
 int KquantDecoder::enqueue_chunk(const int* dev_tokens, int N, int start, cudaStream_t st) {
     const int H = m.hidden_dim, QD = m.n_heads * m.head_dim, KVD = m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
     DCHK(launch_embed_rows(pf_x, m.tok_embd, m.embd_type, dev_tokens, N, H, st));
-    if (!few.layers.empty() && N > MF_MAX_TOKENS) return enqueue_rows_chunk(N, start, st);
+    if (!few.layers.empty() && N > MF_MAX_TOKENS) {
+        DCHK(enqueue_rows_chunk(N, start, st));
+        mmq_mark(st);                        // behind the chunk's lease
+        return JB_OK;
+    }
     const bool by_few = !few.layers.empty() && N > 1;       // one token: integer dots summed in fp32, by the general kernels
     if (by_few) few.place(pf_operands, N);
     if (by_few) DCHK(launch_mf_norm(nullptr, nullptr, pf_x, nullptr, layers[0].rms_attn, m.rms_eps, H, mf_operand(few.layers[0].qkv, few.xh4, few.xh6), N, st));

@@ -5,6 +5,7 @@
 // weight sub-scales as half products, Q6_K keeps fp32 d (mmq_q4k_llama.cu:383-404,
 // :159-163, :321-322; mmq_q6k_llama.cu:424-438, :208, :361).
 #include "mmq.cuh"
+#include "dense.cuh"
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -41,6 +42,18 @@ void* MmqWork::scratch(size_t bytes, bool capturing) {
     }
     held = held || capturing;
     return act;
+}
+// An object whose request was refused does not ask for as much again: it stays with the fused kernel, whose results differ in their last bits.  A captured
+// call asks too, so that it takes the way an uncaptured one takes; what it was given stays.
+void* MmqWork::wide_scratch(size_t weights, bool capturing) {
+    const size_t need = weights + gemm_pair_part_floats() * sizeof(float);
+    if (need <= wide_bytes) return wide;
+    if (need >= wide_refused || (capturing && (!capture_limit || wide))) return nullptr;
+    void* p = nullptr;
+    if (mmq_alloc(&p, need) != cudaSuccess) { wide_refused = need; return nullptr; }
+    if (wide) { const RelaxedCapture relaxed; cudaFree(wide); }
+    wide = p; wide_bytes = need;
+    return wide;
 }
 // one warp per 32-element group of one token
 __global__ void mmq_quantize_kernel(const __half* x, ActQ a, int N, int K, int ds4) {
@@ -122,17 +135,25 @@ int launch_add_half(__half* out, const __half* a, const __half* b, long long n, 
 static int launch_mmq_impl(__half* y, const void* W, int type, const __half* x, int M, int N, int K, int32_t* dbg, const __half* residual,
                            bool same_x, cudaStream_t st, MmqWork* w, bool cap);
 
-// The library's scratch: an object per stream, so that calls on different streams do not meet.  A call holds the lock while it enqueues
-// its launches (quantiser, product, sum), so that threads that share a stream do not mix theirs.  A stream that has none takes one
+// The library's scratch: an object per stream, so that calls on different streams do not meet.  A call holds its object while it enqueues
+// its launches (quantiser, product, sum; a session those of a whole chunk), so that threads that share a stream do not mix theirs; the lock on all of them is
+// held for the look-up alone.  A stream that has none takes one
 // whose last work is known to be over (sessions record an event at the end of a prompt: mmq_mark), else a new one; when there are
 // MMQ_STREAMS, the one that was not used for the longest time, behind its event (every call records one from half of them on).  Nothing
 // here waits on the host: a wait for the device would invalidate any capture in the process.
 // Captured calls have objects apart from these, which their graphs keep: one per stream handle (a stream's id cannot be asked for under
 // capture); a handle beyond MMQ_GRAPHS shares the one that was captured into least recently.
 constexpr int MMQ_STREAMS = 32, MMQ_GRAPHS = 32;
+struct MmqEntry {
+    unsigned long long id = 0, used = 0;
+    cudaEvent_t done = nullptr; bool marked = false;      // all work so far lies before the event: no one is using it (users) since
+    int users = 0;                                        // leases that hold it or wait for it
+    std::recursive_mutex mu;                              // a session's products take theirs inside the chunk's
+    MmqWork work;
+};
 struct MmqPool {
-    struct Entry { unsigned long long id = 0, used = 0; cudaEvent_t done = nullptr; bool marked = false; MmqWork work; };
-    std::mutex mu;
+    typedef MmqEntry Entry;
+    std::mutex mu;                               // everything but the entries' work
     Entry streams[MMQ_STREAMS], graphs[MMQ_GRAPHS];
     int n_streams = 0, n_graphs = 0;
     unsigned long long clock = 0;
@@ -153,16 +174,15 @@ struct MmqPool {
         for (int i = 0; i < n_streams; ++i) if (streams[i].id == id) return &streams[i];
         return nullptr;
     }
-    MmqWork* of_graph(cudaStream_t st) {
+    Entry* of_graph(cudaStream_t st) {
         const unsigned long long id = (unsigned long long)(uintptr_t)st;
         Entry* e = nullptr;
         for (int i = 0; i < n_graphs; ++i) if (graphs[i].id == id) e = &graphs[i];
         if (!e) e = n_graphs < MMQ_GRAPHS ? &graphs[n_graphs++] : oldest(graphs, n_graphs, false);
         e->id = id; e->used = ++clock;
-        e->work.capture_limit = asked;
-        return &e->work;
+        return e;
     }
-    MmqWork* of_stream(cudaStream_t st) {
+    Entry* of_stream(cudaStream_t st) {
         const RelaxedCapture relaxed;
         unsigned long long id;
         if (!id_of(st, id)) return nullptr;
@@ -178,37 +198,44 @@ struct MmqPool {
             e->work.few = e->work.many = MmqOperand();
         }
         e->id = id; e->used = ++clock; e->marked = false;
-        return &e->work;
+        return e;
     }
     void mark(cudaStream_t st) {
         const RelaxedCapture relaxed;
         unsigned long long id;
         Entry* e = id_of(st, id) ? find(id) : nullptr;
-        if (!e || (!e->done && cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming) != cudaSuccess)) { cudaGetLastError(); return; }
+        if (!e || e->users || (!e->done && cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming) != cudaSuccess)) { cudaGetLastError(); return; }
         e->marked = cudaEventRecord(e->done, st) == cudaSuccess;
         if (!e->marked) cudaGetLastError();
     }
 };
 static MmqPool g_mmq_pool[16];                   // per device
-struct MmqLease {
-    std::unique_lock<std::mutex> lock;
-    MmqPool* pool = nullptr;
-    MmqWork* w = nullptr;
-    cudaStream_t st;
-    bool cap;
-    MmqLease(MmqWork* own, cudaStream_t stream) : w(own), st(stream), cap(capturing(stream)) {
-        DeviceCtx* c = own ? nullptr : ctx();
-        if (!c) return;
-        pool = &g_mmq_pool[c->device];
-        lock = std::unique_lock<std::mutex>(pool->mu);
-        w = cap ? pool->of_graph(st) : pool->of_stream(st);
+MmqLease::MmqLease(MmqWork* own, cudaStream_t stream) : w(own), st(stream), cap(capturing(stream)) {
+    DeviceCtx* c = own ? nullptr : ctx();
+    if (!c) return;
+    pool = &g_mmq_pool[c->device];
+    size_t asked;
+    {
+        std::lock_guard<std::mutex> lock(pool->mu);
+        e = cap ? pool->of_graph(st) : pool->of_stream(st);
+        if (!e) return;
+        ++e->users;
+        asked = pool->asked;
     }
-    ~MmqLease() {
-        if (!pool || !w || cap) return;
-        if (w->act_bytes > pool->asked) pool->asked = w->act_bytes;
-        if (pool->n_streams > MMQ_STREAMS / 2) pool->mark(st);
-    }
-};
+    e->mu.lock();
+    w = &e->work;
+    if (cap) w->capture_limit = asked;
+}
+MmqLease::~MmqLease() {
+    if (!e) return;
+    const size_t bytes = w->act_bytes;
+    e->mu.unlock();
+    std::lock_guard<std::mutex> lock(pool->mu);
+    --e->users;
+    if (cap) return;
+    if (bytes > pool->asked) pool->asked = bytes;
+    if (pool->n_streams > MMQ_STREAMS / 2) pool->mark(st);
+}
 
 void mmq_mark(cudaStream_t st) {
     DeviceCtx* c = ctx();
@@ -245,7 +272,7 @@ int launch_mmq_pair(__half* y1, __half* y2, const void* W1, int type1, const voi
     const size_t need = mmq_tc_scratch_bytes_pair(type1, M1, M2, N, K);
     __half* xq = w ? (__half*)w->scratch(need, l.cap) : nullptr;
     if (!xq) return set_error(JB_ERR_NOMEM, "batched gemm: %zu B of activation scratch unavailable", need);
-    return launch_mmq_tc_pair(y1, y2, W1, W2, type1, x, xq, M1, M2, N, K, false, st, *w, mmq_wide_applies(M1, M2, N, K) ? w->wide_scratch(l.cap) : nullptr);
+    return launch_mmq_tc_pair(y1, y2, W1, W2, type1, x, xq, M1, M2, N, K, false, st, *w, mmq_wide_applies(M1, M2, N, K) ? w->wide_scratch(MMQ_WEIGHT_BYTES, l.cap) : nullptr);
 }
 
 int launch_mmq_ready(__half* y1, __half* y2, const void* W1, const void* W2, int type, const __half* xq, int M1, int M2, int N, int K, cudaStream_t st, MmqWork* own) {
@@ -255,7 +282,7 @@ int launch_mmq_ready(__half* y1, __half* y2, const void* W1, const void* W2, int
     __half* scratch = l.w ? (__half*)l.w->scratch(need, l.cap) : nullptr;
     if (!scratch) return set_error(JB_ERR_NOMEM, "batched gemm: %zu B of scratch unavailable", need);
     l.w->few = l.w->many = MmqOperand();         // sums of K ranges may lie where another call left its operand
-    return launch_mmq_tc_pair(y1, y2, W1, W2, type, nullptr, scratch, M1, M2, N, K, false, st, *l.w, mmq_wide_applies(M1, M2, N, K) ? l.w->wide_scratch(l.cap) : nullptr, xq);
+    return launch_mmq_tc_pair(y1, y2, W1, W2, type, nullptr, scratch, M1, M2, N, K, false, st, *l.w, mmq_wide_applies(M1, M2, N, K) ? l.w->wide_scratch(MMQ_WEIGHT_BYTES, l.cap) : nullptr, xq);
 }
 
 static int launch_mmq_impl(__half* y, const void* W, int type, const __half* x, int M, int N, int K, int32_t* dbg, const __half* residual,
@@ -281,7 +308,7 @@ static int launch_mmq_impl(__half* y, const void* W, int type, const __half* x, 
         const size_t need_tc = mmq_tc_scratch_bytes(type, M, N, K);
         __half* xq = w ? (__half*)w->scratch(need_tc, cap) : nullptr;
         if (!xq) return set_error(JB_ERR_NOMEM, "batched gemm: %zu B of activation scratch unavailable", need_tc);
-        return launch_mmq_tc_pair(y, nullptr, W, nullptr, type, x, xq, M, 0, N, K, same_x, st, *w, mmq_wide_applies(M, 0, N, K) ? w->wide_scratch(cap) : nullptr);
+        return launch_mmq_tc_pair(y, nullptr, W, nullptr, type, x, xq, M, 0, N, K, same_x, st, *w, mmq_wide_applies(M, 0, N, K) ? w->wide_scratch(MMQ_WEIGHT_BYTES, cap) : nullptr);
     }
     const size_t need = mmq_scratch_bytes(N, K);
     uint8_t* base = w ? (uint8_t*)w->scratch(need, cap) : nullptr;

@@ -21,6 +21,17 @@ int launch_mmq_pair(__half* y1, __half* y2, const void* W1, int type1, const voi
 // The tensor-core path over activations that are quantised already: xq [N][columns of mmq_tc.cu's operand for `type`]
 int launch_mmq_ready(__half* y1, __half* y2, const void* W1, const void* W2, int type, const __half* xq, int M1, int M2, int N, int K, cudaStream_t st, MmqWork* own = nullptr);
 size_t mmq_scratch_bytes(int N, int K);
+// The library's scratch for a stream (own: a session's), kept from other threads while it lives; w null: there is none to be had
+struct MmqPool; struct MmqEntry;
+struct MmqLease {
+    MmqWork* w; cudaStream_t st; bool cap;       // cap: the stream is being captured
+    MmqLease(MmqWork* own, cudaStream_t stream);
+    ~MmqLease();
+    MmqLease(const MmqLease&) = delete;
+    MmqLease& operator=(const MmqLease&) = delete;
+private:
+    MmqPool* pool = nullptr; MmqEntry* e = nullptr;
+};
 void mmq_mark(cudaStream_t st);       // all products on st so far may be taken for over once the stream has come here
 cudaError_t mmq_alloc(void** p, size_t bytes);      // cudaMalloc, whether this thread or another one captures
 // tensor-core path (mmq_tc.cu): tcgen05.mma over fp16 operands built from the same quantised values
@@ -31,8 +42,9 @@ int    launch_mmq_tc_pair(__half* y, __half* y2, const void* W, const void* W2, 
 size_t mmq_tc_scratch_bytes_pair(int type, int M, int M2, int N, int K);
 // many tokens: the weights are expanded to the fp16 operand once, then multiplied by gemm_pair.cu
 bool   mmq_wide_applies(int M, int M2, int N, int K);
-constexpr size_t MMQ_WEIGHT_BYTES = (size_t)64 << 20;      // expanded weights of a piece
+constexpr size_t MMQ_WEIGHT_BYTES = (size_t)64 << 20;      // expanded weights of a piece, at most
 struct MmqPiece { const void* W; const void* W2; int type, M, M2, K, r0, rows; };      // rows r0 .. of W's and W2's (null: none) rows in a row
+size_t mmq_piece_bytes(const MmqPiece& p);                 // of its expanded weights
 void   mmq_pieces(std::vector<MmqPiece>& out, const void* W1, const void* W2, int type, int M1, int M2, int K);
 int    launch_mmq_expand(const MmqPiece& p, void* wq, bool ahead, cudaStream_t st);
 // behind: launches to go right behind the product, before the sum of its K ranges; part: gemm_pair_part_floats

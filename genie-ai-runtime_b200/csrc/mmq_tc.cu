@@ -521,13 +521,6 @@ constexpr int MW_MIN_TOKENS = 384;      // 256 tokens: Q6_K 2560 x 9728 46 us th
 bool mmq_wide_applies(int M, int M2, int N, int K) {
     return N >= ((long long)M + M2 < 2048 ? MW_MIN_TOKENS + 64 : MW_MIN_TOKENS) && (long long)M + M2 >= 256 && (size_t)(K + K / 16 + TC_K) * sizeof(__half) * 256 <= MW_WEIGHT_BYTES;
 }
-// Asked for once: an object whose request was refused stays with the fused kernel, whose results differ in their last bits.  A captured
-// call asks too, so that it takes the way an uncaptured one takes.
-void* MmqWork::wide_scratch(bool capturing) {
-    if (wide || no_wide || (capturing && !capture_limit)) return wide;
-    no_wide = mmq_alloc(&wide, MW_WEIGHT_BYTES + gemm_pair_part_floats() * sizeof(float)) != cudaSuccess;
-    return wide;
-}
 
 // Rows [r0, r0 + rows) of the operand, Kp halves each; a thread takes 8 bytes of packed codes: 16 weights of a Q4_K block, 32 of a
 // Q6_K block, or 8 of the extra columns.  Bound by the writes (2 bytes per weight, into L2).
@@ -607,6 +600,7 @@ __global__ void __launch_bounds__(256) mmq_expand_kernel(const TcArgs a, __half*
 }
 
 static int mw_width(int type, int K) { return K + (type == T_Q4K ? (2 * (K / 32) + TC_K - 1) / TC_K * TC_K : 0); }
+size_t mmq_piece_bytes(const MmqPiece& p) { return (size_t)p.rows * mw_width(p.type, p.K) * sizeof(__half); }
 void mmq_pieces(std::vector<MmqPiece>& out, const void* W1, const void* W2, int type, int M1, int M2, int K) {
     const long long all = (long long)M1 + M2, most = (long long)(MW_WEIGHT_BYTES / ((size_t)mw_width(type, K) * sizeof(__half))) & ~255ll;
     const long long pieces = (all + most - 1) / most, step = ((all + pieces - 1) / pieces + 255) & ~255ll;

@@ -257,6 +257,54 @@ def test_two_sessions_prompt_at_once():
     assert jb.device_status() == 0
 
 
+def test_a_second_session_takes_over_the_expanded_weights():
+    """Two buffers of expanded weights and the sums of split products are the stream's, not a session's: 147 MB more for each session otherwise."""
+    import torch
+    jb = pkg()
+    m = orc.gen_model(83, n_layers=1, hidden=512, n_heads=4, n_kv=1, hd=128, ffn=1024, vocab=512)
+    w = jb.decoder.upload(m)
+    prompt = np.random.Generator(np.random.PCG64(83)).integers(0, 512, 600)
+    sessions, taken, logits = [], [], []
+    for _ in range(4):
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        d = jb.decoder.Decoder(m["cfg"], w, 700, jb.decoder.FUSED | jb.decoder.PREFILL)
+        d.prefill(prompt, 0, torch.cuda.Stream())
+        logits.append(d.logits())
+        taken.append(free - torch.cuda.mem_get_info()[0])
+        sessions.append(d)
+    # caches of 700 positions and buffers of 600 tokens: a few MB, in whole 2 MB pieces of the driver's
+    assert all(t < 32 << 20 for t in taken[1:]), taken
+    assert all(torch.equal(l, logits[0]) for l in logits)
+    for d in sessions:
+        d.close()
+    assert jb.device_status() == 0
+
+
+def test_two_sessions_prompt_on_one_stream_from_two_threads():
+    """A chunk's expansions run ahead of its products in buffers of the stream: a session on the same stream in another thread waits its turn."""
+    import threading
+    import torch
+    jb = pkg()
+    m = orc.gen_model(84, n_layers=3, hidden=1024, n_heads=8, n_kv=2, hd=128, ffn=2048, vocab=512)
+    w = jb.decoder.upload(m)
+    st = torch.cuda.Stream()
+    d = [jb.decoder.Decoder(m["cfg"], w, 700, jb.decoder.FUSED | jb.decoder.PREFILL) for _ in range(2)]
+    prompts = [np.random.Generator(np.random.PCG64(1400 + i)).integers(0, 512, n) for i, n in enumerate((640, 500))]
+    want = []
+    for i in range(2):
+        d[i].prefill(prompts[i], 0, st)
+        want.append(d[i].logits().clone())
+    for _ in range(10):
+        ts = [threading.Thread(target=lambda i=i: [d[i].prefill(prompts[i], 0, st) for _ in range(5)]) for i in range(2)]
+        for t in ts: t.start()
+        for t in ts: t.join()
+        assert all(torch.equal(d[i].logits(), want[i]) for i in range(2))
+    for x in d:
+        x.close()
+    assert jb.device_status(st) == 0
+
+
 def test_capture_on_another_stream_than_the_warm_up():
     """A product captured on a stream that has no scratch yet: refused while the device has not seen a call that asked for as much (in a process of its own),
     else the graph gives the uncaptured result, by the expanded path too."""
