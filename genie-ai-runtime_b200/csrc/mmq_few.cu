@@ -29,6 +29,7 @@
 #include "mmq_few.cuh"
 #include "mmq.cuh"
 #include "tc.cuh"
+#include <cstdio>
 #include <cstdlib>
 #include <cstring>
 
@@ -757,6 +758,9 @@ static int mf_launch(const MfProduct& p, const MfOperand& x, float* part, __half
         JB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MF_SMEM));
         c->mf_attr[y ? 1 : 0] = true;
     }
+    static const bool verbose = getenv("JLLM_B200_MMQ_DEBUG") != nullptr;
+    for (int i = 0; verbose && i < p.nseg; ++i)
+        fprintf(stderr, "[mmq_few] type %d M=%d N=%d K=%d: %d of %d CTAs, %d tiles of %d super-blocks\n", p.seg[i].q6 ? T_Q6K : T_Q4K, p.seg[i].M, N, p.K, p.seg[i].ctas, grid, p.seg[i].tiles, a.nb);
     JB_CUDA(launch_k(kern, dim3(grid), dim3(MF_THREADS), MF_SMEM, st, pdl_enabled(), p.map[0], p.map[p.nseg > 1 ? 1 : 0], p.map[p.nseg > 2 ? 2 : 0], a));
     count_launch();
     if (y && grid > 1) {
@@ -804,8 +808,12 @@ int launch_mf_quantise(const __half* x, const MfOperand& q, int K, int N, cudaSt
 static size_t mf_align(size_t b) { return (b + 255) & ~(size_t)255; }
 bool MfModel::plan(const jllm_b200_model_desc& m, bool with_out) {
     layers.clear();
-    const char* only = getenv("JLLM_B200_MMQ");            // "cuda" keeps all products on the CUDA cores
-    if (only && !strcmp(only, "cuda")) return false;
+    // the switches that choose among the general kernels are theirs: a session under one of them runs these
+    static const bool off = [] {
+        const char *mmq = getenv("JLLM_B200_MMQ"), *stream = getenv("JLLM_B200_MMQ_STREAM"), *pair = getenv("JLLM_B200_MMQ_PAIR");
+        return (mmq && !strcmp(mmq, "cuda")) || (stream && stream[0] == '0') || (pair && pair[0] == '0');
+    }();
+    if (off) return false;
     hidden = m.hidden_dim; q_dim = m.n_heads * m.head_dim; ffn = m.intermediate_dim;
     const int kv_dim = m.n_kv_heads * m.head_dim;
     // a head is a 128-row tile; norms keep a token in one CTA's registers

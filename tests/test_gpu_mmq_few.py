@@ -9,6 +9,9 @@ maximum 0.43 of the logit RMS against the oracle over the streams of a model of 
 bounds; the logits of one token, where a flipped group weighs more than in the mean over streams, to the error RMS of 0.15 that
 tests/test_gpu_decoder.py derives for them."""
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -132,7 +135,7 @@ def test_streams_as_the_general_kernels(shape, swap, streams):
     jb = pkg()
     cfg, w = weights(shape, swap)
     prompts = np.random.Generator(np.random.PCG64(streams)).integers(0, cfg["vocab"], (streams, 3)).astype(np.int32)
-    sides = []
+    sides, kernels = [], []
     for ws in (w, elsewhere(w)):
         d = jb.decoder.BatchDecoder(cfg, ws, 16, streams)
         st = torch.cuda.Stream()
@@ -141,8 +144,10 @@ def test_streams_as_the_general_kernels(shape, swap, streams):
         d.generate(prompts, 1, st)
         assert torch.equal(first, d.logits())              # a session can be used again, and sums in a fixed order
         sides.append(first.double().cpu().numpy())
+        kernels.append(d.kernels_per_step())
         assert jb.device_status(st) == 0
         d.close()
+    assert kernels[0] < kernels[1]                         # the two sides are two ways
     check_logits(*sides, ERR_RMS)
 
 
@@ -192,3 +197,42 @@ def test_a_missing_norm_vector_is_refused(name):
     with pytest.raises(jb.JllmError):
         d.generate(np.zeros((5, 3), np.int32), 1)
     d.close()
+
+
+@pytest.mark.parametrize("switch", ["JLLM_B200_MMQ_STREAM=0", "JLLM_B200_MMQ_PAIR=0", "JLLM_B200_MMQ=cuda", "JLLM_B200_MMQ_DEBUG=1"])
+def test_switches_of_the_products_hold_for_sessions(switch):
+    """A switch that chooses among the general kernels makes sessions run them, whatever the weights; the one that prints prints here too."""
+    code = """
+import numpy as np, torch
+import test_gpu_mmq_few as t
+jb = t.pkg()
+cfg, w = t.weights("even", False)
+st = torch.cuda.Stream()
+for n in (20, 150):
+    counts = []
+    for ws in (w, t.elsewhere(w)):
+        d = jb.decoder.Decoder(cfg, ws, 256, jb.decoder.FUSED | jb.decoder.PREFILL)
+        n0 = jb.launch_count()
+        d.prefill(np.arange(n, dtype=np.int32), 0, st)
+        counts.append(jb.launch_count() - n0)
+        d.close()
+    b = []
+    for ws in (w, t.elsewhere(w)):
+        d = jb.decoder.BatchDecoder(cfg, ws, 8, 5)
+        d.generate(np.zeros((5, 2), np.int32), 1, st)
+        b.append(d.kernels_per_step())
+        d.close()
+    print("counts", *counts, *b)
+assert jb.device_status(st) == 0
+"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    name, value = switch.split("=")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, PYTHONPATH=os.pathsep.join([os.path.dirname(here), here]), **{name: value}))
+    assert r.returncode == 0, r.stderr[-2000:]
+    counts = [[int(x) for x in l.split()[1:]] for l in r.stdout.splitlines() if l.startswith("counts")]
+    assert len(counts) == 2
+    if name == "JLLM_B200_MMQ_DEBUG":
+        assert "[mmq_few]" in r.stderr and all(c[0] < c[1] and c[2] < c[3] for c in counts)
+    else:
+        assert all(c[0] == c[1] and c[2] == c[3] for c in counts), counts
