@@ -17,7 +17,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as orc
-from gpu_util import pkg
+from gpu_util import pkg, ulp16
 
 pytestmark = pytest.mark.gpu
 
@@ -27,6 +27,10 @@ SHAPES = {
     "even": dict(n_layers=2, hidden=512, n_heads=4, n_kv=2, hd=128, ffn=1024, vocab=2048),
     "odd": dict(n_layers=2, hidden=768, n_heads=6, n_kv=2, hd=128, ffn=1280, vocab=1000),
     "whole": dict(n_layers=1, hidden=2048, n_heads=2, n_kv=1, hd=128, ffn=2048, vocab=2056),
+    # the norms' forms: up to 32, 64 and 128 tiles of a token, up to 32 and 64 super-blocks, the last warps with fewer
+    "w4096": dict(n_layers=1, hidden=4096, n_heads=2, n_kv=1, hd=128, ffn=512, vocab=512),
+    "w4352": dict(n_layers=1, hidden=4352, n_heads=2, n_kv=1, hd=128, ffn=512, vocab=512),
+    "w8448": dict(n_layers=1, hidden=8448, n_heads=2, n_kv=1, hd=128, ffn=512, vocab=512),
 }
 
 
@@ -73,6 +77,14 @@ def device_bytes(ptr, n):
     return out.cpu().numpy()
 
 
+def first_keys(d, n, kv):
+    """Key codes [n][kv][128] and scales [n][kv] of the first layer."""
+    buf = pkg().lib.jllm_b200_decoder_buffer
+    buf.restype = C.c_void_p
+    return (device_bytes(buf(C.c_void_p(d._h), 7), n * kv * 128).view(np.int8).reshape(n, kv, 128).astype(np.int32),
+            device_bytes(buf(C.c_void_p(d._h), 8), n * kv * 4).view(np.float32).reshape(n, kv))
+
+
 def check_logits(got, want, bound):
     rms = float(np.sqrt(np.mean(want ** 2)))
     err = np.abs(got - want)
@@ -80,14 +92,10 @@ def check_logits(got, want, bound):
     assert np.isfinite(got).all() and np.sqrt(np.mean(err ** 2)) <= bound * rms and err.max() <= ERR_MAX * rms
 
 
-# padded to 16 tokens; two accumulators up to 48, three super-blocks of weights in tensor memory up to 96, two above, two accumulators again up to 112
-@pytest.mark.parametrize("shape,swap", [("even", False), ("odd", False), ("odd", True), ("whole", False)])
-# beyond 128: rows of many tokens, tiles of 32..256 tokens with and without K ranges, and from 384 or 448 on the expanded weights
-@pytest.mark.parametrize("n", [2, 16, 17, 48, 49, 96, 97, 112, 113, 128, 129, 257, 450])
-def test_prompt_chunk_as_the_general_kernels(shape, swap, n):
+def chunk_as_the_general_kernels(cfg, w, n):
+    """A prompt of n tokens by both sides: key codes and scales of the first layer, logits."""
     import torch
     jb = pkg()
-    cfg, w = weights(shape, swap)
     prompt = np.random.Generator(np.random.PCG64(n)).integers(0, cfg["vocab"], n)
     kv = cfg["n_kv_heads"]
     sides = []
@@ -97,10 +105,7 @@ def test_prompt_chunk_as_the_general_kernels(shape, swap, n):
         n0 = jb.launch_count()
         d.prefill(prompt, 0, st)
         launches = jb.launch_count() - n0
-        buf = jb.lib.jllm_b200_decoder_buffer
-        buf.restype = C.c_void_p
-        codes = device_bytes(buf(C.c_void_p(d._h), 7), n * kv * 128).view(np.int8).reshape(n, kv, 128).astype(np.int32)
-        scales = device_bytes(buf(C.c_void_p(d._h), 8), n * kv * 4).view(np.float32).reshape(n, kv)
+        codes, scales = first_keys(d, n, kv)
         sides.append((codes, scales, d.logits().cpu().numpy().astype(np.float64), launches))
         assert jb.device_status(st) == 0
         d.close()
@@ -109,6 +114,122 @@ def test_prompt_chunk_as_the_general_kernels(shape, swap, n):
     assert np.all(np.abs(scales - scales0) <= 2.0 ** -10 * np.abs(scales0))
     assert np.abs(codes - codes0).max() <= 1 and np.mean(codes != codes0) <= 0.05
     check_logits(logits, logits0, ONE_TOKEN_RMS)
+
+
+# padded to 16 tokens; two accumulators up to 48, three super-blocks of weights in tensor memory up to 96, two above, two accumulators again up to 112
+@pytest.mark.parametrize("shape,swap", [("even", False), ("odd", False), ("odd", True), ("whole", False)])
+# beyond 128: rows of many tokens, tiles of 32..256 tokens with and without K ranges, and from 384 or 448 on the expanded weights
+@pytest.mark.parametrize("n", [2, 16, 17, 48, 49, 96, 97, 112, 113, 128, 129, 257, 450])
+def test_prompt_chunk_as_the_general_kernels(shape, swap, n):
+    chunk_as_the_general_kernels(*weights(shape, swap), n)
+
+
+@pytest.mark.parametrize("shape", ["w4096", "w4352", "w8448"])
+@pytest.mark.parametrize("n", [17, 129])
+def test_wide_models(shape, n):
+    chunk_as_the_general_kernels(*weights(shape, False), n)
+
+
+@pytest.mark.parametrize("n", [17, 129])
+@pytest.mark.parametrize("neox,norms", [(0, True), (0, False), (1, False)])
+def test_adjacent_pairs_and_heads_without_norms(monkeypatch, neox, norms, n):
+    """rope_neox = 0 turns adjacent elements; models without head norms give null vectors."""
+    jb = pkg()
+
+    class Desc(jb.decoder.ModelDesc):
+        def __setattr__(self, name, value):
+            super().__setattr__(name, neox if name == "rope_neox" else value)
+
+    monkeypatch.setattr(jb.decoder, "ModelDesc", Desc)
+    cfg, w = weights("odd", False)
+    if not norms:
+        w["layers"] = [{k: v for k, v in l.items() if k not in ("q_norm", "k_norm")} for l in w["layers"]]
+    chunk_as_the_general_kernels(cfg, w, n)
+    if n == 17:
+        prompts = np.random.Generator(np.random.PCG64(3)).integers(0, cfg["vocab"], (5, 3)).astype(np.int32)
+        streams_as_the_general_kernels(cfg, w, prompts)
+
+
+@pytest.mark.parametrize("n,at", [(20, 7), (150, 100)])
+def test_an_infinite_token_reaches_no_other_tokens_row(n, at):
+    """Token `at` of a prompt is infinite: every other key of the first layer has the codes and the scale that it has without it."""
+    import torch
+    jb = pkg()
+    cfg, w = weights("odd", False)
+    bad = dict(w, tok_embd=(w["tok_embd"][0].clone(), w["tok_embd"][1]))
+    bad["tok_embd"][0].reshape(cfg["vocab"], -1, 144)[3, 1, 0:2] = torch.tensor([0x00, 0x7C], dtype=torch.uint8, device="cuda")      # an infinite block scale of token 3
+    prompt = np.random.Generator(np.random.PCG64(n)).integers(4, cfg["vocab"], n)
+    prompt[at] = 3
+    st = torch.cuda.Stream()
+    sides = []
+    for ws in (w, bad):
+        d = jb.decoder.Decoder(cfg, ws, 512, jb.decoder.FUSED | jb.decoder.PREFILL)
+        d.prefill(prompt, 0, st)
+        sides.append(first_keys(d, n, cfg["n_kv_heads"]))
+        assert jb.device_status(st) == 0
+        d.close()
+    others = np.arange(n) != at
+    assert all(np.array_equal(a[others], b[others]) for a, b in zip(*sides))
+    assert not np.array_equal(sides[0][0][at], sides[1][0][at])
+
+
+def test_an_infinite_stream_reaches_no_other_stream():
+    import torch
+    jb = pkg()
+    cfg, w = weights("odd", False)
+    bad = dict(w, tok_embd=(w["tok_embd"][0].clone(), w["tok_embd"][1]))
+    bad["tok_embd"][0].reshape(cfg["vocab"], -1, 144)[3, 1, 0:2] = torch.tensor([0x00, 0x7C], dtype=torch.uint8, device="cuda")
+    prompts = np.random.Generator(np.random.PCG64(9)).integers(4, cfg["vocab"], (19, 3)).astype(np.int32)
+    prompts[5, 1] = 3
+    st = torch.cuda.Stream()
+    sides = []
+    for ws in (w, bad):
+        d = jb.decoder.BatchDecoder(cfg, ws, 16, 19)
+        tokens = d.generate(prompts, 1, st)
+        sides.append((d.logits(), tokens))
+        assert jb.device_status(st) == 0
+        d.close()
+    others = torch.arange(19, device="cuda") != 5
+    assert torch.equal(sides[0][0][others], sides[1][0][others])
+    assert not torch.isfinite(sides[1][0][5]).any() and sides[1][1][0, 5] == 0      # no logit is a candidate: token 0
+
+
+# output matrices of Q6_K rows of 2, 3 and 8 super-blocks and of Q4_K ones; fewer units than SMs, and tiles that two and three CTAs share
+@pytest.mark.parametrize("hidden,vocab,q4", [(512, 2048, False), (768, 24000, False), (768, 1000, True), (2048, 2056, False), (1024, 20000, True)])
+@pytest.mark.parametrize("streams", [2, 17, 128])
+def test_logits_product_over_known_activations(hidden, vocab, q4, streams):
+    """Layers that add nothing and tokens of small whole numbers, whose norm is the same in any order of summation: the logits are the output product over
+    activations that the stand-alone product can be given bit for bit."""
+    import torch
+    jb = pkg()
+    m = orc.gen_model(11, n_layers=1, hidden=hidden, n_heads=2, n_kv=1, hd=128, ffn=256, vocab=vocab)
+    w = jb.decoder.upload(m)
+    r = np.random.Generator(np.random.PCG64(12))
+    if q4:
+        w["output"] = (torch.from_numpy(orc.gen_q4k(r, vocab, hidden, orc.model_sigma(orc.Q4_K, hidden), orc.MODEL_MIN_RATIO)).cuda(), orc.Q4_K)
+    for name in ("wo", "down"):
+        w["layers"][0][name][0].zero_()
+    embed = torch.randint(0, 256, (vocab * hidden // 256, 144), dtype=torch.uint8, device="cuda", generator=torch.Generator(device="cuda").manual_seed(13))
+    embed[:, :16] = torch.tensor([0x00, 0x3C, 0, 0] + [1] * 4 + [0] * 4 + [1] * 4, dtype=torch.uint8, device="cuda")      # d = 1, dmin = 0, scales 1: a weight is its code
+    w["tok_embd"] = (embed.reshape(-1), orc.Q4_K)
+    prompts = r.integers(0, vocab, (streams, 1)).astype(np.int32)
+    st = torch.cuda.Stream()
+    d = jb.decoder.BatchDecoder(m["cfg"], w, 8, streams)
+    d.generate(prompts, 1, st)
+    got = d.logits().double().cpu().numpy()
+    assert jb.device_status(st) == 0
+    d.close()
+    codes = embed.reshape(vocab, -1, 144)[torch.from_numpy(prompts[:, 0].astype(np.int64)).cuda()][..., 16:].reshape(streams, -1, 4, 32)
+    x = torch.cat([codes & 15, codes >> 4], -1).reshape(streams, hidden).half()
+    normed, y = torch.empty_like(x), torch.zeros((streams, vocab), dtype=torch.float16, device="cuda")
+    jb.fused_rmsnorm_residual(normed, x, None, w["out_norm"], streams, hidden, m["cfg"]["eps"], 1)
+    jb.gemm_quant_batched(y, w["output"][0], w["output"][1], normed, vocab, streams, hidden)
+    torch.cuda.synchronize()
+    want = y.double().cpu().numpy()
+    # the same fp16 operands, summed in fp32 in another order: hidden 2^-24 of the sum of magnitudes, which is sqrt(hidden) of an output's size or so
+    # (2.4e-3 of the RMS at 2048), and each side rounds to fp16; a super-block too many or too few is 0.3 of it at least
+    rms = np.sqrt(np.mean(want ** 2))
+    assert (np.abs(got - want) <= 2 * ulp16(want) + hidden ** 1.5 * 2.0 ** -24 * rms).all(), np.abs(got - want).max() / rms
 
 
 def test_a_chunk_of_one_token_keeps_its_integer_products():
@@ -121,23 +242,18 @@ def test_a_chunk_of_one_token_keeps_its_integer_products():
     for ws in (w, elsewhere(w)):
         d = jb.decoder.Decoder(cfg, ws, 64, jb.decoder.FUSED | jb.decoder.PREFILL)
         d.prefill(np.array([5, 6, 7]), 0, st, chunk=2)
-        buf = jb.lib.jllm_b200_decoder_buffer
-        buf.restype = C.c_void_p
-        sides.append((device_bytes(buf(C.c_void_p(d._h), 7), 3 * kv * 128)[2 * kv * 128:], device_bytes(buf(C.c_void_p(d._h), 8), 3 * kv * 4)[2 * kv * 4:]))
+        sides.append([a[2] for a in first_keys(d, 3, kv)])
         assert jb.device_status(st) == 0
         d.close()
     assert all(np.array_equal(a, b) for a, b in zip(*sides))
 
 
-@pytest.mark.parametrize("shape,swap,streams", [("even", False, 2), ("odd", True, 33), ("odd", False, 96), ("whole", False, 128), ("even", True, 113)])
-def test_streams_as_the_general_kernels(shape, swap, streams):
+def streams_as_the_general_kernels(cfg, w, prompts):
     import torch
     jb = pkg()
-    cfg, w = weights(shape, swap)
-    prompts = np.random.Generator(np.random.PCG64(streams)).integers(0, cfg["vocab"], (streams, 3)).astype(np.int32)
     sides, kernels = [], []
     for ws in (w, elsewhere(w)):
-        d = jb.decoder.BatchDecoder(cfg, ws, 16, streams)
+        d = jb.decoder.BatchDecoder(cfg, ws, 16, len(prompts))
         st = torch.cuda.Stream()
         d.generate(prompts, 1, st)
         first = d.logits()
@@ -149,6 +265,12 @@ def test_streams_as_the_general_kernels(shape, swap, streams):
         d.close()
     assert kernels[0] < kernels[1]                         # the two sides are two ways
     check_logits(*sides, ERR_RMS)
+
+
+@pytest.mark.parametrize("shape,swap,streams", [("even", False, 2), ("odd", True, 33), ("odd", False, 96), ("whole", False, 128), ("even", True, 113), ("w4352", False, 9)])
+def test_streams_as_the_general_kernels(shape, swap, streams):
+    cfg, w = weights(shape, swap)
+    streams_as_the_general_kernels(cfg, w, np.random.Generator(np.random.PCG64(streams)).integers(0, cfg["vocab"], (streams, 3)).astype(np.int32))
 
 
 @pytest.mark.parametrize("name", ["rms_attn", "rms_ffn", "q_norm", "k_norm", "out_norm"])
