@@ -152,13 +152,13 @@ static int bdec_enqueue_step(jllm_b200_batch_decoder* d, const int* prompt, int 
             BCHK(launch_mf_sums(qkv, mf_operand(qkv, f.xh4, f.xh6), f.part, B, st));
             BCHK(launch_mf_prep(qkv, f.part, pr, m.rope_theta, B, st));
         } else {
-        BCHK(launch_rmsnorm(d->normed, d->x, nullptr, w.rms_attn, true, B, H, m.rms_eps, st));
-        BCHK(launch_mmq(d->q, resolve_weight(w.wq), w.type_wq, d->normed, QD, B, H, nullptr, st, &d->mmq));
-        BCHK(launch_mmq_ex(d->k, resolve_weight(w.wk), w.type_wk, d->normed, KVD, B, H, nullptr, true, st, &d->mmq));      // same activations as Q
-        BCHK(launch_mmq_ex(d->v, resolve_weight(w.wv), w.type_wv, d->normed, KVD, B, H, nullptr, true, st, &d->mmq));
-        BCHK(launch_qkv_prep_batched(d->q, d->k, d->v, w.q_norm, w.k_norm, m.rms_eps, (int8_t* const*)L, (int8_t* const*)(L + B),
-                                     (float* const*)(L + 2 * B), (float* const*)(L + 3 * B), B, m.n_heads, m.n_kv_heads, m.head_dim,
-                                     d->state, m.rope_theta, m.rope_neox != 0, st));
+            BCHK(launch_rmsnorm(d->normed, d->x, nullptr, w.rms_attn, true, B, H, m.rms_eps, st));
+            BCHK(launch_mmq(d->q, resolve_weight(w.wq), w.type_wq, d->normed, QD, B, H, nullptr, st, &d->mmq));
+            BCHK(launch_mmq_ex(d->k, resolve_weight(w.wk), w.type_wk, d->normed, KVD, B, H, nullptr, true, st, &d->mmq));      // same activations as Q
+            BCHK(launch_mmq_ex(d->v, resolve_weight(w.wv), w.type_wv, d->normed, KVD, B, H, nullptr, true, st, &d->mmq));
+            BCHK(launch_qkv_prep_batched(d->q, d->k, d->v, w.q_norm, w.k_norm, m.rms_eps, (int8_t* const*)L, (int8_t* const*)(L + B),
+                                         (float* const*)(L + 2 * B), (float* const*)(L + 3 * B), B, m.n_heads, m.n_kv_heads, m.head_dim,
+                                         d->state, m.rope_theta, m.rope_neox != 0, st));
         }
         AttnCall c;
         c.out = d->att; c.q = d->q; c.k_list = (const void* const*)L; c.v_list = (const void* const*)(L + B);
@@ -188,10 +188,10 @@ static int bdec_enqueue_step(jllm_b200_batch_decoder* d, const int* prompt, int 
         BCHK(launch_mmq_ex(d->x, resolve_weight(w.w_down), w.type_w_down, d->sw, H, B, I, d->x2, false, st, &d->mmq));     // + residual
     }
     if (few) {
-        BCHK(launch_mf_out(f.out, mf_operand(f.out, f.xh4, f.xh6), d->logits, nullptr, f.part, B, st));
+        BCHK(launch_mf_out(f.out, mf_operand(f.out, f.xh4, f.xh6), d->logits, f.part, B, st));
     } else {
-    BCHK(launch_rmsnorm(d->normed, d->x, nullptr, m.output_norm, true, B, H, m.rms_eps, st));
-    BCHK(launch_mmq(d->logits, resolve_weight(m.output), m.output_type, d->normed, V, B, H, nullptr, st, &d->mmq));
+        BCHK(launch_rmsnorm(d->normed, d->x, nullptr, m.output_norm, true, B, H, m.rms_eps, st));
+        BCHK(launch_mmq(d->logits, resolve_weight(m.output), m.output_type, d->normed, V, B, H, nullptr, st, &d->mmq));
     }
     const ArArgs ar = { d->logits, V, B, d->tokens, d->state, d->out_tokens, d->out_cap, d->seq_lens, prompt, n_prompt, d->best, d->best_at, d->tickets };
     const int slices = B >= 2 * AR_SLICES ? (B >= 148 ? 1 : 4) : AR_SLICES;      // one to two CTAs of 1024 threads per SM

@@ -448,11 +448,11 @@ int KquantDecoder::enqueue_chunk(const int* dev_tokens, int N, int start, cudaSt
             DCHK(launch_mf_sums(qkv, mf_operand(qkv, few.xh4, few.xh6), few.part, N, st));
             DCHK(launch_mf_prep(qkv, few.part, pr, m.rope_theta, N, st));
         } else {
-        DCHK(launch_rmsnorm(pf_normed, pf_x, nullptr, w.rms_attn, true, N, H, m.rms_eps, st));
-        DCHK(launch_mmq_pair(pf_q, pf_k, resolve_weight(w.wq), w.type_wq, resolve_weight(w.wk), w.type_wk, pf_normed, QD, KVD, N, H, st));
-        DCHK(launch_mmq_ex(pf_v, resolve_weight(w.wv), w.type_wv, pf_normed, KVD, N, H, nullptr, true, st));      // the operand of the product before
-        DCHK(launch_qkv_prep_tokens(pf_q, pf_k, pf_v, w.q_norm, w.k_norm, m.rms_eps, kc, vc, ks, vs, N, m.n_heads, m.n_kv_heads,
-                                    m.head_dim, start, m.rope_theta, m.rope_neox != 0, st));
+            DCHK(launch_rmsnorm(pf_normed, pf_x, nullptr, w.rms_attn, true, N, H, m.rms_eps, st));
+            DCHK(launch_mmq_pair(pf_q, pf_k, resolve_weight(w.wq), w.type_wq, resolve_weight(w.wk), w.type_wk, pf_normed, QD, KVD, N, H, st));
+            DCHK(launch_mmq_ex(pf_v, resolve_weight(w.wv), w.type_wv, pf_normed, KVD, N, H, nullptr, true, st));      // the operand of the product before
+            DCHK(launch_qkv_prep_tokens(pf_q, pf_k, pf_v, w.q_norm, w.k_norm, m.rms_eps, kc, vc, ks, vs, N, m.n_heads, m.n_kv_heads,
+                                        m.head_dim, start, m.rope_theta, m.rope_neox != 0, st));
         }
         DCHK(enqueue_attention(l, N, start, st));
         if (by_few) {

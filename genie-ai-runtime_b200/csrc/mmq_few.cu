@@ -50,7 +50,7 @@ struct MfArgs {
     int nseg, nb, N, NP, rows;
     const __half* x4; const __half* x6;
     float* part;                          // sums [slot][token][rows], or of the tiles that CTAs share [CTA][2][token][128]
-    __half* y; const __half* res;         // outputs of the product itself
+    __half* y;                            // outputs of the product itself
     int* status;
 };
 
@@ -414,21 +414,8 @@ __global__ void __launch_bounds__(MF_THREADS, 1) mf_kernel(const __grid_constant
                     #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         const int t = (dt >> 4) + 8 * i, r8 = 8 * (dt & 15), row8 = tile * MF_ROWS + r8;
-                        if (t0 + t < a.N && row8 < sg.M) {
-                            uint4 v = *reinterpret_cast<const uint4*>(stage + t * MF_ROWS + r8);
-                            const size_t o = (size_t)(t0 + t) * sg.M + row8;
-                            if (a.res) {
-                                const uint4 rv = *reinterpret_cast<const uint4*>(a.res + o);
-                                uint32_t* vw = reinterpret_cast<uint32_t*>(&v);
-                                const uint32_t* rw = reinterpret_cast<const uint32_t*>(&rv);
-                                #pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&rw[e])), z = __half22float2(*reinterpret_cast<const __half2*>(&vw[e]));
-                                    vw[e] = mf_pack(__float2half_rn(__fadd_rn(x.x, z.x)), __float2half_rn(__fadd_rn(x.y, z.y)));
-                                }
-                            }
-                            *reinterpret_cast<uint4*>(a.y + o) = v;
-                        }
+                        if (t0 + t < a.N && row8 < sg.M)
+                            *reinterpret_cast<uint4*>(a.y + (size_t)(t0 + t) * sg.M + row8) = *reinterpret_cast<const uint4*>(stage + t * MF_ROWS + r8);
                     }
                     asm volatile("bar.sync 2, 128;" ::: "memory");
                 }
@@ -463,10 +450,7 @@ __global__ void __launch_bounds__(256) mf_edge_kernel(const __grid_constant__ Mf
         const int pos = 32 * i + lane, row = tile * MF_ROWS + (pos % per) * s.perm + pos / per;
         float v = a.part[((size_t)(2 * first + 1) * a.N + t) * MF_ROWS + pos];
         for (int c = first + 1; c <= last; ++c) v += a.part[((size_t)(2 * c) * a.N + t) * MF_ROWS + pos];
-        if (row >= s.M) continue;
-        const size_t o = (size_t)t * s.M + row;
-        const __half h = __float2half_rn(v);
-        a.y[o] = a.res ? __float2half_rn(__fadd_rn(__half2float(a.res[o]), __half2float(h))) : h;
+        if (row < s.M) a.y[(size_t)t * s.M + row] = __float2half_rn(v);
     }
 }
 
@@ -745,13 +729,13 @@ bool mf_plan(MfProduct& p, const MfWeight* w, int n, int K) {
 }
 size_t mf_edge_bytes(int N) { DeviceCtx* c = ctx(); return (size_t)(c ? c->sm_count : 148) * 2 * N * MF_ROWS * sizeof(float); }
 
-static int mf_launch(const MfProduct& p, const MfOperand& x, float* part, __half* y, const __half* res, int N, cudaStream_t st) {
+static int mf_launch(const MfProduct& p, const MfOperand& x, float* part, __half* y, int N, cudaStream_t st) {
     DeviceCtx* c = ctx();
     if (!c) return JB_ERR_CUDA;
     MfArgs a = {};
     int grid = 0;
     for (int i = 0; i < p.nseg; ++i) { a.seg[i] = p.seg[i]; grid = p.seg[i].cta0 + p.seg[i].ctas; }
-    a.nseg = p.nseg; a.nb = p.K / QK_K; a.N = N; a.NP = mf_padded(N); a.rows = p.rows; a.x4 = x.x4; a.x6 = x.x6; a.part = part; a.y = y; a.res = res;
+    a.nseg = p.nseg; a.nb = p.K / QK_K; a.N = N; a.NP = mf_padded(N); a.rows = p.rows; a.x4 = x.x4; a.x6 = x.x6; a.part = part; a.y = y;
     a.status = c->d_status;
     auto kern = y ? mf_kernel<true> : mf_kernel<false>;
     if (!c->mf_attr[y ? 1 : 0]) {
@@ -769,8 +753,8 @@ static int mf_launch(const MfProduct& p, const MfOperand& x, float* part, __half
     }
     return JB_OK;
 }
-int launch_mf_sums(const MfProduct& p, const MfOperand& x, float* part, int N, cudaStream_t st) { return mf_launch(p, x, part, nullptr, nullptr, N, st); }
-int launch_mf_out(const MfProduct& p, const MfOperand& x, __half* y, const __half* residual, float* edge, int N, cudaStream_t st) { return mf_launch(p, x, edge, y, residual, N, st); }
+int launch_mf_sums(const MfProduct& p, const MfOperand& x, float* part, int N, cudaStream_t st) { return mf_launch(p, x, part, nullptr, N, st); }
+int launch_mf_out(const MfProduct& p, const MfOperand& x, __half* y, float* edge, int N, cudaStream_t st) { return mf_launch(p, x, edge, y, N, st); }
 
 static MfSums mf_sums(const MfProduct* p, const float* part, int N) {
     MfSums s = {};

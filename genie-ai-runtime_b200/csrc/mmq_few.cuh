@@ -40,8 +40,8 @@ inline MfOperand mf_operand(const MfProduct& p, void* x4, void* x6) {
 
 // Sums [slot][token][rows] into part.
 int launch_mf_sums(const MfProduct& p, const MfOperand& x, float* part, int N, cudaStream_t st);
-// y[token][M] in fp16 of a product of one matrix, plus residual[token][M] when given; edge: mf_edge_bytes of scratch.
-int launch_mf_out(const MfProduct& p, const MfOperand& x, __half* y, const __half* residual, float* edge, int N, cudaStream_t st);
+// y[token][M] in fp16 of a product of one matrix; edge: mf_edge_bytes of scratch.
+int launch_mf_out(const MfProduct& p, const MfOperand& x, __half* y, float* edge, int N, cudaStream_t st);
 
 // The kernels between the products.
 // x (+ the sums of the product in front, when p is given: x_out) -> RMSNorm with weights w, quantised into q (w null: the sum alone)
