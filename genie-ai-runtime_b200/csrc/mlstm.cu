@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(ML_THREADS) mlstm_kernel(const MlArgs p) {
 
 // raw outputs -> over each head's root mean square, times the weight, times sigmoid(g): a warp per (token, head)
 template <typename T>
-__global__ void __launch_bounds__(256) mlstm_out_kernel(const MlstmCall c, int n, bool take_next) {
+__global__ void __launch_bounds__(256) mlstm_out_kernel(const MlstmCall c, int n, bool take_next, bool vec) {
     pdl_wait();
     pdl_launch();
     if (take_next) {                                       // the chunk kernel left the next n and m beside the old ones
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(256) mlstm_out_kernel(const MlstmCall c, int n
     const T* g = reinterpret_cast<const T*>(c.proj) + (size_t)t * c.ld + c.off_g + h * c.vdim;
     T* out = reinterpret_cast<T*>(c.out) + (size_t)t * c.ldo + h * c.vdim;
     float sq = 0.f;
-    if (c.vdim % 4 == 0) {                                 // 16-byte rows of everything
+    if (vec) {                                             // fours of everything from whole boundaries
         const float* w4 = c.norm_w + h * c.vdim;
         for (int d = 4 * lane; d < c.vdim; d += 128) { const float4 v = load4(o + d); sq = fmaf(v.x, v.x, sq); sq = fmaf(v.y, v.y, sq); sq = fmaf(v.z, v.z, sq); sq = fmaf(v.w, v.w, sq); }
         const float rs = 1.0f / sqrtf(warp_sum(sq) / (float)c.vdim + c.eps);
@@ -202,8 +202,10 @@ int launch_mlstm(const MlstmCall& a, int n, int start, const int* d_pos, cudaStr
         if (rc || n == 1) return rc;
     }
     const dim3 og((unsigned)(((long long)n * a.heads * 32 + 255) / 256));
-    if (a.kind == EK_F32) JB_CUDA(launch_k(mlstm_out_kernel<float>, og, dim3(256), 0, st, pdl_enabled(), a, n, chunks));
-    else                  JB_CUDA(launch_k(mlstm_out_kernel<__nv_bfloat16>, og, dim3(256), 0, st, pdl_enabled(), a, n, chunks));
+    const uintptr_t four = a.kind == EK_F32 ? 15 : 7;
+    const bool vec = a.vdim % 4 == 0 && a.ld % 4 == 0 && a.off_g % 4 == 0 && a.ldo % 4 == 0 && !(((uintptr_t)a.raw | (uintptr_t)a.norm_w) & 15) && !(((uintptr_t)a.proj | (uintptr_t)a.out) & four);
+    if (a.kind == EK_F32) JB_CUDA(launch_k(mlstm_out_kernel<float>, og, dim3(256), 0, st, pdl_enabled(), a, n, chunks, vec));
+    else                  JB_CUDA(launch_k(mlstm_out_kernel<__nv_bfloat16>, og, dim3(256), 0, st, pdl_enabled(), a, n, chunks, vec));
     count_launch();
     return JB_OK;
 }

@@ -137,7 +137,8 @@ template <int KC> struct McLayout {
                               n = g + ((2 * (uint32_t)sizeof(McGates) + 127) & ~127u), sum = n + 2 * KC * 64 * 4, nq = sum + 4 * MC_L * 4, bytes = nq + 4 * MC_L * 4;
 };
 
-template <int KC>
+// WHOLE: outputs lie at 16-byte boundaries, else at 8-byte ones
+template <int KC, bool WHOLE>
 __global__ void __launch_bounds__(MC_THREADS, 1) mlstm_chunk_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                                                                     const __grid_constant__ CUtensorMap vmap, const __grid_constant__ McArgs p) {
     extern __shared__ uint8_t mc_raw[];
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mlstm_chunk_kernel(const __grid
             const uint32_t sc = tmem + MC_TM_SC + b * 128u + ((uint32_t)(q * 32) << 16);
             float sum[2] = {0.f, 0.f};
             #pragma unroll 1
-            for (int j = part; j < 8; j += 2) {                      // columns 16 j ..; loops stay rolled: see above
+            for (int j = part; j < 8; j += 2) {                      // columns 16 j ..; rolled, as everything here: unrolled, the roles' code is fetched more slowly than it runs
                 uint32_t x[16];                                      // scores; then first and second parts of the weighted ones
                 __syncwarp();
                 if (j <= 2 * q + 1) {
@@ -554,7 +555,11 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mlstm_chunk_kernel(const __grid
             float* out = c.raw + ((size_t)r * c.heads + h) * c.vdim + col;
             #pragma unroll
             for (int i = 0; i < 8; ++i)
-                if (r + 4 * i < p.n && col < c.vdim) *reinterpret_cast<uint4*>(out + (size_t)(4 * i) * c.heads * c.vdim) = y[i];
+                if (r + 4 * i < p.n && col < c.vdim) {
+                    float* o4 = out + (size_t)(4 * i) * c.heads * c.vdim;
+                    if (WHOLE) *reinterpret_cast<uint4*>(o4) = y[i];
+                    else { *reinterpret_cast<uint2*>(o4) = make_uint2(y[i].x, y[i].y); *reinterpret_cast<uint2*>(o4 + 2) = make_uint2(y[i].z, y[i].w); }
+                }
             __syncwarp();
         }
         if (ch == chunks && blockIdx.x == 0 && id < 32 * KC)         // what the thread itself wrote
@@ -598,7 +603,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mlstm_chunk_kernel(const __grid
 
 bool mlstm_chunks_apply(const MlstmCall& a, int n) {
     return a.kind == EK_BF16 && n >= 16 && a.dim % 8 == 0 && a.dim <= MC_MAX_DIM && a.vdim % 8 == 0 && a.ld % 8 == 0 && a.off_q % 8 == 0 && a.off_k % 8 == 0 && a.off_v % 8 == 0 &&
-           !((uintptr_t)a.proj & 15) && !((uintptr_t)a.state & 15) && (n <= MLSTM_SHORT ? !((uintptr_t)a.raw & 7) : !((uintptr_t)a.raw & 15) && encode_tiled_fn());
+           !((uintptr_t)a.proj & 15) && !((uintptr_t)a.raw & 7) && !((uintptr_t)a.state & 15) && (n <= MLSTM_SHORT || encode_tiled_fn());
 }
 // [head][token][column] of a part of the projections, boxes of 64 columns x a chunk, zero outside a head's columns and behind the last token
 static bool mc_map(CUtensorMap* map, const MlstmCall& a, int off, int cols, int n) {
@@ -607,16 +612,16 @@ static bool mc_map(CUtensorMap* map, const MlstmCall& a, int off, int cols, int 
     return encode_tiled_fn()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<__nv_bfloat16*>(reinterpret_cast<const __nv_bfloat16*>(a.proj)) + off, gdim, gstr, box, estr,
                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-template <int KC>
+template <int KC, bool WHOLE>
 static int mc_go(const MlstmCall& a, int n, int start, int* status, cudaStream_t st) {
     constexpr int smem = (int)McLayout<KC>::bytes + 1024;
     static bool attr = false;
-    if (!attr) { JB_CUDA(cudaFuncSetAttribute(mlstm_chunk_kernel<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); attr = true; }
+    if (!attr) { JB_CUDA(cudaFuncSetAttribute(mlstm_chunk_kernel<KC, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); attr = true; }
     CUtensorMap qm, km, vm;
     if (!mc_map(&qm, a, a.off_q, a.dim, n) || !mc_map(&km, a, a.off_k, a.dim, n) || !mc_map(&vm, a, a.off_v, a.vdim, n))
         return set_error(JB_ERR_CUDA, "mlstm chunks: tensor map refused (%d tokens, heads of %d x %d)", n, a.dim, a.vdim);
     const McArgs p = {a, n, start, status};
-    JB_CUDA(launch_k(mlstm_chunk_kernel<KC>, dim3((a.vdim + MC_V - 1) / MC_V, a.heads), dim3(MC_THREADS), (size_t)smem, st, pdl_enabled(), qm, km, vm, p));
+    JB_CUDA(launch_k(mlstm_chunk_kernel<KC, WHOLE>, dim3((a.vdim + MC_V - 1) / MC_V, a.heads), dim3(MC_THREADS), (size_t)smem, st, pdl_enabled(), qm, km, vm, p));
     count_launch();
     return JB_OK;
 }
@@ -625,7 +630,8 @@ int launch_mlstm_chunks(const MlstmCall& a, int n, int start, cudaStream_t st) {
     if (!x) return set_error(JB_ERR_STATE, "mlstm chunks: library not initialised");
     if (!mlstm_chunks_apply(a, n)) return set_error(JB_ERR_ARG, "mlstm chunks: %d tokens, heads of %d x %d", n, a.dim, a.vdim);
     if (n <= MLSTM_SHORT) return launch_mlstm_short(a, n, start, st);
-    return a.dim <= 128 ? mc_go<2>(a, n, start, x->d_status, st) : mc_go<4>(a, n, start, x->d_status, st);
+    if ((uintptr_t)a.raw & 15) return a.dim <= 128 ? mc_go<2, false>(a, n, start, x->d_status, st) : mc_go<4, false>(a, n, start, x->d_status, st);
+    return a.dim <= 128 ? mc_go<2, true>(a, n, start, x->d_status, st) : mc_go<4, true>(a, n, start, x->d_status, st);
 }
 
 }  // namespace jb

@@ -11,8 +11,16 @@ from test_gpu_layered import as_np, pad8, rng, up
 pytestmark = pytest.mark.gpu
 
 
-def run(jb, q, k, v, zi, zf, cuts):
-    """raw outputs [T][H][V] and the state left behind"""
+def shifted(t, by):
+    """The tensor `by` elements further on than a 16-byte boundary."""
+    import torch
+    buf = torch.empty(t.numel() + by, dtype=t.dtype, device="cuda")
+    buf[by:] = t.reshape(-1)
+    return buf[by:].reshape(t.shape)
+
+
+def run(jb, q, k, v, zi, zf, cuts, shift=None):
+    """raw outputs [T][H][V] and the state left behind; shift: elements by which raw, out and the norm's weights start off a 16-byte boundary"""
     T, H, D = q.shape
     V = v.shape[2]
     a, b = pad8(H * D), pad8(H * V)
@@ -24,8 +32,13 @@ def run(jb, q, k, v, zi, zf, cuts):
     got, at = [], 0
     for c in cuts:
         out, raw = zeros((c, b), "bfloat16"), zeros((c, H * V))
+        if shift:
+            raw, out, wd = shifted(raw, shift[0]), shifted(out, shift[1]), shifted(wd, shift[2])
         jb.mlstm(out, raw, state, pd[at:at + c].contiguous(), gd[at:at + c].contiguous(), bd, wd, H, D, V, 13.0, 1e-4, c, at)
         got.append(as_np(raw).reshape(c, H, V))
+        if np.abs(got[-1]).max() < 1e15:                    # the kernel behind: head norms, and gates of a half
+            x = got[-1] / np.sqrt((got[-1] ** 2).mean(2, keepdims=True) + 1e-4)
+            assert np.abs(as_np(out).reshape(c, -1)[:, :H * V].reshape(c, H, V) - x / 2).max() <= 2.0 ** -8 * np.abs(x).max()
         at += c
     assert at == T
     return np.concatenate(got), as_np(state)
@@ -56,3 +69,17 @@ def test_a_value_that_is_not_finite_reaches_no_earlier_token(T, at, value):
     for a, b in ((got[:at], clean[:at]), (got[:, 0], clean[:, 0]), (got[:, 1, other], clean[:, 1, other])):
         assert np.isfinite(a).all() and np.abs(a - b).max(initial=0) <= 1e-4 * np.abs(clean).max()
     assert not np.isfinite(got[at:, 1, 33]).any()
+
+
+@pytest.mark.parametrize("shift", [(2, 0, 0), (1, 0, 0), (0, 1, 0), (0, 2, 0), (0, 0, 1), (2, 4, 4)])
+@pytest.mark.parametrize("T", [8, 40, 200])
+def test_outputs_may_start_at_any_element(T, shift):
+    """`raw` at 8-byte boundaries is for the prompt kernels, elsewhere for the one that takes token by token; the kernel behind them reads it either way."""
+    jb, (H, D, V) = pkg(), (2, 64, 40)
+    q, k, v, _, zi, zf = memory_case(rng(T), H, D, V, T, "plain", "bfloat16")
+    want, _ = run(jb, q, k, v, zi, zf, [T])
+    got, _ = run(jb, q, k, v, zi, zf, [T], shift)
+    if shift[0] % 2 == 0:
+        assert np.array_equal(got, want)
+    else:
+        assert np.abs(got - want).max() <= 4e-4 * np.abs(want).max()      # both within the 2e-4 of test_edges
