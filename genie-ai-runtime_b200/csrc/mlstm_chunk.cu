@@ -26,12 +26,14 @@ constexpr uint32_t MC_TILE = MC_L * 128;                               // bytes 
 // q S, the chunk's own part of the outputs, k^T v of 128 dimensions each (first parts | second parts, 64 columns)
 constexpr uint32_t MC_TM_SC = 0, MC_TM_QS = 256, MC_TM_PV = 320, MC_TM_U = 384;
 
-// A, M: as two floats, in units of log2 (M less the logarithm of the scores' scale); a = e^(m_0 - M_t), w = e^(A_s - M_L), em = e^(-m_t)
+// A, M: as two floats, in units of log2 (M less the logarithm of the scores' scale over MC_LOW); a = e^(m_0 - M_t), w = e^(A_s - M_L), em = e^(-m_t)
 struct alignas(16) McGates { float2 A[MC_L], M[MC_L]; float a[MC_L], w[MC_L], em[MC_L], decay; };
 struct McArgs { MlstmCall c; int n, start; int* status; };
 
 __device__ __forceinline__ float2 mc_two(double x) { const float hi = (float)x; return make_float2(hi, (float)(x - (double)hi)); }
-// e^(A - M) times the scores' scale; 2^x to 2^-22, zero below 2^-126
+// e^(A - M) times the scores' scale, times 1 / MC_LOW, by which the score it weighs is multiplied first: their product may be a subnormal number, which the
+// exponential alone (2^x to 2^-22, zero below 2^-126; its other form takes four instructions in place of one) would leave out
+constexpr float MC_LOW = 1.0f / (1 << 24);
 __device__ __forceinline__ float mc_weight(float Ax, float Ay, float2 M) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"((Ax - M.x) + (Ay - M.y))); return y; }
 __device__ __forceinline__ void mc_split(float x, float y, uint32_t& hi, uint32_t& lo) {
     hi = fa_pack(x, y);
@@ -122,7 +124,7 @@ __device__ __forceinline__ bool mc_gates(const MlstmCall& c, int h, int t0, int 
     for (int e = 0; e < 4; ++e) {
         const int t = 4 * lane + e;
         Mt = fmax(Mt, a[e]);
-        g->A[t] = mc_two(a[e] * LOG2E); g->M[t] = mc_two(fma(Mt, LOG2E, -scale));
+        g->A[t] = mc_two(a[e] * LOG2E); g->M[t] = mc_two(fma(Mt, LOG2E, -scale - 24.0));
         g->a[t] = expf((float)(m - Mt));
         g->w[t] = t < valid ? expf((float)(a[e] - ML)) : 0.f;
         g->em[t] = expf((float)(-(F[e] + Mt)));
@@ -323,8 +325,8 @@ __global__ void __launch_bounds__(MC_THREADS, 1) mlstm_chunk_kernel(const __grid
                     #pragma unroll
                     for (int i = 0; i < 16; i += 2) {                // those of later tokens too: a branch around each would leave them one behind another
                         const float4 A = *reinterpret_cast<const float4*>(&g.A[16 * j + i]);
-                        v[i] = __uint_as_float(x[i]) * mc_weight(A.x, A.y, Mt);
-                        v[i + 1] = __uint_as_float(x[i + 1]) * mc_weight(A.z, A.w, Mt);
+                        v[i] = (__uint_as_float(x[i]) * MC_LOW) * mc_weight(A.x, A.y, Mt);
+                        v[i + 1] = (__uint_as_float(x[i + 1]) * MC_LOW) * mc_weight(A.z, A.w, Mt);
                     }
                     if (j >= 2 * q) {                                // later tokens weigh nothing
                         #pragma unroll

@@ -71,6 +71,23 @@ def test_a_value_that_is_not_finite_reaches_no_earlier_token(T, at, value):
     assert not np.isfinite(got[at:, 1, 33]).any()
 
 
+@pytest.mark.parametrize("T", [30, 100, 200])
+def test_weights_below_the_normal_numbers(T):
+    """The first token alone meets every query, so much later that its weight is a subnormal number, and its values are large enough to show it."""
+    jb, D, V = pkg(), 64, 32
+    q, k, v = np.zeros((T, 1, D)), np.zeros((T, 1, D)), np.zeros((T, 1, V))
+    q[:, 0, 0], k[0, 0, 0], k[1:, 0, 1], v[0] = 4.0, 1.0, 1.0, 2.0 ** 100
+    # what the next eight tokens forget takes it to 2^-128.5
+    zi, zf = np.zeros((T, 1)), np.full((T, 1), 60.0)
+    zf[1:9, 0] = -16.63
+    want = orc.mlstm_memory(q[:, 0] * D ** -0.5, k[:, 0], v[:, 0], orc.capped(zi[:, 0], 13.0), orc.log_sigmoid(orc.capped(zf[:, 0], 13.0)))[0]
+    got, _ = run(jb, q, k, v, zi, zf, [T])
+    low = np.abs(want[8:]) / 2.0 ** 100
+    assert ((low > 2.0 ** -133) & (low < 2.0 ** -126)).all()                   # what is looked at is where it should be
+    # the weighted score of 2^-129.5 goes into the product as a bf16 number, a multiple of 2^-133: half of that is 2^-4.5 of it
+    assert (np.abs(got[8:, 0] - want[8:]) <= 2.0 ** -4 * np.abs(want[8:])).all(), (got[8:12, 0, 0], want[8:12, 0])
+
+
 @pytest.mark.parametrize("shift", [(2, 0, 0), (1, 0, 0), (0, 1, 0), (0, 2, 0), (0, 0, 1), (2, 4, 4)])
 @pytest.mark.parametrize("T", [8, 40, 200])
 def test_outputs_may_start_at_any_element(T, shift):
