@@ -42,7 +42,7 @@ struct KquantDecoder : jllm_b200_decoder {
     __half *pf_x = nullptr, *pf_x2 = nullptr, *pf_normed = nullptr, *pf_y = nullptr, *pf_q = nullptr, *pf_att = nullptr, *pf_k = nullptr,
            *pf_v = nullptr, *pf_gate = nullptr, *pf_up = nullptr, *pf_sw = nullptr;
     MfModel few;                       // products of chunks of up to MF_MAX_TOKENS tokens
-    void* pf_operands = nullptr;       // in the slab: quantised activations and partial sums of such a chunk, or the operands of a longer one
+    void* pf_operands = nullptr;       // in the slab: the operands of a longer one
 
     ~KquantDecoder() override {
         if (slab) cudaFree(slab);
@@ -54,6 +54,7 @@ struct KquantDecoder : jllm_b200_decoder {
     int enqueue_step(int n_splits, cudaStream_t st) override;
     int reserve_chunk(int tokens, cudaStream_t st) override;
     int enqueue_chunk(const int* dev_tokens, int n, int start, cudaStream_t st) override;
+    int enqueue_few_chunk(int N, int start, cudaStream_t st);
     int enqueue_few_mlp(int l, int N, cudaStream_t st);
     int enqueue_rows_chunk(int N, int start, cudaStream_t st);
     int enqueue_attention(int l, int N, int start, cudaStream_t st, bool* tc = nullptr);      // tc: whether it was attention_tc.cu's
@@ -299,12 +300,11 @@ int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     const size_t N = (size_t)cap, H = m.hidden_dim, QD = (size_t)m.n_heads * m.head_dim, KVD = (size_t)m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
     // Where the weights allow it (by_rows), every chunk goes through the kernels that hand one product's results to the next as its operand: up to
-    // MF_MAX_TOKENS tokens the products of few tokens, beyond those of mmq_tc.cu; the scratch of one serves the other.
+    // MF_MAX_TOKENS tokens the products of few tokens, whose operands and partial sums lie in the stream's scratch, beyond those of mmq_tc.cu.
     const bool by_rows = !few.layers.empty(), many = !by_rows || cap > MF_MAX_TOKENS;
-    const size_t few_bytes = by_rows ? al(few.bytes(cap < MF_MAX_TOKENS ? cap : MF_MAX_TOKENS)) : 0, row_bytes = by_rows && many ? al(few.row_bytes(cap)) : 0;
-    const size_t operands = few_bytes > row_bytes ? few_bytes : row_bytes;
+    const size_t operands = by_rows && many ? al(few.row_bytes(cap)) : 0;
     const size_t rows = many ? N : 1, general = by_rows ? 1 : N;        // a chunk of one token is the general kernels' too
-    const size_t total = 2 * al(N * H * 2) + 2 * al(N * QD * 2) + al(rows * H * 2) + 2 * al(rows * KVD * 2) + 2 * al(rows * I * 2) + al(general * H * 2) + al(general * I * 2) + (by_rows ? operands : 0);
+    const size_t total = 2 * al(N * H * 2) + 2 * al(N * QD * 2) + al(rows * H * 2) + 2 * al(rows * KVD * 2) + 2 * al(rows * I * 2) + al(general * H * 2) + al(general * I * 2) + operands;
     // one allocation for all of it: it is made inside a session's first prompt, where each costs 0.4 - 2 ms (512 tokens: the first prompt
     // took 1064 us more than the next with two, 444 with one)
     size_t codes = cap >= attention_tc_min_tokens(m.n_heads, m.n_kv_heads) && m.max_context <= PF_CODES_MAX && m.head_dim == 128 ? attention_tc_scratch(m.n_kv_heads, m.max_context) : 0;
@@ -319,7 +319,7 @@ int KquantDecoder::reserve_chunk(int cap, cudaStream_t) {
     pf_k = (__half*)take(rows * KVD * 2); pf_v = (__half*)take(rows * KVD * 2);
     pf_gate = (__half*)take(rows * I * 2); pf_up = (__half*)take(rows * I * 2);
     pf_normed = (__half*)take(general * H * 2); pf_sw = (__half*)take(general * I * 2);
-    if (by_rows) pf_operands = take(operands);
+    pf_operands = take(operands);
     pf_cap = cap;
     return JB_OK;
 }
@@ -413,6 +413,27 @@ int KquantDecoder::enqueue_rows_chunk(int N, int start, cudaStream_t st) {
     return JB_OK;
 }
 
+// The layers of a chunk of few tokens.
+int KquantDecoder::enqueue_few_chunk(int N, int start, cudaStream_t st) {
+    const MmqLease lease(nullptr, st);
+    const size_t need = few.bytes(N);
+    void* scratch = lease.w ? lease.w->scratch(need, lease.cap) : nullptr;
+    if (!scratch) return set_error(JB_ERR_NOMEM, "decoder: %zu B of prefill operands", need);
+    lease.w->few = lease.w->many = MmqOperand();        // what lay there is overwritten
+    few.place(scratch, N);
+    DCHK(launch_mf_norm(nullptr, nullptr, pf_x, nullptr, layers[0].rms_attn, m.rms_eps, m.hidden_dim, mf_operand(few.layers[0].qkv, few.xh4, few.xh6), N, st));
+    for (int l = 0; l < m.n_layers; ++l) {
+        const MfProduct& qkv = few.layers[l].qkv;
+        const MfPrep pr = { pf_q, layers[l].q_norm, layers[l].k_norm, m.rms_eps, nullptr, nullptr, nullptr, nullptr, (int8_t*)kv.key_ptr(l, 0), (int8_t*)kv.val_ptr(l, 0),
+                            kv.kv_scale_ptr(l, 0, false), kv.kv_scale_ptr(l, 0, true), nullptr, start, 1, m.n_heads, m.n_kv_heads, m.rope_neox != 0 };
+        DCHK(launch_mf_sums(qkv, mf_operand(qkv, few.xh4, few.xh6), few.part, N, st));
+        DCHK(launch_mf_prep(qkv, few.part, pr, m.rope_theta, N, st));
+        DCHK(enqueue_attention(l, N, start, st));
+        DCHK(enqueue_few_mlp(l, N, st));
+    }
+    return JB_OK;
+}
+
 // what follows attention in a layer of few tokens: Wo, residual and norm, gate and up, SwiGLU, W_down, residual and the next layer's norm
 int KquantDecoder::enqueue_few_mlp(int l, int N, cudaStream_t st) {
     const MfLayer& p = few.layers[l];
@@ -430,35 +451,21 @@ int KquantDecoder::enqueue_few_mlp(int l, int N, cudaStream_t st) {
 int KquantDecoder::enqueue_chunk(const int* dev_tokens, int N, int start, cudaStream_t st) {
     const int H = m.hidden_dim, QD = m.n_heads * m.head_dim, KVD = m.n_kv_heads * m.head_dim, I = m.intermediate_dim;
     DCHK(launch_embed_rows(pf_x, m.tok_embd, m.embd_type, dev_tokens, N, H, st));
-    if (!few.layers.empty() && N > MF_MAX_TOKENS) {
-        DCHK(enqueue_rows_chunk(N, start, st));
+    if (!few.layers.empty() && N > 1) {      // one token: integer dots summed in fp32, by the general kernels
+        DCHK(N > MF_MAX_TOKENS ? enqueue_rows_chunk(N, start, st) : enqueue_few_chunk(N, start, st));
         mmq_mark(st);                        // behind the chunk's lease
         return JB_OK;
     }
-    const bool by_few = !few.layers.empty() && N > 1;       // one token: integer dots summed in fp32, by the general kernels
-    if (by_few) few.place(pf_operands, N);
-    if (by_few) DCHK(launch_mf_norm(nullptr, nullptr, pf_x, nullptr, layers[0].rms_attn, m.rms_eps, H, mf_operand(few.layers[0].qkv, few.xh4, few.xh6), N, st));
     for (int l = 0; l < m.n_layers; ++l) {
         const jllm_b200_layer_desc& w = layers[l];
         int8_t* kc = (int8_t*)kv.key_ptr(l, 0); int8_t* vc = (int8_t*)kv.val_ptr(l, 0);
         float* ks = kv.kv_scale_ptr(l, 0, false); float* vs = kv.kv_scale_ptr(l, 0, true);
-        if (by_few) {
-            const MfProduct& qkv = few.layers[l].qkv;
-            const MfPrep pr = { pf_q, w.q_norm, w.k_norm, m.rms_eps, nullptr, nullptr, nullptr, nullptr, kc, vc, ks, vs, nullptr, start, 1, m.n_heads, m.n_kv_heads, m.rope_neox != 0 };
-            DCHK(launch_mf_sums(qkv, mf_operand(qkv, few.xh4, few.xh6), few.part, N, st));
-            DCHK(launch_mf_prep(qkv, few.part, pr, m.rope_theta, N, st));
-        } else {
-            DCHK(launch_rmsnorm(pf_normed, pf_x, nullptr, w.rms_attn, true, N, H, m.rms_eps, st));
-            DCHK(launch_mmq_pair(pf_q, pf_k, resolve_weight(w.wq), w.type_wq, resolve_weight(w.wk), w.type_wk, pf_normed, QD, KVD, N, H, st));
-            DCHK(launch_mmq_ex(pf_v, resolve_weight(w.wv), w.type_wv, pf_normed, KVD, N, H, nullptr, true, st));      // the operand of the product before
-            DCHK(launch_qkv_prep_tokens(pf_q, pf_k, pf_v, w.q_norm, w.k_norm, m.rms_eps, kc, vc, ks, vs, N, m.n_heads, m.n_kv_heads,
-                                        m.head_dim, start, m.rope_theta, m.rope_neox != 0, st));
-        }
+        DCHK(launch_rmsnorm(pf_normed, pf_x, nullptr, w.rms_attn, true, N, H, m.rms_eps, st));
+        DCHK(launch_mmq_pair(pf_q, pf_k, resolve_weight(w.wq), w.type_wq, resolve_weight(w.wk), w.type_wk, pf_normed, QD, KVD, N, H, st));
+        DCHK(launch_mmq_ex(pf_v, resolve_weight(w.wv), w.type_wv, pf_normed, KVD, N, H, nullptr, true, st));      // the operand of the product before
+        DCHK(launch_qkv_prep_tokens(pf_q, pf_k, pf_v, w.q_norm, w.k_norm, m.rms_eps, kc, vc, ks, vs, N, m.n_heads, m.n_kv_heads,
+                                    m.head_dim, start, m.rope_theta, m.rope_neox != 0, st));
         DCHK(enqueue_attention(l, N, start, st));
-        if (by_few) {
-            DCHK(enqueue_few_mlp(l, N, st));
-            continue;
-        }
         DCHK(launch_mmq(pf_y, resolve_weight(w.wo), w.type_wo, pf_att, H, N, QD, nullptr, st));
         DCHK(launch_add_half(pf_x2, pf_x, pf_y, (long long)N * H, st));
         DCHK(launch_rmsnorm(pf_normed, pf_x2, nullptr, w.rms_ffn, true, N, H, m.rms_eps, st));

@@ -281,8 +281,32 @@ def test_a_second_session_takes_over_the_expanded_weights():
     assert jb.device_status() == 0
 
 
-def test_two_sessions_prompt_on_one_stream_from_two_threads():
-    """A chunk's expansions run ahead of its products in buffers of the stream: a session on the same stream in another thread waits its turn."""
+def test_a_second_session_takes_over_the_scratch_of_short_prompts():
+    """Operands and partial sums of a prompt of few tokens are the stream's too (10 MB at these widths)."""
+    import torch
+    jb = pkg()
+    m = orc.gen_model(85, n_layers=1, hidden=512, n_heads=4, n_kv=1, hd=128, ffn=8192, vocab=512)
+    w = jb.decoder.upload(m)
+    prompt = np.random.Generator(np.random.PCG64(85)).integers(0, 512, 100)
+    sessions, taken, logits = [], [], []
+    for _ in range(4):
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        d = jb.decoder.Decoder(m["cfg"], w, 128, jb.decoder.FUSED | jb.decoder.PREFILL)
+        d.prefill(prompt, 0, torch.cuda.Stream())
+        logits.append(d.logits())
+        taken.append(free - torch.cuda.mem_get_info()[0])
+        sessions.append(d)
+    assert all(t < 6 << 20 for t in taken[1:]), taken
+    assert all(torch.equal(l, logits[0]) for l in logits)
+    for d in sessions:
+        d.close()
+    assert jb.device_status() == 0
+
+
+@pytest.mark.parametrize("lengths", [(640, 500), (640, 60), (60, 100)])
+def test_two_sessions_prompt_on_one_stream_from_two_threads(lengths):
+    """A chunk has its expansions, operands and partial sums in buffers of the stream: a session on the same stream in another thread waits its turn."""
     import threading
     import torch
     jb = pkg()
@@ -290,7 +314,7 @@ def test_two_sessions_prompt_on_one_stream_from_two_threads():
     w = jb.decoder.upload(m)
     st = torch.cuda.Stream()
     d = [jb.decoder.Decoder(m["cfg"], w, 700, jb.decoder.FUSED | jb.decoder.PREFILL) for _ in range(2)]
-    prompts = [np.random.Generator(np.random.PCG64(1400 + i)).integers(0, 512, n) for i, n in enumerate((640, 500))]
+    prompts = [np.random.Generator(np.random.PCG64(1400 + i)).integers(0, 512, n) for i, n in enumerate(lengths)]
     want = []
     for i in range(2):
         d[i].prefill(prompts[i], 0, st)
