@@ -194,7 +194,9 @@ static int bdec_enqueue_step(jllm_b200_batch_decoder* d, const int* prompt, int 
         BCHK(launch_mmq(d->logits, resolve_weight(m.output), m.output_type, d->normed, V, B, H, nullptr, st, &d->mmq));
     }
     const ArArgs ar = { d->logits, V, B, d->tokens, d->state, d->out_tokens, d->out_cap, d->seq_lens, prompt, n_prompt, d->best, d->best_at, d->tickets };
-    const int slices = B >= 2 * AR_SLICES ? (B >= 148 ? 1 : 4) : AR_SLICES;      // one to two CTAs of 1024 threads per SM
+    const DeviceCtx* cx = ctx();
+    if (!cx) return JB_ERR_CUDA;
+    const int slices = B >= 2 * AR_SLICES ? (B >= cx->sm_count ? 1 : 4) : AR_SLICES;      // one to two CTAs of 1024 threads per SM
     JB_CUDA(launch_k(argmax_rows_kernel, dim3(slices, B), dim3(1024), 0, st, pdl_enabled(), ar));
     count_launch();
     d->kernels_per_step = (int)(jllm_b200_launch_count() - l0);

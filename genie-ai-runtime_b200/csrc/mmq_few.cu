@@ -23,7 +23,7 @@
 // Measured with cold weights, us at 8 / 64 / 128 tokens, in brackets what served before (warps streaming rows into mma.sync up to 40 tokens, the
 // 128 x 256 tiles of mmq_tc.cu): gate and up, Q4_K 9728 x 2560 twice, 12.8 / 16.9 / 22.4 (27.2 / 35.4 / -); W_down, Q6_K 2560 x 9728,
 // 11.2 / 13.4 / 18.3 (16.8 / 27.1 / -); Wo, Q4_K 2560 x 4096, 6.7 / 8.9 / 12.4 (7.5 / 20.3 / -); logits, Q6_K 151936 x 2560, 91 / 99 / 123
-// (125 / 280 / -), of which 62 / 75 / 103 are left without the arithmetic on the codes (ALU 63 % and issue slots 73 % busy), and memory needs 49.
+// (125 / 280 / -), of which 62 / 75 / 103 are left without the arithmetic on the codes (at 64 tokens ALU 61 % and issue slots 71 % busy), and memory needs 49.
 // A prompt chunk of 8 layers: 33 tokens 696 us (1283); above 128 tokens an accumulator and two
 // super-blocks of weights no longer fit into tensor memory.
 #include "mmq_few.cuh"
@@ -98,7 +98,8 @@ __device__ __forceinline__ uint32_t mf_u32(__half2 h) { return *reinterpret_cast
 __device__ __forceinline__ __half2 mf_bytes(uint32_t w) { return __hsub2(mf_h2((w & 0x00FF00FFu) | 0x64006400u), mf_h2(0x64006400u)); }
 
 // Two codes of a word (bits 0-3 and 16-19; `high`: bits 4-7 and 20-23) -> (q - 8) * s, both roundings as in mmq_tc.cu: 0x6400 | q is the
-// half 1024 + q, 0x6400 | 16 q is 1024 + 16 q, and (1024 + 16 q) / 16 - 72 = q - 8 is exact.
+// half 1024 + q, 0x6400 | 16 q is 1024 + 16 q, and (1024 + 16 q) / 16 - 72 = q - 8 is exact (numbers put into a half's mantissa: the conversion of
+// Kim et al., "Who Says Elephants Can't Run", 2022).
 __device__ __forceinline__ uint32_t mf_low(uint32_t w, __half2 s) { return mf_u32(__hmul2(__hsub2(mf_h2((w & 0x000F000Fu) | 0x64006400u), mf_h2(0x64086408u)), s)); }
 __device__ __forceinline__ uint32_t mf_high(uint32_t w, __half2 s) { return mf_u32(__hmul2(__hfma2(mf_h2((w & 0x00F000F0u) | 0x64006400u), mf_h2(0x2C002C00u), mf_h2(0xD480D480u)), s)); }
 
