@@ -96,13 +96,15 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dense_gemv_kernel(const DgArgs 
     if (MODE == GEMV_PLAIN && g.late) pdl_wait();
     if (MODE != GEMV_MOE_UP && MODE != GEMV_MOE_DOWN) { if (n_batches > 0) load(0, 0, cur); }
     // The rest of the CTA's first rows on their way into L2 while the input vector is being produced and normed; more than DG_AHEAD delays the loads
-    // behind them (a request of a model with parallel layers, 512 + 16 tokens, us at 0 / 32 / 64 / 128 / 256 KB: 7932 / 7788 / 7778 / 7907 / 8118).
+    // behind them (a request of a model with parallel layers, 512 + 16 tokens, us at 0 / 32 / 64 / 128 / 256 KB: 7932 / 7788 / 7778 / 7907 / 8118).  Not
+    // where a CTA has no more than that, half of it in its first loads: width 1024, 8 + 32 tokens, without / always / so: 8696 / 8721 / 8687 (parallel
+    // layers), 10575 / 10711 / 10663 (the same in fp32), 12995 / 13082 / 13024 (sequential, fp32); width 2560 13960 / 13793 / 13810, 15505 / 15457 / 15448.
     if (MODE != GEMV_MOE_UP && MODE != GEMV_MOE_DOWN && !g.late) {
         const long long row = (long long)p.nchunk * 16;
         const int r0 = MODE == GEMV_PAIR ? 2 * i0 : i0, r1 = MODE == GEMV_PAIR ? min(2 * i1, g.M) : i1;
         const char* at = reinterpret_cast<const char*>(g.W) + r0 * row;
         const long long bytes = min((long long)DG_AHEAD, (r1 - r0) * row);
-        for (long long o = (long long)threadIdx.x * 2048; o < bytes; o += DG_THREADS * 2048)
+        for (long long o = (r1 - r0) * row > DG_AHEAD ? (long long)threadIdx.x * 2048 : bytes; o < bytes; o += DG_THREADS * 2048)
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(at + o), "r"((uint32_t)min(2048ll, bytes - o)) : "memory");
     }
     if (NORM) norm_prefetch<DG_THREADS>(g.norm);
